@@ -263,10 +263,11 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
   ok = ok && h.dalloc(&d.v0x, N, "v0x") && h.dalloc(&d.v0y, N, "v0y") &&
        h.dalloc(&d.v0p, N, "v0p") && h.dalloc(&d.fx, N, "fx") && h.dalloc(&d.fy, N, "fy") &&
        h.dalloc(&d.tau, N, "tau") && h.dalloc(&d.moved, N, "moved");
+  ok = ok && h.dalloc(&d.rec, N, "rec") && h.dalloc(&d.rec_t, N, "rec_t") &&
+       h.dalloc(&d.rf, N, "rf");
   if (h.prec == sc::PREC_MIXED)
-    ok = ok && h.dalloc(&d.rec, N, "rec") && h.dalloc(&d.rec_t, N, "rec_t") &&
-         h.dalloc(&d.mc, N, "mc") && h.dalloc(&d.mv, N, "mv") && h.dalloc(&d.mm, N, "mm") &&
-         h.dalloc(&d.pa, N, "pa") && h.dalloc(&d.rcf, N, "rcf") && h.dalloc(&d.rf, N, "rf") &&
+    ok = ok && h.dalloc(&d.mc, N, "mc") && h.dalloc(&d.mv, N, "mv") && h.dalloc(&d.mm, N, "mm") &&
+         h.dalloc(&d.pa, N, "pa") && h.dalloc(&d.rcf, N, "rcf") &&
          h.dalloc(&d.cellp, N, "cellp") && h.dalloc(&d.gbuild, n_sys, "gbuild") &&
          h.dalloc(&d.ord, N, "ord") && h.dalloc(&d.nbr_p, N * d.maxn, "nbr_p") &&
          h.dalloc(&d.nbr_pn, N, "nbr_pn");
@@ -297,6 +298,22 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
        h.dalloc(&d.nwork, 3, "nwork") &&
        h.dalloc(&d.status, 2, "status");
   if (!ok) return bail(h.last_status ? h.last_status : SC_E_NOMEM);
+  // the FP64 form's pair results, where there is memory for them (a mask word holds 64
+  // list entries)
+  if (h.prec == sc::PREC_FP64 && d.maxn <= 64) {
+    const size_t np = (N + 128) * sc::kPairCap;
+    if (h.dalloc(&d.pr_mask, N, "pair masks") && h.dalloc(&d.pr_info, N, "pair offsets") &&
+        h.dalloc(&d.pr_who, np, "pair partners") && h.dalloc(&d.pr_res, np, "pair results")) {
+      d.pr_win = sc::pair_window(ntot);
+    } else {
+      h.dfree(d.pr_mask);
+      h.dfree(d.pr_info);
+      h.dfree(d.pr_who);
+      h.err.clear();
+      h.last_status = SC_OK;
+      cudaGetLastError();
+    }
+  }
   d.geom = geom;
   d.psys = psys;
   d.pchunk_sys = pcs;
@@ -677,7 +694,8 @@ int sc_get_pairs(sc_handle* H, int sys, int* pairs, long cap, long* n_pairs) {
   for (int k = 0; k < S.n; k++) {
     int c = std::min(nn[k], d.maxn);
     for (int m = 0; m < c; m++) {
-      int j = (int)((unsigned)lst[(size_t)m * S.n + k] & sc::kSlotMask) - S.p0;
+      const unsigned mask = h.prec == sc::PREC_FP64 ? sc::kSlot64Mask : sc::kSlotMask;
+      int j = (int)((unsigned)lst[(size_t)m * S.n + k] & mask) - S.p0;
       if (j < 0 || j >= S.n) continue;
       int a = ids[k], b = ids[j];
       if (a < b) pr.emplace_back(a, b);

@@ -361,7 +361,10 @@ __global__ void k_rb_commit(Dev d, const StepScalars* __restrict__ tab, int row,
     if (!mixed) {
       double sn, cs;
       sincos(phi, &sn, &cs);
-      d.nxy[i] = make_double2(ra.y * cs, ra.y * sn);
+      const double2 n = make_double2(ra.y * cs, ra.y * sn);
+      d.nxy[i] = n;
+      d.rec[i] = screen_record(p, n);
+      d.rf[i] = (float)ra.x;
     }
   });
 }
@@ -421,7 +424,10 @@ __global__ void k_refresh(Dev d) {
   double2 ra = d.ra[i];
   double sn, cs;
   sincos(phi, &sn, &cs);
-  d.nxy[i] = make_double2(ra.y * cs, ra.y * sn);
+  const double2 n = make_double2(ra.y * cs, ra.y * sn);
+  d.nxy[i] = n;
+  d.rec[i] = screen_record(d.xy[i], n);
+  d.rf[i] = (float)ra.x;
 }
 
 // gradient_relax_step, src/cpp/relaxation_dynamics.cpp:11-31
@@ -453,7 +459,9 @@ __global__ void k_gd_update(Dev d, const StepScalars* __restrict__ tab, int row)
   double2 ra = d.ra[i];
   double sn, cs;
   sincos(phi, &sn, &cs);
-  d.nxy[i] = make_double2(ra.y * cs, ra.y * sn);
+  const double2 n = make_double2(ra.y * cs, ra.y * sn);
+  d.nxy[i] = n;
+  d.rec[i] = screen_record(p, n);
   if (!(isfinite(p.x) && isfinite(p.y) && isfinite(phi))) atomicOr(d.status, ST_NAN);
   // the reference tests and rebuilds inside the update loop
   if (m.x > 0.5 * g.pad || m.x < -0.5 * g.pad || m.y > 0.5 * g.pad || m.y < -0.5 * g.pad) {

@@ -187,12 +187,15 @@ __global__ void k_cg_probe(Dev d, CgState c) {
   }
   const double2 p = d.xy[i];
   const double pht = d.ph[i] + q.t * dp;
-  d.xy_t[i] = make_double2(p.x + q.t * dx, p.y + q.t * dy);
+  const double2 pt = make_double2(p.x + q.t * dx, p.y + q.t * dy);
+  d.xy_t[i] = pt;
   d.ph_t[i] = pht;
   const double A = d.ra[i].y;
   double sn, cs;
   sincos(pht, &sn, &cs);
-  d.nxy_t[i] = make_double2(A * cs, A * sn);
+  const double2 n = make_double2(A * cs, A * sn);
+  d.nxy_t[i] = n;
+  d.rec_t[i] = screen_record(pt, n);
 }
 
 // The parabola through (0, E0), (1, E1), (2, E2) in units of the step and its
@@ -321,7 +324,9 @@ __global__ void k_cg_move(Dev d, CgState c) {
   const double A = d.ra[i].y;
   double sn, cs;
   sincos(phi, &sn, &cs);
-  d.nxy[i] = make_double2(A * cs, A * sn);
+  const double2 n = make_double2(A * cs, A * sn);
+  d.nxy[i] = n;
+  d.rec[i] = screen_record(p, n);
   double2 m = d.moved[i];
   m.x += ddx;
   m.y += ddy;

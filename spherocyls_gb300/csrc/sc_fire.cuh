@@ -240,7 +240,9 @@ __device__ __forceinline__ void fire_update(const Dev& d, const FireState& f, in
     double2 ra = d.ra[i];
     double sn, cs;
     sincos(phi, &sn, &cs);
-    d.nxy[i] = make_double2(ra.y * cs, ra.y * sn);
+    const double2 n = make_double2(ra.y * cs, ra.y * sn);
+    d.nxy[i] = n;
+    d.rec[i] = screen_record(p, n);
     double2 m = d.moved[i];
     m.x += ddx;
     m.y += ddy;

@@ -431,14 +431,15 @@ bool Handle::rebuild_all() {
 }
 
 void Handle::launch_pass(int mode, bool se, int row, bool fast) {
-  kernels += (prec == PREC_MIXED && se) ? 3 : 1;  // mixed: the FP64 stress kernels
   Dev dd = d;
   dd.cond = (mode == PASS_CORR_STRAIN || mode == PASS_CORR_RESIZE) ? step_cond : 0;
   dd.skip = pass_skip;
-  if (prec == PREC_MIXED)
+  if (prec == PREC_MIXED) {
     launch_pass_mixed(dd, mode, se, d_tab, row, stream, block);
-  else
-    launch_pass_fp64(dd, mode, se, d_tab, row, stream, fast);
+    kernels += se ? 3 : 1;  // with the FP64 stress kernels
+  } else {
+    kernels += launch_pass_fp64(dd, mode, se, d_tab, row, stream, fast);
+  }
 }
 
 cudaEvent_t Handle::next_event() {
@@ -605,17 +606,17 @@ bool Handle::capture_conditional(bool resize, int nsteps, const std::vector<char
     e = new_cond_handle(&hcond);
     if (e != cudaSuccess) break;
     step_cond = hcond;
+    const long long k1 = kernels;
     enqueue_corr(resize, k, false);
     step_cond = 0;
+    fixed += kernels - k1;
     e = add_cond_body(hcond,
                       [&](cudaStream_t st) { return enqueue_rebuild_body(resize, k, false, st); });
     if (e != cudaSuccess) break;
+    const long long k2 = kernels;
     enqueue_pred(resize, k, se[k] != 0, false);
-    fixed += 2;
-    if (se[k]) {
-      enqueue_se_record(r++);
-      fixed += 3;
-    }
+    if (se[k]) enqueue_se_record(r++);
+    fixed += kernels - k2;
   }
   cudaGraph_t g = nullptr;
   cudaError_t e2 = cudaStreamEndCapture(stream, &g);
@@ -1139,6 +1140,7 @@ bool Handle::run_fire_graph(int iters, double ftol, double dt_max) {
     }
     const bool mixed = prec == PREC_MIXED;
     cudaError_t e = cudaSuccess;
+    const long long k0 = kernels;
     for (int k = 0; k < iters && e == cudaSuccess; k++) {
       pass_skip = fire.done;  // converged systems: no force pass
       launch_pass(PASS_FORCE, false, 0, true);
@@ -1164,7 +1166,8 @@ bool Handle::run_fire_graph(int iters, double ftol, double dt_max) {
     fire_key_iters = iters;
     fire_key_ftol = ftol;
     fire_key_dtmax = dt_max;
-    fire_graph_kernels = 5LL * iters;
+    fire_graph_kernels = kernels - k0 + 4LL * iters;
+    kernels = k0;
   }
   kernels += fire_graph_kernels;
   return cuda_ok(cudaGraphLaunch(fire_exec, stream), "fire graph launch");

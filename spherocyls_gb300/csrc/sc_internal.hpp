@@ -178,7 +178,8 @@ struct Dev {
   double* fy;
   double* tau;
   double2* moved;
-  // mixed form (FP32 state relative to the cell centre, compensated):
+  // mixed form (FP32 state relative to the cell centre, compensated); the FP64 form
+  // keeps its positions rounded to FP32 in rec, rec_t and rf, for its pair screen:
   float4* rec;    // (x_local, y_local, A cos phi, A sin phi) of the state
   float4* rec_t;  // the same for the predictor copy
   float4* mc;     // (x compensation, y compensation, phi, phi compensation)
@@ -193,8 +194,15 @@ struct Dev {
   int* cell_start;          // [ncells] first slot
   int* cell_count;          // [ncells]
   // neighbour list, column-major [k * ntot + slot]
-  int* nbr;
+  int* nbr;                 // FP64 form: slot | kOwner64 where this particle's index is lower
   int* nbr_n;
+  // FP64 form: the pairs of a pass, each evaluated once (k_pairs64).  Windows of
+  // pr_win slots own pr_win * kPairCap results each, in slot and list order.
+  int pr_win;                  // 0: no pair buffers (k_pass64 instead)
+  unsigned long long* pr_mask; // [ntot] list entries that may touch
+  unsigned* pr_info;           // [ntot] offset in the window | owned pairs << 16, or kPairsOver
+  int* pr_who;                 // [window][pr_win * kPairCap] the partner's slot, -1: no contact
+  double4_16a* pr_res;         // same index: force on the owner (x, y), torques (owner, partner)
   // mixed form: the same lists reordered for the force pass.  Within each window
   // of kOrderWindow slots, threads take the slots in order of increasing list
   // length, so a warp's lanes loop over lists of nearly equal length.
@@ -276,6 +284,13 @@ constexpr int kOrderWindow = 128;  // slots per window of the force-pass orderin
 // mixed-form list entries: slot in the low 28 bits, cell offset (dc+1, dr+1) above
 constexpr int kSlotBits = 28;
 constexpr unsigned kSlotMask = (1u << kSlotBits) - 1u;
+// FP64 list entries: slot in the low 30 bits, the top bit set where the listing
+// particle has the lower index (the reference's "p")
+constexpr unsigned kOwner64 = 0x80000000u;
+constexpr unsigned kSlot64Mask = (1u << 30) - 1u;
+constexpr int kPairCap = 5;  // pair results kept per slot of a window (2 to 3 are used)
+constexpr int kSmallPairs = 1 << 16;  // up to this many slots, windows of 32 (see pair_window)
+constexpr unsigned kPairsOver = 0xffffffffu;  // pr_info of a window with more than that
 // tile force pass: entry capacity per particle of a tile (compute and read lists
 // each), particles and pair results held in shared memory, threads per tile; a
 // tile's partner index below kTileInt (bit 27) is a slot, so slots stay below 2^27
@@ -302,8 +317,11 @@ enum PassMode {
 // ---- kernel launchers (defined in the .cu files) ----
 // tab: device table, row `row` holds nsys StepScalars.
 // fast: the minimiser's force evaluation (FORCE mode only), with fewer FP64 divisions
-void launch_pass_fp64(const Dev& d, int mode, bool se, const StepScalars* tab, int row,
-                      cudaStream_t st, bool fast = false);
+// Returns the number of kernels launched.
+int launch_pass_fp64(const Dev& d, int mode, bool se, const StepScalars* tab, int row,
+                     cudaStream_t st, bool fast = false);
+// slots per window of the pair results
+int pair_window(int ntot);
 void launch_pass_mixed(const Dev& d, int mode, bool se, const StepScalars* tab, int row,
                        cudaStream_t st, int block);
 // set-back of the listed systems whose row says so (after launch_rb_worklist)
@@ -426,6 +444,10 @@ __device__ __forceinline__ void mark_pending_rebuilds(const Dev& d,
     }
   if (setback) atomicExch(d.any, 1);
   if (setback || (threadIdx.x == 0 && *d.any != 0)) cudaGraphSetConditional(d.cond, 1u);
+}
+// FP32 copy of an FP64 position and shaft vector, for the FP64 form's pair screen
+__device__ __forceinline__ float4 screen_record(double2 p, double2 n) {
+  return make_float4((float)p.x, (float)p.y, (float)n.x, (float)n.y);
 }
 // A particle of system s needs its list rebuilt: flag the system, raise the pending
 // word, and (the thread that raises it) switch the step's rebuild node on.

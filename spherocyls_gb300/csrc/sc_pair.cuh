@@ -214,9 +214,8 @@ __device__ __forceinline__ bool pair_fp32(float dX, float dY, float nxA, float n
 // the FP32 rounding of the distance stay far below the 1e-4 relative margin.  Both
 // contact rules need the minimum distance below sig for any contact.
 __device__ __forceinline__ bool may_touch_fp32(float dX, float dY, float nxA, float nyA,
-                                               float aP, float nxB, float nyB, float aQ,
-                                               float sig) {
-  float a = aP * aP, c = aQ * aQ;
+                                               float nxB, float nyB, float sig) {
+  float a = fmaf(nxA, nxA, nyA * nyA), c = fmaf(nxB, nxB, nyB * nyB);
   float b = -(nxA * nxB + nyA * nyB);
   float d = nxA * dX + nyA * dY;
   float e = -(nxB * dX + nyB * dY);

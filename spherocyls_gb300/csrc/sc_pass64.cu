@@ -6,11 +6,12 @@
 // (tmarschall/spherocyls src/cpp/strain_dynamics.cpp:17-235,
 // src/cpp/resize_dynamics.cpp:164-243, src/cpp/spherocyl_box.cpp:303-355).
 //
-// One thread per particle slot gathers over the particle's full neighbour list
-// (column-major, one coalesced index load per entry) and computes each pair with
-// the lower particle index as the reference's "p", so the two threads that visit a
-// pair compute bit-identical contributions.  The epilogue fuses the Heun
-// predictor or corrector for the slot.
+// A pass is two kernels.  k_pairs64 screens every list entry in FP32 and evaluates
+// each pair that may touch once, in FP64, with the lower particle index as the
+// reference's "p"; k_step64 sums each particle's contributions in list order and runs
+// the Heun predictor or corrector.  k_pass64 does both in one thread per particle
+// (each pair from both sides): it serves lists longer than a mask word and handles
+// whose pair buffers could not be had, with the same bits.
 #include "sc_internal.hpp"
 #include "sc_pair.cuh"
 
@@ -66,7 +67,8 @@ __global__ void __launch_bounds__(128) k_build_nbrs(Dev d, const StepScalars* __
           bool hit = ip ? nbr_criterion(pi, pj, sig, g.pad, ts.gamma_p, ts.Lx_p, ts.Ly_p)
                         : nbr_criterion(pj, pi, sig, g.pad, ts.gamma_p, ts.Lx_p, ts.Ly_p);
           if (hit) {
-            if (cnt < d.maxn) d.nbr[(size_t)cnt * d.ntot + i] = j;
+            if (cnt < d.maxn)
+              d.nbr[(size_t)cnt * d.ntot + i] = (int)((unsigned)j | (ip ? kOwner64 : 0u));
             cnt++;
           }
         }
@@ -75,6 +77,55 @@ __global__ void __launch_bounds__(128) k_build_nbrs(Dev d, const StepScalars* __
     d.nbr_n[i] = cnt;
     if (cnt > d.maxn) atomicOr(d.status, ST_NBR_OVERFLOW);
   });
+}
+
+// ---- the FP32 screen ----
+//
+// Each particle keeps (x, y, A cos phi, A sin phi) of the state and of the predictor
+// copy rounded to FP32 (Dev::rec, rec_t) and R (rf); 20 bytes a neighbour instead of 48,
+// and no instruction of the FP64 pipe, which bounds the pass.  The rounding moves a
+// displacement by less than 2.5e-7 L per axis (two coordinates of up to L, their
+// difference, the image shift), by up to 1 + |gamma| of it after the shear: `slack`
+// covers both axes twice over, on top of the margins of may_touch_fp32.  In a grid of
+// three or more cells a side a pair at the image boundary (|d| = L/2) is out of reach,
+// so the image may be chosen in FP32; smaller boxes take the FP64 displacement.
+struct Screen64 {
+  double Lx, Ly, gamma;
+  float fLx, fLy, fgamma, slack;
+  bool small;
+};
+__device__ __forceinline__ Screen64 screen_of(const SysGeom& g, const StepScalars& ts, bool pred) {
+  Screen64 c;
+  c.gamma = pred ? ts.gamma_c : ts.gamma_p;
+  c.Lx = pred ? ts.Lx_c : ts.Lx_p;
+  c.Ly = pred ? ts.Ly_c : ts.Ly_p;
+  c.fLx = (float)c.Lx;
+  c.fLy = (float)c.Ly;
+  c.fgamma = (float)c.gamma;
+  c.slack = 5e-7f * (c.fLx + c.fLy) * (1.f + fabsf(c.fgamma));
+  c.small = g.cols < 3 || g.rows < 3;
+  return c;
+}
+// whether the pair (i, j), with FP32 records ri, rj and radius sum sig, may touch
+__device__ __forceinline__ bool screen_pair(const Screen64& c, const double2* __restrict__ XY,
+                                            int i, int j, float4 ri, float4 rj, float sig) {
+  float dx, dy;
+  if (!c.small) {
+    dx = ri.x - rj.x;
+    dy = ri.y - rj.y;
+    dx += c.fLx * (float)((dx < -0.5f * c.fLx) - (dx > 0.5f * c.fLx));
+    dy += c.fLy * (float)((dy < -0.5f * c.fLy) - (dy > 0.5f * c.fLy));
+    dx = fmaf(c.fgamma, dy, dx);
+  } else {
+    const double2 pi = XY[i], pj = XY[j];
+    double dX = pi.x - pj.x, dY = pi.y - pj.y;
+    dX += c.Lx * (double)((dX < -0.5 * c.Lx) - (dX > 0.5 * c.Lx));
+    dY += c.Ly * (double)((dY < -0.5 * c.Ly) - (dY > 0.5 * c.Ly));
+    dX += c.gamma * dY;
+    dx = (float)dX;
+    dy = (float)dY;
+  }
+  return may_touch_fp32(dx, dy, ri.z, ri.w, rj.z, rj.w, sig + c.slack);
 }
 
 // The reference rebuilds inside its corrector loop as soon as particle i has
@@ -88,100 +139,12 @@ __device__ __forceinline__ void flag_moved(const Dev& d, int s, int id, double2 
   }
 }
 
-// The FP64 pass of one slot: its pairs over its full list, then the Heun epilogue.
-template <int MODE, bool SE, bool TWO, bool FAST = false>
-__device__ __forceinline__ void pass64_slot(const Dev& d, const StepScalars* __restrict__ tab,
-                                            int row, int i) {
-  constexpr bool kPred =
-      (MODE == PASS_CORR_STRAIN || MODE == PASS_CORR_RESIZE || MODE == PASS_ENERGY_T);
-  int s = d.psys[i];
-  if (d.skip && d.skip[s]) return;  // a converged minimiser system
-  const SysGeom& g = d.geom[s];
-  const StepScalars ts = tab[row * d.nsys + s];
-  const double2* __restrict__ XY = kPred ? d.xy_t : d.xy;
-  const double2* __restrict__ NXY = kPred ? d.nxy_t : d.nxy;
-  const double gamma = kPred ? ts.gamma_c : ts.gamma_p;
-  const double Lx = kPred ? ts.Lx_c : ts.Lx_p;
-  const double Ly = kPred ? ts.Ly_c : ts.Ly_p;
-  const bool virial = d.stress_mode == STRESS_VIRIAL;
-  constexpr bool two_point = TWO;
-  const double two_n = 2.0 * g.n;
-
-  double2 pi = XY[i];
-  double2 ni = NXY[i];
-  double2 rai = d.ra[i];
-  int idi = d.id[i];
-  double fx = 0.0, fy = 0.0, tq = 0.0;
-  double se0 = 0.0, se1 = 0.0, se2 = 0.0, se3 = 0.0, se4 = 0.0;
-  int cnt = d.nbr_n[i];
-  if (cnt > d.maxn) cnt = d.maxn;
-  const float fpi_x = (float)ni.x, fpi_y = (float)ni.y, fai = (float)rai.y;
-  for (int k0 = 0; k0 < cnt; k0 += 64) {
-    // FP32 screen of up to 64 entries: the FP64 contact code then runs only for the
-    // entries that may touch, in list order, so the sums are unchanged bit for bit
-    unsigned long long cand = 0ull;
-    const int kend = cnt - k0 < 64 ? cnt : k0 + 64;
-    for (int k = k0; k < kend; k++) {
-      const int j = d.nbr[(size_t)k * d.ntot + i];
-      const double2 pj = XY[j];
-      const double2 nj = NXY[j];
-      const double2 raj = d.ra[j];
-      double dX = pi.x - pj.x, dY = pi.y - pj.y;
-      dX += Lx * (double)((dX < -0.5 * Lx) - (dX > 0.5 * Lx));
-      dY += Ly * (double)((dY < -0.5 * Ly) - (dY > 0.5 * Ly));
-      dX += gamma * dY;
-      if (may_touch_fp32((float)dX, (float)dY, fpi_x, fpi_y, fai, (float)nj.x, (float)nj.y,
-                         (float)raj.y, (float)(rai.x + raj.x)))
-        cand |= 1ull << (k - k0);
-    }
-    while (cand) {
-      const int k = k0 + __ffsll((long long)cand) - 1;
-      cand &= cand - 1ull;
-      int j = d.nbr[(size_t)k * d.ntot + i];
-      double2 pj = XY[j];
-      double2 nj = NXY[j];
-      double2 raj = d.ra[j];
-      int idj = d.id[j];
-      // the lower particle index plays the reference's "p": select the operands (one
-      // copy of the pair code per warp) rather than branch into two
-      const bool ip = idi < idj;
-      const double2 pP = ip ? pi : pj, pQ = ip ? pj : pi;
-      const double2 nP = ip ? ni : nj, nQ = ip ? nj : ni;
-      const double2 rP = ip ? rai : raj, rQ = ip ? raj : rai;
-      PairF64 o;
-      const bool hit =
-          two_point ? pair2_fp64<SE, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x,
-                                           nQ.y, rQ.y, rP.x + rQ.x, gamma, Lx, Ly, two_n, o)
-                    : pair_fp64<SE, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x, nQ.y,
-                                          rQ.y, rP.x + rQ.x, gamma, Lx, Ly, virial, two_n, o);
-      if (hit) {
-        if (ip) {
-          fx += o.fx;
-          fy += o.fy;
-          tq += o.tp;
-          if (SE) {
-            se0 += o.e;
-            se1 += o.pxx;
-            se2 += o.pyy;
-            se3 += o.pxy;
-            se4 += o.pyx;
-          }
-        } else {
-          fx -= o.fx;
-          fy -= o.fy;
-          tq += o.tq;
-        }
-      }
-    }
-  }
-  if (SE) {
-    d.se_part[i] = se0;
-    d.se_part[(size_t)d.ntot + i] = se1;
-    d.se_part[(size_t)2 * d.ntot + i] = se2;
-    d.se_part[(size_t)3 * d.ntot + i] = se3;
-    d.se_part[(size_t)4 * d.ntot + i] = se4;
-  }
-
+// The Heun step of slot i after its forces (fx, fy, tq) at the pass's positions are
+// known: predictor, corrector with the rebuild test, or (PASS_FORCE) the forces alone.
+template <int MODE>
+__device__ __forceinline__ void step64_slot(const Dev& d, const StepScalars& ts, const SysGeom& g,
+                                            int s, int i, double2 rai, int idi, double gamma,
+                                            double fx, double fy, double tq) {
   const double2 irc = d.irc[i];  // (I, RC)
   const double dt = ts.step;
   if (MODE == PASS_FORCE) {
@@ -207,7 +170,9 @@ __device__ __forceinline__ void pass64_slot(const Dev& d, const StepScalars* __r
     d.ph_t[i] = pht;
     double sn, cs;
     sincos(pht, &sn, &cs);
-    d.nxy_t[i] = make_double2(rai.y * cs, rai.y * sn);
+    const double2 nt = make_double2(rai.y * cs, rai.y * sn);
+    d.nxy_t[i] = nt;
+    d.rec_t[i] = screen_record(pt, nt);
   } else if (MODE == PASS_CORR_STRAIN) {
     // strain_step corrector, strain_dynamics.cpp:203-219
     double pht = d.ph_t[i];
@@ -237,7 +202,9 @@ __device__ __forceinline__ void pass64_slot(const Dev& d, const StepScalars* __r
     d.moved[i] = m;
     double sn, cs;
     sincos(phi, &sn, &cs);
-    d.nxy[i] = make_double2(rai.y * cs, rai.y * sn);
+    const double2 n1 = make_double2(rai.y * cs, rai.y * sn);
+    d.nxy[i] = n1;
+    d.rec[i] = screen_record(p, n1);
     if (!(isfinite(p.x) && isfinite(p.y) && isfinite(phi))) atomicOr(d.status, ST_NAN);
     flag_moved(d, s, idi, m, g.pad);
   } else if (MODE == PASS_PRED_RESIZE) {
@@ -274,7 +241,9 @@ __device__ __forceinline__ void pass64_slot(const Dev& d, const StepScalars* __r
     d.ph_t[i] = pht;
     double sn, cs;
     sincos(pht, &sn, &cs);
-    d.nxy_t[i] = make_double2(rai.y * cs, rai.y * sn);
+    const double2 nt = make_double2(rai.y * cs, rai.y * sn);
+    d.nxy_t[i] = nt;
+    d.rec_t[i] = screen_record(pt, nt);
   } else if (MODE == PASS_CORR_RESIZE) {
     double2 p0 = d.xy[i];
     const double phi0 = d.ph[i];
@@ -317,10 +286,103 @@ __device__ __forceinline__ void pass64_slot(const Dev& d, const StepScalars* __r
     d.moved[i] = m;
     double sn, cs;
     sincos(phi, &sn, &cs);
-    d.nxy[i] = make_double2(rai.y * cs, rai.y * sn);
+    const double2 n1 = make_double2(rai.y * cs, rai.y * sn);
+    d.nxy[i] = n1;
+    d.rec[i] = screen_record(p, n1);
     if (!(isfinite(p.x) && isfinite(p.y) && isfinite(phi))) atomicOr(d.status, ST_NAN);
     flag_moved(d, s, idi, m, g.pad);
   }
+}
+
+// The FP64 pass of one slot: its pairs over its full list, then the Heun epilogue.
+template <int MODE, bool SE, bool TWO, bool FAST = false>
+__device__ __forceinline__ void pass64_slot(const Dev& d, const StepScalars* __restrict__ tab,
+                                            int row, int i) {
+  constexpr bool kPred =
+      (MODE == PASS_CORR_STRAIN || MODE == PASS_CORR_RESIZE || MODE == PASS_ENERGY_T);
+  int s = d.psys[i];
+  if (d.skip && d.skip[s]) return;  // a converged minimiser system
+  const SysGeom& g = d.geom[s];
+  const StepScalars ts = tab[row * d.nsys + s];
+  const double2* __restrict__ XY = kPred ? d.xy_t : d.xy;
+  const double2* __restrict__ NXY = kPred ? d.nxy_t : d.nxy;
+  const double gamma = kPred ? ts.gamma_c : ts.gamma_p;
+  const double Lx = kPred ? ts.Lx_c : ts.Lx_p;
+  const double Ly = kPred ? ts.Ly_c : ts.Ly_p;
+  const bool virial = d.stress_mode == STRESS_VIRIAL;
+  constexpr bool two_point = TWO;
+  const double two_n = 2.0 * g.n;
+
+  double2 pi = XY[i];
+  double2 ni = NXY[i];
+  double2 rai = d.ra[i];
+  int idi = d.id[i];
+  double fx = 0.0, fy = 0.0, tq = 0.0;
+  double se0 = 0.0, se1 = 0.0, se2 = 0.0, se3 = 0.0, se4 = 0.0;
+  int cnt = d.nbr_n[i];
+  if (cnt > d.maxn) cnt = d.maxn;
+  const Screen64 scr = screen_of(g, ts, kPred);
+  const float4* __restrict__ REC = kPred ? d.rec_t : d.rec;
+  const float4 ri = REC[i];
+  const float Ri = d.rf[i];
+  for (int k0 = 0; k0 < cnt; k0 += 64) {
+    // FP32 screen of up to 64 entries: the FP64 contact code then runs only for the
+    // entries that may touch, in list order, so the sums are unchanged bit for bit
+    unsigned long long cand = 0ull;
+    const int kend = cnt - k0 < 64 ? cnt : k0 + 64;
+    for (int k = k0; k < kend; k++) {
+      const int j = d.nbr[(size_t)k * d.ntot + i] & kSlot64Mask;
+      if (screen_pair(scr, XY, i, j, ri, REC[j], Ri + d.rf[j])) cand |= 1ull << (k - k0);
+    }
+    while (cand) {
+      const int k = k0 + __ffsll((long long)cand) - 1;
+      cand &= cand - 1ull;
+      const unsigned e = (unsigned)d.nbr[(size_t)k * d.ntot + i];
+      const int j = (int)(e & kSlot64Mask);
+      double2 pj = XY[j];
+      double2 nj = NXY[j];
+      double2 raj = d.ra[j];
+      // the lower particle index plays the reference's "p": select the operands (one
+      // copy of the pair code per warp) rather than branch into two
+      const bool ip = (e & kOwner64) != 0u;
+      const double2 pP = ip ? pi : pj, pQ = ip ? pj : pi;
+      const double2 nP = ip ? ni : nj, nQ = ip ? nj : ni;
+      const double2 rP = ip ? rai : raj, rQ = ip ? raj : rai;
+      PairF64 o;
+      const bool hit =
+          two_point ? pair2_fp64<SE, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x,
+                                           nQ.y, rQ.y, rP.x + rQ.x, gamma, Lx, Ly, two_n, o)
+                    : pair_fp64<SE, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x, nQ.y,
+                                          rQ.y, rP.x + rQ.x, gamma, Lx, Ly, virial, two_n, o);
+      if (hit) {
+        if (ip) {
+          fx += o.fx;
+          fy += o.fy;
+          tq += o.tp;
+          if (SE) {
+            se0 += o.e;
+            se1 += o.pxx;
+            se2 += o.pyy;
+            se3 += o.pxy;
+            se4 += o.pyx;
+          }
+        } else {
+          fx -= o.fx;
+          fy -= o.fy;
+          tq += o.tq;
+        }
+      }
+    }
+  }
+  if (SE) {
+    d.se_part[i] = se0;
+    d.se_part[(size_t)d.ntot + i] = se1;
+    d.se_part[(size_t)2 * d.ntot + i] = se2;
+    d.se_part[(size_t)3 * d.ntot + i] = se3;
+    d.se_part[(size_t)4 * d.ntot + i] = se4;
+  }
+
+  step64_slot<MODE>(d, ts, g, s, i, rai, idi, gamma, fx, fy, tq);
 }
 
 template <int MODE, bool SE, bool TWO, bool FAST = false>
@@ -330,6 +392,221 @@ __global__ void __launch_bounds__(128) k_pass64(Dev d, const StepScalars* __rest
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.ntot) return;
   pass64_slot<MODE, SE, TWO, FAST>(d, tab, row, i);
+}
+
+// ---- a pass with each pair evaluated once ----
+//
+// k_pairs64, one block of kPairBlock threads per window of pr_win slots.  Phase 1: TPS
+// threads per slot screen its list in FP32 and leave the mask of the entries that may
+// touch; the pairs the slot owns (its index is the lower one) become the block's jobs,
+// in slot and list order.  Phase 2: one thread per job evaluates it in FP64, on full
+// warps whatever the lists' lengths, and writes the force and both torques to the
+// window's results.  With SE the owners then add their pairs' stress and energy, 128
+// jobs at a time, in list order (2: the energy alone).  RES false: no results wanted.
+//
+// The FP64 pipe (two lanes a cycle and SM) bounds it: about 150 operations a contact.
+// With one thread per particle, each pair evaluated from both sides and the screen's
+// displacement in FP64, a shear pass took 2.66 ms at 2^20 particles and 65 us at 1024
+// (8 blocks, the rest of the GPU idle); here 0.50 + 0.25 ms (k_pairs64 + k_step64) and
+// 10 + 15 us.
+constexpr int kPairBlock = 128;
+
+template <int SE, bool RES, bool TWO, bool FAST, int TPS>
+__global__ void __launch_bounds__(kPairBlock) k_pairs64(Dev d, const StepScalars* __restrict__ tab,
+                                                       int row, int pred) {
+  constexpr int S = kPairBlock / TPS;
+  __shared__ unsigned short job[S * 64];  // slot in the window << 6 | list entry
+  __shared__ int wsum[kPairBlock / 32];
+  __shared__ double res[SE == 1 ? 5 : 1][SE ? kPairBlock : 1];
+  const int t = threadIdx.x, l = t / TPS, sub = t % TPS;
+  const int i0 = blockIdx.x * S, i = i0 + l;
+  const double2* __restrict__ XY = pred ? d.xy_t : d.xy;
+  const double2* __restrict__ NXY = pred ? d.nxy_t : d.nxy;
+  const float4* __restrict__ REC = pred ? d.rec_t : d.rec;
+  const size_t ntot = d.ntot;
+
+  unsigned long long m = 0ull, mo = 0ull;
+  bool live = i < d.ntot;
+  if (live) {
+    const int s = d.psys[i];
+    live = !(d.skip && d.skip[s]);  // converged minimiser systems have no jobs
+    if (live) {
+      const Screen64 scr = screen_of(d.geom[s], tab[row * d.nsys + s], pred != 0);
+      const float4 ri = REC[i];
+      const float Ri = d.rf[i];
+      const int cnt = min(d.nbr_n[i], d.maxn);
+      for (int k = sub; k < cnt; k += TPS) {
+        const unsigned e = (unsigned)d.nbr[k * ntot + i];
+        // a pass without results has no use for the entries it does not own
+        if (!RES && !(e & kOwner64)) continue;
+        const int j = (int)(e & kSlot64Mask);
+        if (screen_pair(scr, XY, i, j, ri, REC[j], Ri + d.rf[j])) {
+          m |= 1ull << k;
+          if (e & kOwner64) mo |= 1ull << k;
+        }
+      }
+    }
+  }
+  for (int o = 1; o < TPS; o <<= 1) {
+    m |= __shfl_xor_sync(0xffffffffu, m, o);
+    mo |= __shfl_xor_sync(0xffffffffu, mo, o);
+  }
+  // exclusive scan of the slots' job counts over the block
+  const int c = sub == 0 ? __popcll(mo) : 0;
+  int v = c;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if ((t & 31) >= o) v += u;
+  }
+  if ((t & 31) == 31) wsum[t >> 5] = v;
+  __syncthreads();
+  int off = v - c, total = 0;
+  for (int w = 0; w < kPairBlock / 32; w++) {
+    if (w < (t >> 5)) off += wsum[w];
+    total += wsum[w];
+  }
+  const bool fits = total <= S * kPairCap;
+  if (sub == 0 && live) {
+    if (RES) {
+      d.pr_mask[i] = m;
+      d.pr_info[i] = fits ? (unsigned)off | (unsigned)c << 16 : kPairsOver;
+    }
+    int q = off;
+    for (unsigned long long b = mo; b; b &= b - 1ull)
+      job[q++] = (unsigned short)(l << 6 | (__ffsll((long long)b) - 1));
+  }
+  __syncthreads();
+
+  double acc[SE == 1 ? 5 : 1] = {};
+  const size_t base = (size_t)i0 * kPairCap;
+  for (int b0 = 0; b0 < total; b0 += kPairBlock) {
+    const int p = b0 + t;
+    if (p < total) {
+      const int io = i0 + (job[p] >> 6), k = job[p] & 63;
+      const int j = (int)((unsigned)d.nbr[k * ntot + io] & kSlot64Mask);
+      const int s = d.psys[io];
+      const StepScalars& ts = tab[row * d.nsys + s];
+      const double gamma = pred ? ts.gamma_c : ts.gamma_p;
+      const double Lx = pred ? ts.Lx_c : ts.Lx_p, Ly = pred ? ts.Ly_c : ts.Ly_p;
+      const double two_n = SE ? 2.0 * d.geom[s].n : 0.0;
+      const double2 pP = XY[io], pQ = XY[j], nP = NXY[io], nQ = NXY[j], rP = d.ra[io], rQ = d.ra[j];
+      PairF64 o;
+      const bool hit =
+          TWO ? pair2_fp64<SE != 0, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x, nQ.y,
+                                          rQ.y, rP.x + rQ.x, gamma, Lx, Ly, two_n, o)
+              : pair_fp64<SE != 0, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x, nQ.y,
+                                         rQ.y, rP.x + rQ.x, gamma, Lx, Ly,
+                                         d.stress_mode == STRESS_VIRIAL, two_n, o);
+      if (RES && fits) {
+        d.pr_who[base + p] = hit ? j : -1;
+        if (hit) {
+          double4_16a r;
+          r.x = o.fx;
+          r.y = o.fy;
+          r.z = o.tp;
+          r.w = o.tq;
+          d.pr_res[base + p] = r;
+        }
+      }
+      if (SE) res[0][t] = hit ? o.e : 0.0;
+      if (SE == 1) {
+        res[1][t] = hit ? o.pxx : 0.0;
+        res[2][t] = hit ? o.pyy : 0.0;
+        res[3][t] = hit ? o.pxy : 0.0;
+        res[4][t] = hit ? o.pyx : 0.0;
+      }
+    }
+    if (SE) {
+      __syncthreads();
+      const int q0 = max(off, b0), q1 = min(off + c, b0 + kPairBlock);
+      for (int q = q0; q < q1; q++)
+        for (int comp = 0; comp < (SE == 1 ? 5 : 1); comp++) acc[comp] += res[comp][q - b0];
+      __syncthreads();
+    }
+  }
+  if (SE && live && sub == 0)
+    for (int comp = 0; comp < (SE == 1 ? 5 : 1); comp++) d.se_part[comp * ntot + i] = acc[comp];
+}
+
+// One pair of a window whose results did not fit, evaluated where it is needed (the same
+// operations, so the same bits); out of line, since it hardly ever runs.
+template <bool TWO, bool FAST>
+__device__ __noinline__ bool pair_again64(const double2* XY, const double2* NXY,
+                                          const double2* ra, int iP, int iQ, double gamma,
+                                          double Lx, double Ly, double4_16a* r) {
+  const double2 pP = XY[iP], pQ = XY[iQ], nP = NXY[iP], nQ = NXY[iQ], rP = ra[iP], rQ = ra[iQ];
+  PairF64 o;
+  const bool hit =
+      TWO ? pair2_fp64<false, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x, nQ.y, rQ.y,
+                                    rP.x + rQ.x, gamma, Lx, Ly, 0.0, o)
+          : pair_fp64<false, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x, nQ.y, rQ.y,
+                                   rP.x + rQ.x, gamma, Lx, Ly, false, 0.0, o);
+  if (hit) {
+    r->x = o.fx;
+    r->y = o.fy;
+    r->z = o.tp;
+    r->w = o.tq;
+  }
+  return hit;
+}
+
+// k_step64, one thread per slot: the slot's contributions from the pair results, in list
+// order (its own pairs follow each other in its window; a pair it does not own is looked
+// up among its partner's two or three), then the Heun epilogue.
+template <int MODE, bool TWO, bool FAST>
+__global__ void __launch_bounds__(128) k_step64(Dev d, const StepScalars* __restrict__ tab,
+                                               int row) {
+  constexpr bool kCorr = MODE == PASS_CORR_STRAIN || MODE == PASS_CORR_RESIZE;
+  if (kCorr) mark_pending_rebuilds(d, tab, row);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= d.ntot) return;
+  const int s = d.psys[i];
+  if (d.skip && d.skip[s]) return;  // a converged minimiser system
+  const StepScalars& ts = tab[row * d.nsys + s];
+  const double gamma = kCorr ? ts.gamma_c : ts.gamma_p;
+  const unsigned info = d.pr_info[i];
+  const int win = d.pr_win;
+  const size_t own = (size_t)(i / win) * win * kPairCap + (info & 0xffffu);
+  double fx = 0.0, fy = 0.0, tq = 0.0;
+  int rank = 0;
+  for (unsigned long long m = d.pr_mask[i]; m; m &= m - 1ull) {
+    const int k = __ffsll((long long)m) - 1;
+    const unsigned e = (unsigned)d.nbr[(size_t)k * d.ntot + i];
+    const int j = (int)(e & kSlot64Mask);
+    const bool ip = (e & kOwner64) != 0u;
+    const unsigned inf = ip ? info : d.pr_info[j];
+    double4_16a r;
+    bool hit = false;
+    if (inf == kPairsOver) {
+      const double Lx = kCorr ? ts.Lx_c : ts.Lx_p, Ly = kCorr ? ts.Ly_c : ts.Ly_p;
+      hit = pair_again64<TWO, FAST>(kCorr ? d.xy_t : d.xy, kCorr ? d.nxy_t : d.nxy, d.ra,
+                                    ip ? i : j, ip ? j : i, gamma, Lx, Ly, &r);
+    } else if (ip) {
+      const size_t q = own + rank++;
+      hit = d.pr_who[q] >= 0;
+      if (hit) r = d.pr_res[q];
+    } else {
+      const size_t q0 = (size_t)(j / win) * win * kPairCap + (inf & 0xffffu);
+      const int n = (int)(inf >> 16);
+      for (int q = 0; q < n; q++)
+        if (d.pr_who[q0 + q] == i) {
+          hit = true;
+          r = d.pr_res[q0 + q];
+          break;
+        }
+    }
+    if (!hit) continue;
+    if (ip) {
+      fx += r.x;
+      fy += r.y;
+      tq += r.z;
+    } else {
+      fx -= r.x;
+      fy -= r.y;
+      tq += r.w;
+    }
+  }
+  step64_slot<MODE>(d, ts, d.geom[s], s, i, d.ra[i], d.id[i], gamma, fx, fy, tq);
 }
 
 // ---- stress and energy of the mixed form, in FP64 ----
@@ -396,7 +673,7 @@ __global__ void __launch_bounds__(kSeBlock) k_mx_se64(Dev d, const StepScalars* 
   const bool valid = i < d.ntot;
   const bool virial = d.stress_mode == STRESS_VIRIAL;
   int cnt = 0, idi = 0;
-  float fnx = 0.f, fny = 0.f, fai = 0.f;
+  float fnx = 0.f, fny = 0.f;
   double px = 0, py = 0, Lx = 1, Ly = 1, gamma = 0, W = 0, H = 0, Ri = 0;
   if (valid) {
     const int s = d.psys[i];
@@ -427,7 +704,6 @@ __global__ void __launch_bounds__(kSeBlock) k_mx_se64(Dev d, const StepScalars* 
     o_i2n[t] = 0.5 * g.inv_n;
     fnx = (float)ni.x;
     fny = (float)ni.y;
-    fai = (float)rai.y;
     idi = d.id[i];
     cnt = min(d.nbr_n[i], d.maxn);
   }
@@ -449,14 +725,14 @@ __global__ void __launch_bounds__(kSeBlock) k_mx_se64(Dev d, const StepScalars* 
       if (!(idi < d.id[j])) continue;
       const double2 pj = d.xy_t[j];
       const double2 nj = d.nxy_t[j];
-      const double Aj = d.ra[j].y, Rj = d.ra[j].x;
+      const double Rj = d.ra[j].x;
       double sx = (px - pj.x) + (double)(1 - (int)((e >> 28) & 3u)) * W;
       double sy = (py - pj.y) + (double)(1 - (int)(e >> 30)) * H;
       sx += Lx * (double)((sx < -0.5 * Lx) - (sx > 0.5 * Lx));
       sy += Ly * (double)((sy < -0.5 * Ly) - (sy > 0.5 * Ly));
       sx += gamma * sy;
-      if (may_touch_fp32((float)sx, (float)sy, fnx, fny, fai, (float)nj.x, (float)nj.y,
-                         (float)Aj, (float)(Ri + Rj)))
+      if (may_touch_fp32((float)sx, (float)sy, fnx, fny, (float)nj.x, (float)nj.y,
+                         (float)(Ri + Rj)))
         m |= 1ull << (k - k0);
     }
     mask[t] = m;
@@ -524,45 +800,88 @@ __global__ void __launch_bounds__(kSeBlock) k_mx_se64(Dev d, const StepScalars* 
     for (int comp = 0; comp < 5; comp++) d.se_part[(size_t)comp * d.ntot + i] = acc[comp];
 }
 
-template <int MODE, bool SE>
-void launch_one(const Dev& d, const StepScalars* tab, int row, cudaStream_t st) {
-  int block = 128;
-  int grid = (d.ntot + block - 1) / block;
+template <int MODE, bool SE, bool FAST = false>
+void launch_whole(const Dev& d, const StepScalars* tab, int row, cudaStream_t st) {
+  const int block = 128, grid = (d.ntot + block - 1) / block;
   if (d.contact_model == 1)
-    k_pass64<MODE, SE, true><<<grid, block, 0, st>>>(d, tab, row);
+    k_pass64<MODE, SE, true, FAST><<<grid, block, 0, st>>>(d, tab, row);
   else
-    k_pass64<MODE, SE, false><<<grid, block, 0, st>>>(d, tab, row);
+    k_pass64<MODE, SE, false, FAST><<<grid, block, 0, st>>>(d, tab, row);
+}
+
+template <int SE, bool RES, bool FAST>
+void launch_pairs(const Dev& d, const StepScalars* tab, int row, bool pred, cudaStream_t st) {
+  const int grid = (d.ntot + d.pr_win - 1) / d.pr_win, p = pred ? 1 : 0;
+  const bool two = d.contact_model == 1;
+  if (d.pr_win == kPairBlock) {
+    two ? k_pairs64<SE, RES, true, FAST, 1><<<grid, kPairBlock, 0, st>>>(d, tab, row, p)
+        : k_pairs64<SE, RES, false, FAST, 1><<<grid, kPairBlock, 0, st>>>(d, tab, row, p);
+  } else {
+    two ? k_pairs64<SE, RES, true, FAST, 4><<<grid, kPairBlock, 0, st>>>(d, tab, row, p)
+        : k_pairs64<SE, RES, false, FAST, 4><<<grid, kPairBlock, 0, st>>>(d, tab, row, p);
+  }
+}
+
+template <int MODE, bool FAST = false>
+void launch_step(const Dev& d, const StepScalars* tab, int row, cudaStream_t st) {
+  const int block = d.pr_win == kPairBlock ? 128 : 32, grid = (d.ntot + block - 1) / block;
+  if (d.contact_model == 1)
+    k_step64<MODE, true, FAST><<<grid, block, 0, st>>>(d, tab, row);
+  else
+    k_step64<MODE, false, FAST><<<grid, block, 0, st>>>(d, tab, row);
+}
+
+// the pass of one mode through the pair buffers, or in one kernel without them
+template <int MODE>
+int launch_mode(const Dev& d, bool se, const StepScalars* tab, int row, cudaStream_t st) {
+  constexpr bool corr = MODE == PASS_CORR_STRAIN || MODE == PASS_CORR_RESIZE;
+  if (d.pr_win == 0) {
+    if constexpr (corr)
+      launch_whole<MODE, false>(d, tab, row, st);
+    else
+      se ? launch_whole<MODE, true>(d, tab, row, st) : launch_whole<MODE, false>(d, tab, row, st);
+    return 1;
+  }
+  if (!corr && se)
+    launch_pairs<1, true, false>(d, tab, row, corr, st);
+  else
+    launch_pairs<0, true, false>(d, tab, row, corr, st);
+  launch_step<MODE>(d, tab, row, st);
+  return 2;
 }
 
 }  // namespace
 
-void launch_pass_fp64(const Dev& d, int mode, bool se, const StepScalars* tab, int row,
-                      cudaStream_t st, bool fast) {
+// Small systems take windows of 32 slots, four threads screening each: 32 blocks at 1024
+// particles instead of 8.  At 131072 the two are within 1% of each other.
+int pair_window(int ntot) { return ntot <= kSmallPairs ? kPairBlock / 4 : kPairBlock; }
+
+int launch_pass_fp64(const Dev& d, int mode, bool se, const StepScalars* tab, int row,
+                     cudaStream_t st, bool fast) {
   if (fast && mode == PASS_FORCE && !se) {
     // the minimiser's force evaluation (shared reciprocals, see qdiv)
-    const int block = 128, grid = (d.ntot + block - 1) / block;
-    if (d.contact_model == 1)
-      k_pass64<PASS_FORCE, false, true, true><<<grid, block, 0, st>>>(d, tab, row);
-    else
-      k_pass64<PASS_FORCE, false, false, true><<<grid, block, 0, st>>>(d, tab, row);
-    return;
+    if (d.pr_win == 0) {
+      launch_whole<PASS_FORCE, false, true>(d, tab, row, st);
+      return 1;
+    }
+    launch_pairs<0, true, true>(d, tab, row, false, st);
+    launch_step<PASS_FORCE, true>(d, tab, row, st);
+    return 2;
   }
   switch (mode) {
-    case PASS_FORCE:
-      se ? launch_one<PASS_FORCE, true>(d, tab, row, st) : launch_one<PASS_FORCE, false>(d, tab, row, st);
-      break;
-    case PASS_CORR_STRAIN: launch_one<PASS_CORR_STRAIN, false>(d, tab, row, st); break;
-    case PASS_PRED_STRAIN:
-      se ? launch_one<PASS_PRED_STRAIN, true>(d, tab, row, st)
-         : launch_one<PASS_PRED_STRAIN, false>(d, tab, row, st);
-      break;
-    case PASS_CORR_RESIZE: launch_one<PASS_CORR_RESIZE, false>(d, tab, row, st); break;
-    case PASS_PRED_RESIZE:
-      se ? launch_one<PASS_PRED_RESIZE, true>(d, tab, row, st)
-         : launch_one<PASS_PRED_RESIZE, false>(d, tab, row, st);
-      break;
-    case PASS_ENERGY_T: launch_one<PASS_ENERGY_T, true>(d, tab, row, st); break;
+    case PASS_FORCE: return launch_mode<PASS_FORCE>(d, se, tab, row, st);
+    case PASS_CORR_STRAIN: return launch_mode<PASS_CORR_STRAIN>(d, false, tab, row, st);
+    case PASS_PRED_STRAIN: return launch_mode<PASS_PRED_STRAIN>(d, se, tab, row, st);
+    case PASS_CORR_RESIZE: return launch_mode<PASS_CORR_RESIZE>(d, false, tab, row, st);
+    case PASS_PRED_RESIZE: return launch_mode<PASS_PRED_RESIZE>(d, se, tab, row, st);
+    case PASS_ENERGY_T:
+      if (d.pr_win == 0)
+        launch_whole<PASS_ENERGY_T, true>(d, tab, row, st);
+      else
+        launch_pairs<2, false, false>(d, tab, row, true, st);
+      return 1;
   }
+  return 0;
 }
 
 void launch_mx_se64(const Dev& d, const StepScalars* tab, int row, cudaStream_t st) {
