@@ -34,15 +34,29 @@ __device__ __forceinline__ bool nbr_criterion(double2 pp, double2 pq, double sig
   return false;
 }
 
+// The padded list of each listed slot: the reference's criterion in FP64, decided in
+// FP32 wherever that is certain.  The FP32 copies of the positions move |dX|, |dX + dY/2|
+// and |dY| by less than `slack` (see Screen64), so a candidate outside the bound by more
+// is out and one inside it by more is in; about one in a thousand is evaluated in FP64.
+// Boxes so small that a candidate at the image boundary (|d| = L/2), where FP32 might
+// choose the other image, can be in reach evaluate all in FP64.  The FP64 pipe
+// bounded the build: 14 operations for each of about 33 candidates a particle took 191 us
+// at 131072 particles (a/R 0.25 to 2), the FP32 test takes 26 us.
 __global__ void __launch_bounds__(128) k_build_nbrs(Dev d, const StepScalars* __restrict__ tab,
                                                    int row) {
   if (*d.any == 0) return;
   for_listed_slots(d, [&](int i, int s) {
-    const SysGeom g = d.geom[s];
-    const StepScalars ts = tab[row * d.nsys + s];
-    double2 pi = d.xy[i];
-    double2 rai = d.ra[i];
-    int idi = d.id[i];
+    const SysGeom& g = d.geom[s];
+    const StepScalars& ts = tab[row * d.nsys + s];
+    const float4 ri = d.rec[i];
+    const float si = d.rsf[i];
+    const int idi = d.id[i];
+    const float gam = (float)ts.gamma_p, fLx = (float)ts.Lx_p, fLy = (float)ts.Ly_p;
+    const float pad = (float)g.pad;
+    const float slack = 5e-7f * (fLx + fLy) * (1.f + fabsf(gam)) + 1e-6f * (2.f * g.smax + pad);
+    const float reach = g.smax + pad + slack;
+    const bool small = !(0.5f * fLx > reach * (1.f + fmaxf(fabsf(gam), 0.5f)) &&
+                         0.5f * fLy > reach);
     int c = d.cell[i] - g.c0;
     int col, rw;
     cell_colrow(g, c, &col, &rw);
@@ -58,19 +72,26 @@ __global__ void __launch_bounds__(128) k_build_nbrs(Dev d, const StepScalars* __
         int st = d.cell_start[cc], nn = d.cell_count[cc];
         for (int j = st; j < st + nn; j++) {
           if (j == i) continue;
-          int idj = d.id[j];
-          double2 pj = d.xy[j];
-          double2 raj = d.ra[j];
-          bool ip = idi < idj;
-          // S = R_p + A_p + R_q + A_q summed in the reference's order
-          double sig = ip ? rai.x + rai.y + raj.x + raj.y : raj.x + raj.y + rai.x + rai.y;
-          bool hit = ip ? nbr_criterion(pi, pj, sig, g.pad, ts.gamma_p, ts.Lx_p, ts.Ly_p)
-                        : nbr_criterion(pj, pi, sig, g.pad, ts.gamma_p, ts.Lx_p, ts.Ly_p);
-          if (hit) {
-            if (cnt < d.maxn)
-              d.nbr[(size_t)cnt * d.ntot + i] = (int)((unsigned)j | (ip ? kOwner64 : 0u));
-            cnt++;
+          const float4 rj = d.rec[j];
+          float dx = ri.x - rj.x, dy = ri.y - rj.y;
+          dx += fLx * (float)((dx < -0.5f * fLx) - (dx > 0.5f * fLx));
+          dy += fLy * (float)((dy < -0.5f * fLy) - (dy > 0.5f * fLy));
+          const float near = fminf(fabsf(fmaf(gam, dy, dx)), fabsf(fmaf(0.5f, dy, dx)));
+          const float over = fmaxf(fabsf(dy), near) - (si + d.rsf[j] + pad);
+          if (!small && over > slack) continue;
+          const int idj = d.id[j];
+          const bool ip = idi < idj;
+          if (small || !(over < -slack)) {
+            const double2 pi = d.xy[i], pj = d.xy[j], rai = d.ra[i], raj = d.ra[j];
+            // S = R_p + A_p + R_q + A_q summed in the reference's order
+            double sig = ip ? rai.x + rai.y + raj.x + raj.y : raj.x + raj.y + rai.x + rai.y;
+            if (!(ip ? nbr_criterion(pi, pj, sig, g.pad, ts.gamma_p, ts.Lx_p, ts.Ly_p)
+                     : nbr_criterion(pj, pi, sig, g.pad, ts.gamma_p, ts.Lx_p, ts.Ly_p)))
+              continue;
           }
+          if (cnt < d.maxn)
+            d.nbr[(size_t)cnt * d.ntot + i] = (int)((unsigned)j | (ip ? kOwner64 : 0u));
+          cnt++;
         }
       }
     }
@@ -86,9 +107,9 @@ __global__ void __launch_bounds__(128) k_build_nbrs(Dev d, const StepScalars* __
 // and no instruction of the FP64 pipe, which bounds the pass.  The rounding moves a
 // displacement by less than 2.5e-7 L per axis (two coordinates of up to L, their
 // difference, the image shift), by up to 1 + |gamma| of it after the shear: `slack`
-// covers both axes twice over, on top of the margins of may_touch_fp32.  In a grid of
-// three or more cells a side a pair at the image boundary (|d| = L/2) is out of reach,
-// so the image may be chosen in FP32; smaller boxes take the FP64 displacement.
+// covers both axes twice over, on top of the margins of may_touch_fp32.  Where a pair at
+// the image boundary (|d| = L/2) is out of reach the image may be chosen in FP32; smaller
+// boxes take the FP64 displacement.
 struct Screen64 {
   double Lx, Ly, gamma;
   float fLx, fLy, fgamma, slack;
@@ -103,7 +124,8 @@ __device__ __forceinline__ Screen64 screen_of(const SysGeom& g, const StepScalar
   c.fLy = (float)c.Ly;
   c.fgamma = (float)c.gamma;
   c.slack = 5e-7f * (c.fLx + c.fLy) * (1.f + fabsf(c.fgamma));
-  c.small = g.cols < 3 || g.rows < 3;
+  const float reach = g.smax + c.slack;
+  c.small = !(0.5f * c.fLx > reach * (1.f + fabsf(c.fgamma)) && 0.5f * c.fLy > reach);
   return c;
 }
 // whether the pair (i, j), with FP32 records ri, rj and radius sum sig, may touch
@@ -852,8 +874,9 @@ int launch_mode(const Dev& d, bool se, const StepScalars* tab, int row, cudaStre
 
 }  // namespace
 
-// Small systems take windows of 32 slots, four threads screening each: 32 blocks at 1024
-// particles instead of 8.  At 131072 the two are within 1% of each other.
+// Small systems take windows of 32 slots, four threads screening each, which puts the
+// pairs on four times the SMs.  A shear step in us, windows of 32 against 128: 63 and 93
+// at 4096 particles, 81 and 96 at 16384, 211 and 214 at 65536, 316 and 304 at 131072.
 int pair_window(int ntot) { return ntot <= kSmallPairs ? kPairBlock / 4 : kPairBlock; }
 
 int launch_pass_fp64(const Dev& d, int mode, bool se, const StepScalars* tab, int row,

@@ -61,3 +61,19 @@ def test_pair_buffers_give_the_same_bits(n, phi, aor, contacts, gamma):
 def test_lists_hold_the_same_pairs():
     a, b = _boxes(777, 0.85, 1.0, 1, 0.2)
     assert np.array_equal(a.pairs(), b.pairs())
+
+
+@pytest.mark.parametrize("n,phi,aor,gamma,pad", [
+    (40, 0.8, 1.0, 0.0, 0.0), (500, 0.85, 1.0, 0.45, 0.1), (500, 0.85, 1.0, -0.3, 0.1),
+    (5000, 0.84, 1.5, 0.3, 0.2), (70000, 0.84, 0.3, 0.1, 0.3)])
+def test_list_equals_the_oracles(oracle_built, n, phi, aor, gamma, pad):
+    """The FP32-decided list is the reference's (check_neighbors,
+    src/cpp/spherocyl_box.cpp:303-318), pair for pair."""
+    from spherocyls_gb300 import generate_packing
+
+    a, _ = _boxes(n, phi, aor, 1, gamma, pad=pad)
+    L, x, y, p, R, A = generate_packing(n, phi, aor, seed=5)
+    ob = oracle_built.OracleBox(L, x, y, p, A, R, pad, gamma=gamma)
+    ob.find_neighbors()
+    ref = ob.pairs()
+    assert np.array_equal(a.pairs(), ref[np.lexsort((ref[:, 1], ref[:, 0]))])
