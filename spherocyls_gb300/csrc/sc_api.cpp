@@ -272,7 +272,7 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
          h.dalloc(&d.ord, N, "ord") && h.dalloc(&d.nbr_p, N * d.maxn, "nbr_p") &&
          h.dalloc(&d.nbr_pn, N, "nbr_pn");
   else
-    ok = ok && h.dalloc(&d.rsf, N, "rsf");
+    ok = ok && h.dalloc(&d.rsf, N, "rsf") && h.dalloc(&d.iaa, N, "iaa");
   if (opt.precision == SC_PREC_MIXED) {
     ok = ok && h.dalloc(&d.gbar, 2, "grid barrier") && h.dalloc(&h.d_persist, 1, "persist out");
     if (ok) ok = h.cuda_ok(cudaMemsetAsync(d.gbar, 0, 2 * sizeof(unsigned), h.stream), "barrier");

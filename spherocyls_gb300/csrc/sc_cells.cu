@@ -366,6 +366,7 @@ __global__ void k_rb_commit(Dev d, const StepScalars* __restrict__ tab, int row,
       d.rec[i] = screen_record(p, n);
       d.rf[i] = (float)ra.x;
       d.rsf[i] = (float)(ra.x + ra.y);
+      d.iaa[i] = shared_rcp(ra.y * ra.y);
     }
   });
 }

@@ -188,6 +188,7 @@ struct Dev {
   float4* pa;     // (R, A, particle index as int bits, 1/I)
   float* rcf;     // isolated-rotation coefficient RC
   float* rf;      // R in FP32: the only per-neighbour constant the force pass gathers
+  double* iaa;    // 1 / A^2 (FP64 form: shared_rcp, sc_pair.cuh)
   float* rsf;     // R + A in FP32 (FP64 form: the list build's reach)
   int* cellp;     // local cell packed as col | row << 16
   float* gbuild;  // [nsys] gamma at which each system's list was built

@@ -227,14 +227,14 @@ __global__ void __launch_bounds__(128) k_na_forces(int* scratch, int n, double L
         PairF64 o;
         if (i < j) {
           if (pair_fp64<false>(xi - x[j], yi - y[j], nxi, nyi, Ai, nxj, nyj, Aj, Ri + R[j], gamma,
-                               L, L, false, 2.0, o)) {
+                               L, L, false, 2.0, o, 0.0, 0.0)) {
             Fx += o.fx;
             Fy += o.fy;
             T += o.tp;
           }
         } else {
           if (pair_fp64<false>(x[j] - xi, y[j] - yi, nxj, nyj, Aj, nxi, nyi, Ai, R[j] + Ri, gamma,
-                               L, L, false, 2.0, o)) {
+                               L, L, false, 2.0, o, 0.0, 0.0)) {
             Fx -= o.fx;
             Fy -= o.fy;
             T += o.tq;

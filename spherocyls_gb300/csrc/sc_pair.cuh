@@ -26,13 +26,63 @@ struct PairF64 {
   double e, pxx, pyy, pxy, pyx;   // stress/energy contributions (when requested)
 };
 
-// x / y, or, in the minimiser's form (FAST), x times a reciprocal of y shared by
-// several quotients.  The FAST form trades the last bits of the reference's
+// ---- FP64 operations taken off the FP64 pipe ----
+//
+// GB300 runs FP64 at about 1/60 of its FP32 rate, and that pipe bounds the pair code.
+// Comparisons with constants and clamps are decided on the bits of the operand by the
+// integer pipe instead, with the same result for every value (NaN as in fmin, fmax).
+
+// d - L where d > L/2, d + L where d < -L/2 (L > 0)
+__device__ __forceinline__ double nearest_image(double d, double L) {
+  if ((__double2hiint(d) & 0x7fffffff) < __double2hiint(0.5 * L)) return d;
+  return d + L * (double)((d < -0.5 * L) - (d > 0.5 * L));
+}
+__device__ __forceinline__ unsigned long long abs_bits(double v) {
+  return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
+constexpr unsigned long long kBitsOne = 0x3ff0000000000000ull, kBitsInf = 0x7ff0000000000000ull;
+// fmin(fmax(v, -1), 1): a NaN becomes -1
+__device__ __forceinline__ double clamp_one(double v) {
+  const unsigned long long b = abs_bits(v);
+  if (b < kBitsOne) return v;
+  return b > kBitsInf || __double2hiint(v) < 0 ? -1.0 : 1.0;
+}
+// |v| > 1 and |v| >= 1 (false for NaN)
+__device__ __forceinline__ bool beyond_one(double v) {
+  const unsigned long long b = abs_bits(v);
+  return b > kBitsOne && b <= kBitsInf;
+}
+__device__ __forceinline__ bool reaches_one(double v) {
+  const unsigned long long b = abs_bits(v);
+  return b >= kBitsOne && b <= kBitsInf;
+}
+// u < v for sums of squares, whose bits order as their values (false where u is NaN)
+__device__ __forceinline__ bool less_square(double u, double v) {
+  return (unsigned long long)__double_as_longlong(u) < (unsigned long long)__double_as_longlong(v);
+}
+
+// Quotients that share a divisor: r = 1/y rounded to nearest, then x r with one correction
+// by its exact remainder, which is the correctly rounded x/y (P. W. Markstein, IBM J. Res.
+// Dev. 34, 111 (1990)); three operations in place of a division's eight or so.  A divisor
+// whose reciprocal is near the ends of the exponent range has r = 0 and is divided by.
+__device__ __forceinline__ double shared_rcp(double y) {
+  const double r = 1.0 / y;
+  const unsigned h = (unsigned)__double2hiint(r);
+  return h - 0x20b00000u < 0x3e800000u ? r : 0.0;  // 2^-500 < r < 2^500
+}
+__device__ __forceinline__ double div_by(double x, double y, double r) {
+  if (__double2hiint(r) == 0) return x / y;
+  const double q = x * r;
+  return fma(fma(-y, q, x), r, q);
+}
+
+// x / y by the shared reciprocal of y, or, in the minimiser's form (FAST), x times a
+// reciprocal of y.  The FAST form trades the last bits of the reference's
 // rounding for fewer FP64 divisions (GB300's FP64 rate is a small fraction of its
 // FP32 rate); the force-evaluation and dynamics paths never use it.
 template <bool FAST>
 __device__ __forceinline__ double qdiv(double x, double y, double inv_y) {
-  return FAST ? x * inv_y : x / y;
+  return FAST ? x * inv_y : div_by(x, y, inv_y);
 }
 
 // Reciprocals of a = |u_A|^2, c = |u_B|^2, delta and sig from one division.
@@ -60,17 +110,18 @@ __device__ __forceinline__ Recip64 recip64(double a, double c, double delta, dou
 }
 
 // dX, dY: raw coordinate differences P - Q (no minimum image yet).
-// Returns true when the spherocylinders overlap.
+// Returns true when the spherocylinders overlap.  inv_aP, inv_aQ: shared_rcp of aP^2, aQ^2
+// (unused with FAST).
 // FAST with SE (the mixed form's FP64 stress): inv_LL = 1/(Lx Ly) and inv_two_n =
 // 1/(2n) from the caller replace the per-term divisions.
 template <bool SE, bool FAST = false>
 __device__ __forceinline__ bool pair_fp64(double dX, double dY, double nxA, double nyA, double aP,
                                           double nxB, double nyB, double aQ, double sig,
                                           double gamma, double Lx, double Ly, bool virial,
-                                          double two_n, PairF64& o, double inv_LL = 0.0,
-                                          double inv_two_n = 0.0) {
-  dX += Lx * (double)((dX < -0.5 * Lx) - (dX > 0.5 * Lx));
-  dY += Ly * (double)((dY < -0.5 * Ly) - (dY > 0.5 * Ly));
+                                          double two_n, PairF64& o, double inv_aP, double inv_aQ,
+                                          double inv_LL = 0.0, double inv_two_n = 0.0) {
+  dX = nearest_image(dX, Lx);
+  dY = nearest_image(dY, Ly);
   dX += gamma * dY;
 
   double a = aP * aP;
@@ -80,20 +131,23 @@ __device__ __forceinline__ bool pair_fp64(double dX, double dY, double nxA, doub
   double e = -nxB * dX - nyB * dY;
   double delta = a * c - b * b;
   Recip64 iv{};
-  if (FAST) iv = recip64(a, c, delta, sig);
+  if (FAST) {
+    iv = recip64(a, c, delta, sig);
+  } else {
+    iv.a = inv_aP;
+    iv.c = inv_aQ;
+  }
 
-  double t = fmin(fmax((FAST && delta > 0) ? (b * d - a * e) * iv.delta
-                                            : (b * d - a * e) / delta,
-                       -1.), 1.);
+  double t = clamp_one((FAST && delta > 0) ? (b * d - a * e) * iv.delta : (b * d - a * e) / delta);
   double s = qdiv<FAST>(-(b * t + d), a, iv.a);
-  double sarg = fabs(s);
-  s = fmin(fmax(s, -1.), 1.);
-  if (sarg > 1) t = fmin(fmax(qdiv<FAST>(-(b * s + e), c, iv.c), -1.), 1.);
+  const bool end = beyond_one(s);
+  s = clamp_one(s);
+  if (end) t = clamp_one(qdiv<FAST>(-(b * s + e), c, iv.c));
 
   double dDx = dX + s * nxA - t * nxB;
   double dDy = dY + s * nyA - t * nyB;
   double dsq = dDx * dDx + dDy * dDy;
-  if (!(dsq < sig * sig)) return false;
+  if (!less_square(dsq, sig * sig)) return false;
   double Fx, Fy, dij, dvij;
   if (FAST) {
     const double rs = rsqrt(dsq);
@@ -129,7 +183,7 @@ __device__ __forceinline__ bool pair_fp64(double dX, double dY, double nxA, doub
       o.pyx = gx * (CyA - CyB);
     }
   } else if (SE) {
-    double LL = Lx * Ly;
+    const double LL = Lx * Ly, rLL = shared_rcp(LL);
     double CxA = s * nxA - 0.5 * dDx;
     double CyA = s * nyA - 0.5 * dDy;
     double CxB = t * nxB + 0.5 * dDx;
@@ -138,16 +192,16 @@ __device__ __forceinline__ bool pair_fp64(double dX, double dY, double nxA, doub
       // the reference's accumulation, slips included: CyB is built from nxB,
       // one Pxy term lands in Pxx, and Pxy misses its B arm.
       double CyB = t * nxB + 0.5 * dDy;
-      o.pxx = Fx * CxA / LL - Fx * CxB / LL - Fy * CxB / LL;
-      o.pyy = Fy * CyA / LL - Fy * CyB / LL;
-      o.pxy = Fy * CxA / LL;
-      o.pyx = Fx * CyA / LL - Fx * CyB / LL;
+      o.pxx = div_by(Fx * CxA, LL, rLL) - div_by(Fx * CxB, LL, rLL) - div_by(Fy * CxB, LL, rLL);
+      o.pyy = div_by(Fy * CyA, LL, rLL) - div_by(Fy * CyB, LL, rLL);
+      o.pxy = div_by(Fy * CxA, LL, rLL);
+      o.pyx = div_by(Fx * CyA, LL, rLL) - div_by(Fx * CyB, LL, rLL);
     } else {
       double CyB = t * nyB + 0.5 * dDy;
-      o.pxx = Fx * CxA / LL - Fx * CxB / LL;
-      o.pyy = Fy * CyA / LL - Fy * CyB / LL;
-      o.pxy = Fy * CxA / LL - Fy * CxB / LL;
-      o.pyx = Fx * CyA / LL - Fx * CyB / LL;
+      o.pxx = div_by(Fx * CxA, LL, rLL) - div_by(Fx * CxB, LL, rLL);
+      o.pyy = div_by(Fy * CyA, LL, rLL) - div_by(Fy * CyB, LL, rLL);
+      o.pxy = div_by(Fy * CxA, LL, rLL) - div_by(Fy * CxB, LL, rLL);
+      o.pyx = div_by(Fx * CyA, LL, rLL) - div_by(Fx * CyB, LL, rLL);
     }
   }
   return true;
@@ -277,62 +331,62 @@ __device__ __forceinline__ Contacts2<double> contacts2_fp64(double a, double b, 
                                                             double e, double delta, double dX,
                                                             double dY, double nxA, double nyA,
                                                             double nxB, double nyB,
-                                                            const Recip64& iv = Recip64{}) {
+                                                            const Recip64& iv) {
   double s1, t1, s2, t2, s3, t3;
   if (delta <= 0) {
-    s1 = fmin(fmax(qdiv<FAST>(-(b + d), a, iv.a), -1.0), 1.0);
-    s2 = fmin(fmax(qdiv<FAST>(-(d - b), a, iv.a), -1.0), 1.0);
-    if (fabs(s1) == 1)
-      t1 = fmin(fmax(qdiv<FAST>(-(b * s1 + e), c, iv.c), -1.0), 1.0);
+    s1 = clamp_one(qdiv<FAST>(-(b + d), a, iv.a));
+    s2 = clamp_one(qdiv<FAST>(-(d - b), a, iv.a));
+    if (abs_bits(s1) == kBitsOne)
+      t1 = clamp_one(qdiv<FAST>(-(b * s1 + e), c, iv.c));
     else if (b < 0)
-      t1 = fmin(fmax(qdiv<FAST>(-(b + e), c, iv.c), -1.0), 1.0);
+      t1 = clamp_one(qdiv<FAST>(-(b + e), c, iv.c));
     else
-      t1 = fmin(fmax(qdiv<FAST>(-(e - b), c, iv.c), -1.0), 1.0);
-    if (fabs(s2) == 1)
-      t2 = fmin(fmax(qdiv<FAST>(-(b * s2 + e), c, iv.c), -1.0), 1.0);
+      t1 = clamp_one(qdiv<FAST>(-(e - b), c, iv.c));
+    if (abs_bits(s2) == kBitsOne)
+      t2 = clamp_one(qdiv<FAST>(-(b * s2 + e), c, iv.c));
     else if (b < 0)
-      t2 = fmin(fmax(qdiv<FAST>(-(e - b), c, iv.c), -1.0), 1.0);
+      t2 = clamp_one(qdiv<FAST>(-(e - b), c, iv.c));
     else
-      t2 = fmin(fmax(qdiv<FAST>(-(b + e), c, iv.c), -1.0), 1.0);
+      t2 = clamp_one(qdiv<FAST>(-(b + e), c, iv.c));
     s3 = s2;
     t3 = t2;
   } else {
-    t1 = fmin(fmax(qdiv<FAST>(b * d - a * e, delta, iv.delta), -1.), 1.);
+    t1 = clamp_one(FAST ? (b * d - a * e) * iv.delta : (b * d - a * e) / delta);
     s1 = qdiv<FAST>(-(b * t1 + d), a, iv.a);
-    double sarg = fabs(s1);
-    s1 = fmin(fmax(s1, -1.), 1.);
-    if (sarg >= 1) {
-      t1 = fmin(fmax(qdiv<FAST>(-(b * s1 + e), c, iv.c), -1.), 1.);
+    bool end = reaches_one(s1);
+    s1 = clamp_one(s1);
+    if (end) {
+      t1 = clamp_one(qdiv<FAST>(-(b * s1 + e), c, iv.c));
       s2 = -s1;
       t2 = qdiv<FAST>(-(b * s2 + e), c, iv.c);
-      double targ = fabs(t2);
-      t2 = fmin(fmax(t2, -1.), 1.);
-      if (targ > 1) {
-        s2 = fmin(fmax(qdiv<FAST>(-(b * t2 + d), a, iv.a), -1.), 1.);
+      const bool out = beyond_one(t2);
+      t2 = clamp_one(t2);
+      if (out) {
+        s2 = clamp_one(qdiv<FAST>(-(b * t2 + d), a, iv.a));
         s3 = s2;
         t3 = t2;
       } else {
         t3 = b < 0 ? -s1 : s1;
         s3 = qdiv<FAST>(-(b * t3 + d), a, iv.a);
-        sarg = fabs(s3);
-        s3 = fmin(fmax(s3, -1.0), 1.0);
-        if (sarg >= 1) t3 = fmin(fmax(qdiv<FAST>(-(b * s3 + e), c, iv.c), -1.0), 1.0);
+        end = reaches_one(s3);
+        s3 = clamp_one(s3);
+        if (end) t3 = clamp_one(qdiv<FAST>(-(b * s3 + e), c, iv.c));
       }
     } else {
       t2 = -t1;
       s2 = qdiv<FAST>(-(b * t2 + d), a, iv.a);
-      sarg = fabs(s2);
-      s2 = fmin(fmax(s2, -1.), 1.);
-      if (sarg > 1) {
-        t2 = fmin(fmax(qdiv<FAST>(-(b * s2 + e), c, iv.c), -1.), 1.);
+      end = beyond_one(s2);
+      s2 = clamp_one(s2);
+      if (end) {
+        t2 = clamp_one(qdiv<FAST>(-(b * s2 + e), c, iv.c));
         s3 = s2;
         t3 = t2;
       } else {
         s3 = b < 0 ? -t1 : t1;
         t3 = qdiv<FAST>(-(b * s3 + e), c, iv.c);
-        double targ = fabs(t3);
-        t3 = fmin(fmax(t3, -1.0), 1.0);
-        if (targ >= 1) s3 = fmin(fmax(qdiv<FAST>(-(b * t3 + d), a, iv.a), -1.0), 1.0);
+        const bool out = reaches_one(t3);
+        t3 = clamp_one(t3);
+        if (out) s3 = clamp_one(qdiv<FAST>(-(b * t3 + d), a, iv.a));
       }
     }
   }
@@ -364,7 +418,7 @@ __device__ __forceinline__ bool contact_fp64(double dX, double dY, double s, dou
   double dDx = dX + s * nxA - t * nxB;
   double dDy = dY + s * nyA - t * nyB;
   double dsq = dDx * dDx + dDy * dDy;
-  if (!(dsq < sig * sig)) return false;
+  if (!less_square(dsq, sig * sig)) return false;
   double dij, dvij, Fx, Fy;
   if (FAST) {
     const double rs = rsqrt(dsq);
@@ -395,10 +449,10 @@ __device__ __forceinline__ bool contact_fp64(double dX, double dY, double s, dou
     double CxA = s * nxA - 0.5 * dDx, CyA = s * nyA - 0.5 * dDy;
     double CxB = t * nxB + 0.5 * dDx, CyB = t * nyB + 0.5 * dDy;
     o.e += dvij * sig * (1.0 - dij / sig) / two_n;
-    o.pxx += Fx * CxA / LL - Fx * CxB / LL;
-    o.pyy += Fy * CyA / LL - Fy * CyB / LL;
-    o.pxy += Fy * CxA / LL - Fy * CxB / LL;
-    o.pyx += Fx * CyA / LL - Fx * CyB / LL;
+    o.pxx += div_by(Fx * CxA, LL, inv_LL) - div_by(Fx * CxB, LL, inv_LL);
+    o.pyy += div_by(Fy * CyA, LL, inv_LL) - div_by(Fy * CyB, LL, inv_LL);
+    o.pxy += div_by(Fy * CxA, LL, inv_LL) - div_by(Fy * CxB, LL, inv_LL);
+    o.pyx += div_by(Fx * CyA, LL, inv_LL) - div_by(Fx * CyB, LL, inv_LL);
   }
   return true;
 }
@@ -409,10 +463,10 @@ template <bool SE, bool FAST = false>
 __device__ __forceinline__ bool pair2_fp64(double dX, double dY, double nxA, double nyA,
                                            double aP, double nxB, double nyB, double aQ,
                                            double sig, double gamma, double Lx, double Ly,
-                                           double two_n, PairF64& o, double inv_LL = 0.0,
-                                           double inv_two_n = 0.0) {
-  dX += Lx * (double)((dX < -0.5 * Lx) - (dX > 0.5 * Lx));
-  dY += Ly * (double)((dY < -0.5 * Ly) - (dY > 0.5 * Ly));
+                                           double two_n, PairF64& o, double inv_aP, double inv_aQ,
+                                           double inv_LL = 0.0, double inv_two_n = 0.0) {
+  dX = nearest_image(dX, Lx);
+  dY = nearest_image(dY, Ly);
   dX += gamma * dY;
   double a = aP * aP;
   double b = -(nxA * nxB + nyA * nyB);
@@ -421,7 +475,13 @@ __device__ __forceinline__ bool pair2_fp64(double dX, double dY, double nxA, dou
   double e = -nxB * dX - nyB * dY;
   double delta = a * c - b * b;
   Recip64 iv{};
-  if (FAST) iv = recip64(a, c, delta, sig);
+  if (FAST) {
+    iv = recip64(a, c, delta, sig);
+  } else {
+    iv.a = inv_aP;
+    iv.c = inv_aQ;
+    if (SE) inv_LL = shared_rcp(Lx * Ly);
+  }
   Contacts2<double> k =
       contacts2_fp64<FAST>(a, b, c, d, e, delta, dX, dY, nxA, nyA, nxB, nyB, iv);
   o.fx = o.fy = o.tp = o.tq = 0.0;

@@ -370,12 +370,15 @@ __device__ __forceinline__ void pass64_slot(const Dev& d, const StepScalars* __r
       const double2 pP = ip ? pi : pj, pQ = ip ? pj : pi;
       const double2 nP = ip ? ni : nj, nQ = ip ? nj : ni;
       const double2 rP = ip ? rai : raj, rQ = ip ? raj : rai;
+      const double ivi = d.iaa[i], ivj = d.iaa[j];
       PairF64 o;
       const bool hit =
           two_point ? pair2_fp64<SE, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x,
-                                           nQ.y, rQ.y, rP.x + rQ.x, gamma, Lx, Ly, two_n, o)
+                                           nQ.y, rQ.y, rP.x + rQ.x, gamma, Lx, Ly, two_n, o,
+                                           ip ? ivi : ivj, ip ? ivj : ivi)
                     : pair_fp64<SE, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x, nQ.y,
-                                          rQ.y, rP.x + rQ.x, gamma, Lx, Ly, virial, two_n, o);
+                                          rQ.y, rP.x + rQ.x, gamma, Lx, Ly, virial, two_n, o,
+                                          ip ? ivi : ivj, ip ? ivj : ivi);
       if (hit) {
         if (ip) {
           fx += o.fx;
@@ -426,11 +429,12 @@ __global__ void __launch_bounds__(128) k_pass64(Dev d, const StepScalars* __rest
 // window's results.  With SE the owners then add their pairs' stress and energy, 128
 // jobs at a time, in list order (2: the energy alone).  RES false: no results wanted.
 //
-// The FP64 pipe (two lanes a cycle and SM) bounds it: about 150 operations a contact.
-// With one thread per particle, each pair evaluated from both sides and the screen's
-// displacement in FP64, a shear pass took 2.66 ms at 2^20 particles and 65 us at 1024
-// (8 blocks, the rest of the GPU idle); here 0.50 + 0.25 ms (k_pairs64 + k_step64) and
-// 10 + 15 us.
+// The FP64 pipe (two lanes a cycle and SM) bounds it: about 115 operations a contact
+// (sc_pair.cuh keeps comparisons, clamps and repeated divisors off the pipe; with them on
+// it, 0.50 ms at 2^20 particles instead of 0.40).  With one thread per particle, each pair
+// evaluated from both sides and the screen's displacement in FP64, a shear pass took 2.66
+// ms at 2^20 particles and 65 us at 1024 (8 blocks, the rest of the GPU idle); here 0.40 +
+// 0.25 ms (k_pairs64 + k_step64) and 10 + 15 us.
 constexpr int kPairBlock = 128;
 
 template <int SE, bool RES, bool TWO, bool FAST, int TPS>
@@ -512,13 +516,14 @@ __global__ void __launch_bounds__(kPairBlock) k_pairs64(Dev d, const StepScalars
       const double Lx = pred ? ts.Lx_c : ts.Lx_p, Ly = pred ? ts.Ly_c : ts.Ly_p;
       const double two_n = SE ? 2.0 * d.geom[s].n : 0.0;
       const double2 pP = XY[io], pQ = XY[j], nP = NXY[io], nQ = NXY[j], rP = d.ra[io], rQ = d.ra[j];
+      const double iP = FAST ? 0.0 : d.iaa[io], iQ = FAST ? 0.0 : d.iaa[j];
       PairF64 o;
       const bool hit =
           TWO ? pair2_fp64<SE != 0, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x, nQ.y,
-                                          rQ.y, rP.x + rQ.x, gamma, Lx, Ly, two_n, o)
+                                          rQ.y, rP.x + rQ.x, gamma, Lx, Ly, two_n, o, iP, iQ)
               : pair_fp64<SE != 0, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x, nQ.y,
                                          rQ.y, rP.x + rQ.x, gamma, Lx, Ly,
-                                         d.stress_mode == STRESS_VIRIAL, two_n, o);
+                                         d.stress_mode == STRESS_VIRIAL, two_n, o, iP, iQ);
       if (RES && fits) {
         d.pr_who[base + p] = hit ? j : -1;
         if (hit) {
@@ -554,15 +559,15 @@ __global__ void __launch_bounds__(kPairBlock) k_pairs64(Dev d, const StepScalars
 // operations, so the same bits); out of line, since it hardly ever runs.
 template <bool TWO, bool FAST>
 __device__ __noinline__ bool pair_again64(const double2* XY, const double2* NXY,
-                                          const double2* ra, int iP, int iQ, double gamma,
-                                          double Lx, double Ly, double4_16a* r) {
+                                          const double2* ra, const double* iaa, int iP, int iQ,
+                                          double gamma, double Lx, double Ly, double4_16a* r) {
   const double2 pP = XY[iP], pQ = XY[iQ], nP = NXY[iP], nQ = NXY[iQ], rP = ra[iP], rQ = ra[iQ];
   PairF64 o;
   const bool hit =
       TWO ? pair2_fp64<false, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x, nQ.y, rQ.y,
-                                    rP.x + rQ.x, gamma, Lx, Ly, 0.0, o)
+                                    rP.x + rQ.x, gamma, Lx, Ly, 0.0, o, iaa[iP], iaa[iQ])
           : pair_fp64<false, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x, nQ.y, rQ.y,
-                                   rP.x + rQ.x, gamma, Lx, Ly, false, 0.0, o);
+                                   rP.x + rQ.x, gamma, Lx, Ly, false, 0.0, o, iaa[iP], iaa[iQ]);
   if (hit) {
     r->x = o.fx;
     r->y = o.fy;
@@ -601,7 +606,7 @@ __global__ void __launch_bounds__(128) k_step64(Dev d, const StepScalars* __rest
     bool hit = false;
     if (inf == kPairsOver) {
       const double Lx = kCorr ? ts.Lx_c : ts.Lx_p, Ly = kCorr ? ts.Ly_c : ts.Ly_p;
-      hit = pair_again64<TWO, FAST>(kCorr ? d.xy_t : d.xy, kCorr ? d.nxy_t : d.nxy, d.ra,
+      hit = pair_again64<TWO, FAST>(kCorr ? d.xy_t : d.xy, kCorr ? d.nxy_t : d.nxy, d.ra, d.iaa,
                                     ip ? i : j, ip ? j : i, gamma, Lx, Ly, &r);
     } else if (ip) {
       const size_t q = own + rank++;
@@ -799,10 +804,10 @@ __global__ void __launch_bounds__(kSeBlock) k_mx_se64(Dev d, const StepScalars* 
         const bool hit =
             TWO ? pair2_fp64<true, true>(dX, dY, o_nx[o], o_ny[o], o_A[o], nj.x, nj.y, raj.y,
                                          o_R[o] + raj.x, o_gam[o], o_Lx[o], o_Ly[o], o_2n[o], r,
-                                         o_iLL[o], o_i2n[o])
+                                         0.0, 0.0, o_iLL[o], o_i2n[o])
                 : pair_fp64<true, true>(dX, dY, o_nx[o], o_ny[o], o_A[o], nj.x, nj.y, raj.y,
                                         o_R[o] + raj.x, o_gam[o], o_Lx[o], o_Ly[o], virial,
-                                        o_2n[o], r, o_iLL[o], o_i2n[o]);
+                                        o_2n[o], r, 0.0, 0.0, o_iLL[o], o_i2n[o]);
         res[0][t] = hit ? r.e : 0.0;
         res[1][t] = hit ? r.pxx : 0.0;
         res[2][t] = hit ? r.pyy : 0.0;

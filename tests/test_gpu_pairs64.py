@@ -77,3 +77,23 @@ def test_list_equals_the_oracles(oracle_built, n, phi, aor, gamma, pad):
     ob.find_neighbors()
     ref = ob.pairs()
     assert np.array_equal(a.pairs(), ref[np.lexsort((ref[:, 1], ref[:, 0]))])
+
+
+@pytest.mark.parametrize("shape", [0.0, 1e-170, 1e-80, 0.02])
+def test_shapes_at_the_end_of_the_range(oracle_built, shape):
+    """Half shafts of zero (discs) and so short that the reciprocal of their square leaves
+    the range of the shared quotients, against the oracle: 1e-12 of the RMS force, the
+    bound of the FP64 form's forces."""
+    from spherocyls_gb300 import SpherocylBox, generate_packing
+
+    L, x, y, p, R, A = generate_packing(600, 0.85, 0.05, seed=9)
+    A = np.full_like(A, shape)
+    b = SpherocylBox(L, x, y, p, A, R, 0.1)
+    b.calc_forces()
+    ob = oracle_built.OracleBox(L, x, y, p, A, R, 0.1)
+    ob.find_neighbors()
+    ob.calc_forces()
+    f = ob.forces()
+    rms = np.sqrt(np.mean([f[0] ** 2, f[1] ** 2]))
+    for u, v in zip(b.forces(), f):
+        assert np.abs(u - v).max() <= 1e-12 * rms
