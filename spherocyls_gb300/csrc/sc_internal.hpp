@@ -291,7 +291,6 @@ constexpr unsigned kSlotMask = (1u << kSlotBits) - 1u;
 constexpr unsigned kOwner64 = 0x80000000u;
 constexpr unsigned kSlot64Mask = (1u << 30) - 1u;
 constexpr int kPairCap = 5;  // pair results kept per slot of a window (2 to 3 are used)
-constexpr int kSmallPairs = 1 << 16;  // up to this many slots, windows of 32 (see pair_window)
 constexpr unsigned kPairsOver = 0xffffffffu;  // pr_info of a window with more than that
 // tile force pass: entry capacity per particle of a tile (compute and read lists
 // each), particles and pair results held in shared memory, threads per tile; a

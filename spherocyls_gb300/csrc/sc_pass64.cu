@@ -163,10 +163,17 @@ __device__ __forceinline__ void flag_moved(const Dev& d, int s, int id, double2 
 
 // The Heun step of slot i after its forces (fx, fy, tq) at the pass's positions are
 // known: predictor, corrector with the rebuild test, or (PASS_FORCE) the forces alone.
+// rot: rot64<MODE> of the slot, which needs no force.
+template <int MODE>
+__device__ __forceinline__ double rot64(const Dev& d, int i) {
+  if (MODE == PASS_PRED_STRAIN) return iso_rot64(d.irc[i].y, d.ph[i]);
+  if (MODE == PASS_CORR_STRAIN) return iso_rot64(d.irc[i].y, d.ph_t[i]);
+  return 0.0;
+}
 template <int MODE>
 __device__ __forceinline__ void step64_slot(const Dev& d, const StepScalars& ts, const SysGeom& g,
                                             int s, int i, double2 rai, int idi, double gamma,
-                                            double fx, double fy, double tq) {
+                                            double rot, double fx, double fy, double tq) {
   const double2 irc = d.irc[i];  // (I, RC)
   const double dt = ts.step;
   if (MODE == PASS_FORCE) {
@@ -181,7 +188,7 @@ __device__ __forceinline__ void step64_slot(const Dev& d, const StepScalars& ts,
     double phi = d.ph[i];
     double v0x = fx - gamma * fy;
     double v0y = fy;
-    double v0p = tq / irc.x - ts.rate * iso_rot64(irc.y, phi);
+    double v0p = tq / irc.x - ts.rate * rot;
     d.v0x[i] = v0x;
     d.v0y[i] = v0y;
     d.v0p[i] = v0p;
@@ -197,10 +204,9 @@ __device__ __forceinline__ void step64_slot(const Dev& d, const StepScalars& ts,
     d.rec_t[i] = screen_record(pt, nt);
   } else if (MODE == PASS_CORR_STRAIN) {
     // strain_step corrector, strain_dynamics.cpp:203-219
-    double pht = d.ph_t[i];
     double v1x = fx - gamma * fy;
     double v1y = fy;
-    double v1p = tq / irc.x - ts.rate * iso_rot64(irc.y, pht);
+    double v1p = tq / irc.x - ts.rate * rot;
     double ddx = 0.5 * dt * (d.v0x[i] + v1x);
     double ddy = 0.5 * dt * (d.v0y[i] + v1y);
     double ddp = 0.5 * dt * (d.v0p[i] + v1p);
@@ -407,7 +413,7 @@ __device__ __forceinline__ void pass64_slot(const Dev& d, const StepScalars* __r
     d.se_part[(size_t)4 * d.ntot + i] = se4;
   }
 
-  step64_slot<MODE>(d, ts, g, s, i, rai, idi, gamma, fx, fy, tq);
+  step64_slot<MODE>(d, ts, g, s, i, rai, idi, gamma, rot64<MODE>(d, i), fx, fy, tq);
 }
 
 template <int MODE, bool SE, bool TWO, bool FAST = false>
@@ -434,7 +440,7 @@ __global__ void __launch_bounds__(128) k_pass64(Dev d, const StepScalars* __rest
 // it, 0.50 ms at 2^20 particles instead of 0.40).  With one thread per particle, each pair
 // evaluated from both sides and the screen's displacement in FP64, a shear pass took 2.66
 // ms at 2^20 particles and 65 us at 1024 (8 blocks, the rest of the GPU idle); here 0.40 +
-// 0.25 ms (k_pairs64 + k_step64) and 10 + 15 us.
+// 0.25 ms (k_pairs64 + k_step64) and 7 + 8 us.
 constexpr int kPairBlock = 128;
 
 template <int SE, bool RES, bool TWO, bool FAST, int TPS>
@@ -577,63 +583,131 @@ __device__ __noinline__ bool pair_again64(const double2* XY, const double2* NXY,
   return hit;
 }
 
-// k_step64, one thread per slot: the slot's contributions from the pair results, in list
-// order (its own pairs follow each other in its window; a pair it does not own is looked
-// up among its partner's two or three), then the Heun epilogue.
+// The contribution of entry e of slot i's list (info: its pr_info, rank: the owned entries
+// before e that may touch) to its force and torque; zero where there is no contact.
 template <int MODE, bool TWO, bool FAST>
-__global__ void __launch_bounds__(128) k_step64(Dev d, const StepScalars* __restrict__ tab,
-                                               int row) {
+__device__ __forceinline__ void pair_result64(const Dev& d, const StepScalars& ts, double gamma,
+                                              int i, unsigned info, unsigned e, int rank,
+                                              double& x, double& y, double& q) {
   constexpr bool kCorr = MODE == PASS_CORR_STRAIN || MODE == PASS_CORR_RESIZE;
-  if (kCorr) mark_pending_rebuilds(d, tab, row);
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= d.ntot) return;
-  const int s = d.psys[i];
-  if (d.skip && d.skip[s]) return;  // a converged minimiser system
-  const StepScalars& ts = tab[row * d.nsys + s];
-  const double gamma = kCorr ? ts.gamma_c : ts.gamma_p;
-  const unsigned info = d.pr_info[i];
   const int win = d.pr_win;
-  const size_t own = (size_t)(i / win) * win * kPairCap + (info & 0xffffu);
-  double fx = 0.0, fy = 0.0, tq = 0.0;
-  int rank = 0;
-  for (unsigned long long m = d.pr_mask[i]; m; m &= m - 1ull) {
-    const int k = __ffsll((long long)m) - 1;
-    const unsigned e = (unsigned)d.nbr[(size_t)k * d.ntot + i];
-    const int j = (int)(e & kSlot64Mask);
-    const bool ip = (e & kOwner64) != 0u;
-    const unsigned inf = ip ? info : d.pr_info[j];
-    double4_16a r;
-    bool hit = false;
-    if (inf == kPairsOver) {
-      const double Lx = kCorr ? ts.Lx_c : ts.Lx_p, Ly = kCorr ? ts.Ly_c : ts.Ly_p;
-      hit = pair_again64<TWO, FAST>(kCorr ? d.xy_t : d.xy, kCorr ? d.nxy_t : d.nxy, d.ra, d.iaa,
-                                    ip ? i : j, ip ? j : i, gamma, Lx, Ly, &r);
-    } else if (ip) {
-      const size_t q = own + rank++;
-      hit = d.pr_who[q] >= 0;
-      if (hit) r = d.pr_res[q];
+  const int j = (int)(e & kSlot64Mask);
+  const bool ip = (e & kOwner64) != 0u;
+  const int o = ip ? i : j;  // the owner
+  const unsigned inf = ip ? info : d.pr_info[j];
+  double4_16a r;
+  bool hit = false;
+  if (inf == kPairsOver) {
+    const double Lx = kCorr ? ts.Lx_c : ts.Lx_p, Ly = kCorr ? ts.Ly_c : ts.Ly_p;
+    hit = pair_again64<TWO, FAST>(kCorr ? d.xy_t : d.xy, kCorr ? d.nxy_t : d.nxy, d.ra, d.iaa, o,
+                                  ip ? j : i, gamma, Lx, Ly, &r);
+  } else {
+    const size_t q0 = (size_t)(o / win) * win * kPairCap + (inf & 0xffffu);
+    if (ip) {
+      hit = d.pr_who[q0 + rank] >= 0;
+      if (hit) r = d.pr_res[q0 + rank];
     } else {
-      const size_t q0 = (size_t)(j / win) * win * kPairCap + (inf & 0xffffu);
       const int n = (int)(inf >> 16);
-      for (int q = 0; q < n; q++)
-        if (d.pr_who[q0 + q] == i) {
+      for (int k = 0; k < n; k++)
+        if (d.pr_who[q0 + k] == i) {
           hit = true;
-          r = d.pr_res[q0 + q];
+          r = d.pr_res[q0 + k];
           break;
         }
     }
-    if (!hit) continue;
-    if (ip) {
-      fx += r.x;
-      fy += r.y;
-      tq += r.z;
-    } else {
-      fx -= r.x;
-      fy -= r.y;
-      tq += r.w;
-    }
   }
-  step64_slot<MODE>(d, ts, d.geom[s], s, i, d.ra[i], d.id[i], gamma, fx, fy, tq);
+  x = hit ? (ip ? r.x : -r.x) : 0.0;
+  y = hit ? (ip ? r.y : -r.y) : 0.0;
+  q = hit ? (ip ? r.z : r.w) : 0.0;
+}
+
+// k_step64: a slot's contributions from the pair results, in list order (its own pairs
+// follow each other in its window; a pair it does not own is looked up among its partner's
+// two or three), then the Heun epilogue.  GL = 1: a thread does all of it for its slot.
+// GL = 8, for small systems, where the gather's chain of dependent loads (four or five
+// contacts of three loads each) is what the kernel waits for: eight threads of a slot
+// fetch a contribution each, a fourth warp meanwhile takes the cosine of the rotation,
+// and one thread a slot sums and steps.
+constexpr int kStepBlock = 128;
+
+template <int MODE, bool TWO, bool FAST, int GL>
+__global__ void __launch_bounds__(kStepBlock) k_step64(Dev d, const StepScalars* __restrict__ tab,
+                                                      int row) {
+  constexpr bool kCorr = MODE == PASS_CORR_STRAIN || MODE == PASS_CORR_RESIZE;
+  constexpr int S = kStepBlock / GL;
+  if (kCorr) mark_pending_rebuilds(d, tab, row);
+  const int t = threadIdx.x, l = t / GL, sub = t % GL;
+  const int i = blockIdx.x * S + l;
+  int s = 0;
+  bool live = i < d.ntot;
+  if (live) {
+    s = d.psys[i];
+    live = !(d.skip && d.skip[s]);  // not a converged minimiser system
+  }
+  if (GL == 1 && !live) return;
+  const StepScalars& ts = tab[row * d.nsys + s];
+  const double gamma = kCorr ? ts.gamma_c : ts.gamma_p;
+  double fx = 0.0, fy = 0.0, tq = 0.0;
+  if constexpr (GL == 1) {
+    const unsigned info = d.pr_info[i];
+    int rank = 0;
+    for (unsigned long long m = d.pr_mask[i]; m; m &= m - 1ull) {
+      const unsigned e = (unsigned)d.nbr[(size_t)(__ffsll((long long)m) - 1) * d.ntot + i];
+      double x, y, q;
+      pair_result64<MODE, TWO, FAST>(d, ts, gamma, i, info, e, rank, x, y, q);
+      rank += (e & kOwner64) != 0u;
+      fx += x;
+      fy += y;
+      tq += q;
+    }
+    step64_slot<MODE>(d, ts, d.geom[s], s, i, d.ra[i], d.id[i], gamma, rot64<MODE>(d, i), fx, fy,
+                      tq);
+  } else {
+    __shared__ double part[3][kStepBlock], rot[S];
+    __shared__ int left[S];
+    // the last S threads: the rotation of the block's slots
+    const int ir = blockIdx.x * S + t - (kStepBlock - S);
+    if (t >= kStepBlock - S && ir < d.ntot) rot[t - (kStepBlock - S)] = rot64<MODE>(d, ir);
+    unsigned long long m = live ? d.pr_mask[i] : 0ull;
+    const unsigned info = live ? d.pr_info[i] : 0u;
+    int rank = 0, more;
+    do {
+      // this thread's entry: the sub-th of the mask's remaining ones
+      unsigned long long b = m;
+      for (int k = 0; k < sub; k++) b &= b - 1ull;
+      unsigned e = 0u;
+      if (b) e = (unsigned)d.nbr[(size_t)(__ffsll((long long)b) - 1) * d.ntot + i];
+      const unsigned group = (__ballot_sync(0xffffffffu, (e & kOwner64) != 0u) >>
+                              ((t & 31) / GL * GL)) & ((1u << GL) - 1u);
+      double x = 0.0, y = 0.0, q = 0.0;
+      if (b)
+        pair_result64<MODE, TWO, FAST>(d, ts, gamma, i, info, e,
+                                       rank + __popc(group & ((1u << sub) - 1u)), x, y, q);
+      rank += __popc(group);
+      part[0][t] = x;
+      part[1][t] = y;
+      part[2][t] = q;
+      if (sub == 0) left[l] = __popcll(m);
+      for (int k = 0; k < GL; k++) m &= m - 1ull;
+      more = __syncthreads_or(m != 0ull);
+      if (t < S) {
+        const int n = min(left[t], GL);
+        for (int k = 0; k < n; k++) {
+          fx += part[0][t * GL + k];
+          fy += part[1][t * GL + k];
+          tq += part[2][t * GL + k];
+        }
+      }
+      if (more) __syncthreads();
+    } while (more);
+    const int io = blockIdx.x * S + t;
+    if (t >= S || io >= d.ntot) return;
+    const int so = d.psys[io];
+    if (d.skip && d.skip[so]) return;
+    const StepScalars& to = tab[row * d.nsys + so];
+    step64_slot<MODE>(d, to, d.geom[so], so, io, d.ra[io], d.id[io],
+                      kCorr ? to.gamma_c : to.gamma_p, rot[t], fx, fy, tq);
+  }
 }
 
 // ---- stress and energy of the mixed form, in FP64 ----
@@ -836,26 +910,41 @@ void launch_whole(const Dev& d, const StepScalars* tab, int row, cudaStream_t st
     k_pass64<MODE, SE, false, FAST><<<grid, block, 0, st>>>(d, tab, row);
 }
 
+template <int SE, bool RES, bool FAST, int TPS>
+void launch_pairs_of(const Dev& d, const StepScalars* tab, int row, int pred, cudaStream_t st) {
+  const int grid = (d.ntot + d.pr_win - 1) / d.pr_win;
+  if (d.contact_model == 1)
+    k_pairs64<SE, RES, true, FAST, TPS><<<grid, kPairBlock, 0, st>>>(d, tab, row, pred);
+  else
+    k_pairs64<SE, RES, false, FAST, TPS><<<grid, kPairBlock, 0, st>>>(d, tab, row, pred);
+}
+
 template <int SE, bool RES, bool FAST>
 void launch_pairs(const Dev& d, const StepScalars* tab, int row, bool pred, cudaStream_t st) {
-  const int grid = (d.ntot + d.pr_win - 1) / d.pr_win, p = pred ? 1 : 0;
-  const bool two = d.contact_model == 1;
-  if (d.pr_win == kPairBlock) {
-    two ? k_pairs64<SE, RES, true, FAST, 1><<<grid, kPairBlock, 0, st>>>(d, tab, row, p)
-        : k_pairs64<SE, RES, false, FAST, 1><<<grid, kPairBlock, 0, st>>>(d, tab, row, p);
-  } else {
-    two ? k_pairs64<SE, RES, true, FAST, 4><<<grid, kPairBlock, 0, st>>>(d, tab, row, p)
-        : k_pairs64<SE, RES, false, FAST, 4><<<grid, kPairBlock, 0, st>>>(d, tab, row, p);
+  switch (kPairBlock / d.pr_win) {
+    case 1: launch_pairs_of<SE, RES, FAST, 1>(d, tab, row, pred, st); break;
+    case 4: launch_pairs_of<SE, RES, FAST, 4>(d, tab, row, pred, st); break;
+    case 16: launch_pairs_of<SE, RES, FAST, 16>(d, tab, row, pred, st); break;
   }
+}
+
+template <int MODE, bool FAST, int GL>
+void launch_step_of(const Dev& d, const StepScalars* tab, int row, cudaStream_t st) {
+  const int grid = (d.ntot + kStepBlock / GL - 1) / (kStepBlock / GL);
+  if (d.contact_model == 1)
+    k_step64<MODE, true, FAST, GL><<<grid, kStepBlock, 0, st>>>(d, tab, row);
+  else
+    k_step64<MODE, false, FAST, GL><<<grid, kStepBlock, 0, st>>>(d, tab, row);
 }
 
 template <int MODE, bool FAST = false>
 void launch_step(const Dev& d, const StepScalars* tab, int row, cudaStream_t st) {
-  const int block = d.pr_win == kPairBlock ? 128 : 32, grid = (d.ntot + block - 1) / block;
-  if (d.contact_model == 1)
-    k_step64<MODE, true, FAST><<<grid, block, 0, st>>>(d, tab, row);
+  // eight threads a slot against one, a shear step in us: 43 and 56 at 1024 particles, 53
+  // and 66 at 8192, 77 and 77 at 16384, 109 and 97 at 32768
+  if (d.ntot <= 8192)
+    launch_step_of<MODE, FAST, 8>(d, tab, row, st);
   else
-    k_step64<MODE, false, FAST><<<grid, block, 0, st>>>(d, tab, row);
+    launch_step_of<MODE, FAST, 1>(d, tab, row, st);
 }
 
 // the pass of one mode through the pair buffers, or in one kernel without them
@@ -879,10 +968,13 @@ int launch_mode(const Dev& d, bool se, const StepScalars* tab, int row, cudaStre
 
 }  // namespace
 
-// Small systems take windows of 32 slots, four threads screening each, which puts the
-// pairs on four times the SMs.  A shear step in us, windows of 32 against 128: 63 and 93
-// at 4096 particles, 81 and 96 at 16384, 211 and 214 at 65536, 316 and 304 at 131072.
-int pair_window(int ntot) { return ntot <= kSmallPairs ? kPairBlock / 4 : kPairBlock; }
+// Slots per window of the pair results: small systems take small windows, several threads
+// screening a slot, which puts the pairs on more SMs.  A shear step in us with windows of
+// 8, 32 and 128 slots: 43, 46 and 72 at 1024 particles, 48, 49 and 76 at 4096, 88, 77 and 91
+// at 16384, 210, 145 and 149 at 65536, 365, 236 and 224 at 131072.
+int pair_window(int ntot) {
+  return ntot <= 4096 ? kPairBlock / 16 : ntot <= 65536 ? kPairBlock / 4 : kPairBlock;
+}
 
 int launch_pass_fp64(const Dev& d, int mode, bool se, const StepScalars* tab, int row,
                      cudaStream_t st, bool fast) {

@@ -29,12 +29,13 @@ def _boxes(n, phi, aor, contacts, gamma, seed=5, pad=0.1):
     return got
 
 
-# one window and less, the window edges (32, 128), grids under three cells a side, the
-# switch of the window size at 65536, windows with more contacts than they keep (3.5)
+# one window and less, the window edges (8, 32, 128), grids under three cells a side, the
+# switches of the kernels' shapes (4096, 8192, 65536), windows with more contacts than they keep (3.5)
 @pytest.mark.parametrize("n,phi,aor,contacts,gamma", [
     (2, 0.05, 1.0, 1, 0.0), (9, 0.8, 1.0, 1, 0.3), (32, 0.8, 1.0, 2, 0.0), (33, 0.7, 1.5, 1, 0.05),
-    (1000, 0.9, 0.3, 2, -0.2), (65536, 0.84, 1.0, 1, 0.1), (65537, 0.84, 1.0, 1, 0.1),
-    (2048, 3.5, 0.05, 1, 0.0), (2048, 3.5, 0.05, 2, 0.2), (70000, 3.5, 0.05, 1, 0.0)])
+    (1000, 0.9, 0.3, 2, -0.2), (4097, 0.84, 1.0, 2, 0.1),
+    (8192, 0.84, 1.0, 1, 0.1), (8201, 0.84, 1.0, 1, 0.1), (65536, 0.84, 1.0, 1, 0.1), (65537, 0.84, 1.0, 1, 0.1),
+    (2048, 3.5, 0.05, 1, 0.0), (2048, 3.5, 0.05, 2, 0.2), (9000, 3.5, 0.05, 2, 0.2), (70000, 3.5, 0.05, 1, 0.0)])
 def test_pair_buffers_give_the_same_bits(n, phi, aor, contacts, gamma):
     a, b = _boxes(n, phi, aor, contacts, gamma)
     assert np.array_equal(a.calc_se(), b.calc_se())
