@@ -264,7 +264,7 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
        h.dalloc(&d.v0p, N, "v0p") && h.dalloc(&d.fx, N, "fx") && h.dalloc(&d.fy, N, "fy") &&
        h.dalloc(&d.tau, N, "tau") && h.dalloc(&d.moved, N, "moved");
   ok = ok && h.dalloc(&d.rec, N, "rec") && h.dalloc(&d.rec_t, N, "rec_t") &&
-       h.dalloc(&d.rf, N, "rf");
+       h.dalloc(&d.rf, N, "rf") && h.dalloc(&d.rsf, N, "rsf");
   if (h.prec == sc::PREC_MIXED)
     ok = ok && h.dalloc(&d.mc, N, "mc") && h.dalloc(&d.mv, N, "mv") && h.dalloc(&d.mm, N, "mm") &&
          h.dalloc(&d.pa, N, "pa") && h.dalloc(&d.rcf, N, "rcf") &&
@@ -272,11 +272,11 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
          h.dalloc(&d.ord, N, "ord") && h.dalloc(&d.nbr_p, N * d.maxn, "nbr_p") &&
          h.dalloc(&d.nbr_pn, N, "nbr_pn");
   else
-    ok = ok && h.dalloc(&d.rsf, N, "rsf") && h.dalloc(&d.iaa, N, "iaa");
-  if (opt.precision == SC_PREC_MIXED) {
-    ok = ok && h.dalloc(&d.gbar, 2, "grid barrier") && h.dalloc(&h.d_persist, 1, "persist out");
-    if (ok) ok = h.cuda_ok(cudaMemsetAsync(d.gbar, 0, 2 * sizeof(unsigned), h.stream), "barrier");
-  }
+    ok = ok && h.dalloc(&d.iaa, N, "iaa") &&
+         h.dalloc(&d.s_mv, N, "s_mv") && h.dalloc(&d.s_nxy, N, "s_nxy");
+  ok = ok && h.dalloc(&d.gbar, sc::BAR_WORDS, "grid barriers") &&
+       h.cuda_ok(cudaMemsetAsync(d.gbar, 0, sc::BAR_WORDS * sizeof *d.gbar, h.stream), "barriers");
+  if (opt.precision == SC_PREC_MIXED) ok = ok && h.dalloc(&h.d_persist, 1, "persist out");
   if (d.pass_kind == 1)
     ok = ok && h.dalloc(&d.t_own, N * sc::kTileEPP, "tile owners") &&
          h.dalloc(&d.t_pe, N * sc::kTileEPP, "tile partners") &&
@@ -295,9 +295,7 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
   ok = ok && h.dalloc(&pcs, d.npchunks, "pchunk") && h.dalloc(&pcp, d.npchunks, "pchunk") &&
        h.dalloc(&pcn, d.npchunks, "pchunk");
   ok = ok && h.dalloc(&d.flags, n_sys, "flags") && h.dalloc(&d.istar, n_sys, "istar") &&
-       h.dalloc(&d.any, 1, "any") && h.dalloc(&d.work, n_sys, "work") &&
-       h.dalloc(&d.woff, n_sys + 1, "woff") && h.dalloc(&d.wcoff, n_sys + 1, "wcoff") &&
-       h.dalloc(&d.nwork, 3, "nwork") &&
+       h.dalloc(&d.any, 1, "any") &&
        h.dalloc(&d.status, 2, "status");
   if (!ok) return bail(h.last_status ? h.last_status : SC_E_NOMEM);
   // the FP64 form's pair results, where there is memory for them (a mask word holds 64
@@ -369,7 +367,6 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
        h.cuda_ok(cudaMemsetAsync(d.flags, 0, n_sys * sizeof(int), st), "memset") &&
        h.cuda_ok(cudaMemsetAsync(d.istar, 0x7f, n_sys * sizeof(int), st), "memset") &&
        h.cuda_ok(cudaMemsetAsync(d.any, 0, sizeof(int), st), "memset") &&
-       h.cuda_ok(cudaMemsetAsync(d.nwork, 0, 3 * sizeof(int), st), "memset") &&
        h.cuda_ok(cudaMemsetAsync(d.status, 0, 2 * sizeof(int), st), "memset") &&
        h.cuda_ok(cudaMemsetAsync(d.nbr_n, 0, N * sizeof(int), st), "memset") &&
        h.cuda_ok(cudaMemsetAsync(d.fx, 0, N * sizeof(double), st), "memset") &&

@@ -337,11 +337,9 @@ __global__ void k_cg_move(Dev d, CgState c) {
     request_rebuild(d, s);
 }
 
-// a finished move returns the system to the idle state (after k_cg_move); a rebuild
-// still pending switches the rebuild node on as well
+// a finished move returns the system to the idle state (after k_cg_move)
 __global__ void k_cg_settle(Dev d, CgState c) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s == 0 && d.cond && *d.any != 0) cudaGraphSetConditional(d.cond, 1u);
   if (s >= d.nsys) return;
   CgSys& q = c.sys[s];
   if (q.phase == CG_MOVE) q.phase = CG_IDLE;

@@ -207,12 +207,15 @@ bool Handle::layout_cells() {
   if (ncells > cell_cap) {
     dfree(d.cell_start);
     dfree(d.cell_count);
+    dfree(d.cell_fill);
     dfree((void*)d.cell_sys);
     int cap = ncells + ncells / 4 + 64;
-    int *cs = nullptr, *cn = nullptr, *csys = nullptr;
+    int *cs = nullptr, *cn = nullptr, *cf = nullptr, *csys = nullptr;
     if (!dalloc(&cs, cap, "cell_start") || !dalloc(&cn, cap, "cell_count") ||
-        !dalloc(&csys, cap, "cell_sys"))
+        !dalloc(&cf, cap, "cell_fill") || !dalloc(&csys, cap, "cell_sys") ||
+        !cuda_ok(cudaMemsetAsync(cf, 0, cap * sizeof(int), stream), "cell_fill"))
       return false;
+    d.cell_fill = cf;
     d.cell_start = cs;
     d.cell_count = cn;
     d.cell_sys = csys;
@@ -220,18 +223,16 @@ bool Handle::layout_cells() {
   }
   if (nchunks > chunk_cap) {
     dfree(d.chunk_sum);
-    dfree(d.chunk_off);
     dfree((void*)d.chunk_sys);
     dfree((void*)d.chunk_c0);
     dfree((void*)d.chunk_nc);
     int cap = nchunks + nchunks / 4 + 16;
-    int *a = nullptr, *b = nullptr, *e = nullptr, *f = nullptr, *g = nullptr;
-    if (!dalloc(&a, cap, "chunk_sum") || !dalloc(&b, cap, "chunk_off") ||
-        !dalloc(&e, cap, "chunk_sys") || !dalloc(&f, cap, "chunk_c0") ||
-        !dalloc(&g, cap, "chunk_nc"))
+    int *a = nullptr, *e = nullptr, *f = nullptr, *g = nullptr;
+    if (!dalloc(&a, cap, "chunk_sum") || !dalloc(&e, cap, "chunk_sys") ||
+        !dalloc(&f, cap, "chunk_c0") || !dalloc(&g, cap, "chunk_nc") ||
+        !cuda_ok(cudaMemsetAsync(a, 0, cap * sizeof(int), stream), "chunk_sum"))
       return false;
     d.chunk_sum = a;
-    d.chunk_off = b;
     d.chunk_sys = e;
     d.chunk_c0 = f;
     d.chunk_nc = g;
@@ -353,7 +354,7 @@ bool Handle::check_status(const char* where) {
     return false;
   }
   if (st & ST_BARRIER_TIMEOUT) {
-    fail(SC_E_TIMEOUT, "%s: a grid barrier of the persistent step kernel timed out", where);
+    fail(SC_E_TIMEOUT, "%s: a grid barrier of a cooperative kernel timed out", where);
     return false;
   }
   return true;
@@ -365,7 +366,7 @@ bool Handle::materialize() {
   std::vector<StepScalars> rows(nsys);
   for (int s = 0; s < nsys; s++) rows[s] = row_current(s);
   if (!upload_table(rows)) return false;
-  launch_mx_materialize(d, d_tab, 0, true, stream);
+  launch_mx_materialize(d, d_tab, 0, stream);
   kernels += 1;
   fp64_valid = true;
   return cuda_ok(cudaGetLastError(), "materialize");
@@ -424,7 +425,7 @@ bool Handle::rebuild_all() {
   for (int s = 0; s < nsys; s++) rows[s] = row_current(s);
   if (!upload_table(rows)) return false;
   launch_force_rebuild_all(d, stream);
-  launch_rebuild(d, prec == PREC_MIXED, d_tab, 0, stream);
+  kernels += 1 + launch_rebuild(d, prec == PREC_MIXED, d_tab, 0, false, stream);
   pred_valid = false;
   rebuilds++;
   return cuda_ok(cudaGetLastError(), "rebuild launch");
@@ -432,7 +433,6 @@ bool Handle::rebuild_all() {
 
 void Handle::launch_pass(int mode, bool se, int row, bool fast) {
   Dev dd = d;
-  dd.cond = (mode == PASS_CORR_STRAIN || mode == PASS_CORR_RESIZE) ? step_cond : 0;
   dd.skip = pass_skip;
   if (prec == PREC_MIXED) {
     launch_pass_mixed(dd, mode, se, d_tab, row, stream, block);
@@ -477,32 +477,16 @@ void Handle::collect_times() {
 }
 
 // One Heun step (row k of the uploaded table), strain or resize form, in three
-// parts: the corrector pass, the rebuild body (run only when a system needs it;
-// every kernel in it also exits at once when none does), the predictor pass.
+// parts: the corrector pass, the rebuild kernel (which returns at once when no system
+// needs it), the predictor pass.
 void Handle::enqueue_corr(bool resize, int k, bool prof) {
   timed(0, prof, [&] { launch_pass(resize ? PASS_CORR_RESIZE : PASS_CORR_STRAIN, false, k); });
 }
 
-int Handle::enqueue_rebuild_body(bool resize, int k, bool prof, cudaStream_t st) {
-  int n = 0;
-  cudaStream_t keep = stream;
-  stream = st;
-  // the systems to rebuild (flagged, or setting gamma back at this row) first, so
-  // that the kernels before the cell sort touch their slots only
-  launch_rb_worklist(d, d_tab, k, st);
-  if (prec == PREC_MIXED) {
-    // FP64 positions of the systems about to be sorted or set back
-    launch_mx_materialize(d, d_tab, k, false, st);
-    n++;
-  }
-  if (!resize) {
-    launch_setback(d, d_tab, k, st);
-    n++;
-  }
-  timed(2, prof, [&] { launch_rebuild(d, prec == PREC_MIXED, d_tab, k, st, true); });
-  n += prec == PREC_MIXED ? 13 : 11;
-  stream = keep;
-  return n;
+void Handle::enqueue_rebuild(int k, bool prof) {
+  timed(2, prof, [&] {
+    kernels += launch_rebuild(d, prec == PREC_MIXED, d_tab, k, true, stream);
+  });
 }
 
 void Handle::enqueue_pred(bool resize, int k, bool se, bool prof) {
@@ -511,7 +495,7 @@ void Handle::enqueue_pred(bool resize, int k, bool se, bool prof) {
 
 void Handle::enqueue_step(bool resize, int k, bool se, bool prof) {
   enqueue_corr(resize, k, prof);
-  kernels += enqueue_rebuild_body(resize, k, prof, stream);
+  enqueue_rebuild(k, prof);
   enqueue_pred(resize, k, se, prof);
 }
 
@@ -532,22 +516,18 @@ void Handle::invalidate_graph() {
 // A conditional handle on the graph being captured on `stream`, reset to 0 at
 // every launch of the graph.
 cudaError_t Handle::new_cond_handle(cudaGraphConditionalHandle* h) {
-  return new_cond_handle(h, 0);
-}
-
-cudaError_t Handle::new_cond_handle(cudaGraphConditionalHandle* h, unsigned int dflt) {
   cudaStreamCaptureStatus cs;
   cudaGraph_t gcap = nullptr;
   cudaError_t e = cudaStreamGetCaptureInfo(stream, &cs, nullptr, &gcap, nullptr, nullptr, nullptr);
   if (e == cudaSuccess)
-    e = cudaGraphConditionalHandleCreate(h, gcap, dflt, cudaGraphCondAssignDefault);
+    e = cudaGraphConditionalHandleCreate(h, gcap, 0, cudaGraphCondAssignDefault);
   return e;
 }
 
 // Inside a capture on `stream`: an IF (or WHILE) node on `hcond` after the work
 // captured so far, whose body `body` records on stream2.
 cudaError_t Handle::add_cond_body(cudaGraphConditionalHandle hcond,
-                                  const std::function<int(cudaStream_t)>& body,
+                                  const std::function<void(cudaStream_t)>& body,
                                   cudaGraphConditionalNodeType type) {
   cudaStreamCaptureStatus cs;
   cudaGraph_t gcap = nullptr;
@@ -572,88 +552,26 @@ cudaError_t Handle::add_cond_body(cudaGraphConditionalHandle hcond,
   e = cudaStreamBeginCaptureToGraph(stream2, bg, nullptr, nullptr, 0,
                                     cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return e;
-  body_kernels = body(stream2);
+  body(stream2);
   return cudaStreamEndCapture(stream2, &bg);
 }
 
-// Inside a capture on `stream` (the FIRE iterations, whose update kernel does not
-// switch the node itself): k_pre_rebuild for table row `row` (systems that set gamma
-// back, or a pending rebuild), then the conditional node it switches on; `body`
-// enqueues the node's contents on stream2 and returns its kernel count.
-cudaError_t Handle::capture_rebuild_node(int row, const std::function<int(cudaStream_t)>& body) {
-  cudaGraphConditionalHandle hcond;
-  cudaError_t e = new_cond_handle(&hcond);
-  if (e != cudaSuccess) return e;
-  launch_pre_rebuild(d, d_tab, row, hcond, stream);
-  return add_cond_body(hcond, body);
-}
-
-// Capture the per-step sequence with the rebuild body inside a conditional graph
-// node (skipped when no system needs a rebuild).  Returns false, with the capture
-// ended, when any capture step fails.
-bool Handle::capture_conditional(bool resize, int nsteps, const std::vector<char>& se,
-                                 cudaGraph_t* out) {
-  if (!stream2 && !cuda_ok(cudaStreamCreateWithFlags(&stream2, cudaStreamNonBlocking), "stream"))
-    return false;
-  if (!cuda_ok(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture"))
-    return false;
-  cudaError_t e = cudaSuccess;
-  int r = 0;
-  long long fixed = 0;
-  for (int k = 1; k <= nsteps && e == cudaSuccess; k++) {
-    // the corrector pass itself switches the step's rebuild node on
-    cudaGraphConditionalHandle hcond;
-    e = new_cond_handle(&hcond);
-    if (e != cudaSuccess) break;
-    step_cond = hcond;
-    const long long k1 = kernels;
-    enqueue_corr(resize, k, false);
-    step_cond = 0;
-    fixed += kernels - k1;
-    e = add_cond_body(hcond,
-                      [&](cudaStream_t st) { return enqueue_rebuild_body(resize, k, false, st); });
-    if (e != cudaSuccess) break;
-    const long long k2 = kernels;
-    enqueue_pred(resize, k, se[k] != 0, false);
-    if (se[k]) enqueue_se_record(r++);
-    fixed += kernels - k2;
-  }
-  cudaGraph_t g = nullptr;
-  cudaError_t e2 = cudaStreamEndCapture(stream, &g);
-  if (e != cudaSuccess || e2 != cudaSuccess) {
-    if (g) cudaGraphDestroy(g);
-    cudaGetLastError();
-    return false;
-  }
-  graph_kernels = fixed;
-  *out = g;
-  return true;
-}
-
 // Capture `nsteps` steps (rows 1..nsteps of the current table pointer; se[k]: step k
-// records stress/energy) and instantiate them.  With conditional nodes the rebuild
-// bodies run only when needed, else every step carries the (early-exiting) chain.
+// records stress/energy) and instantiate them.
 bool Handle::instantiate_steps(bool resize, int nsteps, const std::vector<char>& se,
                                cudaGraphExec_t* exec, long long* nkernels) {
   cudaGraph_t g = nullptr;
   long long k0 = kernels;
-  graph_conditional = use_conditional && capture_conditional(resize, nsteps, se, &g);
-  kernels = k0;
-  if (!graph_conditional) {
-    use_conditional = false;  // plain capture: the rebuild kernels exit early
-    if (!cuda_ok(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal),
-                 "begin capture"))
-      return false;
-    int r = 0;
-    for (int k = 1; k <= nsteps; k++) {
-      enqueue_step(resize, k, se[k] != 0, false);
-      if (se[k]) enqueue_se_record(r++);
-    }
-    graph_kernels = kernels - k0;
-    kernels = k0;
-    body_kernels = 0;
-    if (!cuda_ok(cudaStreamEndCapture(stream, &g), "end capture")) return false;
+  if (!cuda_ok(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture"))
+    return false;
+  int r = 0;
+  for (int k = 1; k <= nsteps; k++) {
+    enqueue_step(resize, k, se[k] != 0, false);
+    if (se[k]) enqueue_se_record(r++);
   }
+  *nkernels = kernels - k0;
+  kernels = k0;
+  if (!cuda_ok(cudaStreamEndCapture(stream, &g), "end capture")) return false;
   *exec = nullptr;
   cudaError_t e = cudaGraphInstantiate(exec, g, 0);
   cudaGraphDestroy(g);
@@ -664,7 +582,6 @@ bool Handle::instantiate_steps(bool resize, int nsteps, const std::vector<char>&
     *exec = nullptr;
     return false;
   }
-  *nkernels = graph_kernels;
   return true;
 }
 
@@ -847,7 +764,7 @@ int Handle::run_steps(int kind, int shrink, int nsteps, int se_every, double* se
   // The first step call of a kind captures the plain sub-chunk graph of that kind,
   // whatever its length, so that later calls (a long run after a short warm-up) do
   // not pay the capture.
-  if (opt.use_graphs && !opt.profile && use_conditional &&
+  if (opt.use_graphs && !opt.profile &&
       !(opt.persist_steps && prec == PREC_MIXED && d.pass_kind == 0 && kind == KIND_STRAIN) &&
       !subgraph(kind != KIND_STRAIN, 0u))
     cudaGetLastError();  // capture failed: the chunks fall back to eager launches
@@ -948,11 +865,9 @@ int Handle::run_steps(int kind, int shrink, int nsteps, int se_every, double* se
         return last_status;
     }
     collect_times();
-    long long rb0 = dev_rebuilds;
     if (!check_status(kind == KIND_PURE ? "pure shear steps"
                                         : (resize ? "resize steps" : "strain steps")))
       return last_status;
-    if (use_graph && graph_conditional) kernels += (dev_rebuilds - rb0) * body_kernels;
     fp64_valid = prec != PREC_MIXED;
     forces_valid = false;
     hs = sim;
@@ -1003,7 +918,7 @@ bool Handle::run_persist(int nk, int done, int se_every) {
       }
       k += m;
       if (v & 1) {  // step k's corrector ran; its rebuild and predictor follow
-        kernels += enqueue_rebuild_body(false, k, false, stream);
+        enqueue_rebuild(k, false);
         enqueue_pred(false, k, false, false);
         k++;
       }
@@ -1050,8 +965,7 @@ int Handle::gd_step(const double* se_now, double e_min) {
   }
   if (!upload_table(rows)) return last_status;
   launch_gd_update(d, prec == PREC_MIXED, d_tab, 0, stream);
-  launch_rebuild(d, prec == PREC_MIXED, d_tab, 0, stream);
-  kernels += 12;
+  kernels += 1 + launch_rebuild(d, prec == PREC_MIXED, d_tab, 0, prec == PREC_FP64, stream);
   pred_valid = false;
   return cuda_ok(cudaGetLastError(), "gd step") ? SC_OK : last_status;
 }
@@ -1114,51 +1028,31 @@ void Handle::enqueue_fire_iteration(double ftol, double dt_max) {
   launch_pass(PASS_FORCE, false, 0, true);
   pass_skip = nullptr;
   launch_fire_iteration_tail(d, fire, ftol, dt_max, mixed, stream);
-  // the mixed form moves only its FP32 local state: the flagged systems'
-  // FP64 copies are refreshed before the cell sort reads them
-  launch_rb_worklist(d, d_tab, 0, stream);
-  if (mixed) launch_mx_materialize(d, d_tab, 0, false, stream);
-  launch_rebuild(d, mixed, d_tab, 0, stream, true);
-  kernels += 4 + (mixed ? 14 : 12);
+  kernels += 3 + launch_rebuild(d, mixed, d_tab, 0, true, stream);
 }
 
 // `iters` FIRE iterations as one CUDA graph: each is force pass, reductions and
-// update, then the rebuild chain inside a conditional node that runs only when a
-// system was flagged.  Captured once per (iters, ftol, dt_max) and relaunched;
-// returns false (nothing launched) when the capture is not possible.
+// update, then the rebuild kernel.  Captured once per (iters, ftol, dt_max) and
+// relaunched; returns false (nothing launched) when the capture is not possible.
 bool Handle::run_fire_graph(int iters, double ftol, double dt_max) {
-  if (!use_conditional) return false;
   if (!fire_exec || fire_key_iters != iters || fire_key_ftol != ftol || fire_key_dtmax != dt_max) {
     if (fire_exec) cudaGraphExecDestroy(fire_exec);
     fire_exec = nullptr;
     fire_key_iters = 0;
-    if (!stream2 && !cuda_ok(cudaStreamCreateWithFlags(&stream2, cudaStreamNonBlocking), "stream"))
-      return false;
     if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
       cudaGetLastError();
       return false;
     }
-    const bool mixed = prec == PREC_MIXED;
-    cudaError_t e = cudaSuccess;
     const long long k0 = kernels;
-    for (int k = 0; k < iters && e == cudaSuccess; k++) {
-      pass_skip = fire.done;  // converged systems: no force pass
-      launch_pass(PASS_FORCE, false, 0, true);
-      pass_skip = nullptr;
-      launch_fire_iteration_tail(d, fire, ftol, dt_max, mixed, stream);
-      e = capture_rebuild_node(0, [&](cudaStream_t st) {
-        launch_rb_worklist(d, d_tab, 0, st);
-        if (mixed) launch_mx_materialize(d, d_tab, 0, false, st);
-        launch_rebuild(d, mixed, d_tab, 0, st, true);
-        return mixed ? 14 : 12;
-      });
-    }
+    for (int k = 0; k < iters; k++) enqueue_fire_iteration(ftol, dt_max);
+    fire_graph_kernels = kernels - k0;
+    kernels = k0;
     cudaGraph_t g = nullptr;
-    cudaError_t e2 = cudaStreamEndCapture(stream, &g);
+    cudaError_t e = cudaStreamEndCapture(stream, &g);
     cudaGraphExec_t ex = nullptr;
-    if (e == cudaSuccess && e2 == cudaSuccess) e = cudaGraphInstantiate(&ex, g, 0);
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&ex, g, 0);
     if (g) cudaGraphDestroy(g);
-    if (e != cudaSuccess || e2 != cudaSuccess) {
+    if (e != cudaSuccess) {
       cudaGetLastError();
       return false;
     }
@@ -1166,8 +1060,6 @@ bool Handle::run_fire_graph(int iters, double ftol, double dt_max) {
     fire_key_iters = iters;
     fire_key_ftol = ftol;
     fire_key_dtmax = dt_max;
-    fire_graph_kernels = kernels - k0 + 4LL * iters;
-    kernels = k0;
   }
   kernels += fire_graph_kernels;
   return cuda_ok(cudaGraphLaunch(fire_exec, stream), "fire graph launch");
@@ -1199,10 +1091,7 @@ bool Handle::run_persist_fire(int iters, double ftol, double dt_max) {
     k += m;
     if (why == 2) break;  // every system has converged
     if (why == 1) {
-      launch_rb_worklist(d, d_tab, 0, stream);
-      launch_mx_materialize(d, d_tab, 0, false, stream);
-      launch_rebuild(d, true, d_tab, 0, stream, true);
-      kernels += 14;
+      kernels += launch_rebuild(d, true, d_tab, 0, true, stream);
     }
   }
   return true;
@@ -1305,19 +1194,16 @@ void Handle::enqueue_cg_probe(unsigned long long search, cudaStream_t st) {
   stream = keep;
 }
 
-// the chosen move (with the rebuild request through `cond` inside a graph)
-void Handle::enqueue_cg_move(unsigned long long cond, cudaStream_t st) {
-  Dev dd = d;
-  dd.cond = cond;
-  launch_cg_move(dd, cg, st);
-  kernels += 2;
+// the chosen move, and the rebuild it may ask for
+void Handle::enqueue_cg_move() {
+  launch_cg_move(d, cg, stream);
+  kernels += 2 + launch_rebuild(d, false, d_tab, 0, true, stream);
 }
 
 // kCgChunk iterations as one graph: per iteration the head, the line search in a
 // WHILE node (switched on by the head, off by the search when no system probes
-// again), the move, and the rebuild chain in an IF node the move switches on.
+// again), the move and the rebuild kernel.
 bool Handle::run_cg_graph(int max_iter) {
-  if (!use_conditional) return false;
   if (!cg_exec || cg_key_iter != max_iter) {
     if (cg_exec) cudaGraphExecDestroy(cg_exec);
     cg_exec = nullptr;
@@ -1331,21 +1217,15 @@ bool Handle::run_cg_graph(int max_iter) {
     long long k0 = kernels;
     cudaError_t e = cudaSuccess;
     for (int k = 0; k < kCgChunk && e == cudaSuccess; k++) {
-      cudaGraphConditionalHandle hs, hr;
-      e = new_cond_handle(&hs, 0);
+      cudaGraphConditionalHandle hs;
+      e = new_cond_handle(&hs);
       if (e != cudaSuccess) break;
       enqueue_cg_head(max_iter, hs, stream);
       e = add_cond_body(
-          hs, [&](cudaStream_t st2) { enqueue_cg_probe(hs, st2); return 4; },
+          hs, [&](cudaStream_t st2) { enqueue_cg_probe(hs, st2); },
           cudaGraphCondTypeWhile);
       if (e != cudaSuccess) break;
-      e = new_cond_handle(&hr, 0);
-      if (e != cudaSuccess) break;
-      enqueue_cg_move(hr, stream);
-      e = add_cond_body(hr, [&](cudaStream_t st2) {
-        launch_rebuild(d, false, d_tab, 0, st2);
-        return 12;
-      });
+      enqueue_cg_move();
     }
     kernels = k0;
     cudaGraph_t g = nullptr;
@@ -1360,7 +1240,7 @@ bool Handle::run_cg_graph(int max_iter) {
     cg_exec = ex;
     cg_key_iter = max_iter;
   }
-  kernels += 7LL * kCgChunk;
+  kernels += 9LL * kCgChunk;
   return cuda_ok(cudaGraphLaunch(cg_exec, stream), "cg graph launch");
 }
 
@@ -1386,9 +1266,7 @@ bool Handle::run_cg_eager(int max_iter) {
       if (!searching) break;
       enqueue_cg_probe(0, stream);
     }
-    enqueue_cg_move(0, stream);
-    launch_rebuild(d, false, d_tab, 0, stream);
-    kernels += 12;
+    enqueue_cg_move();
   }
   return cuda_ok(cudaGetLastError(), "cg launch");
 }

@@ -84,9 +84,8 @@ struct Handle {
   bool forces_valid = false;// mixed form: fx/fy/tau hold the forces of the state
   long long steps = 0, rebuilds = 0;
   int dev_status = 0;
-  long long dev_rebuilds = 0;  // rebuild chains the device executed
+  long long dev_rebuilds = 0;  // rebuilds the device executed
   long long kernels = 0;       // kernels launched (eagerly or inside graphs)
-  long long graph_kernels = 0; // kernels in the last captured graph
   long long chunk_kernels = 0; // kernels in the chunk graph (graph_exec)
   int last_status = SC_OK;
   std::string err;
@@ -109,11 +108,8 @@ struct Handle {
   std::vector<SubGraph> sub_graphs;
   StepScalars* d_win = nullptr;
   double* d_win_se = nullptr;
-  cudaStream_t stream2 = nullptr;  // captures the conditional rebuild bodies
-  bool use_conditional = true;     // conditional graph nodes available
-  bool graph_conditional = false;  // the current graph uses them
-  long long body_kernels = 0;      // kernels in one rebuild body
-  // CUDA graph of one chunk of FIRE iterations (same conditional rebuild node)
+  cudaStream_t stream2 = nullptr;  // captures the line search's loop body
+  // CUDA graph of one chunk of FIRE iterations
   cudaGraphExec_t fire_exec = nullptr;
   int fire_key_iters = 0;
   double fire_key_ftol = 0, fire_key_dtmax = 0;
@@ -164,17 +160,12 @@ struct Handle {
   void collect_times();
   void enqueue_step(bool resize, int k, bool se, bool prof);
   void enqueue_corr(bool resize, int k, bool prof);
-  int enqueue_rebuild_body(bool resize, int k, bool prof, cudaStream_t st);
+  void enqueue_rebuild(int k, bool prof);
   void enqueue_pred(bool resize, int k, bool se, bool prof);
-  cudaError_t capture_rebuild_node(int row, const std::function<int(cudaStream_t)>& body);
   cudaError_t new_cond_handle(cudaGraphConditionalHandle* h);
   cudaError_t add_cond_body(cudaGraphConditionalHandle h,
-                            const std::function<int(cudaStream_t)>& body,
+                            const std::function<void(cudaStream_t)>& body,
                             cudaGraphConditionalNodeType type = cudaGraphCondTypeIf);
-  cudaError_t new_cond_handle(cudaGraphConditionalHandle* h, unsigned int dflt);
-  unsigned long long step_cond = 0;  // rebuild node of the step being captured
-  bool capture_conditional(bool resize, int nsteps, const std::vector<char>& se,
-                           cudaGraph_t* out);
   bool instantiate_steps(bool resize, int nsteps, const std::vector<char>& se,
                          cudaGraphExec_t* exec, long long* nkernels);
   bool run_subgraphs(bool resize, int nsteps, int se_every);
@@ -210,7 +201,7 @@ struct Handle {
   bool ensure_cg();
   void enqueue_cg_head(int max_iter, unsigned long long search, cudaStream_t st);
   void enqueue_cg_probe(unsigned long long search, cudaStream_t st);
-  void enqueue_cg_move(unsigned long long cond, cudaStream_t st);
+  void enqueue_cg_move();
   bool run_cg_graph(int max_iter);
   bool run_cg_eager(int max_iter);
   int cg_minimize(int max_iter, int* iters, double* energy, int* reason);

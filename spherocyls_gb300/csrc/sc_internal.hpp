@@ -189,12 +189,13 @@ struct Dev {
   float* rcf;     // isolated-rotation coefficient RC
   float* rf;      // R in FP32: the only per-neighbour constant the force pass gathers
   double* iaa;    // 1 / A^2 (FP64 form: shared_rcp, sc_pair.cuh)
-  float* rsf;     // R + A in FP32 (FP64 form: the list build's reach)
+  float* rsf;     // R + A in FP32: the list build's reach
   int* cellp;     // local cell packed as col | row << 16
   float* gbuild;  // [nsys] gamma at which each system's list was built
   // cell lists
   int* cell_start;          // [ncells] first slot
   int* cell_count;          // [ncells]
+  int* cell_fill;           // [ncells] arrivals during a rebuild, zero between rebuilds
   // neighbour list, column-major [k * ntot + slot]
   int* nbr;                 // FP64 form: slot | kOwner64 where this particle's index is lower
   int* nbr_n;
@@ -215,7 +216,7 @@ struct Dev {
   // compute entries (owner-major) and read entries live in the slot range of its
   // particles times kTileEPP; a pair inside the tile is computed by its lower slot
   // and read back by the other partner from the pair results.
-  unsigned* gbar;           // [2] grid barrier of the persistent step kernel (count, generation)
+  unsigned long long* gbar; // [BAR_WORDS] counters of the cooperative kernels
   const int* skip;          // [nsys] or null: force passes leave systems with skip[s] != 0
                             // alone (converged minimiser systems)
   int pass_kind;            // 0: one thread per particle over its full list, 1: tiles
@@ -232,8 +233,7 @@ struct Dev {
   int* cell_tmp;
   int* rank;
   int* perm;
-  int* chunk_sum;
-  int* chunk_off;
+  int* chunk_sum;           // [nchunks] particles per scan chunk, zero between rebuilds
   const int* chunk_sys;     // [nchunks] system of each chunk
   const int* chunk_c0;      // [nchunks] first global cell of each chunk
   const int* chunk_nc;      // [nchunks] cells in the chunk
@@ -243,6 +243,8 @@ struct Dev {
   double2* s_irc;
   int* s_id;
   int* s_cell;
+  double2* s_mv;            // FP64 form: displacement counters and shaft vectors on their way
+  double2* s_nxy;
   // stress/energy: per-slot contributions and per-chunk partials
   double* se_part;          // [5][ntot]
   double* se_chunk;         // [5][npchunks]
@@ -260,27 +262,22 @@ struct Dev {
   int* flags;               // [nsys] bit0 moved-rebuild, bit1 forced rebuild
   int* istar;               // [nsys] lowest particle index that triggered a rebuild
   int* any;                 // [1] set when any system needs a rebuild
-  int* work;                // [nsys] rebuild worklist: the flagged systems, ascending
-  int* woff;                // [nsys + 1] first work item (slot) of each listed system
-  int* wcoff;               // [nsys + 1] first work item (cell) of each listed system
-  int* nwork;               // [3] listed systems, their slots, their cells
-  int* status;              // [2] sticky error bits (ST_*), rebuild-chain count
-  // the conditional rebuild node of the step a corrector pass belongs to, inside a
-  // captured chunk (0 elsewhere): the pass switches it on when a rebuild is due
-  unsigned long long cond;
+  int* status;              // [2] sticky error bits (ST_*), rebuild count
 };
 
 // sticky device status bits
 enum { ST_NBR_OVERFLOW = 1, ST_NAN = 2, ST_CELL_OVERFLOW = 4, ST_BARRIER_TIMEOUT = 8 };
-// spins (of about 64 ns each) a block waits at a grid barrier of the persistent
-// step kernel before it gives up, records ST_BARRIER_TIMEOUT and goes on
-constexpr unsigned kBarrierSpins = 1u << 24;
+// loads (of about half a microsecond each) a block waits at a grid barrier before it gives
+// up and records ST_BARRIER_TIMEOUT
+constexpr unsigned kBarrierSpins = 1u << 22;
+// Dev::gbar: the barriers of the rebuild and of the persistent kernels, the blocks that
+// are done with a rebuild
+enum { BAR_REBUILD = 0, BAR_STEPS = 1, BAR_FIRE = 2, BAR_DONE = 3, BAR_WORDS = 4 };
 
 constexpr int kScanChunk = 1024;  // cells per scan chunk
 constexpr int kSeChunk = 1024;    // particles per reduction chunk
 // a system's particle-reduction chunks: [pch0, pch0 + pchunk_count), in slot order
 SC_HDI int pchunk_count(const SysGeom& g) { return (g.n + kSeChunk - 1) / kSeChunk; }
-constexpr int kMaxCellSort = 48;  // cells above this occupancy use the in-place slow sort
 constexpr int kNoTrigger = 0x7f7f7f7f;  // istar value when no particle triggered
 constexpr int kOrderWindow = 128;  // slots per window of the force-pass ordering
 // mixed-form list entries: slot in the low 28 bits, cell offset (dc+1, dr+1) above
@@ -325,17 +322,18 @@ int launch_pass_fp64(const Dev& d, int mode, bool se, const StepScalars* tab, in
 int pair_window(int ntot);
 void launch_pass_mixed(const Dev& d, int mode, bool se, const StepScalars* tab, int row,
                        cudaStream_t st, int block);
-// set-back of the listed systems whose row says so (after launch_rb_worklist)
-void launch_setback(const Dev& d, const StepScalars* tab, int row, cudaStream_t st);
-// the rebuild worklist: flagged systems and those whose row (tab, row) sets gamma back
-void launch_rb_worklist(const Dev& d, const StepScalars* tab, int row, cudaStream_t st);
-// the rebuild chain of the listed systems; `listed`: launch_rb_worklist already ran
-void launch_rebuild(const Dev& d, bool mixed, const StepScalars* tab, int row, cudaStream_t st,
-                    bool listed = false);
+// The rebuild of the flagged systems (cells, records, lists), a cooperative kernel that
+// returns at once when none is flagged; `moved`: the state was left by a pass or a minimiser
+// (mixed form: in its records; FP64 form: the shaft vectors are current), else it is in xy
+// and ph alone.  Returns the number of kernels launched.
+int launch_rebuild(const Dev& d, bool mixed, const StepScalars* tab, int row, bool moved,
+                   cudaStream_t st);
+int launch_rebuild_fp64(const Dev& d, const StepScalars* tab, int row, bool moved,
+                        cudaStream_t st);
+int launch_rebuild_mixed(const Dev& d, const StepScalars* tab, int row, bool moved,
+                         cudaStream_t st);
 void launch_force_rebuild_all(const Dev& d, cudaStream_t st);
 void launch_clear_flags(const Dev& d, cudaStream_t st);
-void launch_pre_rebuild(const Dev& d, const StepScalars* tab, int row,
-                        cudaGraphConditionalHandle cond, cudaStream_t st);
 void launch_se_reduce(const Dev& d, cudaStream_t st);
 void launch_gd_update(const Dev& d, bool mixed, const StepScalars* tab, int row, cudaStream_t st);
 void launch_se_store(const Dev& d, double* dst, cudaStream_t st);
@@ -352,9 +350,6 @@ void launch_ingest(const Dev& d, const double* x, const double* y, const double*
                    const double* R, const double* A, const int* sys_p0, const double* sys_L,
                    int* psys, cudaStream_t st);
 void launch_unsort_forces(const Dev& d, double* out, cudaStream_t st);
-void launch_refresh_geometry(const Dev& d, bool mixed, const StepScalars* tab, int row,
-                             cudaStream_t st);
-void launch_build_nbrs(const Dev& d, const StepScalars* tab, int row, cudaStream_t st);
 // FIRE and affine rescale
 void launch_fire_reset(const Dev& d, const FireState& f, double dt0, cudaStream_t st);
 void launch_fire_iteration_tail(const Dev& d, const FireState& f, double ftol, double dt_max,
@@ -364,16 +359,8 @@ void launch_affine(const Dev& d, const double* factor, cudaStream_t st);
 void launch_reflect(const Dev& d, const double* lx, cudaStream_t st);
 void launch_rotate(const Dev& d, const double* q, cudaStream_t st);
 // mixed form
-// all: every slot; else the slots of the listed systems (after launch_rb_worklist)
-void launch_mx_materialize(const Dev& d, const StepScalars* tab, int row, bool all,
-                           cudaStream_t st);
-void launch_mx_local(const Dev& d, const StepScalars* tab, int row, bool all, cudaStream_t st);
-void launch_mx_order(const Dev& d, bool all, cudaStream_t st);
-// the list build and the ordering in one kernel (the per-particle pass)
-void launch_mx_build_order(const Dev& d, const StepScalars* tab, int row, bool all,
-                           cudaStream_t st);
-void launch_mx_build_list(const Dev& d, const StepScalars* tab, int row, bool all,
-                          cudaStream_t st);
+// FP64 state of every slot from its records
+void launch_mx_materialize(const Dev& d, const StepScalars* tab, int row, cudaStream_t st);
 // Persistent mixed shear steps (per-particle pass): rows row0 .. row0 + nsteps - 1 of
 // the table in one cooperative launch, corrector and predictor passes separated by
 // grid barriers, until a step's corrector asks for a rebuild (or a set-back).
@@ -387,84 +374,65 @@ bool launch_persist_steps(const Dev& d, const StepScalars* tab, int row0, int ns
 // converged).  Returns false when the cooperative launch failed.
 bool launch_persist_fire(const Dev& d, const FireState& f, const StepScalars* tab, double ftol,
                          double dt_max, int iters, int* out, cudaStream_t st);
-// tile lists from the mixed lists (after launch_mx_build_list)
-void launch_tile_lists(const Dev& d, bool all, cudaStream_t st);
 // FP64 stress and energy partials of the mixed state (two kernels)
 void launch_mx_se64(const Dev& d, const StepScalars* tab, int row, cudaStream_t st);
 
-constexpr int kWalkBlocks = 152 * 8;  // fixed grid of the worklist kernels
-
 #ifdef __CUDACC__
-// Grid-stride walks over the slots / cells of the systems on the rebuild worklist
-// (k_rb_worklist), so that a rebuild of a few systems of a large batch costs in
-// proportion to those systems.  f(slot or cell, system).
-// the listed system that work item g belongs to (off: exclusive prefix sums)
-__device__ __forceinline__ int listed_system(const int* __restrict__ off, int nw, int g) {
-  int lo = 0, hi = nw - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (off[mid] <= g)
-      lo = mid;
-    else
-      hi = mid - 1;
+// Grid barrier of a cooperative kernel (thread 0 of each block arrives): a counter that
+// only grows, so that arriving is one reduction and waiting one load, 1.3 us with 152
+// blocks and 1.8 us with 456 (a count and a generation: 2.1 and 2.5 us).  A counter serves
+// one kernel of a handle, whose grid is always the same, so a multiple of the grid is where
+// the launch found it.  The wait is bounded: a barrier that times out records
+// ST_BARRIER_TIMEOUT and returns false.
+struct GridBarrier {
+  unsigned long long* count;
+  unsigned long long target;
+  __device__ __forceinline__ explicit GridBarrier(unsigned long long* c) : count(c), target(0) {
+    if (threadIdx.x == 0) target = load() / gridDim.x * gridDim.x;
   }
-  return lo;
-}
-template <class F>
-__device__ __forceinline__ void for_listed_slots(const Dev& d, F&& f) {
-  const int nw = d.nwork[0], W = d.nwork[1];
-  const int t = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  for (int g = t; g < W; g += stride) {
-    const int w = listed_system(d.woff, nw, g);
-    const int s = d.work[w];
-    f(d.geom[s].p0 + (g - d.woff[w]), s);
+  __device__ __forceinline__ unsigned long long load() const {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(count) : "memory");
+    return v;
   }
-}
-template <class F>
-__device__ __forceinline__ void for_listed_cells(const Dev& d, F&& f) {
-  const int nw = d.nwork[0], W = d.nwork[2];
-  const int t = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  for (int g = t; g < W; g += stride) {
-    const int w = listed_system(d.wcoff, nw, g);
-    const int s = d.work[w];
-    f(d.geom[s].c0 + (g - d.wcoff[w]), s);
+  __device__ __forceinline__ bool wait(int* status) {
+    bool ok = true;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      target += gridDim.x;
+      asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(count) : "memory");
+      unsigned it = 0;
+      while (load() < target) {
+        if (++it > kBarrierSpins) {
+          atomicOr(status, ST_BARRIER_TIMEOUT);
+          ok = false;
+          break;
+        }
+      }
+    }
+    return __syncthreads_and(ok) != 0;
   }
-}
-// Corrector passes inside a captured step (d.cond != 0), block 0 before any early
-// exit: mark the systems that set gamma back at this step (their rows say so) and
-// switch the step's rebuild node on for them, or for a rebuild still pending.
+};
+// Corrector passes, block 0 before any early exit: flag the systems that set gamma back
+// at this step (their rows say so) for the rebuild that follows.
 __device__ __forceinline__ void mark_pending_rebuilds(const Dev& d,
                                                       const StepScalars* __restrict__ tab,
                                                       int row) {
-  if (!d.cond || blockIdx.x != 0) return;
-  bool setback = false;
+  if (blockIdx.x != 0) return;
   for (int s = threadIdx.x; s < d.nsys; s += blockDim.x)
     if (tab[row * d.nsys + s].setback) {
       atomicOr(&d.flags[s], 2);
-      setback = true;
+      atomicExch(d.any, 1);
     }
-  if (setback) atomicExch(d.any, 1);
-  if (setback || (threadIdx.x == 0 && *d.any != 0)) cudaGraphSetConditional(d.cond, 1u);
 }
 // FP32 copy of an FP64 position and shaft vector, for the FP64 form's pair screen
 __device__ __forceinline__ float4 screen_record(double2 p, double2 n) {
   return make_float4((float)p.x, (float)p.y, (float)n.x, (float)n.y);
 }
-// A particle of system s needs its list rebuilt: flag the system, raise the pending
-// word, and (the thread that raises it) switch the step's rebuild node on.
+// A particle of system s needs its list rebuilt: flag the system, raise the pending word.
 __device__ __forceinline__ void request_rebuild(const Dev& d, int s) {
   if (d.flags[s] == 0) atomicOr(&d.flags[s], 1);
-  if (*d.any == 0 && atomicExch(d.any, 1) == 0 && d.cond) cudaGraphSetConditional(d.cond, 1u);
-}
-// all: every slot of every system (forced refreshes), else the worklist
-template <class F>
-__device__ __forceinline__ void for_slots(const Dev& d, bool all, F&& f) {
-  if (!all) {
-    for_listed_slots(d, f);
-    return;
-  }
-  const int t = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  for (int i = t; i < d.ntot; i += stride) f(i, d.psys[i]);
+  if (*d.any == 0) atomicExch(d.any, 1);
 }
 #endif
 

@@ -61,6 +61,25 @@ __device__ __forceinline__ bool less_square(double u, double v) {
   return (unsigned long long)__double_as_longlong(u) < (unsigned long long)__double_as_longlong(v);
 }
 
+// (double)f and (float)d (rounded to nearest even) by the integer pipe; the conversions
+// run at the FP64 pipe's rate.
+__device__ __forceinline__ double widen(float f) {
+  const unsigned b = __float_as_uint(f), e = b & 0x7f800000u;
+  if (e == 0u || e == 0x7f800000u) return (double)f;  // zero, subnormal, infinite, NaN
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)),
+                          (int)(b << 29));
+}
+__device__ __forceinline__ float narrow(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned e = hi & 0x7ff00000u;
+  // exponents whose rounded value is a normal float
+  if (e - 0x38100000u >= 0x0fd00000u) return (float)v;
+  const unsigned m = __funnelshift_l(lo, (hi & 0x7fffffffu) - 0x38000000u, 3);
+  const unsigned rest = lo & 0x1fffffffu;
+  const unsigned up = rest > 0x10000000u || (rest == 0x10000000u && (m & 1u)) ? 1u : 0u;
+  return __uint_as_float((hi & 0x80000000u) | (m + up));
+}
+
 // Quotients that share a divisor: r = 1/y rounded to nearest, then x r with one correction
 // by its exact remainder, which is the correctly rounded x/y (P. W. Markstein, IBM J. Res.
 // Dev. 34, 111 (1990)); three operations in place of a division's eight or so.  A divisor

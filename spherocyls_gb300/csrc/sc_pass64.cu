@@ -14,6 +14,7 @@
 // whose pair buffers could not be had, with the same bits.
 #include "sc_internal.hpp"
 #include "sc_pair.cuh"
+#include "sc_rebuild.cuh"
 
 namespace sc {
 
@@ -34,7 +35,7 @@ __device__ __forceinline__ bool nbr_criterion(double2 pp, double2 pq, double sig
   return false;
 }
 
-// The padded list of each listed slot: the reference's criterion in FP64, decided in
+// The padded list of slot i (system s): the reference's criterion in FP64, decided in
 // FP32 wherever that is certain.  The FP32 copies of the positions move |dX|, |dX + dY/2|
 // and |dY| by less than `slack` (see Screen64), so a candidate outside the bound by more
 // is out and one inside it by more is in; about one in a thousand is evaluated in FP64.
@@ -42,62 +43,120 @@ __device__ __forceinline__ bool nbr_criterion(double2 pp, double2 pq, double sig
 // choose the other image, can be in reach evaluate all in FP64.  The FP64 pipe
 // bounded the build: 14 operations for each of about 33 candidates a particle took 191 us
 // at 131072 particles (a/R 0.25 to 2), the FP32 test takes 26 us.
-__global__ void __launch_bounds__(128) k_build_nbrs(Dev d, const StepScalars* __restrict__ tab,
-                                                   int row) {
-  if (*d.any == 0) return;
-  for_listed_slots(d, [&](int i, int s) {
-    const SysGeom& g = d.geom[s];
-    const StepScalars& ts = tab[row * d.nsys + s];
-    const float4 ri = d.rec[i];
-    const float si = d.rsf[i];
-    const int idi = d.id[i];
-    const float gam = (float)ts.gamma_p, fLx = (float)ts.Lx_p, fLy = (float)ts.Ly_p;
-    const float pad = (float)g.pad;
-    const float slack = 5e-7f * (fLx + fLy) * (1.f + fabsf(gam)) + 1e-6f * (2.f * g.smax + pad);
-    const float reach = g.smax + pad + slack;
-    const bool small = !(0.5f * fLx > reach * (1.f + fmaxf(fabsf(gam), 0.5f)) &&
-                         0.5f * fLy > reach);
-    int c = d.cell[i] - g.c0;
-    int col, rw;
-    cell_colrow(g, c, &col, &rw);
+// GL = 8 threads (sub: which) take the candidates side by side; the list keeps the order of
+// the scan.  With one thread a slot small systems wait for 33 loads in turn: 17 us at 1024
+// particles, 5 with eight.
+template <int GL>
+__device__ __forceinline__ void build_nbrs(const Dev& d, const StepScalars* __restrict__ tab,
+                                           int row, int i, int s, int sub, unsigned lanes,
+                                           Candidates* table) {
+  const SysGeom& g = d.geom[s];
+  const StepScalars& ts = tab[row * d.nsys + s];
+  const float4 ri = d.rec[i];
+  const float si = d.rsf[i];
+  const int idi = d.id[i];
+  const float gam = (float)ts.gamma_p, fLx = (float)ts.Lx_p, fLy = (float)ts.Ly_p;
+  const float pad = g.fpad;
+  const float slack = 5e-7f * (fLx + fLy) * (1.f + fabsf(gam)) + 1e-6f * (2.f * g.smax + pad);
+  const float reach = g.smax + pad + slack;
+  const bool small = !(0.5f * fLx > reach * (1.f + fmaxf(fabsf(gam), 0.5f)) &&
+                       0.5f * fLy > reach);
+  int col, rw;
+  cell_colrow(g, d.cell[i] - g.c0, &col, &rw);
+  int cnt = 0;
+  // whether candidate j is listed, and which of the two has the lower index
+  auto test = [&](int j, bool* ip) {
+    const float4 rj = d.rec[j];
+    float dx = ri.x - rj.x, dy = ri.y - rj.y;
+    dx += fLx * (float)((dx < -0.5f * fLx) - (dx > 0.5f * fLx));
+    dy += fLy * (float)((dy < -0.5f * fLy) - (dy > 0.5f * fLy));
+    const float near = fminf(fabsf(fmaf(gam, dy, dx)), fabsf(fmaf(0.5f, dy, dx)));
+    const float over = fmaxf(fabsf(dy), near) - (si + d.rsf[j] + pad);
+    if (!small && over > slack) return false;
+    *ip = idi < d.id[j];
+    if (small || !(over < -slack)) {
+      const double2 pi = d.xy[i], pj = d.xy[j], rai = d.ra[i], raj = d.ra[j];
+      // S = R_p + A_p + R_q + A_q summed in the reference's order
+      double sig = *ip ? rai.x + rai.y + raj.x + raj.y : raj.x + raj.y + rai.x + rai.y;
+      return *ip ? nbr_criterion(pi, pj, sig, g.pad, ts.gamma_p, ts.Lx_p, ts.Ly_p)
+                 : nbr_criterion(pj, pi, sig, g.pad, ts.gamma_p, ts.Lx_p, ts.Ly_p);
+    }
+    return true;
+  };
+  if (GL == 1) {
     // 3x3 block of cells; a dimension with fewer than three cells is scanned once
     // per distinct cell (the reference would list such cells twice).
-    int ncx = g.cols < 3 ? g.cols : 3, ncy = g.rows < 3 ? g.rows : 3;
-    int cnt = 0;
+    const int ncx = g.cols < 3 ? g.cols : 3, ncy = g.rows < 3 ? g.rows : 3;
     for (int a = 0; a < ncy; a++) {
-      int r2 = ncy == 3 ? wrap_index(rw + a - 1, g.rows) : a;
+      const int r2 = ncy == 3 ? wrap_index(rw + a - 1, g.rows) : a;
       for (int b = 0; b < ncx; b++) {
-        int c2 = ncx == 3 ? wrap_index(col + b - 1, g.cols) : b;
-        int cc = g.c0 + cell_local(g, c2, r2);
-        int st = d.cell_start[cc], nn = d.cell_count[cc];
-        for (int j = st; j < st + nn; j++) {
-          if (j == i) continue;
-          const float4 rj = d.rec[j];
-          float dx = ri.x - rj.x, dy = ri.y - rj.y;
-          dx += fLx * (float)((dx < -0.5f * fLx) - (dx > 0.5f * fLx));
-          dy += fLy * (float)((dy < -0.5f * fLy) - (dy > 0.5f * fLy));
-          const float near = fminf(fabsf(fmaf(gam, dy, dx)), fabsf(fmaf(0.5f, dy, dx)));
-          const float over = fmaxf(fabsf(dy), near) - (si + d.rsf[j] + pad);
-          if (!small && over > slack) continue;
-          const int idj = d.id[j];
-          const bool ip = idi < idj;
-          if (small || !(over < -slack)) {
-            const double2 pi = d.xy[i], pj = d.xy[j], rai = d.ra[i], raj = d.ra[j];
-            // S = R_p + A_p + R_q + A_q summed in the reference's order
-            double sig = ip ? rai.x + rai.y + raj.x + raj.y : raj.x + raj.y + rai.x + rai.y;
-            if (!(ip ? nbr_criterion(pi, pj, sig, g.pad, ts.gamma_p, ts.Lx_p, ts.Ly_p)
-                     : nbr_criterion(pj, pi, sig, g.pad, ts.gamma_p, ts.Lx_p, ts.Ly_p)))
-              continue;
-          }
+        const int c2 = ncx == 3 ? wrap_index(col + b - 1, g.cols) : b;
+        const int cc = g.c0 + cell_local(g, c2, r2);
+        const int st = d.cell_start[cc], en = st + d.cell_count[cc];
+        for (int j = st; j < en; j++) {
+          bool ip = false;
+          if (j == i || !test(j, &ip)) continue;
           if (cnt < d.maxn)
             d.nbr[(size_t)cnt * d.ntot + i] = (int)((unsigned)j | (ip ? kOwner64 : 0u));
           cnt++;
         }
       }
     }
-    d.nbr_n[i] = cnt;
-    if (cnt > d.maxn) atomicOr(d.status, ST_NBR_OVERFLOW);
-  });
+  } else {
+    const int n = list_candidates(d, g, col, rw, *table, sub, lanes);
+    for (int k0 = 0, q = 0; k0 < n; k0 += GL) {
+      const int k = k0 + sub;
+      bool ip = false, hit = false;
+      int j = 0;
+      if (k < n) {
+        while (k >= table->off[q + 1]) q++;
+        j = table->first[q] + k - table->off[q];
+        hit = j != i && test(j, &ip);
+      }
+      const unsigned all = __ballot_sync(lanes, hit) & lanes;
+      const int at = cnt + __popc(all & ((1u << (threadIdx.x & 31)) - 1u));
+      cnt += __popc(all);
+      if (hit && at < d.maxn)
+        d.nbr[(size_t)at * d.ntot + i] = (int)((unsigned)j | (ip ? kOwner64 : 0u));
+    }
+  }
+  if (sub != 0) return;
+  d.nbr_n[i] = cnt;
+  if (cnt > d.maxn) atomicOr(d.status, ST_NBR_OVERFLOW);
+}
+
+// The rebuild of the FP64 form (sc_rebuild.cuh): cells, shaft vectors and FP32 copies, lists.
+template <int BS>
+__global__ void __launch_bounds__(BS, 1024 / BS) k_rebuild64(Dev d,
+                                                             const StepScalars* __restrict__ tab,
+                                                             int row, int moved) {
+  if (!rb::pending(d)) return;
+  GridBarrier bar(d.gbar + BAR_REBUILD);
+  const rb::Work<BS> work(d);
+  const bool ok = rb::sort_cells<false, BS>(
+      d, work, tab, row, moved != 0, bar,
+      [&](int i, int, double2 p, double, double2 ra, double2, int, int) {
+        d.moved[i] = d.s_mv[i];
+        const double2 n = d.s_nxy[i];
+        d.nxy[i] = n;
+        d.rec[i] = screen_record(p, n);
+        d.rf[i] = (float)ra.x;
+        d.rsf[i] = (float)(ra.x + ra.y);
+        d.iaa[i] = shared_rcp(ra.y * ra.y);
+      });
+  if (!ok) return;
+  if (work.items > kLaneItems) {
+    work.each(d, [&](int i, int s) { build_nbrs<1>(d, tab, row, i, s, 0, 0u, nullptr); });
+  } else {
+    __shared__ Candidates table[BS / 8];
+    const unsigned lanes = 0xffu << (threadIdx.x & 24);
+    for (int g = (blockIdx.x * BS + threadIdx.x) / 8; g < work.items; g += gridDim.x * BS / 8) {
+      int i, s;
+      if (work.at(d, g, &i, &s))
+        build_nbrs<8>(d, tab, row, i, s, threadIdx.x & 7, lanes, &table[threadIdx.x / 8]);
+    }
+  }
+  rb::finish(d);
 }
 
 // ---- the FP32 screen ----
@@ -1013,8 +1072,19 @@ void launch_mx_se64(const Dev& d, const StepScalars* tab, int row, cudaStream_t 
     k_mx_se64<false><<<grid, kSeBlock, 0, st>>>(d, tab, row);
 }
 
-void launch_build_nbrs(const Dev& d, const StepScalars* tab, int row, cudaStream_t st) {
-  k_build_nbrs<<<2 * kWalkBlocks, 128, 0, st>>>(d, tab, row);
+int launch_rebuild_fp64(const Dev& d, const StepScalars* tab, int row, bool moved,
+                        cudaStream_t st) {
+  int mv = moved ? 1 : 0;
+  void* args[] = {(void*)&d, (void*)&tab, &row, &mv};
+  if (d.ntot <= kSmallRebuild) {
+    const void* fn = (const void*)k_rebuild64<128>;
+    cudaLaunchCooperativeKernel(fn, coop_blocks<0>(fn, 128, (d.ntot + 15) / 16), 128, args, 0, st);
+  } else {
+    const void* fn = (const void*)k_rebuild64<512>;
+    cudaLaunchCooperativeKernel(fn, coop_blocks<1>(fn, 512, (d.ntot + 63) / 64), 512, args, 0,
+                                st);
+  }
+  return 1;
 }
 
 }  // namespace sc

@@ -27,6 +27,7 @@
 #include "sc_fire.cuh"
 #include "sc_internal.hpp"
 #include "sc_pair.cuh"
+#include "sc_rebuild.cuh"
 
 namespace sc {
 
@@ -279,35 +280,10 @@ __global__ void __launch_bounds__(128, TWO ? 6 : 12) k_pass_mixed(Dev d,
 // and relaunches.  Every wait is bounded (kBarrierSpins): a barrier that times out
 // records ST_BARRIER_TIMEOUT, which the host reports as an error.
 
-// generation barrier over all blocks of the grid (thread 0 of each block arrives)
-__device__ __forceinline__ void grid_barrier(unsigned* bar, int* status) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    volatile unsigned* vgen = bar + 1;
-    const unsigned gen = *vgen;
-    __threadfence();
-    if (atomicAdd(bar, 1u) == gridDim.x - 1) {
-      atomicExch(bar, 0u);
-      __threadfence();
-      atomicAdd(bar + 1, 1u);
-    } else {
-      unsigned it = 0;
-      while (*vgen == gen) {
-        if (++it > kBarrierSpins) {
-          atomicOr(status, ST_BARRIER_TIMEOUT);
-          break;
-        }
-        __nanosleep(64);
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-}
-
 template <bool TWO>
 __global__ void __launch_bounds__(128, TWO ? 6 : 12) k_persist_steps(
     Dev d, const StepScalars* __restrict__ tab, int row0, int nsteps, int* out) {
+  GridBarrier bar(d.gbar + BAR_STEPS);
   const int stride = gridDim.x * blockDim.x;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
   int k = 0, stopped = 0;
@@ -322,14 +298,14 @@ __global__ void __launch_bounds__(128, TWO ? 6 : 12) k_persist_steps(
         }
     for (int pos = t0; pos < d.ntot; pos += stride)
       pass_mixed_position<PASS_CORR_STRAIN, TWO, true>(d, tab, row, pos);
-    grid_barrier(d.gbar, d.status);
+    bar.wait(d.status);
     if (*(volatile int*)d.any != 0) {  // the same value in every block after the barrier
       stopped = 1;
       break;
     }
     for (int pos = t0; pos < d.ntot; pos += stride)
       pass_mixed_position<PASS_PRED_STRAIN, TWO, true>(d, tab, row, pos);
-    grid_barrier(d.gbar, d.status);
+    bar.wait(d.status);
   }
   if (t0 == 0) *out = 2 * k + stopped;
 }
@@ -350,21 +326,22 @@ template <bool TWO>
 __global__ void __launch_bounds__(256, TWO ? 3 : 4) k_persist_fire(
     Dev d, FireState f, const StepScalars* __restrict__ tab, double ftol, double dt_max,
     int iters, int* out) {
+  GridBarrier bar(d.gbar + BAR_FIRE);
   const int stride = gridDim.x * blockDim.x;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
   int k = 0, why = 0;
   while (k < iters) {
     for (int pos = t0; pos < d.ntot; pos += stride)
       pass_mixed_position<PASS_FORCE, TWO, true>(d, tab, 0, pos);
-    grid_barrier(d.gbar, d.status);
+    bar.wait(d.status);
     for (int ch = blockIdx.x; ch < d.npchunks; ch += gridDim.x) {
       fire::fire_chunk<true>(d, f, ch);
       __syncthreads();  // the next chunk reuses the block's shared partials
     }
-    grid_barrier(d.gbar, d.status);
+    bar.wait(d.status);
     // one block per system, as k_fire_sys (the block has kFireBlock threads)
     for (int s = blockIdx.x; s < d.nsys; s += gridDim.x) fire::fire_sys(d, f, s, ftol, dt_max);
-    grid_barrier(d.gbar, d.status);
+    bar.wait(d.status);
     k++;
     // every block sees the same flags: they change only in the phase before the barrier
     int pending = 0;
@@ -374,7 +351,7 @@ __global__ void __launch_bounds__(256, TWO ? 3 : 4) k_persist_fire(
       break;
     }
     for (int i = t0; i < d.ntot; i += stride) fire::fire_update<true>(d, f, i);
-    grid_barrier(d.gbar, d.status);
+    bar.wait(d.status);
     if (*(volatile int*)d.any != 0) {
       why = 1;
       break;
@@ -527,10 +504,10 @@ __device__ __forceinline__ int tile_excl_scan(int v, int* sh, int* total) {
 // offsets by block scans; then every read entry finds the compute entry of its pair
 // among the partner's.  A pair listed by one side only (the capsule test's rounding
 // at the padding's edge, far from contact) is computed by nobody.
-__global__ void __launch_bounds__(kTileThreads) k_tile_lists(Dev d, int all) {
-  if (!all && *d.any == 0) return;
+__global__ void __launch_bounds__(kTileThreads) k_tile_lists(Dev d) {
+  if (*d.any == 0) return;
   const int4 tl = d.tiles[blockIdx.x];
-  if (!all && d.flags[tl.x] == 0) return;
+  if (d.flags[tl.x] == 0) return;
   __shared__ int sh[32];
   const int cl = tl.y + tl.z - 1;
   const int p0 = d.cell_start[tl.y];
@@ -608,59 +585,44 @@ __global__ void __launch_bounds__(kTileThreads) k_tile_lists(Dev d, int all) {
   }
 }
 
-// ---- rebuild support ----
+// ---- rebuild ----
 
-// FP64 absolute state from the compensated local state (flagged systems, systems
-// that set back gamma at this step, or all).
-// FP64 state of slot i from its compensated record and its cell centre
-__device__ __forceinline__ void materialize_slot(const Dev& d, const StepScalars& ts, int i) {
-  int cp = d.cellp[i];
-  float4 r = d.rec[i];
-  float4 c = d.mc[i];
-  double x = ((cp & 0xffff) + 0.5) * ts.W_p + ((double)r.x + (double)c.x);
-  double y = ((cp >> 16) + 0.5) * ts.H_p + ((double)r.y + (double)c.y);
-  d.xy[i] = make_double2(x, y);
-  d.ph[i] = (double)c.z + (double)c.w;
+// FP64 absolute state of every slot from its compensated record and its cell centre
+__global__ void k_mx_materialize(Dev d, const StepScalars* __restrict__ tab, int row) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= d.ntot) return;
+  const float4 c = d.mc[i];
+  d.xy[i] = rb::mixed_position(d, tab[row * d.nsys + d.psys[i]], i, d.rec[i], c);
+  d.ph[i] = widen(c.z) + widen(c.w);
 }
 
-// every slot (all) or, after launch_rb_worklist, the slots of the listed systems
-__global__ void k_mx_materialize(Dev d, const StepScalars* __restrict__ tab, int row, int all) {
-  if (all) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < d.ntot) materialize_slot(d, tab[row * d.nsys + d.psys[i]], i);
-    return;
-  }
-  for_listed_slots(d, [&](int i, int s) { materialize_slot(d, tab[row * d.nsys + s], i); });
-}
-
-// Compensated local state from the FP64 state after a cell sort.
-__global__ void k_mx_local(Dev d, const StepScalars* __restrict__ tab, int row, int all) {
-  if (!all && *d.any == 0) return;
-  for_slots(d, all != 0, [&](int i, int s) {
-    const SysGeom& g = d.geom[s];
-    const StepScalars& ts = tab[row * d.nsys + s];
-    int lc = d.cell[i] - g.c0;
-    int col, rw;
-    cell_colrow(g, lc, &col, &rw);
-    d.cellp[i] = col | (rw << 16);
-    double2 p = d.xy[i];
-    double lx = p.x - (col + 0.5) * ts.W_p;
-    double ly = p.y - (rw + 0.5) * ts.H_p;
-    double phi = d.ph[i];
-    float xl = (float)lx, yl = (float)ly, pf = (float)phi;
-    double2 ra = d.ra[i];
-    double2 irc = d.irc[i];
-    float A = (float)ra.y;
-    float sn, cs;
-    sincosf(pf, &sn, &cs);
-    d.rec[i] = make_float4(xl, yl, A * cs, A * sn);
-    d.mc[i] = make_float4((float)(lx - xl), (float)(ly - yl), pf, (float)(phi - pf));
-    d.mm[i] = make_float4(0.f, 0.f, pf + (float)(phi - pf), 0.f);
-    // 1/I in FP32 (an FP64 division per particle costs more than the whole record)
-    d.pa[i] = make_float4((float)ra.x, A, __int_as_float(d.id[i]), __frcp_rn((float)irc.x));
-    d.rcf[i] = (float)irc.y;
-    d.rf[i] = (float)ra.x;
-  });
+// Compensated local state of a slot from its FP64 state after the cell sort.
+__device__ __forceinline__ void local_record(const Dev& d, const StepScalars* __restrict__ tab,
+                                             int row, int i, int s, double2 p, double phi,
+                                             double2 ra, double2 irc, int id, int cell) {
+  const SysGeom& g = d.geom[s];
+  const StepScalars& ts = tab[row * d.nsys + s];
+  int col, rw;
+  cell_colrow(g, cell - g.c0, &col, &rw);
+  d.cellp[i] = col | (rw << 16);
+  // (conversions between FP32 and FP64 by the integer pipe: 35 of 57 us of this phase at
+  // 2^20 particles were theirs)
+  const double lx = fma(-widen((float)col + 0.5f), ts.W_p, p.x);
+  const double ly = fma(-widen((float)rw + 0.5f), ts.H_p, p.y);
+  float xl = narrow(lx), yl = narrow(ly), pf = narrow(phi);
+  float A = narrow(ra.y);
+  const float pc = narrow(phi - widen(pf));
+  float sn, cs;
+  sincosf(pf, &sn, &cs);
+  d.rec[i] = make_float4(xl, yl, A * cs, A * sn);
+  d.mc[i] = make_float4(narrow(lx - widen(xl)), narrow(ly - widen(yl)), pf, pc);
+  d.mm[i] = make_float4(0.f, 0.f, pf + pc, 0.f);
+  // 1/I in FP32 (an FP64 division per particle costs more than the whole record)
+  const float R = narrow(ra.x);
+  d.pa[i] = make_float4(R, A, __int_as_float(id), __frcp_rn(narrow(irc.x)));
+  d.rcf[i] = narrow(irc.y);
+  d.rf[i] = R;
+  d.rsf[i] = R + A;
 }
 
 // The padded neighbour list in FP32 (see the file comment).  Two stages per
@@ -671,19 +633,21 @@ __global__ void k_mx_local(Dev d, const StepScalars* __restrict__ tab, int row, 
 // by cell, slots ascending) is the scan order either way.
 constexpr int kMxQueue = 24;
 
-// The list of slot i (system s): see the file comment and kMxQueue.
+// The list of slot i (system s): see the file comment and kMxQueue.  SMALL: a grid under
+// three cells a side somewhere.
+template <bool SMALL>
 __device__ __forceinline__ void build_list_slot(const Dev& d, const StepScalars* __restrict__ tab,
                                                 int row, int i, int s) {
   const SysGeom& g = d.geom[s];
   const StepScalars& ts = tab[row * d.nsys + s];
-  const float W = ts.f_Wp, H = ts.f_Hp, gam = ts.f_gamma_p, pad = (float)g.pad;
+  const float W = ts.f_Wp, H = ts.f_Hp, gam = ts.f_gamma_p, pad = g.fpad;
   const float Lxf = W * g.cols, Lyf = H * g.rows;
   const int cp = d.cellp[i];
   const int col = cp & 0xffff, rw = cp >> 16;
   const float4 ri = d.rec[i];
-  const float2 rai = reinterpret_cast<const float2*>(d.pa)[2 * (size_t)i];  // (R, A)
-  const int ncx = g.cols < 3 ? g.cols : 3, ncy = g.rows < 3 ? g.rows : 3;
-  const bool smallx = ncx < 3, smally = ncy < 3;
+  const float Ri = d.rf[i], si = d.rsf[i] + pad;
+  const int ncx = SMALL && g.cols < 3 ? g.cols : 3, ncy = SMALL && g.rows < 3 ? g.rows : 3;
+  const bool smallx = SMALL && ncx < 3, smally = SMALL && ncy < 3;
   unsigned queue[kMxQueue];  // survivors of the centre test: slot | cell offset code
   int nq = 0, cnt = 0;
   // capsule test of the queued candidates, accepted ones appended in queue order
@@ -691,6 +655,7 @@ __device__ __forceinline__ void build_list_slot(const Dev& d, const StepScalars*
     for (int q = 0; q < nq; q++) {
       const unsigned e = queue[q];
       const int j = (int)(e & kSlotMask);
+      if (j == i) continue;
       const float4 rj = d.rec[j];
       const float Rj = d.rf[j];
       float dx = ri.x - rj.x + (float)(1 - (int)((e >> 28) & 3u)) * W;
@@ -698,7 +663,7 @@ __device__ __forceinline__ void build_list_slot(const Dev& d, const StepScalars*
       if (smallx) dx += Lxf * (float)((dx < -0.5f * Lxf) - (dx > 0.5f * Lxf));
       if (smally) dy += Lyf * (float)((dy < -0.5f * Lyf) - (dy > 0.5f * Lyf));
       if (capsules_within(fmaf(gam, dy, dx), dy, ri.z, ri.w, rj.z, rj.w,
-                          (rai.x + Rj + pad) * 1.00002f + 1e-5f)) {
+                          (Ri + Rj + pad) * 1.00002f + 1e-5f)) {
         if (cnt < d.maxn) d.nbr[(size_t)cnt * d.ntot + i] = (int)e;
         cnt++;
       }
@@ -708,24 +673,22 @@ __device__ __forceinline__ void build_list_slot(const Dev& d, const StepScalars*
   for (int a = 0; a < ncy; a++) {
     int dr = smally ? a - rw : a - 1;
     int r2 = smally ? a : wrap_index(rw + dr, g.rows);
+    const float y0 = ri.y - (float)dr * H;
     for (int b = 0; b < ncx; b++) {
       int dc = smallx ? b - col : b - 1;
       int c2 = smallx ? b : wrap_index(col + dc, g.cols);
       int cc = g.c0 + cell_local(g, c2, r2);
       int st = d.cell_start[cc], en = st + d.cell_count[cc];
       unsigned code = ((unsigned)(dc + 1) << 28) | ((unsigned)(dr + 1) << 30);
-      const float ox = (float)dc * W, oy = (float)dr * H;
-      for (int j = st; j < en; j++) {
-        if (j == i) continue;
-        const float4 rj = d.rec[j];
-        const float2 raj = reinterpret_cast<const float2*>(d.pa)[2 * (size_t)j];
-        float dx = ri.x - rj.x - ox;
-        float dy = ri.y - rj.y - oy;
+      const float x0 = ri.x - (float)dc * W;
+      for (int j = st; j < en; j++) {  // (the slot itself is dropped with the queue)
+        const float2 rj = *reinterpret_cast<const float2*>(&d.rec[j]);
+        float dx = x0 - rj.x, dy = y0 - rj.y;
         if (smallx) dx += Lxf * (float)((dx < -0.5f * Lxf) - (dx > 0.5f * Lxf));
         if (smally) dy += Lyf * (float)((dy < -0.5f * Lyf) - (dy > 0.5f * Lyf));
-        const float lim = (rai.x + rai.y + raj.x + raj.y + pad) * 1.00002f + 1e-6f;
+        const float lim = fmaf(si + d.rsf[j], 1.00002f, 1e-6f);
         const float dxl = fmaf(gam, dy, dx);
-        if (dxl * dxl + dy * dy < lim * lim) {
+        if (fmaf(dxl, dxl, dy * dy) < lim * lim) {
           queue[nq++] = (unsigned)j | code;
           if (nq == kMxQueue) flush();
         }
@@ -737,77 +700,147 @@ __device__ __forceinline__ void build_list_slot(const Dev& d, const StepScalars*
   if (cnt > d.maxn) atomicOr(d.status, ST_NBR_OVERFLOW);
   if (i == g.p0) d.gbuild[s] = gam;
 }
+__device__ __forceinline__ void build_list_slot(const Dev& d, const StepScalars* __restrict__ tab,
+                                                int row, int i, int s) {
+  if (d.geom[s].cols < 3 || d.geom[s].rows < 3)
+    build_list_slot<true>(d, tab, row, i, s);
+  else
+    build_list_slot<false>(d, tab, row, i, s);
+}
+
+// The same list with eight threads a slot, for small rebuilds (see build_nbrs): the
+// candidates side by side, both tests at once.
+__device__ __forceinline__ void build_list_lanes(const Dev& d, const StepScalars* __restrict__ tab,
+                                                 int row, int i, int s, int sub, unsigned lanes,
+                                                 Candidates& table) {
+  const SysGeom& g = d.geom[s];
+  const StepScalars& ts = tab[row * d.nsys + s];
+  const float W = ts.f_Wp, H = ts.f_Hp, gam = ts.f_gamma_p, pad = g.fpad;
+  const float Lxf = W * g.cols, Lyf = H * g.rows;
+  const int cp = d.cellp[i];
+  const float4 ri = d.rec[i];
+  const float Ri = d.rf[i], si = d.rsf[i] + pad;
+  const bool smallx = g.cols < 3, smally = g.rows < 3;
+  const int n = list_candidates(d, g, cp & 0xffff, cp >> 16, table, sub, lanes);
+  int cnt = 0;
+  for (int k0 = 0, q = 0; k0 < n; k0 += 8) {
+    const int k = k0 + sub;
+    bool hit = false;
+    unsigned e = 0u;
+    if (k < n) {
+      while (k >= table.off[q + 1]) q++;
+      const int j = table.first[q] + k - table.off[q];
+      e = (unsigned)j | table.code[q];
+      if (j != i) {
+        const float4 rj = d.rec[j];
+        float dx = ri.x - rj.x + (float)(1 - (int)((e >> 28) & 3u)) * W;
+        float dy = ri.y - rj.y + (float)(1 - (int)(e >> 30)) * H;
+        if (smallx) dx += Lxf * (float)((dx < -0.5f * Lxf) - (dx > 0.5f * Lxf));
+        if (smally) dy += Lyf * (float)((dy < -0.5f * Lyf) - (dy > 0.5f * Lyf));
+        const float lim = fmaf(si + d.rsf[j], 1.00002f, 1e-6f);
+        const float dxl = fmaf(gam, dy, dx);
+        if (fmaf(dxl, dxl, dy * dy) < lim * lim)
+          hit = capsules_within(dxl, dy, ri.z, ri.w, rj.z, rj.w,
+                                (Ri + d.rf[j] + pad) * 1.00002f + 1e-5f);
+      }
+    }
+    const unsigned all = __ballot_sync(lanes, hit) & lanes;
+    const int at = cnt + __popc(all & ((1u << (threadIdx.x & 31)) - 1u));
+    cnt += __popc(all);
+    if (hit && at < d.maxn) d.nbr[(size_t)at * d.ntot + i] = (int)e;
+  }
+  if (sub != 0) return;
+  d.nbr_n[i] = cnt;
+  if (cnt > d.maxn) atomicOr(d.status, ST_NBR_OVERFLOW);
+  if (i == g.p0) d.gbuild[s] = gam;
+}
 
 __global__ void __launch_bounds__(128, 12) k_mx_build_list(Dev d, const StepScalars* __restrict__ tab,
-                                                      int row, int all) {
-  if (!all && *d.any == 0) return;
-  for_slots(d, all != 0, [&](int i, int s) { build_list_slot(d, tab, row, i, s); });
+                                                      int row) {
+  if (*d.any == 0) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= d.ntot || d.flags[d.psys[i]] == 0) return;
+  build_list_slot(d, tab, row, i, d.psys[i]);
 }
 
 // Force-pass ordering: within each window of kOrderWindow slots, a stable sort
-// of the slots by list length; the lists are copied to their positions.  A window
-// is redone when any of its slots belongs to a system that was rebuilt.
-__device__ __forceinline__ void order_window(const Dev& d, int base, int i, bool valid) {
-  __shared__ int len[kOrderWindow];
+// of the slots by list length; the lists are copied to their positions.  One group of
+// kOrderWindow threads (w0: its first; bar: its barrier); i: this thread's slot.
+__device__ __forceinline__ void group_sync(int bar) {
+  asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(kOrderWindow) : "memory");
+}
+__device__ __forceinline__ void order_window(const Dev& d, int i, int* len, int w0, int bar) {
+  const bool valid = i < d.ntot;
+  const int in = threadIdx.x - w0;
   int c = 0x7fffffff;  // slots past the end sort last
   if (valid) c = min(d.nbr_n[i], d.maxn);
-  len[threadIdx.x] = c;
-  __syncthreads();
+  group_sync(bar);  // the group's last window is done with len, its lists are complete
+  len[in] = c;
+  group_sync(bar);
   int rank = 0;
   for (int k = 0; k < kOrderWindow; k++) {
     const int o = len[k];
-    rank += (o < c) | ((o == c) & (k < (int)threadIdx.x));
+    rank += (o < c) | ((o == c) & (k < in));
   }
   if (!valid) return;
-  const int pos = base + rank;
+  const int pos = i - in + rank;
   d.ord[pos] = i;
   d.nbr_pn[pos] = c;
   const size_t n = d.ntot;
-  for (int k = 0; k < c; k++) d.nbr_p[k * n + pos] = d.nbr[k * n + i];
+  for (int k = 0; k < c; k += 8) {  // eight loads in flight
+    int e[8];
+    for (int q = 0; q < 8; q++)
+      if (k + q < c) e[q] = d.nbr[(k + q) * n + i];
+    for (int q = 0; q < 8; q++)
+      if (k + q < c) d.nbr_p[(k + q) * n + pos] = e[q];
+  }
 }
 
-__global__ void __launch_bounds__(kOrderWindow) k_mx_order(Dev d, int all) {
-  if (!all && *d.any == 0) return;
-  const int base = blockIdx.x * kOrderWindow;
-  const int i = base + threadIdx.x;
-  const bool valid = i < d.ntot;
-  const bool mine = valid && (all || d.flags[d.psys[i]] != 0);
-  if (!__syncthreads_or(mine)) return;
-  order_window(d, base, i, valid);
-}
-
-// The list build and the force-pass ordering fused (the per-particle pass), one
-// block per window of kOrderWindow slots: the window's slots of rebuilt systems
-// build their lists, then the window is ordered and its lists copied to their
-// positions while they are still in cache.  Same lists and order as
-// k_mx_build_list followed by k_mx_order.
-__global__ void __launch_bounds__(kOrderWindow, 12) k_mx_build_order(
-    Dev d, const StepScalars* __restrict__ tab, int row, int all) {
-  if (!all && *d.any == 0) return;
-  const int base = blockIdx.x * kOrderWindow;
-  const int i = base + threadIdx.x;
-  const bool valid = i < d.ntot;
-  const int s = valid ? d.psys[i] : 0;
-  const bool mine = valid && (all || d.flags[s] != 0);
-  if (!__syncthreads_or(mine)) return;
-  if (mine) build_list_slot(d, tab, row, i, s);
-  __syncthreads();  // the window's lengths and lists are complete
-  order_window(d, base, i, valid);
+// The rebuild of the mixed form (sc_rebuild.cuh): cells, records and, for the per-particle
+// pass, the lists and their ordering (LISTS).  Large rebuilds list and order window by
+// window, a group of kOrderWindow threads each: apart, with a grid barrier between, they
+// took 202 us instead of 147 at 2^20 particles.  Small ones list with eight threads a slot.
+template <bool LISTS, int BS>
+__global__ void __launch_bounds__(BS, 1536 / BS) k_rebuild_mx(Dev d,
+                                                              const StepScalars* __restrict__ tab,
+                                                              int row, int moved) {
+  if (!rb::pending(d)) return;
+  GridBarrier bar(d.gbar + BAR_REBUILD);
+  const rb::Work<BS> work(d);
+  const bool ok = rb::sort_cells<true, BS>(
+      d, work, tab, row, moved != 0, bar,
+      [&](int i, int s, double2 p, double phi, double2 ra, double2 irc, int id, int cell) {
+        local_record(d, tab, row, i, s, p, phi, ra, irc, id, cell);
+      });
+  if (!ok || !LISTS) return;
+  const bool by_lanes = work.items <= kLaneItems;
+  if (by_lanes) {
+    __shared__ Candidates table[BS / 8];
+    const unsigned lanes = 0xffu << (threadIdx.x & 24);
+    for (int g = (blockIdx.x * BS + threadIdx.x) / 8; g < work.items; g += gridDim.x * BS / 8) {
+      int i, s;
+      if (work.at(d, g, &i, &s))
+        build_list_lanes(d, tab, row, i, s, threadIdx.x & 7, lanes, table[threadIdx.x / 8]);
+    }
+    if (!bar.wait(d.status)) return;
+  }
+  __shared__ int len[BS];
+  const int w0 = threadIdx.x / kOrderWindow * kOrderWindow, in = threadIdx.x - w0;
+  for (int g = (blockIdx.x * BS + w0) / kOrderWindow; g < work.windows;
+       g += gridDim.x * BS / kOrderWindow) {
+    const int i = work.window(d, g) * kOrderWindow + in;
+    if (!by_lanes && i < d.ntot) {
+      const int s = d.psys[i];
+      if (d.flags[s] != 0) build_list_slot(d, tab, row, i, s);
+    }
+    order_window(d, i, len + w0, w0, 1 + w0 / kOrderWindow);
+  }
+  rb::finish(d);
 }
 
 inline int nblk(int n, int b) { return (n + b - 1) / b; }
 
 }  // namespace
-
-void launch_mx_order(const Dev& d, bool all, cudaStream_t st) {
-  k_mx_order<<<nblk(d.ntot, kOrderWindow), kOrderWindow, 0, st>>>(d, all ? 1 : 0);
-}
-
-void launch_mx_build_order(const Dev& d, const StepScalars* tab, int row, bool all,
-                           cudaStream_t st) {
-  k_mx_build_order<<<nblk(d.ntot, kOrderWindow), kOrderWindow, 0, st>>>(d, tab, row,
-                                                                         all ? 1 : 0);
-}
 
 void launch_pass_mixed(const Dev& d, int mode, bool se, const StepScalars* tab, int row,
                        cudaStream_t st, int block) {
@@ -845,11 +878,9 @@ bool launch_persist_steps(const Dev& d, const StepScalars* tab, int row0, int ns
       per_sm < 1)
     return false;
   int grid = sms * per_sm;
-  const int need = (d.ntot + 127) / 128;
+  const int need = (d.ntot + 63) / 64;
   if (need < grid) grid = need;
-  Dev dd = d;
-  dd.cond = 0;  // no graph node to switch: the launch ends at a pending rebuild
-  void* args[] = {&dd, (void*)&tab, &row0, &nsteps, &out};
+  void* args[] = {(void*)&d, (void*)&tab, &row0, &nsteps, &out};
   return cudaLaunchCooperativeKernel(fn, grid, 128, args, 0, st) == cudaSuccess;
 }
 
@@ -868,32 +899,36 @@ bool launch_persist_fire(const Dev& d, const FireState& f, const StepScalars* ta
   const int need = (d.ntot + 255) / 256;
   if (need < grid) grid = need;
   Dev dd = d;
-  dd.cond = 0;
   dd.skip = f.done;  // converged systems: no force pass
   FireState ff = f;
   void* args[] = {&dd, &ff, (void*)&tab, &ftol, &dt_max, &iters, &out};
   return cudaLaunchCooperativeKernel(fn, grid, 256, args, 0, st) == cudaSuccess;
 }
 
-void launch_tile_lists(const Dev& d, bool all, cudaStream_t st) {
-  k_tile_lists<<<d.ntiles, kTileThreads, 0, st>>>(d, all ? 1 : 0);
+void launch_mx_materialize(const Dev& d, const StepScalars* tab, int row, cudaStream_t st) {
+  k_mx_materialize<<<nblk(d.ntot, 256), 256, 0, st>>>(d, tab, row);
 }
 
-void launch_mx_materialize(const Dev& d, const StepScalars* tab, int row, bool all,
-                           cudaStream_t st) {
-  if (all)
-    k_mx_materialize<<<nblk(d.ntot, 256), 256, 0, st>>>(d, tab, row, 1);
-  else
-    k_mx_materialize<<<kWalkBlocks, 256, 0, st>>>(d, tab, row, 0);
-}
-
-void launch_mx_local(const Dev& d, const StepScalars* tab, int row, bool all, cudaStream_t st) {
-  k_mx_local<<<kWalkBlocks, 256, 0, st>>>(d, tab, row, all ? 1 : 0);
-}
-
-void launch_mx_build_list(const Dev& d, const StepScalars* tab, int row, bool all,
-                          cudaStream_t st) {
-  k_mx_build_list<<<2 * kWalkBlocks, 128, 0, st>>>(d, tab, row, all ? 1 : 0);
+int launch_rebuild_mixed(const Dev& d, const StepScalars* tab, int row, bool moved,
+                         cudaStream_t st) {
+  const bool tiles = d.pass_kind == 1;
+  int mv = moved ? 1 : 0;
+  void* args[] = {(void*)&d, (void*)&tab, &row, &mv};
+  if (!tiles && d.ntot <= kSmallRebuild) {
+    const void* fn = (const void*)k_rebuild_mx<true, 128>;
+    cudaLaunchCooperativeKernel(fn, coop_blocks<2>(fn, 128, (d.ntot + 15) / 16), 128, args, 0, st);
+    return 1;
+  }
+  const void* fn = tiles ? (const void*)k_rebuild_mx<false, 512>
+                         : (const void*)k_rebuild_mx<true, 512>;
+  const int need = (d.ntot + 63) / 64;
+  const int blocks = tiles ? coop_blocks<3>(fn, 512, need) : coop_blocks<4>(fn, 512, need);
+  cudaLaunchCooperativeKernel(fn, blocks, 512, args, 0, st);
+  if (!tiles) return 1;
+  k_mx_build_list<<<nblk(d.ntot, 128), 128, 0, st>>>(d, tab, row);
+  k_tile_lists<<<d.ntiles, kTileThreads, 0, st>>>(d);
+  launch_clear_flags(d, st);
+  return 4;
 }
 
 }  // namespace sc
