@@ -291,7 +291,7 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
        h.dalloc(&d.s_id, N, "s_id") && h.dalloc(&d.s_cell, N, "s_cell");
   ok = ok && h.dalloc(&d.se_part, 5 * N, "se_part") &&
        h.dalloc(&d.se_chunk, 5 * (size_t)d.npchunks, "se_chunk") &&
-       h.dalloc(&d.se_sys, 5 * (size_t)n_sys, "se_sys");
+       h.dalloc(&d.se_sys, 5 * (size_t)n_sys, "se_sys") && h.dalloc(&d.se_done, n_sys, "se_done");
   ok = ok && h.dalloc(&pcs, d.npchunks, "pchunk") && h.dalloc(&pcp, d.npchunks, "pchunk") &&
        h.dalloc(&pcn, d.npchunks, "pchunk");
   ok = ok && h.dalloc(&d.flags, n_sys, "flags") && h.dalloc(&d.istar, n_sys, "istar") &&
@@ -365,6 +365,7 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
                                  cudaMemcpyHostToDevice, st), "upload") &&
        h.cuda_ok(cudaMemsetAsync(d.moved, 0, N * sizeof(double2), st), "memset") &&
        h.cuda_ok(cudaMemsetAsync(d.flags, 0, n_sys * sizeof(int), st), "memset") &&
+       h.cuda_ok(cudaMemsetAsync(d.se_done, 0, n_sys * sizeof(int), st), "memset") &&
        h.cuda_ok(cudaMemsetAsync(d.istar, 0x7f, n_sys * sizeof(int), st), "memset") &&
        h.cuda_ok(cudaMemsetAsync(d.any, 0, sizeof(int), st), "memset") &&
        h.cuda_ok(cudaMemsetAsync(d.status, 0, 2 * sizeof(int), st), "memset") &&

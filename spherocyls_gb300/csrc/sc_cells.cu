@@ -70,55 +70,62 @@ __global__ void k_gd_update(Dev d, const StepScalars* __restrict__ tab, int row)
   }
 }
 
-// Stress/energy: deterministic two-level reduction of the per-slot contributions.
-__global__ void k_se_chunk(Dev d) {
-  int ch = blockIdx.x;
-  int p0 = d.pchunk_p0[ch], np = d.pchunk_np[ch];
-  __shared__ double sh[5][32];
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int comp = 0; comp < 5; comp++) {
-    const double* src = d.se_part + (size_t)comp * d.ntot + p0;
-    double v = 0.0;
-    for (int k = threadIdx.x; k < np; k += blockDim.x) v += src[k];
-    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) sh[comp][w] = v;
-  }
-  __syncthreads();
-  if (w < 5) {
-    double v = lane < nw ? sh[w][lane] : 0.0;
-    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) d.se_chunk[(size_t)w * d.npchunks + ch] = v;
-  }
-}
+// Stress/energy: deterministic two-level reduction of the per-slot contributions, one
+// block per chunk and component; the block that finishes a system's last one sums its
+// chunks, each thread its strided share in order, then a fixed tree, and stores the record
+// (dst, may be null).  The sums run at the FP64 pipe's rate, so the components are on
+// different SMs.  Systems with d.skip set keep their sums.  As three kernels (chunks with
+// the components in turn, systems, records) it took 15 us at 16384 particles, here 8.
+constexpr int kSeThreads = 256;
 
-// One block per system: each thread sums its strided share of the system's chunk
-// partials in order, then a fixed tree over the block (deterministic).
-__global__ void __launch_bounds__(256) k_se_sys(Dev d) {
-  const int s = blockIdx.x;
+__global__ void __launch_bounds__(kSeThreads) k_se_reduce(Dev d, double* __restrict__ dst) {
+  constexpr int kPer = kSeChunk / kSeThreads, kWarps = kSeThreads / 32;
+  __shared__ double sh[5][kWarps];
+  __shared__ int last;
+  const int ch = blockIdx.x, comp = blockIdx.y, nc = gridDim.y;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int p0 = d.pchunk_p0[ch], np = d.pchunk_np[ch], s = d.pchunk_sys[ch];
+  if (d.skip && d.skip[s]) return;
+  double v[kPer];
+  for (int q = 0; q < kPer; q++) {
+    const int k = t + q * kSeThreads;
+    v[q] = k < np ? d.se_part[(size_t)comp * d.ntot + p0 + k] : 0.0;
+  }
+  double x = 0.0;
+  for (int q = 0; q < kPer; q++) x += v[q];
+  for (int o = 16; o; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+  if (lane == 0) sh[0][w] = x;
+  __syncthreads();
   const SysGeom& g = d.geom[s];
-  const int ch0 = g.pch0, ch1 = g.pch0 + pchunk_count(g);
-  __shared__ double sh[5][8];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int comp = 0; comp < 5; comp++) {
-    double v = 0.0;
-    for (int ch = ch0 + threadIdx.x; ch < ch1; ch += blockDim.x)
-      v += d.se_chunk[(size_t)comp * d.npchunks + ch];
-    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) sh[comp][w] = v;
+  const int nch = pchunk_count(g);
+  if (w == 0) {
+    x = lane < kWarps ? sh[0][lane] : 0.0;
+    for (int o = 16; o; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0) {
+      d.se_chunk[(size_t)comp * d.npchunks + ch] = x;
+      __threadfence();
+      last = atomicAdd(&d.se_done[s], 1) == nch * nc - 1;
+      __threadfence();
+    }
   }
   __syncthreads();
-  if (threadIdx.x < 5) {
-    double v = 0.0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); k++) v += sh[threadIdx.x][k];
-    d.se_sys[(size_t)threadIdx.x * d.nsys + s] = v;
+  if (!last) return;
+  for (int c = 0; c < nc; c++) {
+    x = 0.0;
+    for (int k = t; k < nch; k += kSeThreads)
+      x += __ldcg(&d.se_chunk[(size_t)c * d.npchunks + g.pch0 + k]);
+    if (w * 32 < nch)
+      for (int o = 16; o; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0) sh[c][w] = x;
   }
-}
-
-// se_sys is [5][nsys]; a record is [nsys][5]
-__global__ void k_se_store(Dev d, double* dst) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= d.nsys) return;
-  for (int k = 0; k < 5; k++) dst[5 * s + k] = d.se_sys[(size_t)k * d.nsys + s];
+  __syncthreads();
+  if (t < nc) {
+    x = 0.0;
+    for (int k = 0; k < kWarps; k++) x += sh[t][k];
+    d.se_sys[(size_t)t * d.nsys + s] = x;
+    if (dst) dst[5 * s + t] = x;
+  }
+  if (t == 0) d.se_done[s] = 0;
 }
 
 // set_particle's wrap loop (src/cpp/spherocyl_box.cpp:204-215) for the input state:
@@ -229,13 +236,8 @@ void launch_unsort_forces(const Dev& d, double* out, cudaStream_t st) {
   k_unsort_forces<<<nblk(d.ntot, 256), 256, 0, st>>>(d, out);
 }
 
-void launch_se_store(const Dev& d, double* dst, cudaStream_t st) {
-  k_se_store<<<nblk(d.nsys, 128), 128, 0, st>>>(d, dst);
-}
-
-void launch_se_reduce(const Dev& d, cudaStream_t st) {
-  k_se_chunk<<<d.npchunks, 256, 0, st>>>(d);
-  k_se_sys<<<d.nsys, 256, 0, st>>>(d);
+void launch_se_reduce(const Dev& d, double* dst, bool energy, cudaStream_t st) {
+  k_se_reduce<<<dim3(d.npchunks, energy ? 1 : 5), kSeThreads, 0, st>>>(d, dst);
 }
 
 }  // namespace sc

@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(kCgBlock) k_cg_begin(Dev d, CgState c, int max
                                                        unsigned long long search) {
   const int s = blockIdx.x;
   CgSys& q = c.sys[s];
+  if (threadIdx.x == 0) c.idle[s] = 1;
   if (q.done) return;  // block-uniform
   double F2 = 0, FF0 = 0, F02 = 0;
   const int ch0 = d.geom[s].pch0, ch1 = ch0 + pchunk_count(d.geom[s]);
@@ -136,6 +137,7 @@ __global__ void __launch_bounds__(kCgBlock) k_cg_begin(Dev d, CgState c, int max
   q.probes = 0;
   q.t = q.step;
   q.phase = CG_TOP;
+  c.idle[s] = 0;
   *c.searching = 1;
   if (search) cudaGraphSetConditional(search, 1u);
 }
@@ -295,7 +297,9 @@ __global__ void k_cg_search(Dev d, CgState c, unsigned long long search) {
         q.done = 1;
         q.reason = CG_PROBES;
       }
-      again = again || (!q.done && q.phase >= CG_TOP && q.phase <= CG_FINAL);
+      const bool on = !q.done && q.phase >= CG_TOP && q.phase <= CG_FINAL;
+      if (!on) c.idle[s] = 1;
+      again = again || on;
     }
   }
   // one block: the loop switch is decided once

@@ -128,8 +128,9 @@ bool HostSys::grid_changes_xy(double Lx_now, double Ly_now) const {
   return r != rows || c != cols;
 }
 
-// FP32 copies of a row, for the mixed form
+// FP32 copies of a row, for the mixed form, and the box area's reciprocal
 static void fill_f32(StepScalars& t) {
+  t.inv_area = 1.0 / (t.Lx_p * t.Ly_p);
   t.f_gamma_c = (float)t.gamma_c;
   t.f_gamma_p = (float)t.gamma_p;
   t.f_Wc = (float)t.W_c;
@@ -675,9 +676,8 @@ bool Handle::ensure_se_hist(int nrec) {
 }
 
 void Handle::enqueue_se_record(int rec) {
-  kernels += 3;
-  launch_se_reduce(d, stream);
-  launch_se_store(d, d_se_hist + (size_t)rec * nsys * 5, stream);
+  kernels += 1;
+  launch_se_reduce(d, d_se_hist + (size_t)rec * nsys * 5, false, stream);
 }
 
 // ---- protocols ----
@@ -939,7 +939,8 @@ int Handle::calc(bool se, double* se_out) {
   launch_pass(PASS_FORCE, se, 0);
   forces_valid = true;
   if (se) {
-    launch_se_reduce(d, stream);
+    launch_se_reduce(d, nullptr, false, stream);
+    kernels += 1;
     if (!cuda_ok(cudaMemcpyAsync(h_pinned + 8, d.se_sys, 5 * nsys * sizeof(double),
                                  cudaMemcpyDeviceToHost, stream),
                  "read se"))
@@ -1154,12 +1155,13 @@ bool Handle::ensure_cg() {
   if (cg.sys) return true;
   double *x0 = nullptr, *y0 = nullptr, *p0 = nullptr, *part = nullptr;
   CgSys* sys = nullptr;
-  int* searching = nullptr;
+  int *searching = nullptr, *idle = nullptr;
   if (!dalloc(&x0, ntot, "cg f0x") || !dalloc(&y0, ntot, "cg f0y") ||
       !dalloc(&p0, ntot, "cg f0p") || !dalloc(&sys, nsys, "cg sys") ||
       !dalloc(&part, 3 * (size_t)d.npchunks, "cg partials") ||
-      !dalloc(&searching, 1, "cg flag"))
+      !dalloc(&searching, 1, "cg flag") || !dalloc(&idle, nsys, "cg idle"))
     return false;
+  cg.idle = idle;
   cg.sys = sys;
   cg.part = part;
   cg.searching = searching;
@@ -1176,9 +1178,9 @@ void Handle::enqueue_cg_head(int max_iter, unsigned long long search, cudaStream
   cudaStream_t keep = stream;
   stream = st;
   launch_pass(PASS_FORCE, true, 0);
-  launch_se_reduce(d, st);
+  launch_se_reduce(d, nullptr, true, st);
   launch_cg_begin(d, cg, max_iter, search, st);
-  kernels += 5;
+  kernels += 4;
   stream = keep;
 }
 
@@ -1187,10 +1189,15 @@ void Handle::enqueue_cg_probe(unsigned long long search, cudaStream_t st) {
   cudaStream_t keep = stream;
   stream = st;
   launch_cg_probe(d, cg, st);
+  // systems that are not probing keep their energies
+  pass_skip = cg.idle;
   launch_pass(PASS_ENERGY_T, true, 0);
-  launch_se_reduce(d, st);
+  pass_skip = nullptr;
+  Dev probing = d;
+  probing.skip = cg.idle;
+  launch_se_reduce(probing, nullptr, true, st);
   launch_cg_search(d, cg, search, st);
-  kernels += 4;
+  kernels += 3;
   stream = keep;
 }
 
@@ -1222,7 +1229,12 @@ bool Handle::run_cg_graph(int max_iter) {
       if (e != cudaSuccess) break;
       enqueue_cg_head(max_iter, hs, stream);
       e = add_cond_body(
-          hs, [&](cudaStream_t st2) { enqueue_cg_probe(hs, st2); },
+          hs,
+          // several probes an iteration of the loop, which costs 12 us by itself; past the
+          // end of every search a probe's kernels find nothing to do, about 9 us
+          [&](cudaStream_t st2) {
+            for (int q = 0; q < kCgUnroll; q++) enqueue_cg_probe(hs, st2);
+          },
           cudaGraphCondTypeWhile);
       if (e != cudaSuccess) break;
       enqueue_cg_move();

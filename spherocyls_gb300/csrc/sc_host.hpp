@@ -196,6 +196,7 @@ struct Handle {
   // Polak-Ribiere conjugate gradient with the reference's line search
   CgState cg{};
   static constexpr int kCgChunk = 10;  // iterations per captured graph
+  static constexpr int kCgUnroll = 4;  // probes per iteration of the line search's loop
   cudaGraphExec_t cg_exec = nullptr;
   int cg_key_iter = -1;
   bool ensure_cg();

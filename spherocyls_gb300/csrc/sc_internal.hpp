@@ -94,6 +94,7 @@ struct StepScalars {
   double rate;       // strain rate
   double step;       // integration step
   double scale;      // resize factor pow(1-rate, dt)
+  double inv_area;   // 1 / (Lx_p Ly_p)
   int mode;          // 0 none, 1 multiply by scale (shrink), 2 divide by scale (grow),
                      // 3 pure shear (x stretched and y compressed at the strain rate)
   int setback;       // set back gamma at the end of this step
@@ -146,6 +147,7 @@ struct CgState {
   CgSys* sys;      // [nsys]
   double* part;    // [3 * npchunks] chunk partials of |F|^2, F.F0, |F0|^2
   int* searching;  // any system probing (for the host-driven loop)
+  int* idle;       // [nsys] systems that are not probing (Dev::skip of the probes' passes)
   int max_probes;  // a line search that needs more probes ends the system (CG_PROBES)
 };
 
@@ -249,6 +251,7 @@ struct Dev {
   double* se_part;          // [5][ntot]
   double* se_chunk;         // [5][npchunks]
   double* se_sys;           // [5][nsys]
+  int* se_done;             // [nsys] chunks of a system summed so far (zero between uses)
   const int* pchunk_sys;    // particle chunks for reductions
   const int* pchunk_p0;
   const int* pchunk_np;
@@ -334,9 +337,10 @@ int launch_rebuild_mixed(const Dev& d, const StepScalars* tab, int row, bool mov
                          cudaStream_t st);
 void launch_force_rebuild_all(const Dev& d, cudaStream_t st);
 void launch_clear_flags(const Dev& d, cudaStream_t st);
-void launch_se_reduce(const Dev& d, cudaStream_t st);
+// per-system sums of the stress/energy partials into se_sys and, when given, dst
+// ([nsys][5]); energy: the first of the five alone (no dst)
+void launch_se_reduce(const Dev& d, double* dst, bool energy, cudaStream_t st);
 void launch_gd_update(const Dev& d, bool mixed, const StepScalars* tab, int row, cudaStream_t st);
-void launch_se_store(const Dev& d, double* dst, cudaStream_t st);
 // per-slot values back to input order: out[k * ntot + input index] (k = 0, 1, 2)
 void launch_unsort_state(const Dev& d, double* out, cudaStream_t st);
 void launch_cg_reset(const Dev& d, const CgState& c, cudaStream_t st);

@@ -787,160 +787,115 @@ __global__ void k_mx_se_prep(Dev d) {
   if (i >= d.ntot) return;
   const float4 r = d.rec[i];
   const float4 c = d.mc[i];
-  const double phi = (double)c.z + (double)c.w;
+  const double phi = widen(c.z) + widen(c.w);
   const double A = d.ra[i].y;
   double sn, cs;
   sincos(phi, &sn, &cs);
-  d.xy_t[i] = make_double2((double)r.x + (double)c.x, (double)r.y + (double)c.y);
+  d.xy_t[i] = make_double2(widen(r.x) + widen(c.x), widen(r.y) + widen(c.y));
   d.nxy_t[i] = make_double2(A * cs, A * sn);
 }
 
-// The mixed form's FP64 stress and energy of the state, one block per 128 slots.
-// Each pair is taken once, from its lower particle index, over the mixed list
-// (entries: slot | cell offset code), with the state's scalars (the _p fields).
-// Phase 1: each thread marks, in windows of 64 list entries, the entries it owns
-// that pass an FP32 screen (a conservative bound on the segment distance, see
-// may_touch_fp32).  Phase 2: the block evaluates the marked pairs 128 at a time,
-// one per thread whatever the lane owning it, in FP64 with shared reciprocals
-// (FAST: this stress is the mixed form's, checked against the FP64 form to 1e-9, not
-// the reference's rounding).  Phase 3: each owner adds the results of its own pairs
-// in list order.  The sums are those of a per-slot loop over the list, and
-// deterministic; the FP64 work runs on full warps instead of the lanes that happen
-// to own a touching pair.
-constexpr int kSeBlock = 128;
-
-// position of set bit r (0-based, counted from bit 0) of m; m has more than r bits set
-__device__ __forceinline__ int nth_set_bit64(unsigned long long m, int r) {
-  for (int q = 0; q < r; q++) m &= m - 1ull;
-  return __ffsll((long long)m) - 1;
-}
-
-template <bool TWO>
-__global__ void __launch_bounds__(kSeBlock) k_mx_se64(Dev d, const StepScalars* __restrict__ tab,
-                                                     int row) {
-  // the owners' particle data and system scalars, for whichever thread evaluates
-  // their pairs
-  __shared__ double o_px[kSeBlock], o_py[kSeBlock], o_nx[kSeBlock], o_ny[kSeBlock];
-  __shared__ double o_R[kSeBlock], o_A[kSeBlock];
-  __shared__ double o_W[kSeBlock], o_H[kSeBlock], o_gam[kSeBlock], o_Lx[kSeBlock],
-      o_Ly[kSeBlock], o_iLL[kSeBlock], o_2n[kSeBlock], o_i2n[kSeBlock];
-  __shared__ unsigned long long mask[kSeBlock];
-  __shared__ int off[kSeBlock + 1];
-  __shared__ int sh_scan[kSeBlock / 32];
-  __shared__ double res[5][kSeBlock];
-  const int t = threadIdx.x;
-  const int i = blockIdx.x * kSeBlock + t;
+// The mixed form's FP64 stress and energy of the state, one block per window of
+// kPairBlock / TPS slots, in the phases of k_pairs64: TPS threads per slot screen the mixed
+// list (entries: slot | cell offset code) with the FP32 records and mark the pairs that
+// the slot owns (its index is the lower one) and that may touch; one thread a pair evaluates
+// them, 128 at a time, in FP64 with shared reciprocals (FAST: this stress is the mixed
+// form's, checked against the FP64 form to 1e-9, not the reference's rounding); each
+// owner adds the results of its own pairs in list order, so the sums are deterministic.
+// Systems whose grid has under three cells a side evaluate every pair they own: their
+// image is chosen in FP64.
+// With the screen's displacements in FP64 and one thread a slot it took 35 us at 16384
+// particles and 942 us at 2^20; now 18 and 446.
+template <bool TWO, int TPS>
+__global__ void __launch_bounds__(kPairBlock) k_mx_se64(Dev d, const StepScalars* __restrict__ tab,
+                                                       int row) {
+  constexpr int S = kPairBlock / TPS;
+  __shared__ unsigned short job[S * 64];  // slot in the window << 6 | entry of the 64
+  __shared__ int wsum[kPairBlock / 32];
+  __shared__ int longest;
+  __shared__ double res[5][kPairBlock];
+  const int t = threadIdx.x, l = t / TPS, sub = t % TPS;
+  const int i0 = blockIdx.x * S, i = i0 + l;
   const bool valid = i < d.ntot;
-  const bool virial = d.stress_mode == STRESS_VIRIAL;
+  const size_t ntot = d.ntot;
   int cnt = 0, idi = 0;
-  float fnx = 0.f, fny = 0.f;
-  double px = 0, py = 0, Lx = 1, Ly = 1, gamma = 0, W = 0, H = 0, Ri = 0;
+  float4 ri = make_float4(0.f, 0.f, 0.f, 0.f);
+  float Ri = 0.f, W = 0.f, H = 0.f, gam = 0.f;
+  bool small = false;
   if (valid) {
     const int s = d.psys[i];
     const SysGeom& g = d.geom[s];
     const StepScalars& ts = tab[row * d.nsys + s];
-    W = ts.W_p;
-    H = ts.H_p;
-    gamma = ts.gamma_p;
-    Lx = ts.Lx_p;
-    Ly = ts.Ly_p;
-    const double2 pi = d.xy_t[i], ni = d.nxy_t[i], rai = d.ra[i];
-    px = pi.x;
-    py = pi.y;
-    Ri = rai.x;
-    o_px[t] = pi.x;
-    o_py[t] = pi.y;
-    o_nx[t] = ni.x;
-    o_ny[t] = ni.y;
-    o_R[t] = rai.x;
-    o_A[t] = rai.y;
-    o_W[t] = W;
-    o_H[t] = H;
-    o_gam[t] = gamma;
-    o_Lx[t] = Lx;
-    o_Ly[t] = Ly;
-    o_iLL[t] = 1.0 / (Lx * Ly);
-    o_2n[t] = 2.0 * g.n;
-    o_i2n[t] = 0.5 * g.inv_n;
-    fnx = (float)ni.x;
-    fny = (float)ni.y;
+    W = ts.f_Wp;
+    H = ts.f_Hp;
+    gam = ts.f_gamma_p;
+    small = g.cols < 3 || g.rows < 3;
+    ri = d.rec[i];
+    Ri = d.rf[i];
     idi = d.id[i];
     cnt = min(d.nbr_n[i], d.maxn);
   }
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  // the block's longest list sets the number of 64-entry windows
-  int kmax = cnt;
-  for (int o = 16; o; o >>= 1) kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
-  if ((t & 31) == 0) sh_scan[t >> 5] = kmax;
+  if (t == 0) longest = 0;
   __syncthreads();
-  kmax = 0;
-  for (int w = 0; w < kSeBlock / 32; w++) kmax = max(kmax, sh_scan[w]);
-  for (int k0 = 0; k0 < kmax; k0 += 64) {
-    // phase 1: this window's owned entries that may touch
+  if (cnt > 64) atomicMax(&longest, cnt);  // more than one window of 64 entries: rare
+  for (int k0 = 0;; k0 += 64) {
     unsigned long long m = 0ull;
     const int kend = min(cnt, k0 + 64);
-    for (int k = k0; k < kend; k++) {
-      const unsigned e = (unsigned)d.nbr[(size_t)k * d.ntot + i];
+    for (int k = k0 + sub; k < kend; k += TPS) {
+      const unsigned e = (unsigned)d.nbr[k * ntot + i];
       const int j = (int)(e & kSlotMask);
       if (!(idi < d.id[j])) continue;
-      const double2 pj = d.xy_t[j];
-      const double2 nj = d.nxy_t[j];
-      const double Rj = d.ra[j].x;
-      double sx = (px - pj.x) + (double)(1 - (int)((e >> 28) & 3u)) * W;
-      double sy = (py - pj.y) + (double)(1 - (int)(e >> 30)) * H;
-      sx += Lx * (double)((sx < -0.5 * Lx) - (sx > 0.5 * Lx));
-      sy += Ly * (double)((sy < -0.5 * Ly) - (sy > 0.5 * Ly));
-      sx += gamma * sy;
-      if (may_touch_fp32((float)sx, (float)sy, fnx, fny, (float)nj.x, (float)nj.y,
-                         (float)(Ri + Rj)))
+      const float4 rj = d.rec[j];
+      const float dx = ri.x - rj.x + (float)(1 - (int)((e >> 28) & 3u)) * W;
+      const float dy = ri.y - rj.y + (float)(1 - (int)(e >> 30)) * H;
+      if (small || may_touch_fp32(fmaf(gam, dy, dx), dy, ri.z, ri.w, rj.z, rj.w, Ri + d.rf[j]))
         m |= 1ull << (k - k0);
     }
-    mask[t] = m;
-    const int c = __popcll(m);
-    // exclusive scan of the counts over the block
+    for (int o = 1; o < TPS; o <<= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
+    // exclusive scan of the slots' job counts over the block
+    const int c = sub == 0 ? __popcll(m) : 0;
     int v = c;
     for (int o = 1; o < 32; o <<= 1) {
       const int u = __shfl_up_sync(0xffffffffu, v, o);
       if ((t & 31) >= o) v += u;
     }
-    __syncthreads();  // sh_scan is free again
-    if ((t & 31) == 31) sh_scan[t >> 5] = v;
+    if ((t & 31) == 31) wsum[t >> 5] = v;
     __syncthreads();
-    int base_w = 0;
-    for (int w = 0; w < (t >> 5); w++) base_w += sh_scan[w];
-    off[t] = base_w + v - c;
-    int total = 0;
-    for (int w = 0; w < kSeBlock / 32; w++) total += sh_scan[w];
-    if (t == 0) off[kSeBlock] = total;
+    int off = v - c, total = 0;
+    for (int w = 0; w < kPairBlock / 32; w++) {
+      if (w < (t >> 5)) off += wsum[w];
+      total += wsum[w];
+    }
+    if (sub == 0) {
+      int q = off;
+      for (unsigned long long b = m; b; b &= b - 1ull)
+        job[q++] = (unsigned short)(l << 6 | (__ffsll((long long)b) - 1));
+    }
     __syncthreads();
-    // phases 2 and 3, 128 pairs at a time
-    for (int b0 = 0; b0 < total; b0 += kSeBlock) {
+    for (int b0 = 0; b0 < total; b0 += kPairBlock) {
       const int p = b0 + t;
       if (p < total) {
-        // the owner: the last thread whose offset is at most p
-        int lo = 0, hi = kSeBlock - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (off[mid] <= p) lo = mid; else hi = mid - 1;
-        }
-        const int o = lo;
-        const int k = k0 + nth_set_bit64(mask[o], p - off[o]);
-        const int io = blockIdx.x * kSeBlock + o;
-        const unsigned e = (unsigned)d.nbr[(size_t)k * d.ntot + io];
+        const int io = i0 + (job[p] >> 6), k = k0 + (job[p] & 63);
+        const unsigned e = (unsigned)d.nbr[k * ntot + io];
         const int j = (int)(e & kSlotMask);
-        const double2 pj = d.xy_t[j];
-        const double2 nj = d.nxy_t[j];
-        const double2 raj = d.ra[j];
-        const double dX = (o_px[o] - pj.x) + (double)(1 - (int)((e >> 28) & 3u)) * o_W[o];
-        const double dY = (o_py[o] - pj.y) + (double)(1 - (int)(e >> 30)) * o_H[o];
+        const int s = d.psys[io];
+        const SysGeom& g = d.geom[s];
+        const StepScalars& ts = tab[row * d.nsys + s];
+        const double2 pi = d.xy_t[io], pj = d.xy_t[j], ni = d.nxy_t[io], nj = d.nxy_t[j];
+        const double2 rai = d.ra[io], raj = d.ra[j];
+        const double dX = (pi.x - pj.x) + (double)(1 - (int)((e >> 28) & 3u)) * ts.W_p;
+        const double dY = (pi.y - pj.y) + (double)(1 - (int)(e >> 30)) * ts.H_p;
+        const double two_n = 2.0 * g.n, i2n = 0.5 * g.inv_n;
         PairF64 r;
         const bool hit =
-            TWO ? pair2_fp64<true, true>(dX, dY, o_nx[o], o_ny[o], o_A[o], nj.x, nj.y, raj.y,
-                                         o_R[o] + raj.x, o_gam[o], o_Lx[o], o_Ly[o], o_2n[o], r,
-                                         0.0, 0.0, o_iLL[o], o_i2n[o])
-                : pair_fp64<true, true>(dX, dY, o_nx[o], o_ny[o], o_A[o], nj.x, nj.y, raj.y,
-                                        o_R[o] + raj.x, o_gam[o], o_Lx[o], o_Ly[o], virial,
-                                        o_2n[o], r, 0.0, 0.0, o_iLL[o], o_i2n[o]);
+            TWO ? pair2_fp64<true, true>(dX, dY, ni.x, ni.y, rai.y, nj.x, nj.y, raj.y,
+                                         rai.x + raj.x, ts.gamma_p, ts.Lx_p, ts.Ly_p, two_n, r,
+                                         0.0, 0.0, ts.inv_area, i2n)
+                : pair_fp64<true, true>(dX, dY, ni.x, ni.y, rai.y, nj.x, nj.y, raj.y,
+                                        rai.x + raj.x, ts.gamma_p, ts.Lx_p, ts.Ly_p,
+                                        d.stress_mode == STRESS_VIRIAL, two_n, r, 0.0, 0.0,
+                                        ts.inv_area, i2n);
         res[0][t] = hit ? r.e : 0.0;
         res[1][t] = hit ? r.pxx : 0.0;
         res[2][t] = hit ? r.pyy : 0.0;
@@ -949,15 +904,17 @@ __global__ void __launch_bounds__(kSeBlock) k_mx_se64(Dev d, const StepScalars* 
       }
       __syncthreads();
       // each owner adds its pairs of this batch, in list order (a pair that does
-      // not touch adds zeros, as the per-slot loop skipped it)
-      const int q0 = max(off[t], b0), q1 = min(off[t] + c, b0 + kSeBlock);
+      // not touch adds zeros)
+      const int q0 = max(off, b0), q1 = min(off + c, b0 + kPairBlock);
       for (int q = q0; q < q1; q++)
         for (int comp = 0; comp < 5; comp++) acc[comp] += res[comp][q - b0];
       __syncthreads();
     }
+    __syncthreads();  // longest is complete, the jobs are done with
+    if (k0 + 64 >= longest) break;
   }
-  if (valid)
-    for (int comp = 0; comp < 5; comp++) d.se_part[(size_t)comp * d.ntot + i] = acc[comp];
+  if (valid && sub == 0)
+    for (int comp = 0; comp < 5; comp++) d.se_part[comp * ntot + i] = acc[comp];
 }
 
 template <int MODE, bool SE, bool FAST = false>
@@ -1063,13 +1020,22 @@ int launch_pass_fp64(const Dev& d, int mode, bool se, const StepScalars* tab, in
   return 0;
 }
 
-void launch_mx_se64(const Dev& d, const StepScalars* tab, int row, cudaStream_t st) {
-  const int grid = (d.ntot + kSeBlock - 1) / kSeBlock;
-  k_mx_se_prep<<<grid, kSeBlock, 0, st>>>(d);
+template <int TPS>
+static void launch_mx_se64_of(const Dev& d, const StepScalars* tab, int row, cudaStream_t st) {
+  const int grid = (d.ntot + kPairBlock / TPS - 1) / (kPairBlock / TPS);
   if (d.contact_model == 1)
-    k_mx_se64<true><<<grid, kSeBlock, 0, st>>>(d, tab, row);
+    k_mx_se64<true, TPS><<<grid, kPairBlock, 0, st>>>(d, tab, row);
   else
-    k_mx_se64<false><<<grid, kSeBlock, 0, st>>>(d, tab, row);
+    k_mx_se64<false, TPS><<<grid, kPairBlock, 0, st>>>(d, tab, row);
+}
+
+void launch_mx_se64(const Dev& d, const StepScalars* tab, int row, cudaStream_t st) {
+  k_mx_se_prep<<<(d.ntot + 127) / 128, 128, 0, st>>>(d);
+  switch (kPairBlock / pair_window(d.ntot)) {
+    case 1: launch_mx_se64_of<1>(d, tab, row, st); break;
+    case 4: launch_mx_se64_of<4>(d, tab, row, st); break;
+    case 16: launch_mx_se64_of<16>(d, tab, row, st); break;
+  }
 }
 
 int launch_rebuild_fp64(const Dev& d, const StepScalars* tab, int row, bool moved,
