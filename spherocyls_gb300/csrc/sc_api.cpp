@@ -254,7 +254,16 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
   d.npchunks = (int)pchunk_sys.size();
   bool ok = true;
   sc::SysGeom* geom = nullptr;
-  int *psys = nullptr, *pcs = nullptr, *pcp = nullptr, *pcn = nullptr;
+  int *psys = nullptr, *pcs = nullptr, *pcp = nullptr, *pcn = nullptr, *wsys = nullptr;
+  std::vector<int> win_sys((N + sc::kOrderWindow - 1) / sc::kOrderWindow, -1);
+  for (int s = 0; s < n_sys; s++) {
+    const sc::HostSys& S = h.hs[s];
+    const int last = S.p0 + S.n;
+    for (int w = (S.p0 + sc::kOrderWindow - 1) / sc::kOrderWindow;
+         w < (int)win_sys.size() && std::min((w + 1) * sc::kOrderWindow, ntot) <= last; w++)
+      win_sys[w] = s;
+  }
+  ok = ok && h.dalloc(&wsys, win_sys.size(), "window systems");
   ok = ok && h.dalloc(&geom, n_sys, "geom") && h.dalloc(&psys, N, "psys");
   ok = ok && h.dalloc(&d.xy, N, "xy") && h.dalloc(&d.ph, N, "ph") && h.dalloc(&d.ra, N, "ra") &&
        h.dalloc(&d.irc, N, "irc") && h.dalloc(&d.id, N, "id") && h.dalloc(&d.cell, N, "cell");
@@ -266,11 +275,10 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
   ok = ok && h.dalloc(&d.rec, N, "rec") && h.dalloc(&d.rec_t, N, "rec_t") &&
        h.dalloc(&d.rf, N, "rf") && h.dalloc(&d.rsf, N, "rsf");
   if (h.prec == sc::PREC_MIXED)
-    ok = ok && h.dalloc(&d.mc, N, "mc") && h.dalloc(&d.mv, N, "mv") && h.dalloc(&d.mm, N, "mm") &&
-         h.dalloc(&d.pa, N, "pa") && h.dalloc(&d.rcf, N, "rcf") &&
+    ok = ok && h.dalloc(&d.mc, N, "mc") && h.dalloc(&d.mv, N, "mv") && h.dalloc(&d.mvp, N, "mvp") && h.dalloc(&d.mvr, N, "mvr") && h.dalloc(&d.mm, N, "mm") &&
+         h.dalloc(&d.mph, N, "mph") && h.dalloc(&d.pa, N, "pa") &&
          h.dalloc(&d.cellp, N, "cellp") && h.dalloc(&d.gbuild, n_sys, "gbuild") &&
-         h.dalloc(&d.ord, N, "ord") && h.dalloc(&d.nbr_p, N * d.maxn, "nbr_p") &&
-         h.dalloc(&d.nbr_pn, N, "nbr_pn");
+         h.dalloc(&d.ord, N, "ord") && h.dalloc(&d.nbr_p, N * d.maxn, "nbr_p");
   else
     ok = ok && h.dalloc(&d.iaa, N, "iaa") &&
          h.dalloc(&d.s_mv, N, "s_mv") && h.dalloc(&d.s_nxy, N, "s_nxy");
@@ -316,6 +324,7 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
   }
   d.geom = geom;
   d.psys = psys;
+  d.wsys = wsys;
   d.pchunk_sys = pcs;
   d.pchunk_p0 = pcp;
   d.pchunk_np = pcn;
@@ -362,6 +371,8 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
        h.cuda_ok(cudaMemcpyAsync(pcp, pchunk_p0.data(), d.npchunks * sizeof(int),
                                  cudaMemcpyHostToDevice, st), "upload") &&
        h.cuda_ok(cudaMemcpyAsync(pcn, pchunk_np.data(), d.npchunks * sizeof(int),
+                                 cudaMemcpyHostToDevice, st), "upload") &&
+       h.cuda_ok(cudaMemcpyAsync(wsys, win_sys.data(), win_sys.size() * sizeof(int),
                                  cudaMemcpyHostToDevice, st), "upload") &&
        h.cuda_ok(cudaMemsetAsync(d.moved, 0, N * sizeof(double2), st), "memset") &&
        h.cuda_ok(cudaMemsetAsync(d.flags, 0, n_sys * sizeof(int), st), "memset") &&

@@ -169,7 +169,7 @@ __device__ __forceinline__ void fire_update(const Dev& d, const FireState& f, in
   if (q.done) return;
   const SysGeom& g = d.geom[s];
   if (MIXED) {
-    const float4 pa = d.pa[i];  // (R, A, index bits, 1/I)
+    const float4 pa = d.pa[i];  // (R, A, RC, 1/I)
     const float A = pa.y;
     const float fx = (float)d.fx[i], fy = (float)d.fy[i], ap = (float)d.tau[i] * pa.w;
     float vx = (float)f.vx[i], vy = (float)f.vy[i], vp = (float)f.vp[i];
@@ -199,7 +199,7 @@ __device__ __forceinline__ void fire_update(const Dev& d, const FireState& f, in
     r.w = A * sn;
     d.rec[i] = r;
     d.mc[i] = c;
-    float4 m = d.mm[i];
+    float2 m = d.mm[i];
     m.x += ddx;
     m.y += ddy;
     d.mm[i] = m;
@@ -207,7 +207,7 @@ __device__ __forceinline__ void fire_update(const Dev& d, const FireState& f, in
     // (centre plus A times the rotation) and the next step's allowance within half
     // the padding
     float dd = sqrtf(fmaf(ddx, ddx, ddy * ddy)) + A * fabsf(ddp);
-    float moved = sqrtf(m.x * m.x + m.y * m.y) + A * fabsf((c.z + c.w) - m.z);
+    float moved = sqrtf(m.x * m.x + m.y * m.y) + A * fabsf((c.z + c.w) - d.mph[i]);
     if (!(moved + dd < 0.5f * g.fpad)) {
       if (d.flags[s] == 0) atomicOr(&d.flags[s], 1);
       if (*d.any == 0) atomicExch(d.any, 1);

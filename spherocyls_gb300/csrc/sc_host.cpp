@@ -253,6 +253,8 @@ bool Handle::layout_cells() {
   d.ntiles = ntiles;
   d.ncells = ncells;
   d.nchunks = nchunks;
+  d.small_grid = 0;
+  for (const HostSys& h : hs) d.small_grid |= h.cols < 3 || h.rows < 3;
   invalidate_graph();  // captured kernels hold the old layout
   std::vector<SysGeom> g(nsys);
   int pch = 0;

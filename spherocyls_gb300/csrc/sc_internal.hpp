@@ -159,6 +159,7 @@ struct Dev {
   int contact_model;        // 0 one contact point (src/cpp), 1 two points (src/cuda 2p)
   const SysGeom* geom;      // [nsys]
   const int* psys;          // [ntot] system of each slot
+  const int* wsys;          // system of each window of kOrderWindow slots, -1: several
   const int* cell_sys;      // [ncells] system of each cell
   // state
   double2* xy;
@@ -185,10 +186,12 @@ struct Dev {
   float4* rec;    // (x_local, y_local, A cos phi, A sin phi) of the state
   float4* rec_t;  // the same for the predictor copy
   float4* mc;     // (x compensation, y compensation, phi, phi compensation)
-  float4* mv;     // (v0x, v0y, v0phi, predicted phi)
-  float4* mm;     // (x, y displacement since the last rebuild, angle at it, unused)
-  float4* pa;     // (R, A, particle index as int bits, 1/I)
-  float* rcf;     // isolated-rotation coefficient RC
+  float2* mv;     // v0x, v0y of the predictor
+  float* mvp;     // v0phi of the predictor
+  float* mvr;     // pure shear: the flow's rotation rate at the predictor
+  float2* mm;     // x, y displacement since the last rebuild
+  float* mph;     // angle at the last rebuild
+  float4* pa;     // (R, A, isolated-rotation coefficient RC, 1/I)
   float* rf;      // R in FP32: the only per-neighbour constant the force pass gathers
   double* iaa;    // 1 / A^2 (FP64 form: shared_rcp, sc_pair.cuh)
   float* rsf;     // R + A in FP32: the list build's reach
@@ -211,9 +214,8 @@ struct Dev {
   // mixed form: the same lists reordered for the force pass.  Within each window
   // of kOrderWindow slots, threads take the slots in order of increasing list
   // length, so a warp's lanes loop over lists of nearly equal length.
-  int* ord;     // [ntot] position -> slot
-  int* nbr_p;   // column-major [k * ntot + position]
-  int* nbr_pn;  // [ntot] list length at each position (capped at maxn)
+  unsigned* ord;  // [ntot] position -> slot in the window | list length << 7 (capped at maxn)
+  int* nbr_p;     // column-major [k * ntot + position]
   // mixed form, tile force pass (pass_kind 1): each tile's pairs once.  The tile's
   // compute entries (owner-major) and read entries live in the slot range of its
   // particles times kTileEPP; a pair inside the tile is computed by its lower slot
@@ -221,6 +223,7 @@ struct Dev {
   unsigned long long* gbar; // [BAR_WORDS] counters of the cooperative kernels
   const int* skip;          // [nsys] or null: force passes leave systems with skip[s] != 0
                             // alone (converged minimiser systems)
+  int small_grid;           // some system's grid has fewer than three cells a side
   int pass_kind;            // 0: one thread per particle over its full list, 1: tiles
   int ntiles;
   const int4* tiles;        // [ntiles] (system, first global cell, cells, 0)
@@ -282,7 +285,7 @@ constexpr int kSeChunk = 1024;    // particles per reduction chunk
 // a system's particle-reduction chunks: [pch0, pch0 + pchunk_count), in slot order
 SC_HDI int pchunk_count(const SysGeom& g) { return (g.n + kSeChunk - 1) / kSeChunk; }
 constexpr int kNoTrigger = 0x7f7f7f7f;  // istar value when no particle triggered
-constexpr int kOrderWindow = 128;  // slots per window of the force-pass ordering
+constexpr int kOrderWindow = 128;  // slots per window of the force-pass ordering (Dev::ord)
 // mixed-form list entries: slot in the low 28 bits, cell offset (dc+1, dr+1) above
 constexpr int kSlotBits = 28;
 constexpr unsigned kSlotMask = (1u << kSlotBits) - 1u;

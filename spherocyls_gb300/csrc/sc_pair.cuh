@@ -226,6 +226,26 @@ __device__ __forceinline__ bool pair_fp64(double dX, double dY, double nxA, doub
   return true;
 }
 
+// Approximate quotient, reciprocal and reciprocal square root of normal numbers: those of
+// __fdividef and rsqrtf without the scaling around subnormal operands, about a dozen
+// instructions a pair.
+__device__ __forceinline__ float rcp_fast(float y) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return r;
+}
+__device__ __forceinline__ float div_fast(float x, float y) { return x * rcp_fast(y); }
+__device__ __forceinline__ float rsqrt_fast(float y) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return r;
+}
+// Cell offset 1 - code of a mixed list entry as a float: code is the low two bits of c.
+// (8388608 + code is exact; a conversion would take the slow pipe)
+__device__ __forceinline__ float cell_offset(unsigned c) {
+  return 8388609.f - __uint_as_float(0x4b000000u | (c & 3u));
+}
+
 struct PairF32 {
   float fx, fy, tp, tq;
   float ov;                      // overlap 1 - d/sigma
@@ -251,17 +271,17 @@ __device__ __forceinline__ bool pair_fp32(float dX, float dY, float nxA, float n
   float uxv = fmaf(nxA, nyB, -w) + fmaf(-nyA, nxB, w);  // cross(u_A, u_B), error-compensated
   float w2 = nyA * dX;
   float uxD = fmaf(nxA, dY, -w2) + fmaf(-nyA, dX, w2);  // cross(u_A, D)
-  float t = uxv == 0.f ? -1.f : fminf(fmaxf(__fdividef(uxD, uxv), -1.f), 1.f);
-  float s = -__fdividef(b * t + d, a);
+  float t = uxv == 0.f ? -1.f : fminf(fmaxf(div_fast(uxD, uxv), -1.f), 1.f);
+  float s = -div_fast(b * t + d, a);
   float sarg = fabsf(s);
   s = fminf(fmaxf(s, -1.f), 1.f);
-  if (sarg > 1.f) t = fminf(fmaxf(-__fdividef(b * s + e, c), -1.f), 1.f);
+  if (sarg > 1.f) t = fminf(fmaxf(-div_fast(b * s + e, c), -1.f), 1.f);
   float dDx = dX + s * nxA - t * nxB;
   float dDy = dY + s * nyA - t * nyB;
   float dsq = dDx * dDx + dDy * dDy;
   if (!(dsq < sig * sig)) return false;
-  float inv_d = rsqrtf(dsq);
-  float inv_sig = __fdividef(1.f, sig);
+  float inv_d = rsqrt_fast(dsq);
+  float inv_sig = rcp_fast(sig);
   float ov = 1.f - dsq * inv_d * inv_sig;   // 1 - d/sigma
   float f = ov * inv_sig * inv_d;           // (1 - d/sigma)/(sigma d)
   float Fx = dDx * f, Fy = dDy * f;
@@ -523,8 +543,8 @@ __device__ __forceinline__ bool contact_fp32(float dX, float dY, float s, float 
   float dDy = dY + s * nyA - t * nyB;
   float dsq = dDx * dDx + dDy * dDy;
   if (!(dsq < sig * sig)) return false;
-  float inv_d = rsqrtf(dsq);
-  float inv_sig = __fdividef(1.f, sig);
+  float inv_d = rsqrt_fast(dsq);
+  float inv_sig = rcp_fast(sig);
   float ov = 1.f - dsq * inv_d * inv_sig;
   float f = ov * inv_sig * inv_d;
   float Fx = dDx * f, Fy = dDy * f;
@@ -558,55 +578,55 @@ __device__ __forceinline__ bool pair2_fp32(float dX, float dY, float nxA, float 
   float s1, t1, s2, t2, s3, t3;
   auto cl = [](float v) { return fminf(fmaxf(v, -1.f), 1.f); };
   if (uxv == 0.f) {
-    s1 = cl(-__fdividef(b + d, a));
-    s2 = cl(-__fdividef(d - b, a));
+    s1 = cl(-div_fast(b + d, a));
+    s2 = cl(-div_fast(d - b, a));
     if (fabsf(s1) == 1.f)
-      t1 = cl(-__fdividef(b * s1 + e, c));
+      t1 = cl(-div_fast(b * s1 + e, c));
     else
-      t1 = cl(b < 0.f ? -__fdividef(b + e, c) : -__fdividef(e - b, c));
+      t1 = cl(b < 0.f ? -div_fast(b + e, c) : -div_fast(e - b, c));
     if (fabsf(s2) == 1.f)
-      t2 = cl(-__fdividef(b * s2 + e, c));
+      t2 = cl(-div_fast(b * s2 + e, c));
     else
-      t2 = cl(b < 0.f ? -__fdividef(e - b, c) : -__fdividef(b + e, c));
+      t2 = cl(b < 0.f ? -div_fast(e - b, c) : -div_fast(b + e, c));
     s3 = s2;
     t3 = t2;
   } else {
-    t1 = cl(__fdividef(uxD, uxv));
-    s1 = -__fdividef(b * t1 + d, a);
+    t1 = cl(div_fast(uxD, uxv));
+    s1 = -div_fast(b * t1 + d, a);
     float sarg = fabsf(s1);
     s1 = cl(s1);
     if (sarg >= 1.f) {
-      t1 = cl(-__fdividef(b * s1 + e, c));
+      t1 = cl(-div_fast(b * s1 + e, c));
       s2 = -s1;
-      t2 = -__fdividef(b * s2 + e, c);
+      t2 = -div_fast(b * s2 + e, c);
       float targ = fabsf(t2);
       t2 = cl(t2);
       if (targ > 1.f) {
-        s2 = cl(-__fdividef(b * t2 + d, a));
+        s2 = cl(-div_fast(b * t2 + d, a));
         s3 = s2;
         t3 = t2;
       } else {
         t3 = b < 0.f ? -s1 : s1;
-        s3 = -__fdividef(b * t3 + d, a);
+        s3 = -div_fast(b * t3 + d, a);
         sarg = fabsf(s3);
         s3 = cl(s3);
-        if (sarg >= 1.f) t3 = cl(-__fdividef(b * s3 + e, c));
+        if (sarg >= 1.f) t3 = cl(-div_fast(b * s3 + e, c));
       }
     } else {
       t2 = -t1;
-      s2 = -__fdividef(b * t2 + d, a);
+      s2 = -div_fast(b * t2 + d, a);
       sarg = fabsf(s2);
       s2 = cl(s2);
       if (sarg > 1.f) {
-        t2 = cl(-__fdividef(b * s2 + e, c));
+        t2 = cl(-div_fast(b * s2 + e, c));
         s3 = s2;
         t3 = t2;
       } else {
         s3 = b < 0.f ? -t1 : t1;
-        t3 = -__fdividef(b * s3 + e, c);
+        t3 = -div_fast(b * s3 + e, c);
         float targ = fabsf(t3);
         t3 = cl(t3);
-        if (targ >= 1.f) s3 = cl(-__fdividef(b * t3 + d, a));
+        if (targ >= 1.f) s3 = cl(-div_fast(b * t3 + d, a));
       }
     }
   }

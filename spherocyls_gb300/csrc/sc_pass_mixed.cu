@@ -75,7 +75,7 @@ __device__ __forceinline__ void mixed_epilogue(const Dev& d, const StepScalars& 
     if (MODE == PASS_PRED_STRAIN) {
       // strain_step predictor, strain_dynamics.cpp:187-199
       float phi = c.z + c.w;
-      const float RC = d.rcf[i];
+      const float RC = pai.z;
       v0x = fx - gam * fy;
       v0y = fy;
       v0p = tq * invI - ts.f_rate * (0.5f * (1.f - RC * __cosf(2.f * phi)));
@@ -88,7 +88,7 @@ __device__ __forceinline__ void mixed_epilogue(const Dev& d, const StepScalars& 
     // pure shear: isolated rotation in the flow (+x/2, -y/2) at the strain rate
     // (pure_euler_est_2p, src/cuda/2point_dynamics.cu:1889-1891)
     const float rot = (MODE == PASS_PRED_RESIZE && ts.mode == 3)
-                          ? ts.f_rate * (-0.5f * d.rcf[i] * __sinf(2.f * (c.z + c.w)))
+                          ? ts.f_rate * (-0.5f * pai.z * __sinf(2.f * (c.z + c.w)))
                           : 0.f;
     float xt = ri.x + (c.x + dt * v0x);
     float yt = ri.y + (c.y + dt * v0y);
@@ -106,22 +106,27 @@ __device__ __forceinline__ void mixed_epilogue(const Dev& d, const StepScalars& 
     float sn, cs;
     sincosf(pt, &sn, &cs);
     d.rec_t[i] = make_float4(xt, yt, A * cs, A * sn);
-    // pure shear keeps the rotation rate of the flow in place of the predicted angle
-    d.mv[i] = make_float4(v0x, v0y, v0p, (MODE == PASS_PRED_RESIZE && ts.mode == 3) ? rot : pt);
+    d.mv[i] = make_float2(v0x, v0y);
+    d.mvp[i] = v0p;
+    // pure shear keeps the rotation rate of the flow as well
+    if (MODE == PASS_PRED_RESIZE && ts.mode == 3) d.mvr[i] = rot;
   } else {
-    const float4 v0 = d.mv[i];
+    const float2 v0 = d.mv[i];
+    const float v0p = d.mvp[i];
     float4 c = d.mc[i];
     float4 r = d.rec[i];
     float ddx, ddy, ddp;
     if (MODE == PASS_CORR_STRAIN) {
       // strain_step corrector, strain_dynamics.cpp:203-219
-      const float RC = d.rcf[i];
+      const float RC = pai.z;
       float v1x = fx - gam * fy;
       float v1y = fy;
-      float v1p = tq * invI - ts.f_rate * (0.5f * (1.f - RC * __cosf(2.f * v0.w)));
+      // the predicted angle, as the predictor formed it
+      const float pt = c.z + fmaf(dt, v0p + 0.f, c.w);
+      float v1p = tq * invI - ts.f_rate * (0.5f * (1.f - RC * __cosf(2.f * pt)));
       ddx = 0.5f * dt * (v0.x + v1x);
       ddy = 0.5f * dt * (v0.y + v1y);
-      ddp = 0.5f * dt * (v0.z + v1p);
+      ddp = 0.5f * dt * (v0p + v1p);
     } else {
       // resize_step corrector, resize_dynamics.cpp:194-218.  Pure shear
       // (pure_heun_corr_2p, src/cuda/2point_dynamics.cu:2140-2173) ends at the
@@ -129,10 +134,10 @@ __device__ __forceinline__ void mixed_epilogue(const Dev& d, const StepScalars& 
       // forces, with the flow's displacement and rotation taken by Euler.
       ddx = 0.5f * dt * (v0.x + fx);
       ddy = 0.5f * dt * (v0.y + fy);
-      ddp = 0.5f * dt * (v0.z + tq * invI);
-      if (ts.mode == 3) ddp = fmaf(dt, v0.w, ddp);
+      ddp = 0.5f * dt * (v0p + tq * invI);
+      if (ts.mode == 3) ddp = fmaf(dt, d.mvr[i], ddp);
     }
-    float4 m = d.mm[i];
+    float2 m = d.mm[i];
     float aff = 0.f;  // the next step's affine displacement, for the rebuild test
     if (MODE == PASS_CORR_RESIZE) {
       const float gx = ts.f_gx, gy = ts.f_gy;
@@ -171,7 +176,7 @@ __device__ __forceinline__ void mixed_epilogue(const Dev& d, const StepScalars& 
     float h = 0.5f * (g.fpad - dg * (g.smax + g.fpad));
     // a spine end moves by at most the centre's displacement plus A times the
     // rotation; the next step's move is allowed for as well
-    float reach = sqrtf(m.x * m.x + m.y * m.y) + A * fabsf((c.z + c.w) - m.z) +
+    float reach = sqrtf(m.x * m.x + m.y * m.y) + A * fabsf((c.z + c.w) - d.mph[i]) +
                   sqrtf(ddx * ddx + ddy * ddy) + aff + A * fabsf(ddp);
     if (!(reach < h)) request_rebuild(d, s);
   }
@@ -182,13 +187,22 @@ __device__ __forceinline__ void mixed_epilogue(const Dev& d, const StepScalars& 
 // records were written by other blocks of the same (persistent) launch, so they are
 // loaded through L2 (ld.global.cg) and never through the read-only path, which holds
 // only data that stays unchanged for a whole launch.
-template <int MODE, bool TWO, bool COH = false>
+// SMALL: some system's grid has under three cells a side, where the offset between two cells
+// does not settle the image.  ONE: the handle holds one system.
+template <int MODE, bool TWO, bool SMALL, bool ONE, bool COH = false>
 __device__ __forceinline__ void pass_mixed_position(const Dev& d,
                                                     const StepScalars* __restrict__ tab,
                                                     int row, int pos) {
   constexpr bool kPred = (MODE == PASS_CORR_STRAIN || MODE == PASS_CORR_RESIZE);
-  const int i = d.ord[pos];  // the slot this thread works on (lists ordered by length)
-  const int s = d.psys[i];
+  // the slot this thread works on (lists ordered by length) and its list's length
+  const unsigned on = d.ord[pos];
+  const int i = pos - pos % kOrderWindow + (int)(on % kOrderWindow);
+  const int cnt = (int)(on / kOrderWindow);
+  int s = 0;
+  if (!ONE) {
+    s = d.wsys[pos / kOrderWindow];  // (a window of one system, mostly)
+    if (s < 0) s = d.psys[i];
+  }
   if (d.skip && d.skip[s]) return;  // a converged minimiser system
   const SysGeom& g = d.geom[s];
   const StepScalars& ts = tab[row * d.nsys + s];
@@ -196,14 +210,13 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
   const float W = kPred ? ts.f_Wc : ts.f_Wp;
   const float H = kPred ? ts.f_Hc : ts.f_Hp;
   const float gam = kPred ? ts.f_gamma_c : ts.f_gamma_p;
-  const bool smallx = g.cols < 3, smally = g.rows < 3;
-  const float Lxf = W * g.cols, Lyf = H * g.rows;
+  const bool smallx = SMALL && g.cols < 3, smally = SMALL && g.rows < 3;
+  const float Lxf = SMALL ? W * g.cols : 0.f, Lyf = SMALL ? H * g.rows : 0.f;
   constexpr bool two_point = TWO;
 
 #define SC_REC(k) (COH ? __ldcg(REC + (k)) : REC[(k)])
   const float4 ri = SC_REC(i);
-  const float4 pai = d.pa[i];  // (R, A, index bits, 1/I)
-  const int cnt = d.nbr_pn[pos];
+  const float4 pai = d.pa[i];  // (R, A, RC, 1/I)
   // the list is column-major: entry k of this slot sits k * ntot words further on;
   // Lst walks it, two entries ahead of the pair being computed
   const unsigned* __restrict__ Lst = reinterpret_cast<const unsigned*>(d.nbr_p) + pos;
@@ -234,8 +247,8 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
     }
     Lst += stride;
     if (k + 2 < cnt) e2 = __ldg(Lst);
-    float dx = ri.x - rj.x + (float)(1 - (int)((e >> 28) & 3u)) * W;
-    float dy = ri.y - rj.y + (float)(1 - (int)(e >> 30)) * H;
+    float dx = fmaf(cell_offset(e >> 28), W, ri.x - rj.x);
+    float dy = fmaf(cell_offset(e >> 30), H, ri.y - rj.y);
     if (smallx) dx += Lxf * (float)((dx < -0.5f * Lxf) - (dx > 0.5f * Lxf));
     if (smally) dy += Lyf * (float)((dy < -0.5f * Lyf) - (dy > 0.5f * Lyf));
     // Each thread evaluates the pair from its own particle's side (i as "p"): the
@@ -258,15 +271,26 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
   mixed_epilogue<MODE>(d, ts, g, s, i, ri, pai, gam, fx, fy, tq);
 }
 
-template <int MODE, bool TWO>
-__global__ void __launch_bounds__(128, TWO ? 6 : 12) k_pass_mixed(Dev d,
+// k_pass_mixed: one thread per list position.  It waits for dependent gathers (10 of 18
+// resident warps) and issues in 57 to 63% of the cycles, so what counts is instructions a
+// pair and bytes a particle: quotients without the scaling around subnormals, offsets
+// without conversions, no image test and no system lookup where they are not needed, and a
+// state of 115 B a particle, which at 2^20 particles about fits the L2 (129 MB; it was 141
+// B).  45 -> 37 us a pass at 2^20 particles (corrector and predictor, mean), 37 -> 31 on the
+// 512-system ensemble.  Blocks an SM: 12 (40 registers) against 10, 1905 and 1933 us for 20
+// steps at 2^20; the affine passes, which spill more, 305 and 297 us at 49999.  Prefetching
+// the epilogue's state before the loop was 3% slower.
+template <int MODE, bool TWO, bool SMALL, bool ONE>
+__global__ void __launch_bounds__(
+    128, TWO ? 6 : (MODE == PASS_PRED_RESIZE || MODE == PASS_CORR_RESIZE) ? 10 : 12)
+    k_pass_mixed(Dev d,
                                                        const StepScalars* __restrict__ tab,
                                                        int row) {
   constexpr bool kPred = (MODE == PASS_CORR_STRAIN || MODE == PASS_CORR_RESIZE);
   if (kPred) mark_pending_rebuilds(d, tab, row);
   const int pos = blockIdx.x * blockDim.x + threadIdx.x;
   if (pos >= d.ntot) return;
-  pass_mixed_position<MODE, TWO>(d, tab, row, pos);
+  pass_mixed_position<MODE, TWO, SMALL, ONE>(d, tab, row, pos);
 }
 
 // ---- persistent shear steps ----
@@ -297,14 +321,14 @@ __global__ void __launch_bounds__(128, TWO ? 6 : 12) k_persist_steps(
           atomicExch(d.any, 1);
         }
     for (int pos = t0; pos < d.ntot; pos += stride)
-      pass_mixed_position<PASS_CORR_STRAIN, TWO, true>(d, tab, row, pos);
+      pass_mixed_position<PASS_CORR_STRAIN, TWO, true, false, true>(d, tab, row, pos);
     bar.wait(d.status);
     if (*(volatile int*)d.any != 0) {  // the same value in every block after the barrier
       stopped = 1;
       break;
     }
     for (int pos = t0; pos < d.ntot; pos += stride)
-      pass_mixed_position<PASS_PRED_STRAIN, TWO, true>(d, tab, row, pos);
+      pass_mixed_position<PASS_PRED_STRAIN, TWO, true, false, true>(d, tab, row, pos);
     bar.wait(d.status);
   }
   if (t0 == 0) *out = 2 * k + stopped;
@@ -332,7 +356,7 @@ __global__ void __launch_bounds__(256, TWO ? 3 : 4) k_persist_fire(
   int k = 0, why = 0;
   while (k < iters) {
     for (int pos = t0; pos < d.ntot; pos += stride)
-      pass_mixed_position<PASS_FORCE, TWO, true>(d, tab, 0, pos);
+      pass_mixed_position<PASS_FORCE, TWO, true, false, true>(d, tab, 0, pos);
     bar.wait(d.status);
     for (int ch = blockIdx.x; ch < d.npchunks; ch += gridDim.x) {
       fire::fire_chunk<true>(d, f, ch);
@@ -360,13 +384,22 @@ __global__ void __launch_bounds__(256, TWO ? 3 : 4) k_persist_fire(
   if (t0 == 0) *out = 4 * k + why;
 }
 
+template <int MODE, bool TWO>
+void launch_of(const Dev& d, const StepScalars* tab, int row, cudaStream_t st, int block) {
+  const int grid = (d.ntot + block - 1) / block;
+  if (d.small_grid)
+    k_pass_mixed<MODE, TWO, true, false><<<grid, block, 0, st>>>(d, tab, row);
+  else if (d.nsys > 1)
+    k_pass_mixed<MODE, TWO, false, false><<<grid, block, 0, st>>>(d, tab, row);
+  else
+    k_pass_mixed<MODE, TWO, false, true><<<grid, block, 0, st>>>(d, tab, row);
+}
 template <int MODE>
 void launch_one(const Dev& d, const StepScalars* tab, int row, cudaStream_t st, int block) {
-  int grid = (d.ntot + block - 1) / block;
   if (d.contact_model == 1)
-    k_pass_mixed<MODE, true><<<grid, block, 0, st>>>(d, tab, row);
+    launch_of<MODE, true>(d, tab, row, st, block);
   else
-    k_pass_mixed<MODE, false><<<grid, block, 0, st>>>(d, tab, row);
+    launch_of<MODE, false>(d, tab, row, st, block);
 }
 
 // ---- tile force pass ----
@@ -599,7 +632,7 @@ __global__ void k_mx_materialize(Dev d, const StepScalars* __restrict__ tab, int
 // Compensated local state of a slot from its FP64 state after the cell sort.
 __device__ __forceinline__ void local_record(const Dev& d, const StepScalars* __restrict__ tab,
                                              int row, int i, int s, double2 p, double phi,
-                                             double2 ra, double2 irc, int id, int cell) {
+                                             double2 ra, double2 irc, int cell) {
   const SysGeom& g = d.geom[s];
   const StepScalars& ts = tab[row * d.nsys + s];
   int col, rw;
@@ -616,11 +649,11 @@ __device__ __forceinline__ void local_record(const Dev& d, const StepScalars* __
   sincosf(pf, &sn, &cs);
   d.rec[i] = make_float4(xl, yl, A * cs, A * sn);
   d.mc[i] = make_float4(narrow(lx - widen(xl)), narrow(ly - widen(yl)), pf, pc);
-  d.mm[i] = make_float4(0.f, 0.f, pf + pc, 0.f);
+  d.mm[i] = make_float2(0.f, 0.f);
+  d.mph[i] = pf + pc;
   // 1/I in FP32 (an FP64 division per particle costs more than the whole record)
   const float R = narrow(ra.x);
-  d.pa[i] = make_float4(R, A, __int_as_float(id), __frcp_rn(narrow(irc.x)));
-  d.rcf[i] = narrow(irc.y);
+  d.pa[i] = make_float4(R, A, narrow(irc.y), __frcp_rn(narrow(irc.x)));
   d.rf[i] = R;
   d.rsf[i] = R + A;
 }
@@ -784,8 +817,7 @@ __device__ __forceinline__ void order_window(const Dev& d, int i, int* len, int 
   }
   if (!valid) return;
   const int pos = i - in + rank;
-  d.ord[pos] = i;
-  d.nbr_pn[pos] = c;
+  d.ord[pos] = (unsigned)in | (unsigned)c << 7;
   const size_t n = d.ntot;
   for (int k = 0; k < c; k += 8) {  // eight loads in flight
     int e[8];
@@ -809,8 +841,8 @@ __global__ void __launch_bounds__(BS, 1536 / BS) k_rebuild_mx(Dev d,
   const rb::Work<BS> work(d);
   const bool ok = rb::sort_cells<true, BS>(
       d, work, tab, row, moved != 0, bar,
-      [&](int i, int s, double2 p, double phi, double2 ra, double2 irc, int id, int cell) {
-        local_record(d, tab, row, i, s, p, phi, ra, irc, id, cell);
+      [&](int i, int s, double2 p, double phi, double2 ra, double2 irc, int, int cell) {
+        local_record(d, tab, row, i, s, p, phi, ra, irc, cell);
       });
   if (!ok || !LISTS) return;
   const bool by_lanes = work.items <= kLaneItems;
