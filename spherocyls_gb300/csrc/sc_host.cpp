@@ -836,6 +836,8 @@ int Handle::run_steps(int kind, int shrink, int nsteps, int se_every, double* se
     for (int k = 1; k <= nk; k++)
       if (se_every > 0 && (done + k) % se_every == 0) nrec++;
     if (nrec > 0 && !ensure_se_hist(nrec)) return last_status;
+    // (also where a step fails: the rebuild keeps the records alone up to date)
+    if (prec == PREC_MIXED) fp64_valid = false;
     const int pkind = kind == KIND_PURE ? 4 : (resize ? (shrink ? 2 : 3) : 1);
     if (!pred_valid || pred_kind != pkind) {
       launch_pass(resize ? PASS_PRED_RESIZE : PASS_PRED_STRAIN, false, 0);
@@ -870,7 +872,6 @@ int Handle::run_steps(int kind, int shrink, int nsteps, int se_every, double* se
     if (!check_status(kind == KIND_PURE ? "pure shear steps"
                                         : (resize ? "resize steps" : "strain steps")))
       return last_status;
-    fp64_valid = prec != PREC_MIXED;
     forces_valid = false;
     hs = sim;
     rec_done += nrec;
@@ -1031,7 +1032,7 @@ void Handle::enqueue_fire_iteration(double ftol, double dt_max) {
   launch_pass(PASS_FORCE, false, 0, true);
   pass_skip = nullptr;
   launch_fire_iteration_tail(d, fire, ftol, dt_max, mixed, stream);
-  kernels += 3 + launch_rebuild(d, mixed, d_tab, 0, true, stream);
+  kernels += 2 + launch_rebuild(d, mixed, d_tab, 0, true, stream);
 }
 
 // `iters` FIRE iterations as one CUDA graph: each is force pass, reductions and
@@ -1117,6 +1118,7 @@ int Handle::fire_minimize(double ftol, int max_iter, double dt0, double dt_max, 
   std::vector<FireSys> hsys(nsys);
   const bool mixed = prec == PREC_MIXED;
   const bool persist = opt.persist_steps && mixed && d.pass_kind == 0 && d_persist;
+  if (mixed) fp64_valid = false;
   int it = 0;
   bool all_done = false;
   while (it < max_iter && !all_done) {
@@ -1137,7 +1139,6 @@ int Handle::fire_minimize(double ftol, int max_iter, double dt0, double dt_max, 
   }
   pred_valid = false;
   forces_valid = false;
-  if (mixed) fp64_valid = false;
   int max_it = 0;
   fire_iters.assign(nsys, 0);
   for (int s = 0; s < nsys; s++) {

@@ -254,7 +254,8 @@ struct Dev {
   double* se_part;          // [5][ntot]
   double* se_chunk;         // [5][npchunks]
   double* se_sys;           // [5][nsys]
-  int* se_done;             // [nsys] chunks of a system summed so far (zero between uses)
+  int* se_done;             // [nsys] chunks of a system summed so far, by the stress/energy
+                            // and FIRE reductions (zero between uses)
   const int* pchunk_sys;    // particle chunks for reductions
   const int* pchunk_p0;
   const int* pchunk_np;

@@ -66,9 +66,9 @@ __device__ __forceinline__ void mixed_epilogue(const Dev& d, const StepScalars& 
   const float dt = ts.f_step;
   const float A = pai.y, invI = pai.w;
   if (MODE == PASS_FORCE) {
-    d.fx[i] = fx;
-    d.fy[i] = fy;
-    d.tau[i] = tq;
+    d.fx[i] = widen(fx);
+    d.fy[i] = widen(fy);
+    d.tau[i] = widen(tq);
   } else if (MODE == PASS_PRED_STRAIN || MODE == PASS_PRED_RESIZE) {
     const float4 c = d.mc[i];
     float v0x, v0y, v0p;
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(128, TWO ? 6 : 12) k_persist_steps(
 // FIRE iterations of the mixed form in one cooperative launch: the force pass over
 // all positions, the chunk partials, the per-system FIRE update and the particle
 // update, each followed by a grid barrier.  The blocks have the 256 threads of the
-// launch-per-kernel reductions (k_fire_chunk), so each chunk sums in the same order
+// launch-per-kernel reductions (k_fire_sums), so each chunk sums in the same order
 // and the iterates equal those of the graph and eager paths bit for bit.  The launch
 // ends after `iters` iterations, after the iteration whose update asks for a
 // rebuild (the host runs it), or at the iteration in which the last system
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(256, TWO ? 3 : 4) k_persist_fire(
       __syncthreads();  // the next chunk reuses the block's shared partials
     }
     bar.wait(d.status);
-    // one block per system, as k_fire_sys (the block has kFireBlock threads)
+    // one block per system (the block has kFireBlock threads)
     for (int s = blockIdx.x; s < d.nsys; s += gridDim.x) fire::fire_sys(d, f, s, ftol, dt_max);
     bar.wait(d.status);
     k++;

@@ -427,15 +427,18 @@ __device__ __forceinline__ void place(const Dev& d, const Work<BS>& work) {
 }
 
 // Back from scratch; f(slot, system, position, angle, (R, A), (I, RC), index, cell) then
-// makes the records that the form's passes read.
+// makes the records that the form's passes read.  records: the state is in them alone
+// (the FP64 positions and angles are not read before they are next made).
 template <int BS, class F>
-__device__ __forceinline__ void put_back(const Dev& d, const Work<BS>& work, F&& f) {
+__device__ __forceinline__ void put_back(const Dev& d, const Work<BS>& work, bool records, F&& f) {
   work.each(d, [&](int i, int s) {
     const double2 p = d.s_xy[i], ra = d.s_ra[i], irc = d.s_irc[i];
     const double phi = d.s_ph[i];
     const int id = d.s_id[i], c = d.s_cell[i];
-    d.xy[i] = p;
-    d.ph[i] = phi;
+    if (!records) {
+      d.xy[i] = p;
+      d.ph[i] = phi;
+    }
     d.ra[i] = ra;
     d.irc[i] = irc;
     d.id[i] = id;
@@ -496,7 +499,7 @@ __device__ __forceinline__ bool sort_cells(const Dev& d, const Work<BS>& work,
   if (!bar.wait(d.status)) return false;
   place<MIXED>(d, work);
   if (!bar.wait(d.status)) return false;
-  put_back(d, work, records);
+  put_back(d, work, MIXED && moved, records);
   return bar.wait(d.status);
 }
 
