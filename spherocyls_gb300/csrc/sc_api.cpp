@@ -119,11 +119,39 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
     return SC_E_ARG;
   }
   const int ntot = (int)ntot_ll;
+  // Each system's filled area, summed in particle order (calculate_packing_fraction
+  // src/cpp/spherocyl_box.cpp:357-366): a dependent chain of additions, 1.4 ms at 2^20
+  // particles, on a thread of its own beside the device work of the creation, which does
+  // not need it; joined before this function returns.
+  struct Area {
+    std::vector<double> sum;
+    std::thread thread;
+    ~Area() { join(); }
+    void join() {
+      if (thread.joinable()) thread.join();
+    }
+  } filled;
+  filled.sum.assign(n_sys, 0.0);
+  auto sum_areas = [&] {
+    for (int s = 0, i = 0; s < n_sys; s++) {
+      double f = 0.0;
+      for (int k = 0; k < n_per_sys[s]; k++, i++) f += (kRefPi * R[i] + 4.0 * A[i]) * R[i];
+      filled.sum[s] = f;
+    }
+  };
+  bool summing = false;
+  if (ntot >= (1 << 16)) {
+    try {
+      filled.thread = std::thread(sum_areas);
+      summing = true;
+    } catch (...) {  // no thread to be had: summed here
+    }
+  }
+  if (!summing) sum_areas();
   // The input checks and per system the largest R and A (set_particle,
   // src/cpp/spherocyl_box.cpp:216-219) on worker threads over slices of the caller's
-  // arrays, while this thread sums each system's filled area in particle order
-  // (calculate_packing_fraction :357-366; a dependent chain of additions).
-  std::vector<double> rmax(n_sys, 0.0), amax(n_sys, 0.0), filled(n_sys, 0.0);
+  // arrays.
+  std::vector<double> rmax(n_sys, 0.0), amax(n_sys, 0.0);
   {
     std::vector<int> p0s(n_sys + 1, 0);
     for (int s = 0; s < n_sys; s++) p0s[s + 1] = p0s[s] + n_per_sys[s];
@@ -165,11 +193,6 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
     }
     for (int w = 0; w < nthreads; w++)
       if (!on_worker[w]) scan(w);
-    for (int s = 0, i = 0; s < n_sys; s++) {
-      double f = 0.0;
-      for (int k = 0; k < n_per_sys[s]; k++, i++) f += (kRefPi * R[i] + 4.0 * A[i]) * R[i];
-      filled[s] = f;
-    }
     for (auto& t : workers) t.join();
     bool finite = true, shapes = true;
     for (const Part& P : parts) {
@@ -225,8 +248,6 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
     S.pad = pad ? pad[s] : 0.0;
     S.Amax = amax[s];
     S.Rmax = rmax[s];
-    const double filled_s = filled[s];
-    S.packing = filled_s / (S.Lx * S.Ly);
     S.configure(true);
     p0 += S.n;
   }
@@ -390,6 +411,9 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
   h.dfree(d_sys_L);
   if (!h.layout_cells() || !h.rebuild_all() || !h.check_status("create"))
     return bail(h.last_status);
+  filled.join();
+  for (int s = 0; s < n_sys; s++)
+    h.hs[s].packing = filled.sum[s] / (h.hs[s].Lx * h.hs[s].Ly);
   *out = H;
   return SC_OK;
 }

@@ -170,7 +170,7 @@ StepScalars Handle::row_current(int s) const {
 bool Handle::layout_cells() {
   // cells, scan chunks and particle chunks for all systems
   int c = 0, ch = 0;
-  std::vector<int> chunk_sys, chunk_c0, chunk_nc, cell_sys;
+  std::vector<int> chunk_sys, chunk_c0, chunk_nc;
   std::vector<int4> tiles;
   // tiles of about tile_target particles for the tile pass (one tile per system
   // otherwise): square blocks of cells at the system's mean occupancy
@@ -200,7 +200,6 @@ bool Handle::layout_cells() {
       chunk_c0.push_back(c + k * kScanChunk);
       chunk_nc.push_back(std::min(kScanChunk, nc - k * kScanChunk));
     }
-    for (int k = 0; k < nc; k++) cell_sys.push_back(s);
     c += nc;
     ch += h.nchunks;
   }
@@ -209,17 +208,15 @@ bool Handle::layout_cells() {
     dfree(d.cell_start);
     dfree(d.cell_count);
     dfree(d.cell_fill);
-    dfree((void*)d.cell_sys);
     int cap = ncells + ncells / 4 + 64;
-    int *cs = nullptr, *cn = nullptr, *cf = nullptr, *csys = nullptr;
+    int *cs = nullptr, *cn = nullptr, *cf = nullptr;
     if (!dalloc(&cs, cap, "cell_start") || !dalloc(&cn, cap, "cell_count") ||
-        !dalloc(&cf, cap, "cell_fill") || !dalloc(&csys, cap, "cell_sys") ||
+        !dalloc(&cf, cap, "cell_fill") ||
         !cuda_ok(cudaMemsetAsync(cf, 0, cap * sizeof(int), stream), "cell_fill"))
       return false;
     d.cell_fill = cf;
     d.cell_start = cs;
     d.cell_count = cn;
-    d.cell_sys = csys;
     cell_cap = cap;
   }
   if (nchunks > chunk_cap) {
@@ -280,8 +277,6 @@ bool Handle::layout_cells() {
   }
   bool ok = cuda_ok(cudaMemcpyAsync((void*)d.geom, g.data(), nsys * sizeof(SysGeom),
                                     cudaMemcpyHostToDevice, stream), "upload geometry") &&
-            cuda_ok(cudaMemcpyAsync((void*)d.cell_sys, cell_sys.data(), ncells * sizeof(int),
-                                    cudaMemcpyHostToDevice, stream), "upload cell map") &&
             cuda_ok(cudaMemcpyAsync((void*)d.chunk_sys, chunk_sys.data(), nchunks * sizeof(int),
                                     cudaMemcpyHostToDevice, stream), "upload chunks") &&
             cuda_ok(cudaMemcpyAsync((void*)d.chunk_c0, chunk_c0.data(), nchunks * sizeof(int),

@@ -160,7 +160,6 @@ struct Dev {
   const SysGeom* geom;      // [nsys]
   const int* psys;          // [ntot] system of each slot
   const int* wsys;          // system of each window of kOrderWindow slots, -1: several
-  const int* cell_sys;      // [ncells] system of each cell
   // state
   double2* xy;
   double* ph;
