@@ -167,7 +167,7 @@ __device__ __forceinline__ bool pair_fp64(double dX, double dY, double nxA, doub
   double dDy = dY + s * nyA - t * nyB;
   double dsq = dDx * dDx + dDy * dDy;
   if (!less_square(dsq, sig * sig)) return false;
-  double Fx, Fy, dij, dvij;
+  double Fx, Fy, dij, dvij, inv_sig = 0.0;
   if (FAST) {
     const double rs = rsqrt(dsq);
     dij = dsq * rs;
@@ -176,9 +176,11 @@ __device__ __forceinline__ bool pair_fp64(double dX, double dY, double nxA, doub
     Fy = dDy * (dvij * rs);
   } else {
     dij = sqrt(dsq);
-    dvij = (1.0 - dij / sig) / sig;
-    Fx = dDx * dvij / dij;
-    Fy = dDy * dvij / dij;
+    inv_sig = shared_rcp(sig);
+    const double rd = shared_rcp(dij);
+    dvij = div_by(1.0 - div_by(dij, sig, inv_sig), sig, inv_sig);
+    Fx = div_by(dDx * dvij, dij, rd);
+    Fy = div_by(dDy * dvij, dij, rd);
   }
   o.fx = Fx;
   o.fy = Fy;
@@ -206,7 +208,7 @@ __device__ __forceinline__ bool pair_fp64(double dX, double dY, double nxA, doub
     double CxA = s * nxA - 0.5 * dDx;
     double CyA = s * nyA - 0.5 * dDy;
     double CxB = t * nxB + 0.5 * dDx;
-    o.e = dvij * sig * (1.0 - dij / sig) / two_n;
+    o.e = dvij * sig * (1.0 - div_by(dij, sig, inv_sig)) / two_n;
     if (!virial) {
       // the reference's accumulation, slips included: CyB is built from nxB,
       // one Pxy term lands in Pxx, and Pxy misses its B arm.
@@ -467,9 +469,10 @@ __device__ __forceinline__ bool contact_fp64(double dX, double dY, double s, dou
     Fy = dDy * (dvij * rs);
   } else {
     dij = sqrt(dsq);
-    dvij = (1.0 - dij / sig) / sig;
-    Fx = dDx * dvij / dij;
-    Fy = dDy * dvij / dij;
+    const double rd = shared_rcp(dij);
+    dvij = div_by(1.0 - div_by(dij, sig, inv_sig), sig, inv_sig);
+    Fx = div_by(dDx * dvij, dij, rd);
+    Fy = div_by(dDy * dvij, dij, rd);
   }
   o.fx += Fx;
   o.fy += Fy;
@@ -487,7 +490,7 @@ __device__ __forceinline__ bool contact_fp64(double dX, double dY, double s, dou
   } else if (SE) {
     double CxA = s * nxA - 0.5 * dDx, CyA = s * nyA - 0.5 * dDy;
     double CxB = t * nxB + 0.5 * dDx, CyB = t * nyB + 0.5 * dDy;
-    o.e += dvij * sig * (1.0 - dij / sig) / two_n;
+    o.e += dvij * sig * (1.0 - div_by(dij, sig, inv_sig)) / two_n;
     o.pxx += div_by(Fx * CxA, LL, inv_LL) - div_by(Fx * CxB, LL, inv_LL);
     o.pyy += div_by(Fy * CyA, LL, inv_LL) - div_by(Fy * CyB, LL, inv_LL);
     o.pxy += div_by(Fy * CxA, LL, inv_LL) - div_by(Fy * CxB, LL, inv_LL);
@@ -519,6 +522,7 @@ __device__ __forceinline__ bool pair2_fp64(double dX, double dY, double nxA, dou
   } else {
     iv.a = inv_aP;
     iv.c = inv_aQ;
+    iv.sig = shared_rcp(sig);
     if (SE) inv_LL = shared_rcp(Lx * Ly);
   }
   Contacts2<double> k =
