@@ -318,11 +318,11 @@ __device__ __forceinline__ bool may_touch_fp32(float dX, float dY, float nxA, fl
   float uxv = fmaf(nxA, nyB, -w) + fmaf(-nyA, nxB, w);
   float w2 = nyA * dX;
   float uxD = fmaf(nxA, dY, -w2) + fmaf(-nyA, dX, w2);
-  float t = uxv == 0.f ? -1.f : fminf(fmaxf(__fdividef(uxD, uxv), -1.f), 1.f);
-  float s = a > 0.f ? -__fdividef(b * t + d, a) : 0.f;
+  float t = uxv == 0.f ? -1.f : fminf(fmaxf(div_fast(uxD, uxv), -1.f), 1.f);
+  float s = a > 0.f ? -div_fast(b * t + d, a) : 0.f;
   float sarg = fabsf(s);
   s = fminf(fmaxf(s, -1.f), 1.f);
-  if (sarg > 1.f && c > 0.f) t = fminf(fmaxf(-__fdividef(b * s + e, c), -1.f), 1.f);
+  if (sarg > 1.f && c > 0.f) t = fminf(fmaxf(-div_fast(b * s + e, c), -1.f), 1.f);
   float dDx = dX + s * nxA - t * nxB;
   float dDy = dY + s * nyA - t * nyB;
   float lim = sig * 1.0001f + 1e-5f;
@@ -343,11 +343,11 @@ __device__ __forceinline__ bool capsules_within(float dX, float dY, float nxA, f
   const float uxv = fmaf(nxA, nyB, -w) + fmaf(-nyA, nxB, w);
   const float w2 = nyA * dX;
   const float uxD = fmaf(nxA, dY, -w2) + fmaf(-nyA, dX, w2);
-  float t = uxv == 0.f ? -1.f : fminf(fmaxf(__fdividef(uxD, uxv), -1.f), 1.f);
-  float s = a > 0.f ? -__fdividef(b * t + d, a) : 0.f;
+  float t = uxv == 0.f ? -1.f : fminf(fmaxf(div_fast(uxD, uxv), -1.f), 1.f);
+  float s = a > 0.f ? -div_fast(b * t + d, a) : 0.f;
   const float sarg = fabsf(s);
   s = fminf(fmaxf(s, -1.f), 1.f);
-  if (sarg > 1.f && c > 0.f) t = fminf(fmaxf(-__fdividef(b * s + e, c), -1.f), 1.f);
+  if (sarg > 1.f && c > 0.f) t = fminf(fmaxf(-div_fast(b * s + e, c), -1.f), 1.f);
   const float x = dX + s * nxA - t * nxB, y = dY + s * nyA - t * nyB;
   return x * x + y * y < lim * lim;
 }

@@ -691,8 +691,8 @@ __device__ __forceinline__ void build_list_slot(const Dev& d, const StepScalars*
       if (j == i) continue;
       const float4 rj = d.rec[j];
       const float Rj = d.rf[j];
-      float dx = ri.x - rj.x + (float)(1 - (int)((e >> 28) & 3u)) * W;
-      float dy = ri.y - rj.y + (float)(1 - (int)(e >> 30)) * H;
+      float dx = fmaf(cell_offset(e >> 28), W, ri.x - rj.x);
+      float dy = fmaf(cell_offset(e >> 30), H, ri.y - rj.y);
       if (smallx) dx += Lxf * (float)((dx < -0.5f * Lxf) - (dx > 0.5f * Lxf));
       if (smally) dy += Lyf * (float)((dy < -0.5f * Lyf) - (dy > 0.5f * Lyf));
       if (capsules_within(fmaf(gam, dy, dx), dy, ri.z, ri.w, rj.z, rj.w,
@@ -766,8 +766,8 @@ __device__ __forceinline__ void build_list_lanes(const Dev& d, const StepScalars
       e = (unsigned)j | table.code[q];
       if (j != i) {
         const float4 rj = d.rec[j];
-        float dx = ri.x - rj.x + (float)(1 - (int)((e >> 28) & 3u)) * W;
-        float dy = ri.y - rj.y + (float)(1 - (int)(e >> 30)) * H;
+        float dx = fmaf(cell_offset(e >> 28), W, ri.x - rj.x);
+        float dy = fmaf(cell_offset(e >> 30), H, ri.y - rj.y);
         if (smallx) dx += Lxf * (float)((dx < -0.5f * Lxf) - (dx > 0.5f * Lxf));
         if (smally) dy += Lyf * (float)((dy < -0.5f * Lyf) - (dy > 0.5f * Lyf));
         const float lim = fmaf(si + d.rsf[j], 1.00002f, 1e-6f);
@@ -798,22 +798,61 @@ __global__ void __launch_bounds__(128, 12) k_mx_build_list(Dev d, const StepScal
 
 // Force-pass ordering: within each window of kOrderWindow slots, a stable sort
 // of the slots by list length; the lists are copied to their positions.  One group of
-// kOrderWindow threads (w0: its first; bar: its barrier); i: this thread's slot.
+// kOrderWindow threads (w0: its first; bar: its barrier); i: this thread's slot.  The ranks
+// come from a ballot per length and warp; lists of 64 entries and more are ranked by
+// comparing with every slot of the window, which took half the instructions of a rebuild
+// when all were.
+constexpr int kOrderWarps = kOrderWindow / 32;
+struct OrderScratch {
+  int hist[64 * kOrderWarps];  // by length and warp: how many, then how many before
+  int len[kOrderWindow];
+  int top[kOrderWarps];
+};
 __device__ __forceinline__ void group_sync(int bar) {
   asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(kOrderWindow) : "memory");
 }
-__device__ __forceinline__ void order_window(const Dev& d, int i, int* len, int w0, int bar) {
+__device__ __forceinline__ void order_window(const Dev& d, int i, OrderScratch& sc, int w0,
+                                             int bar) {
+  const unsigned full = 0xffffffffu;
   const bool valid = i < d.ntot;
-  const int in = threadIdx.x - w0;
-  int c = 0x7fffffff;  // slots past the end sort last
-  if (valid) c = min(d.nbr_n[i], d.maxn);
-  group_sync(bar);  // the group's last window is done with len, its lists are complete
-  len[in] = c;
+  const int in = threadIdx.x - w0, lane = in & 31, w = in >> 5;
+  const int c = valid ? min(d.nbr_n[i], d.maxn) : -1;  // slots past the end have no rank
+  const int mine = __reduce_max_sync(full, c);
+  group_sync(bar);  // the group's last window is done with the scratch
+  if (lane == 0) sc.top[w] = mine;
+  sc.len[in] = valid ? c : 0x7fffffff;
   group_sync(bar);
+  int top = 0;
+  for (int q = 0; q < kOrderWarps; q++) top = max(top, sc.top[q]);
   int rank = 0;
-  for (int k = 0; k < kOrderWindow; k++) {
-    const int o = len[k];
-    rank += (o < c) | ((o == c) & (k < in));
+  if (top < 64) {
+    for (int v = 0; v <= top; v++) {
+      const unsigned b = __ballot_sync(full, c == v);
+      if (lane == 0) sc.hist[v * kOrderWarps + w] = __popc(b);
+      if (c == v) rank = __popc(b & ((1u << lane) - 1u));
+    }
+    group_sync(bar);
+    if (w == 0) {
+      int before = 0;
+      for (int e0 = 0; e0 < (top + 1) * kOrderWarps; e0 += 32) {
+        const int e = e0 + lane;
+        const int n = e < (top + 1) * kOrderWarps ? sc.hist[e] : 0;
+        int x = n;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(full, x, o);
+          if (lane >= o) x += y;
+        }
+        if (e < (top + 1) * kOrderWarps) sc.hist[e] = before + x - n;
+        before += __shfl_sync(full, x, 31);
+      }
+    }
+    group_sync(bar);
+    if (valid) rank += sc.hist[c * kOrderWarps + w];
+  } else {
+    for (int k = 0; k < kOrderWindow; k++) {
+      const int o = sc.len[k];
+      rank += (o < c) | ((o == c) & (k < in));
+    }
   }
   if (!valid) return;
   const int pos = i - in + rank;
@@ -856,7 +895,7 @@ __global__ void __launch_bounds__(BS, 1536 / BS) k_rebuild_mx(Dev d,
     }
     if (!bar.wait(d.status)) return;
   }
-  __shared__ int len[BS];
+  __shared__ OrderScratch scratch[BS / kOrderWindow];
   const int w0 = threadIdx.x / kOrderWindow * kOrderWindow, in = threadIdx.x - w0;
   for (int g = (blockIdx.x * BS + w0) / kOrderWindow; g < work.windows;
        g += gridDim.x * BS / kOrderWindow) {
@@ -865,7 +904,7 @@ __global__ void __launch_bounds__(BS, 1536 / BS) k_rebuild_mx(Dev d,
       const int s = d.psys[i];
       if (d.flags[s] != 0) build_list_slot(d, tab, row, i, s);
     }
-    order_window(d, i, len + w0, w0, 1 + w0 / kOrderWindow);
+    order_window(d, i, scratch[w0 / kOrderWindow], w0, 1 + w0 / kOrderWindow);
   }
   rb::finish(d);
 }
