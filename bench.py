@@ -98,10 +98,10 @@ def bytes_per_pass(precision: str, nbar: float) -> float:
 
 
 # DRAM bytes (read + write) per particle of one mixed force pass, the mean of the
-# predictor (113.6 MB) and corrector (172.4 MB) launches in one ncu capture of the
+# predictor (96.9 MB) and corrector (142.8 MB) launches in one ncu capture of the
 # default workload at the padding the autotuner picks for it, 0.6
 # (profiles/k_pass_mixed_n1048576.md).
-PASS_DRAM_BYTES_PER_PARTICLE = {"shear_n1048576_phi084": 143.0e6 / (1 << 20)}
+PASS_DRAM_BYTES_PER_PARTICLE = {"shear_n1048576_phi084": 119.9e6 / (1 << 20)}
 
 
 def _peaks():
@@ -574,7 +574,7 @@ def main():
                     help="padding factor of the mixed form when not autotuned")
     ap.add_argument("--no-graphs", action="store_true",
                     help="launch eagerly instead of through CUDA graphs (profiler captures: "
-                         "kernels inside graphs with conditional nodes cannot be profiled)")
+                         "one launch of a kernel at a time instead of a whole graph)")
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3)
     legs = set() if args.legs == "none" else set(args.legs.split(","))
@@ -658,7 +658,7 @@ def main():
         secs = time_steps(b, args.steps, torch)
         c1 = b.counters()
         # forced full rebuilds of the sorted state in an NVTX range (profiler captures
-        # of the rebuild chain select it with --nvtx-include forced_rebuild/)
+        # of the rebuild kernel select it with --nvtx-include forced_rebuild/)
         torch.cuda.nvtx.range_push("forced_rebuild")
         for _ in range(args.forced_rebuilds):
             b.find_neighbors()

@@ -20,7 +20,7 @@ __global__ void k_rb_clear(Dev d) {
   __syncthreads();
   if (threadIdx.x == 0) {
     *d.any = 0;
-    d.status[1] += 1;  // rebuild chains executed
+    d.status[1] += 1;  // rebuilds executed
   }
 }
 

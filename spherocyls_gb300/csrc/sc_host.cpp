@@ -1019,7 +1019,7 @@ bool Handle::ensure_fire() {
   return true;
 }
 
-// One FIRE iteration, eagerly: force pass, reductions and update, rebuild chain.
+// One FIRE iteration, eagerly: force pass, reductions and update, rebuild.
 void Handle::enqueue_fire_iteration(double ftol, double dt_max) {
   const bool mixed = prec == PREC_MIXED;
   // converged systems keep their forces and state: their force passes are skipped
@@ -1066,8 +1066,7 @@ bool Handle::run_fire_graph(int iters, double ftol, double dt_max) {
 
 // `iters` FIRE iterations with the persistent kernel of the mixed form.  A launch
 // returns after the iteration that asks for a rebuild, which is launched here before
-// the next one (as the graph's conditional node does), or once every system has
-// converged.  One host synchronisation per launch, to read where it ended.
+// the next one, or once every system has converged.  One host synchronisation per launch, to read where it ended.
 bool Handle::run_persist_fire(int iters, double ftol, double dt_max) {
   for (int k = 0; k < iters;) {
     if (!launch_persist_fire(d, fire, d_tab, ftol, dt_max, iters - k, d_persist, stream)) {
