@@ -299,7 +299,7 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
     ok = ok && h.dalloc(&d.mc, N, "mc") && h.dalloc(&d.mv, N, "mv") && h.dalloc(&d.mvp, N, "mvp") && h.dalloc(&d.mvr, N, "mvr") && h.dalloc(&d.mm, N, "mm") &&
          h.dalloc(&d.mph, N, "mph") && h.dalloc(&d.pa, N, "pa") &&
          h.dalloc(&d.cellp, N, "cellp") && h.dalloc(&d.gbuild, n_sys, "gbuild") &&
-         h.dalloc(&d.ord, N, "ord") && h.dalloc(&d.nbr_p, N * d.maxn, "nbr_p");
+         h.dalloc(&d.ord, N, "ord") && h.dalloc(&d.nbr_p, N * std::max(d.maxn, 2), "nbr_p");
   else
     ok = ok && h.dalloc(&d.iaa, N, "iaa") &&
          h.dalloc(&d.s_mv, N, "s_mv") && h.dalloc(&d.s_nxy, N, "s_nxy");

@@ -194,6 +194,15 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
                                                     const StepScalars* __restrict__ tab,
                                                     int row, int pos) {
   constexpr bool kPred = (MODE == PASS_CORR_STRAIN || MODE == PASS_CORR_RESIZE);
+  // the list is column-major: entry k of this slot sits k * ntot words further on; Lst walks
+  // it, two entries ahead.  The first two are loaded beside the list's length, not after it
+  // (a list has room for two entries at least; they are used up to its length): 1.88 ->
+  // 1.84 ms for 20 steps at 2^20 particles.
+  const unsigned* __restrict__ Lst = reinterpret_cast<const unsigned*>(d.nbr_p) + pos;
+  const int stride = d.ntot;
+  unsigned e1 = __ldg(Lst);
+  Lst += stride;
+  unsigned e2 = __ldg(Lst);
   // the slot this thread works on (lists ordered by length) and its list's length
   const unsigned on = d.ord[pos];
   const int i = pos - pos % kOrderWindow + (int)(on % kOrderWindow);
@@ -217,18 +226,15 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
 #define SC_REC(k) (COH ? __ldcg(REC + (k)) : REC[(k)])
   const float4 ri = SC_REC(i);
   const float4 pai = d.pa[i];  // (R, A, RC, 1/I)
-  // the list is column-major: entry k of this slot sits k * ntot words further on;
-  // Lst walks it, two entries ahead of the pair being computed
-  const unsigned* __restrict__ Lst = reinterpret_cast<const unsigned*>(d.nbr_p) + pos;
-  const int stride = d.ntot;
-
   float fx = 0.f, fy = 0.f, tq = 0.f;
-  // software pipeline: the list entry two ahead and the neighbour data one ahead
-  // are in flight while the current pair is computed
-  unsigned e1 = cnt > 0 ? __ldg(Lst) : 0u;
-  Lst += stride;
-  unsigned e2 = cnt > 1 ? __ldg(Lst) : 0u;
-  // the neighbour's record and radius (its A^2 is |shaft|^2 from the record)
+  // kAhead: the next neighbour's record and radius (its A^2 is |shaft|^2 from the record)
+  // are in flight while a pair is computed; else they are loaded after it, which takes fewer
+  // registers and moves.  Without it 20 shear steps take 1.68 ms instead of 1.84 at 2^20
+  // particles and 2.66 instead of 2.72 on the 512-system ensemble; with it 20 affine steps
+  // take 0.296 ms instead of 0.306 at 49999, and 50 two-point FIRE iterations (long pairs)
+  // 4.38 ms instead of 4.41 at 524288.  The persistent kernels, whose few blocks need their
+  // loads in flight, keep it too.
+  constexpr bool kAhead = COH || TWO || MODE == PASS_PRED_RESIZE || MODE == PASS_CORR_RESIZE;
   float4 r1 = make_float4(0.f, 0.f, 0.f, 0.f);
   float R1 = 0.f;
   if (cnt > 0) {
@@ -241,7 +247,7 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
     const float4 rj = r1;
     const float Rj = R1;
     e1 = e2;
-    if (k + 1 < cnt) {
+    if (kAhead && k + 1 < cnt) {
       r1 = SC_REC(e1 & kSlotMask);
       R1 = d.rf[e1 & kSlotMask];
     }
@@ -261,10 +267,16 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
         two_point ? pair2_fp32(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, pai.x + Rj, gam, o)
                   : pair_fp32<false>(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, pai.x + Rj, gam,
                                      false, o);
-    if (!touch) continue;
-    fx += o.fx;
-    fy += o.fy;
-    tq += o.tp;
+    if (touch) {
+      fx += o.fx;
+      fy += o.fy;
+      tq += o.tp;
+    }
+    if (!kAhead) {
+      if (k + 1 == cnt) break;
+      r1 = SC_REC(e1 & kSlotMask);
+      R1 = d.rf[e1 & kSlotMask];
+    }
   }
 
 #undef SC_REC
@@ -276,7 +288,7 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
 // pair and bytes a particle: quotients without the scaling around subnormals, offsets
 // without conversions, no image test and no system lookup where they are not needed, and a
 // state of 115 B a particle, which at 2^20 particles about fits the L2 (129 MB; it was 141
-// B).  45 -> 37 us a pass at 2^20 particles (corrector and predictor, mean), 37 -> 31 on the
+// B).  45 -> 33 us a pass at 2^20 particles (corrector and predictor, mean), 37 -> 29 on the
 // 512-system ensemble.  Blocks an SM: 12 (40 registers) against 10, 1905 and 1933 us for 20
 // steps at 2^20; the affine passes, which spill more, 305 and 297 us at 49999.  Prefetching
 // the epilogue's state before the loop was 3% slower.
