@@ -559,7 +559,10 @@ __device__ __forceinline__ int list_candidates(const Dev& d, const SysGeom& g, i
 // Small handles rebuild in blocks of 128 threads, large ones in blocks of 512 (the fewer
 // blocks, the cheaper a barrier); eight threads a slot where there are that many, up to the
 // blocks that are resident.  Up to kLaneItems work items, eight threads list a slot's
-// neighbours: one or two rounds of them.
+// neighbours, at most two and a half rounds of them.  A forced rebuild with its call, us,
+// with eight and with one thread a slot: FP64 52 and 64 at 8192 particles, 60 and 76 at
+// 16384, 64 and 76 at 30000, 67 and 76 at 45000, 77 and 77 at 70000; mixed 52 and 54, 53
+// and 64, 64 and 64, 66 and 66, 77 and 66.
 constexpr int kSmallRebuild = 4096;
 constexpr int kLaneItems = 49152;
 
