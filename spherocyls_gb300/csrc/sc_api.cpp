@@ -303,8 +303,8 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
   else
     ok = ok && h.dalloc(&d.iaa, N, "iaa") &&
          h.dalloc(&d.s_mv, N, "s_mv") && h.dalloc(&d.s_nxy, N, "s_nxy");
-  ok = ok && h.dalloc(&d.gbar, sc::BAR_WORDS, "grid barriers") &&
-       h.cuda_ok(cudaMemsetAsync(d.gbar, 0, sc::BAR_WORDS * sizeof *d.gbar, h.stream), "barriers");
+  ok = ok && h.dalloc(&d.gbar, 2, "grid barrier") &&
+       h.cuda_ok(cudaMemsetAsync(d.gbar, 0, 2 * sizeof *d.gbar, h.stream), "barrier");
   if (opt.precision == SC_PREC_MIXED) ok = ok && h.dalloc(&h.d_persist, 1, "persist out");
   if (d.pass_kind == 1)
     ok = ok && h.dalloc(&d.t_own, N * sc::kTileEPP, "tile owners") &&
@@ -578,27 +578,8 @@ int sc_autotune(sc_handle* H, int steps, double* pad_factor, int* block) {
   const int kind = best.kind == SC_PASS_TILE ? 1 : 0;
   const bool relayout = best.f != 1.0 || kind != h.d.pass_kind ||
                         (kind == 1 && best.target != h.opt.tile_target);
-  if (relayout) {
-    if (!h.materialize()) return h.last_status;
-    if (kind == 1 && !h.d.t_own) {
-      const size_t N = h.ntot;
-      if (!h.dalloc(&h.d.t_own, N * sc::kTileEPP, "tile owners") ||
-          !h.dalloc(&h.d.t_pe, N * sc::kTileEPP, "tile partners") ||
-          !h.dalloc(&h.d.t_rd, N * sc::kTileEPP, "tile reads") ||
-          !h.dalloc(&h.d.t_meta, N, "tile meta") ||
-          !h.dalloc(&h.d.t_pb, N * sc::kTileEPP, "tile pair results"))
-        return h.last_status;
-    }
-    h.d.pass_kind = kind;
-    h.opt.pass_kind = best.kind;
-    h.opt.tile_target = best.target;
-    for (int s = 0; s < ns; s++) {
-      h.hs[s].pad = best.f * pad0[s];
-      h.hs[s].configure(false);
-    }
-    if (!h.layout_cells() || !h.rebuild_all() || !h.check_status("sc_autotune"))
-      return h.last_status;
-  }
+  for (int s = 0; s < ns; s++) pads[s] = best.f * pad0[s];
+  if (relayout && !h.set_pass(kind, best.target, pads)) return h.last_status;
   h.block = best.block;
   h.opt.block = best.block;
   h.opt.persist_steps = best.persist;

@@ -429,6 +429,26 @@ bool Handle::rebuild_all() {
   return cuda_ok(cudaGetLastError(), "rebuild launch");
 }
 
+bool Handle::set_pass(int kind, int target, const std::vector<double>& pads) {
+  if (!materialize()) return false;
+  if (kind == 1 && !d.t_own) {
+    const size_t N = ntot;
+    if (!dalloc(&d.t_own, N * kTileEPP, "tile owners") ||
+        !dalloc(&d.t_pe, N * kTileEPP, "tile partners") ||
+        !dalloc(&d.t_rd, N * kTileEPP, "tile reads") || !dalloc(&d.t_meta, N, "tile meta") ||
+        !dalloc(&d.t_pb, N * kTileEPP, "tile pair results"))
+      return false;
+  }
+  d.pass_kind = kind;
+  opt.pass_kind = kind == 1 ? SC_PASS_TILE : SC_PASS_LIST;
+  opt.tile_target = target;
+  for (int s = 0; s < nsys; s++) {
+    hs[s].pad = pads[s];
+    hs[s].configure(false);
+  }
+  return layout_cells() && rebuild_all() && check_status("pass change");
+}
+
 void Handle::launch_pass(int mode, bool se, int row, bool fast) {
   Dev dd = d;
   dd.skip = pass_skip;

@@ -154,6 +154,8 @@ struct Handle {
   bool ensure_se_hist(int nrec);
   bool check_status(const char* where);
   bool rebuild_all();
+  // mixed form: change the force pass (0 list, 1 tile), its tile size and the paddings
+  bool set_pass(int kind, int target, const std::vector<double>& pads);
   void launch_pass(int mode, bool se, int row, bool fast = false);
   cudaEvent_t next_event();
   void timed(int kind, bool on, const std::function<void()>& f);

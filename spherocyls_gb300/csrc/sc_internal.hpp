@@ -219,7 +219,7 @@ struct Dev {
   // compute entries (owner-major) and read entries live in the slot range of its
   // particles times kTileEPP; a pair inside the tile is computed by its lower slot
   // and read back by the other partner from the pair results.
-  unsigned long long* gbar; // [BAR_WORDS] counters of the cooperative kernels
+  unsigned long long* gbar; // [2] counters of the running cooperative kernel (GridBarrier)
   const int* skip;          // [nsys] or null: force passes leave systems with skip[s] != 0
                             // alone (converged minimiser systems)
   int small_grid;           // some system's grid has fewer than three cells a side
@@ -276,9 +276,6 @@ enum { ST_NBR_OVERFLOW = 1, ST_NAN = 2, ST_CELL_OVERFLOW = 4, ST_BARRIER_TIMEOUT
 // loads (of about half a microsecond each) a block waits at a grid barrier before it gives
 // up and records ST_BARRIER_TIMEOUT
 constexpr unsigned kBarrierSpins = 1u << 22;
-// Dev::gbar: the barriers of the rebuild and of the persistent kernels, the blocks that
-// are done with a rebuild
-enum { BAR_REBUILD = 0, BAR_STEPS = 1, BAR_FIRE = 2, BAR_DONE = 3, BAR_WORDS = 4 };
 
 constexpr int kScanChunk = 1024;  // cells per scan chunk
 constexpr int kSeChunk = 1024;    // particles per reduction chunk
@@ -386,17 +383,16 @@ void launch_mx_se64(const Dev& d, const StepScalars* tab, int row, cudaStream_t 
 
 #ifdef __CUDACC__
 // Grid barrier of a cooperative kernel (thread 0 of each block arrives): a counter that
-// only grows, so that arriving is one reduction and waiting one load, 1.3 us with 152
-// blocks and 1.8 us with 456 (a count and a generation: 2.1 and 2.5 us).  A counter serves
-// one kernel of a handle, whose grid is always the same, so a multiple of the grid is where
-// the launch found it.  The wait is bounded: a barrier that times out records
+// only grows during a launch, so that arriving is one reduction and waiting one load, 1.3 us
+// with 152 blocks and 1.8 us with 456 (a count and a generation: 2.1 and 2.5 us).  A launch
+// finds it at zero: every block leaves (leave), and the last one out takes the counters back
+// for the next launch, which may be another kernel with another grid (the force pass of a
+// handle can change).  The wait is bounded: a barrier that times out records
 // ST_BARRIER_TIMEOUT and returns false.
 struct GridBarrier {
-  unsigned long long* count;
+  unsigned long long* count;  // [0] arrivals, [1] blocks that have left
   unsigned long long target;
-  __device__ __forceinline__ explicit GridBarrier(unsigned long long* c) : count(c), target(0) {
-    if (threadIdx.x == 0) target = load() / gridDim.x * gridDim.x;
-  }
+  __device__ __forceinline__ explicit GridBarrier(unsigned long long* c) : count(c), target(0) {}
   __device__ __forceinline__ unsigned long long load() const {
     unsigned long long v;
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(count) : "memory");
@@ -418,6 +414,23 @@ struct GridBarrier {
       }
     }
     return __syncthreads_and(ok) != 0;
+  }
+  // Once per block, after its last wait; true (in all its threads) for the last block out,
+  // which sees what every block wrote.
+  __device__ __forceinline__ bool leave() {
+    __shared__ int last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      last = atomicAdd(&count[1], 1ull) == gridDim.x - 1;
+      if (last) {
+        count[0] = 0;
+        count[1] = 0;
+        __threadfence();
+      }
+    }
+    __syncthreads();
+    return last != 0;
   }
 };
 // Corrector passes, block 0 before any early exit: flag the systems that set gamma back

@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_rebuild64(Dev d,
                                                              const StepScalars* __restrict__ tab,
                                                              int row, int moved) {
   if (!rb::pending(d)) return;
-  GridBarrier bar(d.gbar + BAR_REBUILD);
+  GridBarrier bar(d.gbar);
   const rb::Work<BS> work(d);
   const bool ok = rb::sort_cells<false, BS>(
       d, work, tab, row, moved != 0, bar,
@@ -144,7 +144,10 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_rebuild64(Dev d,
         d.rsf[i] = (float)(ra.x + ra.y);
         d.iaa[i] = shared_rcp(ra.y * ra.y);
       });
-  if (!ok) return;
+  if (!ok) {
+    bar.leave();
+    return;
+  }
   if (work.items > kLaneItems) {
     work.each(d, [&](int i, int s) { build_nbrs<1>(d, tab, row, i, s, 0, 0u, nullptr); });
   } else {
@@ -156,7 +159,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_rebuild64(Dev d,
         build_nbrs<8>(d, tab, row, i, s, threadIdx.x & 7, lanes, &table[threadIdx.x / 8]);
     }
   }
-  rb::finish(d);
+  rb::finish(d, bar);
 }
 
 // ---- the FP32 screen ----

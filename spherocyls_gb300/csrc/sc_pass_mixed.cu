@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(
 template <bool TWO>
 __global__ void __launch_bounds__(128, TWO ? 6 : 12) k_persist_steps(
     Dev d, const StepScalars* __restrict__ tab, int row0, int nsteps, int* out) {
-  GridBarrier bar(d.gbar + BAR_STEPS);
+  GridBarrier bar(d.gbar);
   const int stride = gridDim.x * blockDim.x;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
   int k = 0, stopped = 0;
@@ -343,6 +343,7 @@ __global__ void __launch_bounds__(128, TWO ? 6 : 12) k_persist_steps(
       pass_mixed_position<PASS_PRED_STRAIN, TWO, true, false, true>(d, tab, row, pos);
     bar.wait(d.status);
   }
+  bar.leave();
   if (t0 == 0) *out = 2 * k + stopped;
 }
 
@@ -362,7 +363,7 @@ template <bool TWO>
 __global__ void __launch_bounds__(256, TWO ? 3 : 4) k_persist_fire(
     Dev d, FireState f, const StepScalars* __restrict__ tab, double ftol, double dt_max,
     int iters, int* out) {
-  GridBarrier bar(d.gbar + BAR_FIRE);
+  GridBarrier bar(d.gbar);
   const int stride = gridDim.x * blockDim.x;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
   int k = 0, why = 0;
@@ -393,6 +394,7 @@ __global__ void __launch_bounds__(256, TWO ? 3 : 4) k_persist_fire(
       break;
     }
   }
+  bar.leave();
   if (t0 == 0) *out = 4 * k + why;
 }
 
@@ -891,14 +893,17 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_rebuild_mx(Dev d,
                                                               const StepScalars* __restrict__ tab,
                                                               int row, int moved) {
   if (!rb::pending(d)) return;
-  GridBarrier bar(d.gbar + BAR_REBUILD);
+  GridBarrier bar(d.gbar);
   const rb::Work<BS> work(d);
   const bool ok = rb::sort_cells<true, BS>(
       d, work, tab, row, moved != 0, bar,
       [&](int i, int s, double2 p, double phi, double2 ra, double2 irc, int, int cell) {
         local_record(d, tab, row, i, s, p, phi, ra, irc, cell);
       });
-  if (!ok || !LISTS) return;
+  if (!ok || !LISTS) {
+    bar.leave();
+    return;
+  }
   const bool by_lanes = work.items <= kLaneItems;
   if (by_lanes) {
     __shared__ Candidates table[BS / 8];
@@ -908,7 +913,10 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_rebuild_mx(Dev d,
       if (work.at(d, g, &i, &s))
         build_list_lanes(d, tab, row, i, s, threadIdx.x & 7, lanes, table[threadIdx.x / 8]);
     }
-    if (!bar.wait(d.status)) return;
+    if (!bar.wait(d.status)) {
+      bar.leave();
+      return;
+    }
   }
   __shared__ OrderScratch scratch[BS / kOrderWindow];
   const int w0 = threadIdx.x / kOrderWindow * kOrderWindow, in = threadIdx.x - w0;
@@ -921,7 +929,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_rebuild_mx(Dev d,
     }
     order_window(d, i, scratch[w0 / kOrderWindow], w0, 1 + w0 / kOrderWindow);
   }
-  rb::finish(d);
+  rb::finish(d, bar);
 }
 
 inline int nblk(int n, int b) { return (n + b - 1) / b; }

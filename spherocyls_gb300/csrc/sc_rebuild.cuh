@@ -458,23 +458,16 @@ __device__ __forceinline__ void put_back(const Dev& d, const Work<BS>& work, boo
   });
 }
 
-// The last block to arrive takes back the flags and counts the rebuild.
-__device__ __forceinline__ void finish(const Dev& d) {
-  __shared__ int last;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(&d.gbar[BAR_DONE], 1ull) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last) return;
+// The end of a rebuild: the last block out takes back the flags and counts it, unless a
+// barrier timed out on the way.
+__device__ __forceinline__ void finish(const Dev& d, GridBarrier& bar) {
+  if (!bar.leave() || (*(volatile int*)d.status & ST_BARRIER_TIMEOUT)) return;
   for (int s = threadIdx.x; s < d.nsys; s += blockDim.x) {
     d.flags[s] = 0;
     d.istar[s] = kNoTrigger;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    d.gbar[BAR_DONE] = 0;
     *d.any = 0;
     d.status[1] += 1;  // rebuilds executed
   }
