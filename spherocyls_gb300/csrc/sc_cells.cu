@@ -12,7 +12,7 @@ namespace {
 constexpr double kRefPi = 3.14159265358979;  // src/cpp/spherocyl_box.cpp:12
 
 __global__ void k_rb_clear(Dev d) {
-  if (*d.any == 0) return;
+  if (!rebuild_pending(d)) return;
   for (int s = threadIdx.x; s < d.nsys; s += blockDim.x) {
     d.flags[s] = 0;
     d.istar[s] = kNoTrigger;

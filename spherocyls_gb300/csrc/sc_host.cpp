@@ -212,6 +212,8 @@ bool Handle::layout_cells() {
     int *cs = nullptr, *cn = nullptr, *cf = nullptr;
     if (!dalloc(&cs, cap, "cell_start") || !dalloc(&cn, cap, "cell_count") ||
         !dalloc(&cf, cap, "cell_fill") ||
+        !cuda_ok(cudaMemsetAsync(cs, 0, cap * sizeof(int), stream), "cell_start") ||
+        !cuda_ok(cudaMemsetAsync(cn, 0, cap * sizeof(int), stream), "cell_count") ||
         !cuda_ok(cudaMemsetAsync(cf, 0, cap * sizeof(int), stream), "cell_fill"))
       return false;
     d.cell_fill = cf;
@@ -931,6 +933,7 @@ bool Handle::run_persist(int nk, int done, int se_every) {
       const int v = h_pinned[3];
       const int m = v >> 1;
       if (m < 0 || m > kp - k + 1 || (m == kp - k + 1 && (v & 1))) {
+        if (!check_status("persistent steps")) return false;
         fail(SC_E_STATE, "persistent step kernel returned %d", v);
         return false;
       }

@@ -382,6 +382,14 @@ bool launch_persist_fire(const Dev& d, const FireState& f, const StepScalars* ta
 void launch_mx_se64(const Dev& d, const StepScalars* tab, int row, cudaStream_t st);
 
 #ifdef __CUDACC__
+// Whether there is anything to rebuild.  After a barrier that timed out the cells may be
+// incomplete, and nothing is rebuilt any more (the host reports the status).
+__device__ __forceinline__ bool timed_out(const Dev& d) {
+  return (*(const volatile int*)d.status & ST_BARRIER_TIMEOUT) != 0;
+}
+__device__ __forceinline__ bool rebuild_pending(const Dev& d) {
+  return *d.any != 0 && !timed_out(d);
+}
 // Grid barrier of a cooperative kernel (thread 0 of each block arrives): a counter that
 // only grows during a launch, so that arriving is one reduction and waiting one load, 1.3 us
 // with 152 blocks and 1.8 us with 456 (a count and a generation: 2.1 and 2.5 us).  A launch

@@ -130,7 +130,7 @@ template <int BS>
 __global__ void __launch_bounds__(BS, 1024 / BS) k_rebuild64(Dev d,
                                                              const StepScalars* __restrict__ tab,
                                                              int row, int moved) {
-  if (!rb::pending(d)) return;
+  if (!rebuild_pending(d)) return;
   GridBarrier bar(d.gbar);
   const rb::Work<BS> work(d);
   const bool ok = rb::sort_cells<false, BS>(

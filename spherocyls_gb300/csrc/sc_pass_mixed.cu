@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(
 // barrier.  A step whose corrector requests a rebuild (or whose row sets gamma back)
 // ends the launch after that corrector; the host runs the rebuild and the predictor
 // and relaunches.  Every wait is bounded (kBarrierSpins): a barrier that times out
-// records ST_BARRIER_TIMEOUT, which the host reports as an error.
+// records ST_BARRIER_TIMEOUT and ends the launch, which the host reports as an error.
 
 template <bool TWO>
 __global__ void __launch_bounds__(128, TWO ? 6 : 12) k_persist_steps(
@@ -323,7 +323,8 @@ __global__ void __launch_bounds__(128, TWO ? 6 : 12) k_persist_steps(
   const int stride = gridDim.x * blockDim.x;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
   int k = 0, stopped = 0;
-  for (; k < nsteps; k++) {
+  bool ok = __syncthreads_and(!timed_out(d)) != 0;  // (a wait of an earlier launch: stop here)
+  for (; ok && k < nsteps; k++) {
     const int row = row0 + k;
     // systems that set gamma back at this step rebuild after its corrector
     if (blockIdx.x == 0)
@@ -334,17 +335,17 @@ __global__ void __launch_bounds__(128, TWO ? 6 : 12) k_persist_steps(
         }
     for (int pos = t0; pos < d.ntot; pos += stride)
       pass_mixed_position<PASS_CORR_STRAIN, TWO, true, false, true>(d, tab, row, pos);
-    bar.wait(d.status);
+    if (!(ok = bar.wait(d.status))) break;
     if (*(volatile int*)d.any != 0) {  // the same value in every block after the barrier
       stopped = 1;
       break;
     }
     for (int pos = t0; pos < d.ntot; pos += stride)
       pass_mixed_position<PASS_PRED_STRAIN, TWO, true, false, true>(d, tab, row, pos);
-    bar.wait(d.status);
+    if (!(ok = bar.wait(d.status))) break;
   }
   bar.leave();
-  if (t0 == 0) *out = 2 * k + stopped;
+  if (t0 == 0) *out = ok ? 2 * k + stopped : -1;
 }
 
 // ---- persistent FIRE ----
@@ -356,7 +357,8 @@ __global__ void __launch_bounds__(128, TWO ? 6 : 12) k_persist_steps(
 // and the iterates equal those of the graph and eager paths bit for bit.  The launch
 // ends after `iters` iterations, after the iteration whose update asks for a
 // rebuild (the host runs it), or at the iteration in which the last system
-// converges: *out = 4 * iterations + (0 all ran, 1 rebuild pending, 2 all converged).
+// converges: *out = 4 * iterations + (0 all ran, 1 rebuild pending, 2 all converged), -1
+// after a barrier that timed out.
 static_assert(fire::kFireBlock == 256, "the persistent FIRE blocks are the reduction blocks");
 
 template <bool TWO>
@@ -367,18 +369,19 @@ __global__ void __launch_bounds__(256, TWO ? 3 : 4) k_persist_fire(
   const int stride = gridDim.x * blockDim.x;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
   int k = 0, why = 0;
-  while (k < iters) {
+  bool ok = __syncthreads_and(!timed_out(d)) != 0;  // (a wait of an earlier launch: stop here)
+  while (ok && k < iters) {
     for (int pos = t0; pos < d.ntot; pos += stride)
       pass_mixed_position<PASS_FORCE, TWO, true, false, true>(d, tab, 0, pos);
-    bar.wait(d.status);
+    if (!(ok = bar.wait(d.status))) break;
     for (int ch = blockIdx.x; ch < d.npchunks; ch += gridDim.x) {
       fire::fire_chunk<true>(d, f, ch);
       __syncthreads();  // the next chunk reuses the block's shared partials
     }
-    bar.wait(d.status);
+    if (!(ok = bar.wait(d.status))) break;
     // one block per system (the block has kFireBlock threads)
     for (int s = blockIdx.x; s < d.nsys; s += gridDim.x) fire::fire_sys(d, f, s, ftol, dt_max);
-    bar.wait(d.status);
+    if (!(ok = bar.wait(d.status))) break;
     k++;
     // every block sees the same flags: they change only in the phase before the barrier
     int pending = 0;
@@ -388,14 +391,14 @@ __global__ void __launch_bounds__(256, TWO ? 3 : 4) k_persist_fire(
       break;
     }
     for (int i = t0; i < d.ntot; i += stride) fire::fire_update<true>(d, f, i);
-    bar.wait(d.status);
+    if (!(ok = bar.wait(d.status))) break;
     if (*(volatile int*)d.any != 0) {
       why = 1;
       break;
     }
   }
   bar.leave();
-  if (t0 == 0) *out = 4 * k + why;
+  if (t0 == 0) *out = ok ? 4 * k + why : -1;
 }
 
 template <int MODE, bool TWO>
@@ -552,7 +555,7 @@ __device__ __forceinline__ int tile_excl_scan(int v, int* sh, int* total) {
 // among the partner's.  A pair listed by one side only (the capsule test's rounding
 // at the padding's edge, far from contact) is computed by nobody.
 __global__ void __launch_bounds__(kTileThreads) k_tile_lists(Dev d) {
-  if (*d.any == 0) return;
+  if (!rebuild_pending(d)) return;
   const int4 tl = d.tiles[blockIdx.x];
   if (d.flags[tl.x] == 0) return;
   __shared__ int sh[32];
@@ -804,7 +807,7 @@ __device__ __forceinline__ void build_list_lanes(const Dev& d, const StepScalars
 
 __global__ void __launch_bounds__(128, 12) k_mx_build_list(Dev d, const StepScalars* __restrict__ tab,
                                                       int row) {
-  if (*d.any == 0) return;
+  if (!rebuild_pending(d)) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.ntot || d.flags[d.psys[i]] == 0) return;
   build_list_slot(d, tab, row, i, d.psys[i]);
@@ -892,7 +895,7 @@ template <bool LISTS, int BS>
 __global__ void __launch_bounds__(BS, 1024 / BS) k_rebuild_mx(Dev d,
                                                               const StepScalars* __restrict__ tab,
                                                               int row, int moved) {
-  if (!rb::pending(d)) return;
+  if (!rebuild_pending(d)) return;
   GridBarrier bar(d.gbar);
   const rb::Work<BS> work(d);
   const bool ok = rb::sort_cells<true, BS>(

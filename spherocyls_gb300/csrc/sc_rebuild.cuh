@@ -461,7 +461,7 @@ __device__ __forceinline__ void put_back(const Dev& d, const Work<BS>& work, boo
 // The end of a rebuild: the last block out takes back the flags and counts it, unless a
 // barrier timed out on the way.
 __device__ __forceinline__ void finish(const Dev& d, GridBarrier& bar) {
-  if (!bar.leave() || (*(volatile int*)d.status & ST_BARRIER_TIMEOUT)) return;
+  if (!bar.leave() || timed_out(d)) return;
   for (int s = threadIdx.x; s < d.nsys; s += blockDim.x) {
     d.flags[s] = 0;
     d.istar[s] = kNoTrigger;
@@ -471,12 +471,6 @@ __device__ __forceinline__ void finish(const Dev& d, GridBarrier& bar) {
     *d.any = 0;
     d.status[1] += 1;  // rebuilds executed
   }
-}
-
-// Whether there is anything to rebuild.  After a barrier that timed out the cells may be
-// incomplete, and nothing is rebuilt any more (the host reports the status).
-__device__ __forceinline__ bool pending(const Dev& d) {
-  return *d.any != 0 && !(d.status[0] & ST_BARRIER_TIMEOUT);
 }
 
 // The phases up to the records; false when a barrier timed out.
