@@ -301,13 +301,17 @@ __device__ __forceinline__ bool pair_fp32(float dX, float dY, float nxA, float n
   return true;
 }
 
+constexpr float kMinNormal = 1.17549435e-38f;  // the smallest normal FP32 number
+
 // Conservative FP32 screen: false only when the two spines (P at the origin, Q at
 // -D in the sheared, minimum-image frame) are certainly farther apart than sig.
 // The closest-point parameters come from the cross-product form; an error in them
 // only moves the evaluated point pair along the spines, which can only raise the
 // distance by the spines' misalignment angle times their length, and both that and
 // the FP32 rounding of the distance stay far below the 1e-4 relative margin.  Both
-// contact rules need the minimum distance below sig for any contact.
+// contact rules need the minimum distance below sig for any contact.  A spine P whose
+// squared length is no normal number is a point (a disc), and the closest point to it is
+// looked for on Q: the first formula, which looks along P, says nothing about Q then.
 __device__ __forceinline__ bool may_touch_fp32(float dX, float dY, float nxA, float nyA,
                                                float nxB, float nyB, float sig) {
   float a = fmaf(nxA, nxA, nyA * nyA), c = fmaf(nxB, nxB, nyB * nyB);
@@ -319,8 +323,8 @@ __device__ __forceinline__ bool may_touch_fp32(float dX, float dY, float nxA, fl
   float w2 = nyA * dX;
   float uxD = fmaf(nxA, dY, -w2) + fmaf(-nyA, dX, w2);
   float t = uxv == 0.f ? -1.f : fminf(fmaxf(div_fast(uxD, uxv), -1.f), 1.f);
-  float s = a > 0.f ? -div_fast(b * t + d, a) : 0.f;
-  float sarg = fabsf(s);
+  float s = a >= kMinNormal ? -div_fast(b * t + d, a) : 0.f;
+  float sarg = a >= kMinNormal ? fabsf(s) : 2.f;
   s = fminf(fmaxf(s, -1.f), 1.f);
   if (sarg > 1.f && c > 0.f) t = fminf(fmaxf(-div_fast(b * s + e, c), -1.f), 1.f);
   float dDx = dX + s * nxA - t * nxB;
@@ -344,8 +348,8 @@ __device__ __forceinline__ bool capsules_within(float dX, float dY, float nxA, f
   const float w2 = nyA * dX;
   const float uxD = fmaf(nxA, dY, -w2) + fmaf(-nyA, dX, w2);
   float t = uxv == 0.f ? -1.f : fminf(fmaxf(div_fast(uxD, uxv), -1.f), 1.f);
-  float s = a > 0.f ? -div_fast(b * t + d, a) : 0.f;
-  const float sarg = fabsf(s);
+  float s = a >= kMinNormal ? -div_fast(b * t + d, a) : 0.f;
+  const float sarg = a >= kMinNormal ? fabsf(s) : 2.f;  // a point: see may_touch_fp32
   s = fminf(fmaxf(s, -1.f), 1.f);
   if (sarg > 1.f && c > 0.f) t = fminf(fmaxf(-div_fast(b * s + e, c), -1.f), 1.f);
   const float x = dX + s * nxA - t * nxB, y = dY + s * nyA - t * nyB;
