@@ -104,22 +104,29 @@ __device__ __forceinline__ double qdiv(double x, double y, double inv_y) {
   return FAST ? x * inv_y : div_by(x, y, inv_y);
 }
 
-// Reciprocals of a = |u_A|^2, c = |u_B|^2, delta and sig from one division.
+// Reciprocals of a = |u_A|^2, c = |u_B|^2, delta and sig from one division; from one each
+// where their product is zero (a disc has a = 0) or near the ends of the exponent range.
 struct Recip64 {
   double a, c, delta, sig;
 };
 __device__ __forceinline__ Recip64 recip64(double a, double c, double delta, double sig) {
   Recip64 r;
   const double ac = a * c;
-  if (delta > 0) {
-    const double inv = 1.0 / (ac * delta * sig);
+  const double all = delta > 0 ? ac * delta * sig : ac * sig;
+  if ((unsigned)__double2hiint(all) - 0x01700000u >= 0x7d200000u) {  // not 2^-1000 to 2^1000
+    r.a = 1.0 / a;
+    r.c = 1.0 / c;
+    r.delta = delta > 0 ? 1.0 / delta : 0.0;
+    r.sig = 1.0 / sig;
+  } else if (delta > 0) {
+    const double inv = 1.0 / all;
     const double i_ac = delta * sig * inv;
     r.delta = ac * sig * inv;
     r.sig = ac * delta * inv;
     r.a = c * i_ac;
     r.c = a * i_ac;
   } else {
-    const double inv = 1.0 / (ac * sig);
+    const double inv = 1.0 / all;
     r.delta = 0.0;
     r.sig = ac * inv;
     r.a = c * sig * inv;

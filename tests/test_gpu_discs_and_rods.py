@@ -61,3 +61,37 @@ def test_forces_of_discs_among_rods(sc, oracle_built, precision, contacts, kw, o
                          **kw) as b:
         b.calc_forces()
         _check(np.array(b.forces()), want, TOL[precision])
+
+
+def _shapes(sc, order):
+    pack = _pack(sc, 600, "mixed" if order in ("all", "short") else order)
+    if order in ("all", "short"):  # discs alone; shafts whose squares' products underflow
+        pack = (*pack[:5], np.full_like(pack[5], 0.0 if order == "all" else 1e-80))
+    return pack
+
+
+@pytest.mark.parametrize("contacts", [1, 2])
+@pytest.mark.parametrize("order", ["mixed", "low", "high", "all", "short"])
+def test_minimiser_forces_of_discs(sc, oracle_built, order, contacts):
+    """The minimiser's form of the FP64 pair code (shared reciprocals): the largest force of
+    the first FIRE iteration, to 1e-9."""
+    pack = _shapes(sc, order)
+    L, x, y, p, R, A = pack
+    want = _oracle(oracle_built, pack, 0.3, contacts)
+    inertia = oracle_built.OracleBox(L, x, y, p, A, R, 0.3).consts()[0]
+    big = np.sqrt(np.maximum(want[0] ** 2 + want[1] ** 2, want[2] ** 2 / inertia).max())
+    with sc.SpherocylBox(L, x, y, p, A, R, 0.3, contacts=contacts) as b:
+        _, fm, _ = b.fire_minimize(1e-30, 1, dt0=1e-9, dt_max=1e-9)
+    assert abs(fm[0] - big) <= 1e-9 * big
+
+
+@pytest.mark.parametrize("contacts", [1, 2])
+@pytest.mark.parametrize("order", ["mixed", "low", "high", "all"])
+def test_mixed_stress_of_discs(sc, order, contacts):
+    """The mixed form's FP64 stress record against the FP64 form's, to 1e-9."""
+    L, x, y, p, R, A = _shapes(sc, order)
+    se = []
+    for precision in ("fp64", "mixed"):
+        with sc.SpherocylBox(L, x, y, p, A, R, 0.3, precision=precision, contacts=contacts) as b:
+            se.append(np.array(b.calc_se()).ravel())
+    assert np.abs(se[1] - se[0]).max() <= 1e-9 * np.abs(se[0]).max()
