@@ -149,9 +149,9 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
   }
   if (!summing) sum_areas();
   // The input checks and per system the largest R and A (set_particle,
-  // src/cpp/spherocyl_box.cpp:216-219) on worker threads over slices of the caller's
-  // arrays.
-  std::vector<double> rmax(n_sys, 0.0), amax(n_sys, 0.0);
+  // src/cpp/spherocyl_box.cpp:216-219) and the smallest A, on worker threads over slices of
+  // the caller's arrays.
+  std::vector<double> rmax(n_sys, 0.0), amax(n_sys, 0.0), amin(n_sys, HUGE_VAL);
   {
     std::vector<int> p0s(n_sys + 1, 0);
     for (int s = 0; s < n_sys; s++) p0s[s + 1] = p0s[s] + n_per_sys[s];
@@ -159,13 +159,14 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
     const int nthreads = ntot < (1 << 16) ? 1 : (int)std::min(8u, std::max(1u, hw));
     struct Part {
       int fin = 1, shp = 1;  // all finite; every R > 0 and A >= 0
-      std::vector<double> rm, am;
+      std::vector<double> rm, am, an;
     };
     std::vector<Part> parts(nthreads);
     auto scan = [&](int w) {
       Part& P = parts[w];
       P.rm.assign(n_sys, 0.0);
       P.am.assign(n_sys, 0.0);
+      P.an.assign(n_sys, HUGE_VAL);
       const int a0 = (int)((long long)ntot * w / nthreads);
       const int a1 = (int)((long long)ntot * (w + 1) / nthreads);
       int s = (int)(std::upper_bound(p0s.begin(), p0s.end(), a0) - p0s.begin()) - 1;
@@ -177,6 +178,7 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
                (int)std::isfinite(phi[i]) & (int)std::isfinite(r) & (int)std::isfinite(a);
         shp &= (int)(r > 0) & (int)(a >= 0);
         if (a > P.am[s]) P.am[s] = a;
+        if (a < P.an[s]) P.an[s] = a;
         if (r > P.rm[s]) P.rm[s] = r;
       }
       P.fin = fin;
@@ -201,6 +203,7 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
       for (int s = 0; s < n_sys; s++) {
         rmax[s] = std::max(rmax[s], P.rm[s]);
         amax[s] = std::max(amax[s], P.am[s]);
+        amin[s] = std::min(amin[s], P.an[s]);
       }
     }
     if (!finite) {
@@ -247,6 +250,7 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
     S.Ly = Ly[s];
     S.pad = pad ? pad[s] : 0.0;
     S.Amax = amax[s];
+    S.Amin = amin[s];
     S.Rmax = rmax[s];
     S.configure(true);
     p0 += S.n;
@@ -258,6 +262,8 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
   d.ntot = ntot;
   d.nsys = n_sys;
   d.stress_mode = opt.stress_mode == SC_STRESS_VIRIAL ? sc::STRESS_VIRIAL : sc::STRESS_COMPAT;
+  d.discs = 0;
+  for (const sc::HostSys& S : h.hs) d.discs |= S.Amin == 0.0 && S.Amax > 0.0;
   d.contact_model = opt.contact_model == SC_CONTACT_TWO ? 1 : 0;
   d.maxn = opt.max_nbrs > 0 ? opt.max_nbrs : 64;
   // the tile pass keeps slots below 2^27 in its entries (kTileInt)

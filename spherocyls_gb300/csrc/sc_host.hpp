@@ -21,7 +21,7 @@ struct HostSys {
   double strain_rate = 0, resize_rate = 0;
   double step = 0.05;  // set_defaults, src/cpp/spherocyl_box.cpp:24
   double pad = 0;
-  double Rmax = 0, Amax = 0;
+  double Rmax = 0, Amax = 0, Amin = 0;
   double packing = 0;
   int rows = 1, cols = 1;
   int ntx = 1, nty = 1;  // tiles across and down (the tile pass's cell numbering)

@@ -223,6 +223,7 @@ struct Dev {
   const int* skip;          // [nsys] or null: force passes leave systems with skip[s] != 0
                             // alone (converged minimiser systems)
   int small_grid;           // some system's grid has fewer than three cells a side
+  int discs;                // some system has discs (A = 0) among rods
   int pass_kind;            // 0: one thread per particle over its full list, 1: tiles
   int ntiles;
   const int4* tiles;        // [ntiles] (system, first global cell, cells, 0)

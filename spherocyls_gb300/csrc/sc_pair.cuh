@@ -263,10 +263,14 @@ struct PairF32 {
 
 // dX, dY: displacement P - Q already reduced to the minimum image (FP32);
 // a = |u_A|^2 and c = |u_B|^2 are the squared half shaft lengths.
-template <bool SE>
+// Either particle may be A, except where one of the two is a disc and the other a rod: the
+// reference's rule then depends on which has the lower index (its "p").  DISCS, q_first (B has
+// the lower index, looked at only for such a pair): the closest point on the rod B where the
+// disc is A, the -1 end of the rod A where the disc is B.
+template <bool SE, bool DISCS = false>
 __device__ __forceinline__ bool pair_fp32(float dX, float dY, float nxA, float nyA, float a,
                                           float nxB, float nyB, float c, float sig, float gamma,
-                                          bool virial, PairF32& o) {
+                                          bool virial, PairF32& o, bool q_first = false) {
   dX = fmaf(gamma, dY, dX);
   float b = -(nxA * nxB + nyA * nyB);
   float d = nxA * dX + nyA * dY;
@@ -285,6 +289,12 @@ __device__ __forceinline__ bool pair_fp32(float dX, float dY, float nxA, float n
   float sarg = fabsf(s);
   s = fminf(fmaxf(s, -1.f), 1.f);
   if (sarg > 1.f) t = fminf(fmaxf(-div_fast(b * s + e, c), -1.f), 1.f);
+  if (DISCS && q_first) {
+    if (a == 0.f)
+      t = fminf(fmaxf(-div_fast(e, c), -1.f), 1.f);
+    else
+      s = -1.f;
+  }
   float dDx = dX + s * nxA - t * nxB;
   float dDy = dY + s * nyA - t * nyB;
   float dsq = dDx * dDx + dDy * dDy;

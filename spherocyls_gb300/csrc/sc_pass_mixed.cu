@@ -188,7 +188,7 @@ __device__ __forceinline__ void mixed_epilogue(const Dev& d, const StepScalars& 
 // loaded through L2 (ld.global.cg) and never through the read-only path, which holds
 // only data that stays unchanged for a whole launch.
 // SMALL: some system's grid has under three cells a side, where the offset between two cells
-// does not settle the image.  ONE: the handle holds one system.
+// does not settle the image, or discs among its rods.  ONE: the handle holds one system.
 template <int MODE, bool TWO, bool SMALL, bool ONE, bool COH = false>
 __device__ __forceinline__ void pass_mixed_position(const Dev& d,
                                                     const StepScalars* __restrict__ tab,
@@ -263,10 +263,13 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
     // record them they come from the FP64 evaluation of the state (k_mx_se64).
     PairF32 o;
     const float cj = fmaf(rj.z, rj.z, rj.w * rj.w);
+    bool q_first = false;
+    if (SMALL && !two_point && d.discs && (ai == 0.f) != (cj == 0.f))
+      q_first = d.id[e & kSlotMask] < d.id[i];
     const bool touch =
         two_point ? pair2_fp32(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, pai.x + Rj, gam, o)
-                  : pair_fp32<false>(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, pai.x + Rj, gam,
-                                     false, o);
+                  : pair_fp32<false, SMALL>(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, pai.x + Rj,
+                                            gam, false, o, q_first);
     if (touch) {
       fx += o.fx;
       fy += o.fy;
@@ -404,7 +407,7 @@ __global__ void __launch_bounds__(256, TWO ? 3 : 4) k_persist_fire(
 template <int MODE, bool TWO>
 void launch_of(const Dev& d, const StepScalars* tab, int row, cudaStream_t st, int block) {
   const int grid = (d.ntot + block - 1) / block;
-  if (d.small_grid)
+  if (d.small_grid || d.discs)
     k_pass_mixed<MODE, TWO, true, false><<<grid, block, 0, st>>>(d, tab, row);
   else if (d.nsys > 1)
     k_pass_mixed<MODE, TWO, false, false><<<grid, block, 0, st>>>(d, tab, row);
@@ -482,10 +485,13 @@ __global__ void __launch_bounds__(kTileThreads, TWO ? 2 : 4) k_tile_pass(
     PairF32 res;
     const float ai = fmaf(ri.z, ri.z, ri.w * ri.w);
     const float cj = fmaf(rj.z, rj.z, rj.w * rj.w);
+    bool q_first = false;
+    if (!TWO && d.discs && (ai == 0.f) != (cj == 0.f))
+      q_first = d.id[(pe & kTileInt) ? p0 + (int)pl : (int)pl] < d.id[p0 + o];
     const bool touch =
         TWO ? pair2_fp32(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, Ri + Rj, gam, res)
-            : pair_fp32<false>(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, Ri + Rj, gam, false,
-                               res);
+            : pair_fp32<false, true>(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, Ri + Rj, gam, false,
+                                     res, q_first);
     pb[e] = touch ? make_float4(res.fx, res.fy, res.tp, res.tq) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __syncthreads();

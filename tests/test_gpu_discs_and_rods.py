@@ -48,7 +48,8 @@ def _check(forces, want, tol):
 
 
 CASES = [("fp64", 1, {}), ("fp64", 1, dict(max_nbrs=80)), ("fp64", 2, {}), ("mixed", 2, {}),
-         ("mixed", 2, dict(pass_kind="tile"))]
+         ("mixed", 2, dict(pass_kind="tile")), ("mixed", 1, {}),
+         ("mixed", 1, dict(pass_kind="tile")), ("mixed", 1, dict(pass_kind="tile", tile_target=16))]
 
 
 @pytest.mark.parametrize("order", ["mixed", "low", "high"])
@@ -95,3 +96,17 @@ def test_mixed_stress_of_discs(sc, order, contacts):
         with sc.SpherocylBox(L, x, y, p, A, R, 0.3, precision=precision, contacts=contacts) as b:
             se.append(np.array(b.calc_se()).ravel())
     assert np.abs(se[1] - se[0]).max() <= 1e-9 * np.abs(se[0]).max()
+
+
+def test_persistent_steps_of_discs(sc):
+    """The persistent kernel against the graph path, bit for bit."""
+    L, x, y, p, R, A = _pack(sc, 600, "mixed")
+    out = []
+    for persist in (False, True):
+        with sc.SpherocylBox(L, x, y, p, A, R, 0.3, precision="mixed",
+                             persist_steps=persist) as b:
+            b.set_strain_rate(1e-2)
+            b.set_step(0.02)
+            b.strain_steps(60)
+            out.append(np.array(b.state()))
+    assert np.array_equal(out[0], out[1])
