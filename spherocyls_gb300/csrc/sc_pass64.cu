@@ -57,7 +57,9 @@ __device__ __forceinline__ void build_nbrs(const Dev& d, const StepScalars* __re
   const int idi = d.id[i];
   const float gam = (float)ts.gamma_p, fLx = (float)ts.Lx_p, fLy = (float)ts.Ly_p;
   const float pad = g.fpad;
-  const float slack = 5e-7f * (fLx + fLy) * (1.f + fabsf(gam)) + 1e-6f * (2.f * g.smax + pad);
+  const float slack = 5e-7f * (fmaxf(fLx, fabsf(ri.x)) + fmaxf(fLy, fabsf(ri.y))) *
+                          (1.f + fabsf(gam)) +
+                      1e-6f * (2.f * g.smax + pad);
   const float reach = g.smax + pad + slack;
   const bool small = !(0.5f * fLx > reach * (1.f + fmaxf(fabsf(gam), 0.5f)) &&
                        0.5f * fLy > reach);
@@ -167,9 +169,11 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_rebuild64(Dev d,
 // Each particle keeps (x, y, A cos phi, A sin phi) of the state and of the predictor
 // copy rounded to FP32 (Dev::rec, rec_t) and R (rf); 20 bytes a neighbour instead of 48,
 // and no instruction of the FP64 pipe, which bounds the pass.  The rounding moves a
-// displacement by less than 2.5e-7 L per axis (two coordinates of up to L, their
-// difference, the image shift), by up to 1 + |gamma| of it after the shear: `slack`
-// covers both axes twice over, on top of the margins of may_touch_fp32.  Where a pair at
+// displacement by less than 3.5e-7 X per axis, X the larger of L and the particle's own
+// coordinate (that coordinate, a partner's within L and the reach of it, their difference, the
+// image shift), by up to 1 + |gamma| of it after the shear: `slack` covers both axes, on top
+// of the margins of may_touch_fp32.  (A long step takes particles many boxes out, where the
+// pair's own displacement may still be a contact.)  Where a pair at
 // the image boundary (|d| = L/2) is out of reach the image may be chosen in FP32; smaller
 // boxes take the FP64 displacement.
 struct Screen64 {
@@ -177,7 +181,9 @@ struct Screen64 {
   float fLx, fLy, fgamma, slack;
   bool small;
 };
-__device__ __forceinline__ Screen64 screen_of(const SysGeom& g, const StepScalars& ts, bool pred) {
+// of a particle with FP32 record ri
+__device__ __forceinline__ Screen64 screen_of(const SysGeom& g, const StepScalars& ts, bool pred,
+                                              float4 ri) {
   Screen64 c;
   c.gamma = pred ? ts.gamma_c : ts.gamma_p;
   c.Lx = pred ? ts.Lx_c : ts.Lx_p;
@@ -185,7 +191,8 @@ __device__ __forceinline__ Screen64 screen_of(const SysGeom& g, const StepScalar
   c.fLx = (float)c.Lx;
   c.fLy = (float)c.Ly;
   c.fgamma = (float)c.gamma;
-  c.slack = 5e-7f * (c.fLx + c.fLy) * (1.f + fabsf(c.fgamma));
+  c.slack = 5e-7f * (fmaxf(c.fLx, fabsf(ri.x)) + fmaxf(c.fLy, fabsf(ri.y))) *
+            (1.f + fabsf(c.fgamma));
   const float reach = g.smax + c.slack;
   c.small = !(0.5f * c.fLx > reach * (1.f + fabsf(c.fgamma)) && 0.5f * c.fLy > reach);
   return c;
@@ -411,9 +418,9 @@ __device__ __forceinline__ void pass64_slot(const Dev& d, const StepScalars* __r
   double se0 = 0.0, se1 = 0.0, se2 = 0.0, se3 = 0.0, se4 = 0.0;
   int cnt = d.nbr_n[i];
   if (cnt > d.maxn) cnt = d.maxn;
-  const Screen64 scr = screen_of(g, ts, kPred);
   const float4* __restrict__ REC = kPred ? d.rec_t : d.rec;
   const float4 ri = REC[i];
+  const Screen64 scr = screen_of(g, ts, kPred, ri);
   const float Ri = d.rf[i];
   for (int k0 = 0; k0 < cnt; k0 += 64) {
     // FP32 screen of up to 64 entries: the FP64 contact code then runs only for the
@@ -525,8 +532,8 @@ __global__ void __launch_bounds__(kPairBlock) k_pairs64(Dev d, const StepScalars
     const int s = d.psys[i];
     live = !(d.skip && d.skip[s]);  // converged minimiser systems have no jobs
     if (live) {
-      const Screen64 scr = screen_of(d.geom[s], tab[row * d.nsys + s], pred != 0);
       const float4 ri = REC[i];
+      const Screen64 scr = screen_of(d.geom[s], tab[row * d.nsys + s], pred != 0, ri);
       const float Ri = d.rf[i];
       const int cnt = min(d.nbr_n[i], d.maxn);
       for (int k = sub; k < cnt; k += TPS) {
