@@ -262,8 +262,11 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
   d.ntot = ntot;
   d.nsys = n_sys;
   d.stress_mode = opt.stress_mode == SC_STRESS_VIRIAL ? sc::STRESS_VIRIAL : sc::STRESS_COMPAT;
-  d.discs = 0;
-  for (const sc::HostSys& S : h.hs) d.discs |= S.Amin == 0.0 && S.Amax > 0.0;
+  d.discs = d.tiny = 0;
+  for (const sc::HostSys& S : h.hs) {
+    d.discs |= S.Amin == 0.0 && S.Amax > 0.0;
+    d.tiny |= sc::tiny_unit(S.Rmax + S.Amax) != 1.f;
+  }
   d.contact_model = opt.contact_model == SC_CONTACT_TWO ? 1 : 0;
   d.maxn = opt.max_nbrs > 0 ? opt.max_nbrs : 64;
   // the tile pass keeps slots below 2^27 in its entries (kTileInt)

@@ -276,6 +276,7 @@ bool Handle::layout_cells() {
     o.inv_n = 1.0 / h.n;
     o.smax = (float)(2.0 * (h.Rmax + h.Amax));
     o.fpad = (float)h.pad;
+    o.unit = tiny_unit(h.Rmax + h.Amax);
   }
   bool ok = cuda_ok(cudaMemcpyAsync((void*)d.geom, g.data(), nsys * sizeof(SysGeom),
                                     cudaMemcpyHostToDevice, stream), "upload geometry") &&
@@ -784,7 +785,7 @@ int Handle::run_steps(int kind, int shrink, int nsteps, int se_every, double* se
   // whatever its length, so that later calls (a long run after a short warm-up) do
   // not pay the capture.
   if (opt.use_graphs && !opt.profile &&
-      !(opt.persist_steps && prec == PREC_MIXED && d.pass_kind == 0 && kind == KIND_STRAIN) &&
+      !(persistent() && kind == KIND_STRAIN) &&
       !subgraph(kind != KIND_STRAIN, 0u))
     cudaGetLastError();  // capture failed: the chunks fall back to eager launches
   int nrec_total = (se_every > 0) ? nsteps / se_every : 0;
@@ -862,8 +863,7 @@ int Handle::run_steps(int kind, int shrink, int nsteps, int se_every, double* se
       pred_kind = pkind;
     }
     bool aligned = se_every == 0 || done % se_every == 0;
-    const bool use_persist = opt.persist_steps && prec == PREC_MIXED && d.pass_kind == 0 &&
-                             kind == KIND_STRAIN && !opt.profile && d_persist;
+    const bool use_persist = persistent() && kind == KIND_STRAIN && !opt.profile;
     bool use_graph = !use_persist && opt.use_graphs && !opt.profile && nk >= 16 && aligned;
     if (use_persist) {
       if (!run_persist(nk, done, se_every)) return last_status;
@@ -1134,7 +1134,7 @@ int Handle::fire_minimize(double ftol, int max_iter, double dt0, double dt_max, 
   launch_fire_reset(d, fire, dt0, stream);
   std::vector<FireSys> hsys(nsys);
   const bool mixed = prec == PREC_MIXED;
-  const bool persist = opt.persist_steps && mixed && d.pass_kind == 0 && d_persist;
+  const bool persist = persistent();
   if (mixed) fp64_valid = false;
   int it = 0;
   bool all_done = false;

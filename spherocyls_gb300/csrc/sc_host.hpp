@@ -154,6 +154,10 @@ struct Handle {
   bool ensure_se_hist(int nrec);
   bool check_status(const char* where);
   bool rebuild_all();
+  // whether runs of steps or iterations go to the persistent kernels
+  bool persistent() const {
+    return opt.persist_steps && prec == PREC_MIXED && d.pass_kind == 0 && !d.tiny && d_persist;
+  }
   // mixed form: change the force pass (0 list, 1 tile), its tile size and the paddings
   bool set_pass(int kind, int target, const std::vector<double>& pads);
   void launch_pass(int mode, bool se, int row, bool fast = false);

@@ -37,7 +37,13 @@ struct SysGeom {
   double inv_n;        // 1/n, energy normalisation
   float smax;          // largest R_i + A_i + R_j + A_j of the system
   float fpad;          // pad in FP32
+  float unit;          // mixed form: lengths are multiplied by it for the pair code (tiny_unit)
 };
+
+// The FP32 pair code takes reciprocals without subnormal numbers, which products of lengths
+// are where lengths are below 1e-16 or so (cross products of nearly parallel spines first).
+// Systems with lengths (R + A) under 1e-9 are scaled by a power of two, which is exact.
+SC_HDI float tiny_unit(double len) { return len < 1e-9 ? 0x1p60f : 1.f; }
 
 // Cell numbering of a system.  The grid is cut into ntx x nty tiles of nearly
 // equal size (tile k along a dimension of n cells covers [k n / nt, (k+1) n / nt));
@@ -224,6 +230,7 @@ struct Dev {
                             // alone (converged minimiser systems)
   int small_grid;           // some system's grid has fewer than three cells a side
   int discs;                // some system has discs (A = 0) among rods
+  int tiny;                 // some system's SysGeom::unit is not 1
   int pass_kind;            // 0: one thread per particle over its full list, 1: tiles
   int ntiles;
   const int4* tiles;        // [ntiles] (system, first global cell, cells, 0)

@@ -188,7 +188,8 @@ __device__ __forceinline__ void mixed_epilogue(const Dev& d, const StepScalars& 
 // loaded through L2 (ld.global.cg) and never through the read-only path, which holds
 // only data that stays unchanged for a whole launch.
 // SMALL: some system's grid has under three cells a side, where the offset between two cells
-// does not settle the image, or discs among its rods.  ONE: the handle holds one system.
+// does not settle the image, or discs among its rods, or lengths to be scaled (which the
+// persistent kernels leave to the other path).  ONE: the handle holds one system.
 template <int MODE, bool TWO, bool SMALL, bool ONE, bool COH = false>
 __device__ __forceinline__ void pass_mixed_position(const Dev& d,
                                                     const StepScalars* __restrict__ tab,
@@ -241,7 +242,8 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
     r1 = SC_REC(e1 & kSlotMask);
     R1 = d.rf[e1 & kSlotMask];
   }
-  const float ai = pai.y * pai.y;
+  const float unit = SMALL && !COH ? g.unit : 1.f;
+  const float ux = unit * ri.z, uy = unit * ri.w, ai = (unit * pai.y) * (unit * pai.y);
   for (int k = 0; k < cnt; k++) {
     const unsigned e = e1;
     const float4 rj = r1;
@@ -262,14 +264,17 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
     // FP32 rounding.  Stress and energy are not summed here: on the steps that
     // record them they come from the FP64 evaluation of the state (k_mx_se64).
     PairF32 o;
-    const float cj = fmaf(rj.z, rj.z, rj.w * rj.w);
+    const float vx = unit * rj.z, vy = unit * rj.w, sig = unit * (pai.x + Rj);
+    const float cj = fmaf(vx, vx, vy * vy);
+    dx *= unit;
+    dy *= unit;
     bool q_first = false;
     if (SMALL && !two_point && d.discs && (ai == 0.f) != (cj == 0.f))
       q_first = d.id[e & kSlotMask] < d.id[i];
     const bool touch =
-        two_point ? pair2_fp32(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, pai.x + Rj, gam, o)
-                  : pair_fp32<false, SMALL>(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, pai.x + Rj,
-                                            gam, false, o, q_first);
+        two_point ? pair2_fp32(dx, dy, ux, uy, ai, vx, vy, cj, sig, gam, o)
+                  : pair_fp32<false, SMALL>(dx, dy, ux, uy, ai, vx, vy, cj, sig, gam, false, o,
+                                            q_first);
     if (touch) {
       fx += o.fx;
       fy += o.fy;
@@ -283,7 +288,7 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
   }
 
 #undef SC_REC
-  mixed_epilogue<MODE>(d, ts, g, s, i, ri, pai, gam, fx, fy, tq);
+  mixed_epilogue<MODE>(d, ts, g, s, i, ri, pai, gam, unit * fx, unit * fy, tq);
 }
 
 // k_pass_mixed: one thread per list position.  It waits for dependent gathers (10 of 18
@@ -407,7 +412,7 @@ __global__ void __launch_bounds__(256, TWO ? 3 : 4) k_persist_fire(
 template <int MODE, bool TWO>
 void launch_of(const Dev& d, const StepScalars* tab, int row, cudaStream_t st, int block) {
   const int grid = (d.ntot + block - 1) / block;
-  if (d.small_grid || d.discs)
+  if (d.small_grid || d.discs || d.tiny)
     k_pass_mixed<MODE, TWO, true, false><<<grid, block, 0, st>>>(d, tab, row);
   else if (d.nsys > 1)
     k_pass_mixed<MODE, TWO, false, false><<<grid, block, 0, st>>>(d, tab, row);
@@ -455,6 +460,7 @@ __global__ void __launch_bounds__(kTileThreads, TWO ? 2 : 4) k_tile_pass(
   const float gam = kCorr ? ts.f_gamma_c : ts.f_gamma_p;
   const bool smallx = g.cols < 3, smally = g.rows < 3;
   const float Lxf = W * g.cols, Lyf = H * g.rows;
+  const float unit = g.unit;
   const int nst = nown < kTileCap ? nown : kTileCap;
   for (int l = threadIdx.x; l < nst; l += blockDim.x) {
     s_rec[l] = REC[p0 + l];
@@ -466,7 +472,7 @@ __global__ void __launch_bounds__(kTileThreads, TWO ? 2 : 4) k_tile_pass(
   for (int e = threadIdx.x; e < ne; e += blockDim.x) {
     const int o = d.t_own[ebase + e];
     const unsigned pe = d.t_pe[ebase + e];
-    const float4 ri = o < kTileCap ? s_rec[o] : REC[p0 + o];
+    float4 ri = o < kTileCap ? s_rec[o] : REC[p0 + o];
     const float Ri = o < kTileCap ? s_R[o] : d.rf[p0 + o];
     const unsigned pl = pe & kTilePayload;
     float4 rj;
@@ -482,6 +488,16 @@ __global__ void __launch_bounds__(kTileThreads, TWO ? 2 : 4) k_tile_pass(
     float dy = ri.y - rj.y + (float)(1 - (int)(pe >> 30)) * H;
     if (smallx) dx += Lxf * (float)((dx < -0.5f * Lxf) - (dx > 0.5f * Lxf));
     if (smally) dy += Lyf * (float)((dy < -0.5f * Lyf) - (dy > 0.5f * Lyf));
+    float sig = Ri + Rj;
+    if (unit != 1.f) {
+      dx *= unit;
+      dy *= unit;
+      ri.z *= unit;
+      ri.w *= unit;
+      rj.z *= unit;
+      rj.w *= unit;
+      sig *= unit;
+    }
     PairF32 res;
     const float ai = fmaf(ri.z, ri.z, ri.w * ri.w);
     const float cj = fmaf(rj.z, rj.z, rj.w * rj.w);
@@ -489,10 +505,10 @@ __global__ void __launch_bounds__(kTileThreads, TWO ? 2 : 4) k_tile_pass(
     if (!TWO && d.discs && (ai == 0.f) != (cj == 0.f))
       q_first = d.id[(pe & kTileInt) ? p0 + (int)pl : (int)pl] < d.id[p0 + o];
     const bool touch =
-        TWO ? pair2_fp32(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, Ri + Rj, gam, res)
-            : pair_fp32<false, true>(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, Ri + Rj, gam, false,
+        TWO ? pair2_fp32(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, sig, gam, res)
+            : pair_fp32<false, true>(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, sig, gam, false,
                                      res, q_first);
-    pb[e] = touch ? make_float4(res.fx, res.fy, res.tp, res.tq) : make_float4(0.f, 0.f, 0.f, 0.f);
+    pb[e] = touch ? make_float4(unit * res.fx, unit * res.fy, res.tp, res.tq) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __syncthreads();
   for (int l = threadIdx.x; l < nown; l += blockDim.x) {
