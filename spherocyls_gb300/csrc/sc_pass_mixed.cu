@@ -242,8 +242,12 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
     r1 = SC_REC(e1 & kSlotMask);
     R1 = d.rf[e1 & kSlotMask];
   }
-  const float unit = SMALL && !COH ? g.unit : 1.f;
-  const float ux = unit * ri.z, uy = unit * ri.w, ai = (unit * pai.y) * (unit * pai.y);
+  // (the products with the unit are kept from being fused into the sums they enter, which
+  // would change the bits where the unit is 1)
+  constexpr bool kUnit = SMALL && !COH;
+  const float unit = kUnit ? g.unit : 1.f;
+  auto scaled = [&](float v) { return kUnit ? __fmul_rn(unit, v) : v; };
+  const float ux = scaled(ri.z), uy = scaled(ri.w), ai = scaled(pai.y) * scaled(pai.y);
   for (int k = 0; k < cnt; k++) {
     const unsigned e = e1;
     const float4 rj = r1;
@@ -264,10 +268,10 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
     // FP32 rounding.  Stress and energy are not summed here: on the steps that
     // record them they come from the FP64 evaluation of the state (k_mx_se64).
     PairF32 o;
-    const float vx = unit * rj.z, vy = unit * rj.w, sig = unit * (pai.x + Rj);
+    const float vx = scaled(rj.z), vy = scaled(rj.w), sig = scaled(pai.x + Rj);
     const float cj = fmaf(vx, vx, vy * vy);
-    dx *= unit;
-    dy *= unit;
+    dx = scaled(dx);
+    dy = scaled(dy);
     bool q_first = false;
     if (SMALL && !two_point && d.discs && (ai == 0.f) != (cj == 0.f))
       q_first = d.id[e & kSlotMask] < d.id[i];
@@ -288,7 +292,7 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
   }
 
 #undef SC_REC
-  mixed_epilogue<MODE>(d, ts, g, s, i, ri, pai, gam, unit * fx, unit * fy, tq);
+  mixed_epilogue<MODE>(d, ts, g, s, i, ri, pai, gam, scaled(fx), scaled(fy), tq);
 }
 
 // k_pass_mixed: one thread per list position.  It waits for dependent gathers (10 of 18
@@ -490,13 +494,13 @@ __global__ void __launch_bounds__(kTileThreads, TWO ? 2 : 4) k_tile_pass(
     if (smally) dy += Lyf * (float)((dy < -0.5f * Lyf) - (dy > 0.5f * Lyf));
     float sig = Ri + Rj;
     if (unit != 1.f) {
-      dx *= unit;
-      dy *= unit;
-      ri.z *= unit;
-      ri.w *= unit;
-      rj.z *= unit;
-      rj.w *= unit;
-      sig *= unit;
+      dx = __fmul_rn(dx, unit);
+      dy = __fmul_rn(dy, unit);
+      ri.z = __fmul_rn(ri.z, unit);
+      ri.w = __fmul_rn(ri.w, unit);
+      rj.z = __fmul_rn(rj.z, unit);
+      rj.w = __fmul_rn(rj.w, unit);
+      sig = __fmul_rn(sig, unit);
     }
     PairF32 res;
     const float ai = fmaf(ri.z, ri.z, ri.w * ri.w);
@@ -508,7 +512,8 @@ __global__ void __launch_bounds__(kTileThreads, TWO ? 2 : 4) k_tile_pass(
         TWO ? pair2_fp32(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, sig, gam, res)
             : pair_fp32<false, true>(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, sig, gam, false,
                                      res, q_first);
-    pb[e] = touch ? make_float4(unit * res.fx, unit * res.fy, res.tp, res.tq) : make_float4(0.f, 0.f, 0.f, 0.f);
+    pb[e] = touch ? make_float4(__fmul_rn(unit, res.fx), __fmul_rn(unit, res.fy), res.tp, res.tq)
+                  : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __syncthreads();
   for (int l = threadIdx.x; l < nown; l += blockDim.x) {

@@ -39,3 +39,21 @@ def test_forces_in_other_units(sc, scale, contacts, kw):
     rms = np.sqrt(np.mean(out["fp64"][:2] ** 2))
     assert np.abs(out["mixed"] - out["fp64"]).max() <= 1e-4 * rms
     assert abs(out["mixedfire"] - out["fp64fire"]) <= 1e-4 * out["fp64fire"]
+
+
+@pytest.mark.parametrize("n,phi", [(8, 0.5), (16, 0.7), (24, 0.7)])
+def test_small_grids_keep_their_bits(sc, n, phi):
+    """Boxes under three cells a side run the variant that scales, with a unit of 1: the
+    persistent kernel, which does not scale, gives the same bits."""
+    L, x, y, p, R, A = sc.generate_packing(n, phi, 1.0, seed=n)
+    out = []
+    for persist in (False, True):
+        with sc.SpherocylBox(L, x, y, p, A, R, 0.2, precision="mixed",
+                             persist_steps=persist) as b:
+            b.set_strain_rate(1e-2)
+            b.set_step(0.02)
+            b.strain_steps(60)
+            out.append(np.array(b.state()))
+            cols = b.box()["cols"]
+    assert cols < 3
+    assert np.array_equal(out[0], out[1])
