@@ -149,9 +149,10 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
   }
   if (!summing) sum_areas();
   // The input checks and per system the largest R and A (set_particle,
-  // src/cpp/spherocyl_box.cpp:216-219) and the smallest A, on worker threads over slices of
-  // the caller's arrays.
-  std::vector<double> rmax(n_sys, 0.0), amax(n_sys, 0.0), amin(n_sys, HUGE_VAL);
+  // src/cpp/spherocyl_box.cpp:216-219) on worker threads over slices of the caller's
+  // arrays.
+  std::vector<double> rmax(n_sys, 0.0), amax(n_sys, 0.0);
+  bool any_disc = false, any_rod = false, any_odd = false;
   {
     std::vector<int> p0s(n_sys + 1, 0);
     for (int s = 0; s < n_sys; s++) p0s[s + 1] = p0s[s] + n_per_sys[s];
@@ -159,30 +160,40 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
     const int nthreads = ntot < (1 << 16) ? 1 : (int)std::min(8u, std::max(1u, hw));
     struct Part {
       int fin = 1, shp = 1;  // all finite; every R > 0 and A >= 0
-      std::vector<double> rm, am, an;
+      int disc = 0, odd = 0;  // some A = 0; some R or A that Dev::odd_shapes asks about
+      std::vector<double> rm, am;
     };
     std::vector<Part> parts(nthreads);
     auto scan = [&](int w) {
       Part& P = parts[w];
       P.rm.assign(n_sys, 0.0);
       P.am.assign(n_sys, 0.0);
-      P.an.assign(n_sys, HUGE_VAL);
       const int a0 = (int)((long long)ntot * w / nthreads);
       const int a1 = (int)((long long)ntot * (w + 1) / nthreads);
       int s = (int)(std::upper_bound(p0s.begin(), p0s.end(), a0) - p0s.begin()) - 1;
-      int fin = 1, shp = 1;
-      for (int i = a0; i < a1; i++) {
-        while (i >= p0s[s + 1]) s++;
-        const double r = R[i], a = A[i];
-        fin &= (int)std::isfinite(x[i]) & (int)std::isfinite(y[i]) &
-               (int)std::isfinite(phi[i]) & (int)std::isfinite(r) & (int)std::isfinite(a);
-        shp &= (int)(r > 0) & (int)(a >= 0);
-        if (a > P.am[s]) P.am[s] = a;
-        if (a < P.an[s]) P.an[s] = a;
-        if (r > P.rm[s]) P.rm[s] = r;
+      int fin = 1, shp = 1, disc = 0, odd = 0;
+      for (int i = a0; i < a1; s++) {
+        const int end = std::min(a1, p0s[s + 1]);
+        double rlo = HUGE_VAL, rhi = 0.0, alo = HUGE_VAL, ahi = 0.0;
+        for (; i < end; i++) {
+          const double r = R[i], a = A[i];
+          fin &= (int)std::isfinite(x[i]) & (int)std::isfinite(y[i]) &
+                 (int)std::isfinite(phi[i]) & (int)std::isfinite(r) & (int)std::isfinite(a);
+          rlo = r < rlo ? r : rlo;
+          rhi = r > rhi ? r : rhi;
+          alo = a < alo ? a : alo;
+          ahi = a > ahi ? a : ahi;
+        }
+        shp &= (int)(rlo > 0) & (int)(alo >= 0);
+        disc |= (int)(alo == 0);
+        odd |= (int)!(std::min(rlo, alo) >= 1e-25) | (int)!(std::max(rhi, ahi) <= 1e25);
+        P.rm[s] = rhi;
+        P.am[s] = ahi;
       }
       P.fin = fin;
       P.shp = shp;
+      P.disc = disc;
+      P.odd = odd;
     };
     std::vector<std::thread> workers;
     std::vector<char> on_worker(nthreads, 0);
@@ -200,10 +211,11 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
     for (const Part& P : parts) {
       finite = finite && P.fin;
       shapes = shapes && P.shp;
+      any_disc = any_disc || P.disc;
+      any_odd = any_odd || P.odd;
       for (int s = 0; s < n_sys; s++) {
         rmax[s] = std::max(rmax[s], P.rm[s]);
         amax[s] = std::max(amax[s], P.am[s]);
-        amin[s] = std::min(amin[s], P.an[s]);
       }
     }
     if (!finite) {
@@ -250,7 +262,6 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
     S.Ly = Ly[s];
     S.pad = pad ? pad[s] : 0.0;
     S.Amax = amax[s];
-    S.Amin = amin[s];
     S.Rmax = rmax[s];
     S.configure(true);
     p0 += S.n;
@@ -262,11 +273,13 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
   d.ntot = ntot;
   d.nsys = n_sys;
   d.stress_mode = opt.stress_mode == SC_STRESS_VIRIAL ? sc::STRESS_VIRIAL : sc::STRESS_COMPAT;
-  d.discs = d.tiny = 0;
+  d.tiny = 0;
   for (const sc::HostSys& S : h.hs) {
-    d.discs |= S.Amin == 0.0 && S.Amax > 0.0;
+    any_rod = any_rod || S.Amax > 0.0;
     d.tiny |= sc::tiny_unit(S.Rmax + S.Amax) != 1.f;
   }
+  d.discs = any_disc && any_rod;
+  d.odd_shapes = any_odd;
   d.contact_model = opt.contact_model == SC_CONTACT_TWO ? 1 : 0;
   d.maxn = opt.max_nbrs > 0 ? opt.max_nbrs : 64;
   // the tile pass keeps slots below 2^27 in its entries (kTileInt)

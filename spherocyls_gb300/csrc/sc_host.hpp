@@ -21,7 +21,7 @@ struct HostSys {
   double strain_rate = 0, resize_rate = 0;
   double step = 0.05;  // set_defaults, src/cpp/spherocyl_box.cpp:24
   double pad = 0;
-  double Rmax = 0, Amax = 0, Amin = 0;
+  double Rmax = 0, Amax = 0;
   double packing = 0;
   int rows = 1, cols = 1;
   int ntx = 1, nty = 1;  // tiles across and down (the tile pass's cell numbering)
@@ -156,7 +156,8 @@ struct Handle {
   bool rebuild_all();
   // whether runs of steps or iterations go to the persistent kernels
   bool persistent() const {
-    return opt.persist_steps && prec == PREC_MIXED && d.pass_kind == 0 && !d.tiny && d_persist;
+    return opt.persist_steps && prec == PREC_MIXED && d.pass_kind == 0 && !d.discs && !d.tiny &&
+           d_persist;
   }
   // mixed form: change the force pass (0 list, 1 tile), its tile size and the paddings
   bool set_pass(int kind, int target, const std::vector<double>& pads);

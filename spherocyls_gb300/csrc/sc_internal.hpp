@@ -229,7 +229,8 @@ struct Dev {
   const int* skip;          // [nsys] or null: force passes leave systems with skip[s] != 0
                             // alone (converged minimiser systems)
   int small_grid;           // some system's grid has fewer than three cells a side
-  int discs;                // some system has discs (A = 0) among rods
+  int discs;                // there are discs (A = 0) and rods
+  int odd_shapes;           // some R or A, discs among them, is outside 1e-25 to 1e25
   int tiny;                 // some system's SysGeom::unit is not 1
   int pass_kind;            // 0: one thread per particle over its full list, 1: tiles
   int ntiles;
@@ -442,7 +443,6 @@ struct GridBarrier {
       if (last) {
         count[0] = 0;
         count[1] = 0;
-        __threadfence();
       }
     }
     __syncthreads();

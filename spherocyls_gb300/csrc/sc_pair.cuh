@@ -104,29 +104,24 @@ __device__ __forceinline__ double qdiv(double x, double y, double inv_y) {
   return FAST ? x * inv_y : div_by(x, y, inv_y);
 }
 
-// Reciprocals of a = |u_A|^2, c = |u_B|^2, delta and sig from one division; from one each
-// where their product is zero (a disc has a = 0) or near the ends of the exponent range.
+// Reciprocals of a = |u_A|^2, c = |u_B|^2, delta and sig from one division.  Their product is
+// zero for a disc and out of range for some other shapes: handles with such particles
+// (Dev::odd_shapes) take the form with a division each.
 struct Recip64 {
   double a, c, delta, sig;
 };
 __device__ __forceinline__ Recip64 recip64(double a, double c, double delta, double sig) {
   Recip64 r;
   const double ac = a * c;
-  const double all = delta > 0 ? ac * delta * sig : ac * sig;
-  if ((unsigned)__double2hiint(all) - 0x01700000u >= 0x7d200000u) {  // not 2^-1000 to 2^1000
-    r.a = 1.0 / a;
-    r.c = 1.0 / c;
-    r.delta = delta > 0 ? 1.0 / delta : 0.0;
-    r.sig = 1.0 / sig;
-  } else if (delta > 0) {
-    const double inv = 1.0 / all;
+  if (delta > 0) {
+    const double inv = 1.0 / (ac * delta * sig);
     const double i_ac = delta * sig * inv;
     r.delta = ac * sig * inv;
     r.sig = ac * delta * inv;
     r.a = c * i_ac;
     r.c = a * i_ac;
   } else {
-    const double inv = 1.0 / all;
+    const double inv = 1.0 / (ac * sig);
     r.delta = 0.0;
     r.sig = ac * inv;
     r.a = c * sig * inv;
@@ -328,7 +323,8 @@ constexpr float kMinNormal = 1.17549435e-38f;  // the smallest normal FP32 numbe
 // the FP32 rounding of the distance stay far below the 1e-4 relative margin.  Both
 // contact rules need the minimum distance below sig for any contact.  A spine P whose
 // squared length is no normal number is a point (a disc), and the closest point to it is
-// looked for on Q: the first formula, which looks along P, says nothing about Q then.
+// looked for on Q (as past an end of P): the first formula, which looks along P, says nothing
+// about Q then.
 __device__ __forceinline__ bool may_touch_fp32(float dX, float dY, float nxA, float nyA,
                                                float nxB, float nyB, float sig) {
   float a = fmaf(nxA, nxA, nyA * nyA), c = fmaf(nxB, nxB, nyB * nyB);
@@ -340,8 +336,8 @@ __device__ __forceinline__ bool may_touch_fp32(float dX, float dY, float nxA, fl
   float w2 = nyA * dX;
   float uxD = fmaf(nxA, dY, -w2) + fmaf(-nyA, dX, w2);
   float t = uxv == 0.f ? -1.f : fminf(fmaxf(div_fast(uxD, uxv), -1.f), 1.f);
-  float s = a >= kMinNormal ? -div_fast(b * t + d, a) : 0.f;
-  float sarg = a >= kMinNormal ? fabsf(s) : 2.f;
+  float s = a >= kMinNormal ? -div_fast(b * t + d, a) : 2.f;
+  float sarg = fabsf(s);
   s = fminf(fmaxf(s, -1.f), 1.f);
   if (sarg > 1.f && c > 0.f) t = fminf(fmaxf(-div_fast(b * s + e, c), -1.f), 1.f);
   float dDx = dX + s * nxA - t * nxB;
@@ -365,8 +361,8 @@ __device__ __forceinline__ bool capsules_within(float dX, float dY, float nxA, f
   const float w2 = nyA * dX;
   const float uxD = fmaf(nxA, dY, -w2) + fmaf(-nyA, dX, w2);
   float t = uxv == 0.f ? -1.f : fminf(fmaxf(div_fast(uxD, uxv), -1.f), 1.f);
-  float s = a >= kMinNormal ? -div_fast(b * t + d, a) : 0.f;
-  const float sarg = a >= kMinNormal ? fabsf(s) : 2.f;  // a point: see may_touch_fp32
+  float s = a >= kMinNormal ? -div_fast(b * t + d, a) : 2.f;  // (a point: see may_touch_fp32)
+  const float sarg = fabsf(s);
   s = fminf(fmaxf(s, -1.f), 1.f);
   if (sarg > 1.f && c > 0.f) t = fminf(fmaxf(-div_fast(b * s + e, c), -1.f), 1.f);
   const float x = dX + s * nxA - t * nxB, y = dY + s * nyA - t * nyB;

@@ -816,7 +816,7 @@ __global__ void k_mx_se_prep(Dev d) {
 // image is chosen in FP64.
 // With the screen's displacements in FP64 and one thread a slot it took 35 us at 16384
 // particles and 942 us at 2^20; now 18 and 446.
-template <bool TWO, int TPS>
+template <bool TWO, bool FAST, int TPS>
 __global__ void __launch_bounds__(kPairBlock) k_mx_se64(Dev d, const StepScalars* __restrict__ tab,
                                                        int row) {
   constexpr int S = kPairBlock / TPS;
@@ -899,10 +899,10 @@ __global__ void __launch_bounds__(kPairBlock) k_mx_se64(Dev d, const StepScalars
         const double two_n = 2.0 * g.n, i2n = 0.5 * g.inv_n;
         PairF64 r;
         const bool hit =
-            TWO ? pair2_fp64<true, true>(dX, dY, ni.x, ni.y, rai.y, nj.x, nj.y, raj.y,
+            TWO ? pair2_fp64<true, FAST>(dX, dY, ni.x, ni.y, rai.y, nj.x, nj.y, raj.y,
                                          rai.x + raj.x, ts.gamma_p, ts.Lx_p, ts.Ly_p, two_n, r,
                                          0.0, 0.0, ts.inv_area, i2n)
-                : pair_fp64<true, true>(dX, dY, ni.x, ni.y, rai.y, nj.x, nj.y, raj.y,
+                : pair_fp64<true, FAST>(dX, dY, ni.x, ni.y, rai.y, nj.x, nj.y, raj.y,
                                         rai.x + raj.x, ts.gamma_p, ts.Lx_p, ts.Ly_p,
                                         d.stress_mode == STRESS_VIRIAL, two_n, r, 0.0, 0.0,
                                         ts.inv_area, i2n);
@@ -1004,7 +1004,7 @@ int pair_window(int ntot) {
 
 int launch_pass_fp64(const Dev& d, int mode, bool se, const StepScalars* tab, int row,
                      cudaStream_t st, bool fast) {
-  if (fast && mode == PASS_FORCE && !se) {
+  if (fast && !d.odd_shapes && mode == PASS_FORCE && !se) {
     // the minimiser's force evaluation (shared reciprocals, see qdiv)
     if (d.pr_win == 0) {
       launch_whole<PASS_FORCE, false, true>(d, tab, row, st);
@@ -1034,9 +1034,11 @@ template <int TPS>
 static void launch_mx_se64_of(const Dev& d, const StepScalars* tab, int row, cudaStream_t st) {
   const int grid = (d.ntot + kPairBlock / TPS - 1) / (kPairBlock / TPS);
   if (d.contact_model == 1)
-    k_mx_se64<true, TPS><<<grid, kPairBlock, 0, st>>>(d, tab, row);
+    (d.odd_shapes ? k_mx_se64<true, false, TPS> : k_mx_se64<true, true, TPS>)<<<
+        grid, kPairBlock, 0, st>>>(d, tab, row);
   else
-    k_mx_se64<false, TPS><<<grid, kPairBlock, 0, st>>>(d, tab, row);
+    (d.odd_shapes ? k_mx_se64<false, false, TPS> : k_mx_se64<false, true, TPS>)<<<
+        grid, kPairBlock, 0, st>>>(d, tab, row);
 }
 
 void launch_mx_se64(const Dev& d, const StepScalars* tab, int row, cudaStream_t st) {

@@ -188,8 +188,8 @@ __device__ __forceinline__ void mixed_epilogue(const Dev& d, const StepScalars& 
 // loaded through L2 (ld.global.cg) and never through the read-only path, which holds
 // only data that stays unchanged for a whole launch.
 // SMALL: some system's grid has under three cells a side, where the offset between two cells
-// does not settle the image, or discs among its rods, or lengths to be scaled (which the
-// persistent kernels leave to the other path).  ONE: the handle holds one system.
+// does not settle the image, or discs among its rods, or lengths to be scaled (the last two
+// take no persistent kernel).  ONE: the handle holds one system.
 template <int MODE, bool TWO, bool SMALL, bool ONE, bool COH = false>
 __device__ __forceinline__ void pass_mixed_position(const Dev& d,
                                                     const StepScalars* __restrict__ tab,
@@ -244,9 +244,9 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
   }
   // (the products with the unit are kept from being fused into the sums they enter, which
   // would change the bits where the unit is 1)
-  constexpr bool kUnit = SMALL && !COH;
-  const float unit = kUnit ? g.unit : 1.f;
-  auto scaled = [&](float v) { return kUnit ? __fmul_rn(unit, v) : v; };
+  constexpr bool kGeneral = SMALL && !COH;
+  const float unit = kGeneral ? g.unit : 1.f;
+  auto scaled = [&](float v) { return kGeneral ? __fmul_rn(unit, v) : v; };
   const float ux = scaled(ri.z), uy = scaled(ri.w), ai = scaled(pai.y) * scaled(pai.y);
   for (int k = 0; k < cnt; k++) {
     const unsigned e = e1;
@@ -273,12 +273,12 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
     dx = scaled(dx);
     dy = scaled(dy);
     bool q_first = false;
-    if (SMALL && !two_point && d.discs && (ai == 0.f) != (cj == 0.f))
+    if (kGeneral && !two_point && d.discs && (ai == 0.f) != (cj == 0.f))
       q_first = d.id[e & kSlotMask] < d.id[i];
     const bool touch =
         two_point ? pair2_fp32(dx, dy, ux, uy, ai, vx, vy, cj, sig, gam, o)
-                  : pair_fp32<false, SMALL>(dx, dy, ux, uy, ai, vx, vy, cj, sig, gam, false, o,
-                                            q_first);
+                  : pair_fp32<false, kGeneral>(dx, dy, ux, uy, ai, vx, vy, cj, sig, gam, false, o,
+                                               q_first);
     if (touch) {
       fx += o.fx;
       fy += o.fy;
@@ -306,7 +306,7 @@ __device__ __forceinline__ void pass_mixed_position(const Dev& d,
 // the epilogue's state before the loop was 3% slower.
 template <int MODE, bool TWO, bool SMALL, bool ONE>
 __global__ void __launch_bounds__(
-    128, TWO ? 6 : (MODE == PASS_PRED_RESIZE || MODE == PASS_CORR_RESIZE) ? 10 : 12)
+    128, TWO ? 6 : SMALL ? 8 : (MODE == PASS_PRED_RESIZE || MODE == PASS_CORR_RESIZE) ? 10 : 12)
     k_pass_mixed(Dev d,
                                                        const StepScalars* __restrict__ tab,
                                                        int row) {
@@ -443,7 +443,8 @@ void launch_one(const Dev& d, const StepScalars* tab, int row, cudaStream_t st, 
 // entries of the pairs whose lower partner computed them (its read entries, in
 // list order).  The sums are deterministic.  A tile with more particles or pair
 // entries than shared memory holds uses global memory for the excess.
-template <int MODE, bool TWO>
+// GENERAL: discs among rods, or lengths to be scaled, in some system.
+template <int MODE, bool TWO, bool GENERAL>
 __global__ void __launch_bounds__(kTileThreads, TWO ? 2 : 4) k_tile_pass(
     Dev d, const StepScalars* __restrict__ tab, int row) {
   constexpr bool kCorr = (MODE == PASS_CORR_STRAIN || MODE == PASS_CORR_RESIZE);
@@ -464,7 +465,7 @@ __global__ void __launch_bounds__(kTileThreads, TWO ? 2 : 4) k_tile_pass(
   const float gam = kCorr ? ts.f_gamma_c : ts.f_gamma_p;
   const bool smallx = g.cols < 3, smally = g.rows < 3;
   const float Lxf = W * g.cols, Lyf = H * g.rows;
-  const float unit = g.unit;
+  const float unit = GENERAL ? g.unit : 1.f;
   const int nst = nown < kTileCap ? nown : kTileCap;
   for (int l = threadIdx.x; l < nst; l += blockDim.x) {
     s_rec[l] = REC[p0 + l];
@@ -493,7 +494,7 @@ __global__ void __launch_bounds__(kTileThreads, TWO ? 2 : 4) k_tile_pass(
     if (smallx) dx += Lxf * (float)((dx < -0.5f * Lxf) - (dx > 0.5f * Lxf));
     if (smally) dy += Lyf * (float)((dy < -0.5f * Lyf) - (dy > 0.5f * Lyf));
     float sig = Ri + Rj;
-    if (unit != 1.f) {
+    if (GENERAL) {
       dx = __fmul_rn(dx, unit);
       dy = __fmul_rn(dy, unit);
       ri.z = __fmul_rn(ri.z, unit);
@@ -506,14 +507,17 @@ __global__ void __launch_bounds__(kTileThreads, TWO ? 2 : 4) k_tile_pass(
     const float ai = fmaf(ri.z, ri.z, ri.w * ri.w);
     const float cj = fmaf(rj.z, rj.z, rj.w * rj.w);
     bool q_first = false;
-    if (!TWO && d.discs && (ai == 0.f) != (cj == 0.f))
+    if (GENERAL && !TWO && d.discs && (ai == 0.f) != (cj == 0.f))
       q_first = d.id[(pe & kTileInt) ? p0 + (int)pl : (int)pl] < d.id[p0 + o];
     const bool touch =
         TWO ? pair2_fp32(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, sig, gam, res)
-            : pair_fp32<false, true>(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, sig, gam, false,
-                                     res, q_first);
-    pb[e] = touch ? make_float4(__fmul_rn(unit, res.fx), __fmul_rn(unit, res.fy), res.tp, res.tq)
-                  : make_float4(0.f, 0.f, 0.f, 0.f);
+            : pair_fp32<false, GENERAL>(dx, dy, ri.z, ri.w, ai, rj.z, rj.w, cj, sig, gam, false,
+                                        res, q_first);
+    if (GENERAL) {
+      res.fx = __fmul_rn(unit, res.fx);
+      res.fy = __fmul_rn(unit, res.fy);
+    }
+    pb[e] = touch ? make_float4(res.fx, res.fy, res.tp, res.tq) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __syncthreads();
   for (int l = threadIdx.x; l < nown; l += blockDim.x) {
@@ -544,10 +548,13 @@ __global__ void __launch_bounds__(kTileThreads, TWO ? 2 : 4) k_tile_pass(
 
 template <int MODE>
 void launch_tile(const Dev& d, const StepScalars* tab, int row, cudaStream_t st) {
+  const bool general = d.discs || d.tiny;
   if (d.contact_model == 1)
-    k_tile_pass<MODE, true><<<d.ntiles, kTileThreads, 0, st>>>(d, tab, row);
+    (general ? k_tile_pass<MODE, true, true> : k_tile_pass<MODE, true, false>)<<<
+        d.ntiles, kTileThreads, 0, st>>>(d, tab, row);
   else
-    k_tile_pass<MODE, false><<<d.ntiles, kTileThreads, 0, st>>>(d, tab, row);
+    (general ? k_tile_pass<MODE, false, true> : k_tile_pass<MODE, false, false>)<<<
+        d.ntiles, kTileThreads, 0, st>>>(d, tab, row);
 }
 
 // block-wide exclusive scan of one int per thread; *total the block's sum

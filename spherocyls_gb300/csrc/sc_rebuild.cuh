@@ -461,13 +461,13 @@ __device__ __forceinline__ void put_back(const Dev& d, const Work<BS>& work, boo
 // The end of a rebuild: the last block out takes back the flags and counts it, unless a
 // barrier timed out on the way.
 __device__ __forceinline__ void finish(const Dev& d, GridBarrier& bar) {
-  if (!bar.leave() || timed_out(d)) return;
+  if (!bar.leave()) return;
   for (int s = threadIdx.x; s < d.nsys; s += blockDim.x) {
     d.flags[s] = 0;
     d.istar[s] = kNoTrigger;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && !timed_out(d)) {
     *d.any = 0;
     d.status[1] += 1;  // rebuilds executed
   }
