@@ -312,19 +312,15 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
        h.dalloc(&d.irc, N, "irc") && h.dalloc(&d.id, N, "id") && h.dalloc(&d.cell, N, "cell");
   ok = ok && h.dalloc(&d.nxy, N, "nxy") && h.dalloc(&d.xy_t, N, "xy_t") &&
        h.dalloc(&d.ph_t, N, "ph_t") && h.dalloc(&d.nxy_t, N, "nxy_t");
-  ok = ok && h.dalloc(&d.v0x, N, "v0x") && h.dalloc(&d.v0y, N, "v0y") &&
-       h.dalloc(&d.v0p, N, "v0p") && h.dalloc(&d.fx, N, "fx") && h.dalloc(&d.fy, N, "fy") &&
+  ok = ok && h.dalloc(&d.v0x, 2 * N, "v0x, v0y") && h.dalloc(&d.v0p, N, "v0p") && h.dalloc(&d.fx, N, "fx") && h.dalloc(&d.fy, N, "fy") &&
        h.dalloc(&d.tau, N, "tau") && h.dalloc(&d.moved, N, "moved");
-  ok = ok && h.dalloc(&d.rec, N, "rec") && h.dalloc(&d.rec_t, N, "rec_t") &&
-       h.dalloc(&d.rf, N, "rf") && h.dalloc(&d.rsf, N, "rsf");
   if (h.prec == sc::PREC_MIXED)
-    ok = ok && h.dalloc(&d.mc, N, "mc") && h.dalloc(&d.mv, N, "mv") && h.dalloc(&d.mvp, N, "mvp") && h.dalloc(&d.mvr, N, "mvr") && h.dalloc(&d.mm, N, "mm") &&
-         h.dalloc(&d.mph, N, "mph") && h.dalloc(&d.pa, N, "pa") &&
+    ok = ok && h.dalloc(&d.rec, N, "rec") && h.dalloc(&d.rec_t, N, "rec_t") &&
+         h.dalloc(&d.rf, N, "rf") && h.dalloc(&d.rsf, N, "rsf") && h.dalloc(&d.mc, N, "mc") &&
+         h.dalloc(&d.mv, N, "mv") && h.dalloc(&d.mvp, N, "mvp") && h.dalloc(&d.mvr, N, "mvr") &&
+         h.dalloc(&d.mm, N, "mm") && h.dalloc(&d.mph, N, "mph") && h.dalloc(&d.pa, N, "pa") &&
          h.dalloc(&d.cellp, N, "cellp") && h.dalloc(&d.gbuild, n_sys, "gbuild") &&
          h.dalloc(&d.ord, N, "ord") && h.dalloc(&d.nbr_p, N * std::max(d.maxn, 2), "nbr_p");
-  else
-    ok = ok && h.dalloc(&d.iaa, N, "iaa") &&
-         h.dalloc(&d.s_mv, N, "s_mv") && h.dalloc(&d.s_nxy, N, "s_nxy");
   ok = ok && h.dalloc(&d.gbar, 2, "grid barrier") &&
        h.cuda_ok(cudaMemsetAsync(d.gbar, 0, 2 * sizeof *d.gbar, h.stream), "barrier");
   if (opt.precision == SC_PREC_MIXED) ok = ok && h.dalloc(&h.d_persist, 1, "persist out");
@@ -349,21 +345,14 @@ int sc_create_rect(const sc_options* opt_in, int n_sys, const int* n_per_sys, co
        h.dalloc(&d.any, 1, "any") &&
        h.dalloc(&d.status, 2, "status");
   if (!ok) return bail(h.last_status ? h.last_status : SC_E_NOMEM);
-  // the FP64 form's pair results, where there is memory for them (a mask word holds 64
-  // list entries)
-  if (h.prec == sc::PREC_FP64 && d.maxn <= 64) {
-    const size_t np = (N + 128) * sc::kPairCap;
-    if (h.dalloc(&d.pr_mask, N, "pair masks") && h.dalloc(&d.pr_info, N, "pair offsets") &&
-        h.dalloc(&d.pr_who, np, "pair partners") && h.dalloc(&d.pr_res, np, "pair results")) {
-      d.pr_win = sc::pair_window(ntot);
-    } else {
-      h.dfree(d.pr_mask);
-      h.dfree(d.pr_info);
-      h.dfree(d.pr_who);
-      h.err.clear();
-      h.last_status = SC_OK;
-      cudaGetLastError();
-    }
+  d.v0y = d.v0x + N;
+  if (h.prec == sc::PREC_FP64) {
+    d.s_nxy = reinterpret_cast<double2*>(d.v0x);
+    d.rec = reinterpret_cast<float4*>(d.s_ra);
+    d.rec_t = reinterpret_cast<float4*>(d.s_irc);
+    d.rf = reinterpret_cast<float*>(d.s_id);
+    d.rsf = reinterpret_cast<float*>(d.s_cell);
+    h.take_extras();
   }
   d.geom = geom;
   d.psys = psys;

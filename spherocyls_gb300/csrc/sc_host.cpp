@@ -57,6 +57,52 @@ void Handle::dfree(void* p) {
     cudaFree(p);
 }
 
+void Handle::take_extras() {
+  if (prec != PREC_FP64) return;
+  const bool pairs = d.maxn <= 64;  // a mask word holds 64 list entries
+  const size_t N = ntot, np = (N + 128) * kPairCap, bytes = 8 * N + (pairs ? 12 * N + 36 * np : 0);
+  // large ones leave some of the device's free memory to the runtime, which loads kernels as
+  // they are first used
+  constexpr size_t kLeave = 256u << 20;
+  if (bytes >= kLeave / 4) {
+    uint64_t have = 0, used = 0;
+    if (use_pool) {
+      cudaMemPoolGetAttribute(device_pool(device), cudaMemPoolAttrReservedMemCurrent, &have);
+      cudaMemPoolGetAttribute(device_pool(device), cudaMemPoolAttrUsedMemCurrent, &used);
+    }
+    size_t free_bytes = 0, total = 0;
+    if (have < used + bytes &&  // (else from the pool's own, which nobody uses)
+        (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess ||
+         free_bytes + (have - used) < bytes + kLeave))
+      return;
+  }
+  auto got = [](cudaError_t e) { return e == cudaSuccess; };
+  if (!got(try_alloc(&d.iaa, N)) || !pairs) return;
+  if (got(try_alloc(&d.pr_mask, N)) && got(try_alloc(&d.pr_info, N)) &&
+      got(try_alloc(&d.pr_who, np)) && got(try_alloc(&d.pr_res, np)))
+    d.pr_win = pair_window(ntot);
+  else
+    give_back();
+}
+
+bool Handle::give_back() {
+  if (prec != PREC_FP64 || !d.iaa) return false;
+  auto drop = [&](auto*& p) {
+    dfree(p);
+    p = nullptr;
+  };
+  invalidate_graph();  // captured kernels hold the pointers
+  d.pr_win = 0;
+  drop(d.iaa);
+  drop(d.pr_mask);
+  drop(d.pr_info);
+  drop(d.pr_who);
+  drop(d.pr_res);
+  cudaStreamSynchronize(stream);
+  if (use_pool) cudaMemPoolTrimTo(device_pool(device), 0);
+  return true;
+}
+
 cudaMemPool_t device_pool(int device) {
   static std::mutex mu;
   static std::map<int, cudaMemPool_t> pools;
@@ -206,20 +252,17 @@ bool Handle::layout_cells() {
   int ncells = c, nchunks = ch;
   if (ncells > cell_cap) {
     dfree(d.cell_start);
-    dfree(d.cell_count);
-    dfree(d.cell_fill);
-    int cap = ncells + ncells / 4 + 64;
-    int *cs = nullptr, *cn = nullptr, *cf = nullptr;
-    if (!dalloc(&cs, cap, "cell_start") || !dalloc(&cn, cap, "cell_count") ||
-        !dalloc(&cf, cap, "cell_fill") ||
-        !cuda_ok(cudaMemsetAsync(cs, 0, cap * sizeof(int), stream), "cell_start") ||
-        !cuda_ok(cudaMemsetAsync(cn, 0, cap * sizeof(int), stream), "cell_count") ||
-        !cuda_ok(cudaMemsetAsync(cf, 0, cap * sizeof(int), stream), "cell_fill"))
+    d.cell_start = nullptr;
+    cell_cap = 0;
+    const size_t cap = ((size_t)ncells + ncells / 4 + 127) / 64 * 64;  // (aligned thirds)
+    int* cells = nullptr;
+    if (!dalloc(&cells, 3 * cap, "cells") ||
+        !cuda_ok(cudaMemsetAsync(cells, 0, 3 * cap * sizeof(int), stream), "cells"))
       return false;
-    d.cell_fill = cf;
-    d.cell_start = cs;
-    d.cell_count = cn;
-    cell_cap = cap;
+    d.cell_start = cells;
+    d.cell_count = cells + cap;
+    d.cell_fill = cells + 2 * cap;
+    cell_cap = (int)cap;
   }
   if (nchunks > chunk_cap) {
     dfree(d.chunk_sum);

@@ -131,20 +131,34 @@ struct Handle {
   bool use_pool = false;  // device memory comes from the device's cached pool
   template <class T>
   bool dalloc(T** p, size_t count, const char* what) {
+    cudaError_t e;
+    while ((e = try_alloc(p, count)) != cudaSuccess)
+      if (!give_back()) {
+        fail(SC_E_NOMEM, "cudaMalloc %s (%zu bytes): %s", what, count * sizeof(T),
+             cudaGetErrorString(e));
+        return false;
+      }
+    return true;
+  }
+  template <class T>
+  cudaError_t try_alloc(T** p, size_t count) {
     *p = nullptr;
     if (count == 0) count = 1;
     cudaError_t e = use_pool ? cudaMallocFromPoolAsync((void**)p, count * sizeof(T),
                                                        device_pool(device), stream)
                              : cudaMalloc((void**)p, count * sizeof(T));
     if (e != cudaSuccess) {
-      fail(SC_E_NOMEM, "cudaMalloc %s (%zu bytes): %s", what, count * sizeof(T),
-           cudaGetErrorString(e));
+      cudaGetLastError();
       *p = nullptr;
-      return false;
+    } else {
+      allocs.push_back((void*)*p);
     }
-    allocs.push_back((void*)*p);
-    return true;
+    return e;
   }
+  // The FP64 form's pair results and reciprocals only make it faster: taken where there is
+  // memory for them, and given back to an allocation that finds none (false: nothing to give).
+  void take_extras();
+  bool give_back();
   void dfree(void* p);
 
   StepScalars row_current(int s) const;

@@ -187,7 +187,9 @@ struct Dev {
   double* tau;
   double2* moved;
   // mixed form (FP32 state relative to the cell centre, compensated); the FP64 form
-  // keeps its positions rounded to FP32 in rec, rec_t and rf, for its pair screen:
+  // keeps its positions rounded to FP32 in rec, rec_t and rf, for its pair screen, in the
+  // memory of the rebuild's scratch s_ra, s_irc, s_id and s_cell (rsf), which is free between
+  // rebuilds and holds a slot's scratch only where the rebuild makes the slot's records anew:
   float4* rec;    // (x_local, y_local, A cos phi, A sin phi) of the state
   float4* rec_t;  // the same for the predictor copy
   float4* mc;     // (x compensation, y compensation, phi, phi compensation)
@@ -198,7 +200,7 @@ struct Dev {
   float* mph;     // angle at the last rebuild
   float4* pa;     // (R, A, isolated-rotation coefficient RC, 1/I)
   float* rf;      // R in FP32: the only per-neighbour constant the force pass gathers
-  double* iaa;    // 1 / A^2 (FP64 form: shared_rcp, sc_pair.cuh)
+  double* iaa;    // 1 / A^2 (FP64 form: shared_rcp, sc_pair.cuh), null where there was no room
   float* rsf;     // R + A in FP32: the list build's reach
   int* cellp;     // local cell packed as col | row << 16
   float* gbuild;  // [nsys] gamma at which each system's list was built
@@ -256,8 +258,7 @@ struct Dev {
   double2* s_irc;
   int* s_id;
   int* s_cell;
-  double2* s_mv;            // FP64 form: displacement counters and shaft vectors on their way
-  double2* s_nxy;
+  double2* s_nxy;           // FP64 form: shaft vectors on their way, in v0x and v0y's memory
   // stress/energy: per-slot contributions and per-chunk partials
   double* se_part;          // [5][ntot]
   double* se_chunk;         // [5][npchunks]

@@ -138,13 +138,12 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_rebuild64(Dev d,
   const bool ok = rb::sort_cells<false, BS>(
       d, work, tab, row, moved != 0, bar,
       [&](int i, int, double2 p, double, double2 ra, double2, int, int) {
-        d.moved[i] = d.s_mv[i];
         const double2 n = d.s_nxy[i];
         d.nxy[i] = n;
         d.rec[i] = screen_record(p, n);
         d.rf[i] = (float)ra.x;
         d.rsf[i] = (float)(ra.x + ra.y);
-        d.iaa[i] = shared_rcp(ra.y * ra.y);
+        if (d.iaa) d.iaa[i] = shared_rcp(ra.y * ra.y);
       });
   if (!ok) {
     bar.leave();
@@ -445,7 +444,7 @@ __device__ __forceinline__ void pass64_slot(const Dev& d, const StepScalars* __r
       const double2 pP = ip ? pi : pj, pQ = ip ? pj : pi;
       const double2 nP = ip ? ni : nj, nQ = ip ? nj : ni;
       const double2 rP = ip ? rai : raj, rQ = ip ? raj : rai;
-      const double ivi = d.iaa[i], ivj = d.iaa[j];
+      const double ivi = d.iaa ? d.iaa[i] : 0.0, ivj = d.iaa ? d.iaa[j] : 0.0;
       PairF64 o;
       const bool hit =
           two_point ? pair2_fp64<SE, FAST>(pP.x - pQ.x, pP.y - pQ.y, nP.x, nP.y, rP.y, nQ.x,

@@ -411,7 +411,9 @@ __device__ __forceinline__ void place(const Dev& d, const Work<BS>& work) {
     d.s_id[i] = id;
     d.s_cell[i] = c;
     if (!MIXED) {
-      d.s_mv[i] = d.nxy_t[src];
+      // nobody reads the counters themselves here, and the predictor's velocities (s_nxy) are
+      // made anew after a rebuild
+      d.moved[i] = d.nxy_t[src];
       d.s_nxy[i] = d.nxy[src];
     }
     if (d.fvx) {  // minimiser velocities travel with their particles (predictor copy is dead here)
@@ -427,7 +429,8 @@ __device__ __forceinline__ void place(const Dev& d, const Work<BS>& work) {
 }
 
 // Back from scratch; f(slot, system, position, angle, (R, A), (I, RC), index, cell) then
-// makes the records that the form's passes read.  records: the state is in them alone
+// makes the records that the form's passes read (the FP64 form's in the scratch that the same
+// slot has just been read from).  records: the state is in them alone
 // (the FP64 positions and angles are not read before they are next made).
 template <int BS, class F>
 __device__ __forceinline__ void put_back(const Dev& d, const Work<BS>& work, bool records, F&& f) {
@@ -435,6 +438,7 @@ __device__ __forceinline__ void put_back(const Dev& d, const Work<BS>& work, boo
     const double2 p = d.s_xy[i], ra = d.s_ra[i], irc = d.s_irc[i];
     const double phi = d.s_ph[i];
     const int id = d.s_id[i], c = d.s_cell[i];
+    asm volatile("" ::: "memory");  // no store of the records' types before these loads
     if (!records) {
       d.xy[i] = p;
       d.ph[i] = phi;

@@ -15,3 +15,20 @@ extern "C" int probe_or_status(sc_handle* H, int bits) {
   st |= bits;
   return cudaMemcpy(h.d.status, &st, sizeof st, cudaMemcpyHostToDevice) == cudaSuccess ? 0 : -1;
 }
+
+// whether the FP64 form has its pair results (2), its reciprocals alone (1), or neither
+extern "C" int probe_extras(sc_handle* H) { return H->h.d.pr_win > 0 ? 2 : H->h.d.iaa != nullptr; }
+extern "C" int probe_give_back(sc_handle* H) { return H->h.give_back() ? 0 : -1; }
+
+// all device memory but `left` bytes; null when it cannot be had
+extern "C" void* probe_fill(size_t left) {
+  size_t free_bytes = 0, total = 0;
+  void* p = nullptr;
+  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || free_bytes <= left) return nullptr;
+  if (cudaMalloc(&p, free_bytes - left) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return p;
+}
+extern "C" int probe_free(void* p) { return cudaFree(p) == cudaSuccess ? 0 : -1; }

@@ -21,4 +21,9 @@ def load(out_dir) -> ctypes.CDLL:
     lib = ctypes.CDLL(so)
     lib.probe_set_pass.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_double]
     lib.probe_or_status.argtypes = [ctypes.c_void_p, ctypes.c_int]
+    lib.probe_extras.argtypes = [ctypes.c_void_p]
+    lib.probe_give_back.argtypes = [ctypes.c_void_p]
+    lib.probe_fill.argtypes = [ctypes.c_size_t]
+    lib.probe_fill.restype = ctypes.c_void_p
+    lib.probe_free.argtypes = [ctypes.c_void_p]
     return lib
