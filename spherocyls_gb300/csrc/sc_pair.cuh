@@ -80,10 +80,20 @@ __device__ __forceinline__ float narrow(double v) {
   return __uint_as_float((hi & 0x80000000u) | (m + up));
 }
 
-// Quotients that share a divisor: r = 1/y rounded to nearest, then x r with one correction
-// by its exact remainder, which is the correctly rounded x/y (P. W. Markstein, IBM J. Res.
-// Dev. 34, 111 (1990)); three operations in place of a division's eight or so.  A divisor
-// whose reciprocal is near the ends of the exponent range has r = 0 and is divided by.
+// Quotients that share a divisor: r = 1/y rounded to nearest, then q = x r with one correction
+// by its remainder (P. W. Markstein, IBM J. Res. Dev. 34, 111 (1990)); three operations in
+// place of a division's eight or so.  The result is the correctly rounded x/y.  With the
+// mantissas 1 <= x, y < 2: a q within one ulp of x/y has an exact remainder, and Markstein's
+// theorem holds; that covers x >= y (|q - x/y| <= x 2^-54 + 2^-53) and, with 2^-54 (x + 1),
+// x <= 1.  For 1 < x < y, q may be up to 1.5 ulp (of 2^-53) off.  Past one ulp the remainder
+// is rounded once, by at most 2^-105, and the corrected value is within 2^-104 of x/y, so
+// that it rounds otherwise only if x/y - q is within 2^-104 of 1.5 ulp: x > 2 - 2^-50, which
+// leaves (x, y) = 2 - (m, n) 2^-52 with n < m < 4, and those round right.
+// That is for |x| within 2^-500 to 2^500, like r; a divisor out of that range has r = 0 and is
+// divided by.  The pair code's dividends are products of its lengths and forces, in range
+// where its divisors are; an x of -0 gives +0, which no sum of forces that starts at +0 can
+// tell, and an infinite one NaN, which only a state that is already non-finite has (a test of
+// x's exponent as well costs 2 to 7% of k_pairs64).
 __device__ __forceinline__ double shared_rcp(double y) {
   const double r = 1.0 / y;
   const unsigned h = (unsigned)__double2hiint(r);
