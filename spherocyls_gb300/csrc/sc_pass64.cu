@@ -840,7 +840,8 @@ __global__ void __launch_bounds__(kPairBlock) k_mx_se64(Dev d, const StepScalars
     gam = ts.f_gamma_p;
     small = g.cols < 3 || g.rows < 3;
     ri = d.rec[i];
-    Ri = d.rf[i];
+    // with what the rounding of local positions (up to a cell) and shaft vectors may add
+    Ri = d.rf[i] + 1e-6f * g.smax * (1.f + fabsf(gam));
     idi = d.id[i];
     cnt = min(d.nbr_n[i], d.maxn);
   }
