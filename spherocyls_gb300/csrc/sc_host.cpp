@@ -588,11 +588,10 @@ cudaError_t Handle::new_cond_handle(cudaGraphConditionalHandle* h) {
   return e;
 }
 
-// Inside a capture on `stream`: an IF (or WHILE) node on `hcond` after the work
-// captured so far, whose body `body` records on stream2.
-cudaError_t Handle::add_cond_body(cudaGraphConditionalHandle hcond,
-                                  const std::function<void(cudaStream_t)>& body,
-                                  cudaGraphConditionalNodeType type) {
+// Inside a capture on `stream`: a WHILE node on `hcond` after the work captured so far,
+// whose body `body` records on stream2.
+cudaError_t Handle::add_loop(cudaGraphConditionalHandle hcond,
+                             const std::function<void(cudaStream_t)>& body) {
   cudaStreamCaptureStatus cs;
   cudaGraph_t gcap = nullptr;
   const cudaGraphNode_t* deps = nullptr;
@@ -604,7 +603,7 @@ cudaError_t Handle::add_cond_body(cudaGraphConditionalHandle hcond,
   cudaGraphNodeParams& cp = *reinterpret_cast<cudaGraphNodeParams*>(cp_buf);
   cp.type = cudaGraphNodeTypeConditional;
   cp.conditional.handle = hcond;
-  cp.conditional.type = type;
+  cp.conditional.type = cudaGraphCondTypeWhile;
   cp.conditional.size = 1;
   cudaGraphNode_t cn;
   e = cudaGraphAddNode(&cn, gcap, deps, nullptr, nd, &cp);
@@ -1291,14 +1290,13 @@ bool Handle::run_cg_graph(int max_iter) {
       e = new_cond_handle(&hs);
       if (e != cudaSuccess) break;
       enqueue_cg_head(max_iter, hs, stream);
-      e = add_cond_body(
+      e = add_loop(
           hs,
           // several probes an iteration of the loop, which costs 12 us by itself; past the
           // end of every search a probe's kernels find nothing to do, about 9 us
           [&](cudaStream_t st2) {
             for (int q = 0; q < kCgUnroll; q++) enqueue_cg_probe(hs, st2);
-          },
-          cudaGraphCondTypeWhile);
+          });
       if (e != cudaSuccess) break;
       enqueue_cg_move();
     }

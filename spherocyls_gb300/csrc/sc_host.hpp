@@ -184,9 +184,7 @@ struct Handle {
   void enqueue_rebuild(int k, bool prof);
   void enqueue_pred(bool resize, int k, bool se, bool prof);
   cudaError_t new_cond_handle(cudaGraphConditionalHandle* h);
-  cudaError_t add_cond_body(cudaGraphConditionalHandle h,
-                            const std::function<void(cudaStream_t)>& body,
-                            cudaGraphConditionalNodeType type = cudaGraphCondTypeIf);
+  cudaError_t add_loop(cudaGraphConditionalHandle h, const std::function<void(cudaStream_t)>& body);
   bool instantiate_steps(bool resize, int nsteps, const std::vector<char>& se,
                          cudaGraphExec_t* exec, long long* nkernels);
   bool run_subgraphs(bool resize, int nsteps, int se_every);

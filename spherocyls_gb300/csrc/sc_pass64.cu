@@ -694,8 +694,8 @@ __device__ __forceinline__ void pair_result64(const Dev& d, const StepScalars& t
 // two or three), then the Heun epilogue.  GL = 1: a thread does all of it for its slot.
 // GL = 8, for small systems, where the gather's chain of dependent loads (four or five
 // contacts of three loads each) is what the kernel waits for: eight threads of a slot
-// fetch a contribution each, a fourth warp meanwhile takes the cosine of the rotation,
-// and one thread a slot sums and steps.
+// fetch a contribution each (the last sixteen of the block take the cosine of the rotation
+// first, beside the other warps' fetches), and one thread a slot sums and steps.
 constexpr int kStepBlock = 128;
 
 template <int MODE, bool TWO, bool FAST, int GL>
