@@ -250,10 +250,11 @@ bool Handle::layout_cells() {
     ch += h.nchunks;
   }
   int ncells = c, nchunks = ch;
+  layout_ok = false;
   if (ncells > cell_cap) {
     dfree(d.cell_start);
     d.cell_start = nullptr;
-    cell_cap = 0;
+    cell_cap = 0;  // (until the new arrays are there, here and below)
     const size_t cap = ((size_t)ncells + ncells / 4 + 127) / 64 * 64;  // (aligned thirds)
     int* cells = nullptr;
     if (!dalloc(&cells, 3 * cap, "cells") ||
@@ -265,6 +266,7 @@ bool Handle::layout_cells() {
     cell_cap = (int)cap;
   }
   if (nchunks > chunk_cap) {
+    chunk_cap = 0;
     dfree(d.chunk_sum);
     dfree((void*)d.chunk_sys);
     dfree((void*)d.chunk_c0);
@@ -283,6 +285,7 @@ bool Handle::layout_cells() {
   }
   const int ntiles = (int)tiles.size();
   if (ntiles > tile_cap) {
+    tile_cap = 0;
     dfree((void*)d.tiles);
     dfree(d.tinfo);
     int cap = ntiles + ntiles / 4 + 16;
@@ -334,7 +337,8 @@ bool Handle::layout_cells() {
             cuda_ok(cudaMemsetAsync(d.tinfo, 0, ntiles * sizeof(int4), stream), "tile info");
   if (!ok) return false;
   // host copies must outlive the async copies
-  return cuda_ok(cudaStreamSynchronize(stream), "layout sync");
+  layout_ok = cuda_ok(cudaStreamSynchronize(stream), "layout sync");
+  return layout_ok;
 }
 
 // The step table holds at least a full chunk from its first allocation, so that a
@@ -344,13 +348,12 @@ bool Handle::layout_cells() {
 // stay valid.
 bool Handle::ensure_table(int rows) {
   if (rows * nsys <= tab_cap) return true;
-  dfree(d_tab);
-  int cap = std::max(std::max(rows, kChunk + 1) * nsys, 2 * tab_cap);
-  StepScalars* t = nullptr;
-  if (!dalloc(&t, cap, "step table")) return false;
-  d_tab = t;
-  tab_cap = cap;
+  const int cap = std::max(std::max(rows, kChunk + 1) * nsys, 2 * tab_cap);
   invalidate_table_graphs();
+  dfree(d_tab);
+  tab_cap = 0;
+  if (!dalloc(&d_tab, cap, "step table")) return false;
+  tab_cap = cap;
   return true;
 }
 
@@ -368,6 +371,10 @@ void Handle::invalidate_table_graphs() {
 
 bool Handle::upload_table(const std::vector<StepScalars>& rows) {
   int nrows = (int)(rows.size() / nsys);
+  if (!layout_ok) {
+    fail(SC_E_NOMEM, "no cell arrays: an earlier call found no memory for them");
+    return false;
+  }
   if (!ensure_table(nrows)) return false;
   // the host table is a member, so it outlives the asynchronous copy
   h_tab = rows;
@@ -477,14 +484,14 @@ bool Handle::rebuild_all() {
 
 bool Handle::set_pass(int kind, int target, const std::vector<double>& pads) {
   if (!materialize()) return false;
-  if (kind == 1 && !d.t_own) {
-    const size_t N = ntot;
-    if (!dalloc(&d.t_own, N * kTileEPP, "tile owners") ||
-        !dalloc(&d.t_pe, N * kTileEPP, "tile partners") ||
-        !dalloc(&d.t_rd, N * kTileEPP, "tile reads") || !dalloc(&d.t_meta, N, "tile meta") ||
-        !dalloc(&d.t_pb, N * kTileEPP, "tile pair results"))
-      return false;
-  }
+  const size_t N = ntot, ne = N * kTileEPP;
+  if (kind == 1 &&  // (those an earlier call got before it failed are there)
+      !((d.t_own || dalloc(&d.t_own, ne, "tile owners")) &&
+        (d.t_pe || dalloc(&d.t_pe, ne, "tile partners")) &&
+        (d.t_rd || dalloc(&d.t_rd, ne, "tile reads")) &&
+        (d.t_meta || dalloc(&d.t_meta, N, "tile meta")) &&
+        (d.t_pb || dalloc(&d.t_pb, ne, "tile pair results"))))
+    return false;
   d.pass_kind = kind;
   opt.pass_kind = kind == 1 ? SC_PASS_TILE : SC_PASS_LIST;
   opt.tile_target = target;
@@ -675,8 +682,8 @@ bool Handle::run_graph(bool resize, int nsteps, int se_every) {
 // captured on first use against the step and record windows.
 Handle::SubGraph* Handle::subgraph(bool resize, unsigned mask) {
   const int G = kGraphSteps;
-  if (!d_win && (!dalloc(&d_win, (size_t)(G + 1) * nsys, "step window") ||
-                 !dalloc(&d_win_se, (size_t)G * nsys * 5, "record window")))
+  if (!(d_win || dalloc(&d_win, (size_t)(G + 1) * nsys, "step window")) ||
+      !(d_win_se || dalloc(&d_win_se, (size_t)G * nsys * 5, "record window")))
     return nullptr;
   for (auto& c : sub_graphs)
     if (c.resize == resize && c.se_mask == mask && c.prec == prec) return &c;
@@ -727,13 +734,12 @@ bool Handle::run_subgraphs(bool resize, int nsteps, int se_every) {
 
 bool Handle::ensure_se_hist(int nrec) {
   if (nrec * nsys * 5 <= se_hist_cap) return true;
-  dfree(d_se_hist);
-  int cap = std::max(nrec * nsys * 5, 2 * se_hist_cap);
-  double* p = nullptr;
-  if (!dalloc(&p, cap, "se history")) return false;
-  d_se_hist = p;
-  se_hist_cap = cap;
+  const int cap = std::max(nrec * nsys * 5, 2 * se_hist_cap);
   invalidate_table_graphs();  // the sub-chunk graphs record into their own window
+  dfree(d_se_hist);
+  se_hist_cap = 0;
+  if (!dalloc(&d_se_hist, cap, "se history")) return false;
+  se_hist_cap = cap;
   return true;
 }
 

@@ -69,6 +69,7 @@ struct Handle {
   Dev d{};
   std::vector<void*> allocs;
   int cell_cap = 0, chunk_cap = 0, tile_cap = 0;
+  bool layout_ok = false;  // the cell arrays are those of the host's grids
   const int* pass_skip = nullptr;  // Dev::skip of the force passes being enqueued
   int* d_persist = nullptr;        // result word of the persistent step kernel
   StepScalars* d_tab = nullptr;

@@ -32,3 +32,25 @@ extern "C" void* probe_fill(size_t left) {
   return p;
 }
 extern "C" int probe_free(void* p) { return cudaFree(p) == cudaSuccess ? 0 : -1; }
+
+// what is left of the handle's memory pool after probe_fill, in pieces of down to 4 KB
+static std::vector<void*> g_pieces;
+extern "C" int probe_exhaust(sc_handle* H) {
+  sc::Handle& h = H->h;
+  if (!h.use_pool) return -1;
+  for (size_t n = size_t(1) << 30; n >= 4096; n /= 2)
+    for (;;) {
+      void* p = nullptr;
+      if (cudaMallocFromPoolAsync(&p, n, sc::device_pool(h.device), h.stream) != cudaSuccess) {
+        cudaGetLastError();
+        break;
+      }
+      g_pieces.push_back(p);
+    }
+  return cudaStreamSynchronize(h.stream) == cudaSuccess ? (int)g_pieces.size() : -1;
+}
+extern "C" int probe_release(sc_handle* H) {
+  for (void* p : g_pieces) cudaFreeAsync(p, H->h.stream);
+  g_pieces.clear();
+  return cudaStreamSynchronize(H->h.stream) == cudaSuccess ? 0 : -1;
+}

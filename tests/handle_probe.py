@@ -26,4 +26,6 @@ def load(out_dir) -> ctypes.CDLL:
     lib.probe_fill.argtypes = [ctypes.c_size_t]
     lib.probe_fill.restype = ctypes.c_void_p
     lib.probe_free.argtypes = [ctypes.c_void_p]
+    lib.probe_exhaust.argtypes = [ctypes.c_void_p]
+    lib.probe_release.argtypes = [ctypes.c_void_p]
     return lib

@@ -120,3 +120,78 @@ def test_a_full_device(sc, probe):
             assert block and probe.probe_free(ctypes.c_void_p(block)) == 0
             _lib.lib().sc_trim_memory(0)
         assert np.array_equal(got, want, equal_nan=True)
+
+
+class _NoMemory:
+    """No device memory for the handle while it lasts."""
+
+    def __init__(self, probe, b):
+        self.probe, self.b = probe, b
+
+    def __enter__(self):
+        from spherocyls_gb300 import _lib
+
+        _lib.lib().sc_trim_memory(0)
+        self.block = self.probe.probe_fill(64 << 20)
+        assert self.block and self.probe.probe_exhaust(self.b.h) >= 0
+
+    def __exit__(self, *exc):
+        from spherocyls_gb300 import _lib
+
+        assert self.probe.probe_release(self.b.h) == 0
+        assert self.probe.probe_free(ctypes.c_void_p(self.block)) == 0
+        _lib.lib().sc_trim_memory(0)
+
+
+def _mixed(sc, n=20000, **kw):
+    L, x, y, p, R, A = sc.generate_packing(n, 0.6, 1.0, seed=8)
+    b = sc.SpherocylBox(L, x, y, p, A, R, 0.2, precision="mixed", **kw)
+    b.set_strain_rate(0.05)
+    b.set_step(0.02)
+    return b
+
+
+def test_tile_arrays_after_a_refusal(sc, probe):
+    """A pass change that finds no memory for all of the tile pass's arrays is an error, and the
+    next one gets those that are missing."""
+    from spherocyls_gb300 import _lib
+
+    with _mixed(sc) as b, _mixed(sc, pass_kind="tile") as want:
+        with _NoMemory(probe, b):
+            assert probe.probe_set_pass(b.h, 1, 0, 0.2) == _lib.SC_E_NOMEM
+        assert b.options()["pass_kind"] == "auto"  # as it was
+        assert probe.probe_set_pass(b.h, 1, 0, 0.2) == 0
+        for box in (b, want):
+            box.strain_steps(20)
+        assert np.array_equal(np.array(b.state()), np.array(want.state()))
+
+
+def test_step_arrays_after_a_refusal(sc, probe):
+    """Steps and records whose windows and tables find no memory are an error; later ones run."""
+    from spherocyls_gb300 import _lib
+
+    with _mixed(sc) as b, _mixed(sc) as want:
+        with _NoMemory(probe, b):
+            with pytest.raises(sc.ScError) as ei:
+                b.strain_steps(100, se_every=1)
+            assert ei.value.status in (_lib.SC_E_NOMEM, _lib.SC_E_CUDA)
+        a, c = (box.strain_steps(100, se_every=1) for box in (b, want))
+        assert np.array_equal(a, c) and np.array_equal(np.array(b.state()), np.array(want.state()))
+
+
+def test_no_cells_after_a_refusal(sc, probe):
+    """A grid that outgrows its cell arrays where there is no memory is an error, and so is every
+    later call that needs cells; the state can still be read."""
+    from spherocyls_gb300 import _lib
+
+    with _mixed(sc, n=200000) as b:
+        s0 = np.array(b.state())
+        with _NoMemory(probe, b):
+            with pytest.raises(sc.ScError) as ei:
+                b.affine_scale(2.0)
+            assert ei.value.status == _lib.SC_E_NOMEM
+        for call in (b.find_neighbors, b.calc_forces, lambda: b.strain_steps(1), b.calc_se):
+            with pytest.raises(sc.ScError) as ei:
+                call()
+            assert ei.value.status == _lib.SC_E_NOMEM
+        assert np.abs(np.array(b.state())[:2] - 2.0 * s0[:2]).max() <= 1e-9 * 2.0 * s0[:2].max()
