@@ -98,10 +98,10 @@ def bytes_per_pass(precision: str, nbar: float) -> float:
 
 
 # DRAM bytes (read + write) per particle of one mixed force pass, the mean of the
-# predictor (96.9 MB) and corrector (142.8 MB) launches in one ncu capture of the
+# predictor (96.7 MB) and corrector (142.3 MB) launches in one ncu capture of the
 # default workload at the padding the autotuner picks for it, 0.6
 # (profiles/k_pass_mixed_n1048576.md).
-PASS_DRAM_BYTES_PER_PARTICLE = {"shear_n1048576_phi084": 119.9e6 / (1 << 20)}
+PASS_DRAM_BYTES_PER_PARTICLE = {"shear_n1048576_phi084": 119.5e6 / (1 << 20)}
 
 
 def _peaks():
