@@ -922,7 +922,7 @@ __device__ __forceinline__ void order_window(const Dev& d, int i, OrderScratch& 
 // pass, the lists and their ordering (LISTS).  Large rebuilds list and order window by
 // window, a group of kOrderWindow threads each: apart, with a grid barrier between, they
 // took 202 us instead of 147 at 2^20 particles.  Small ones list with eight threads a slot.
-// 1024 threads an SM (61 registers) against 1536 (40, spilling): 20 steps of the 512-system
+// 1024 threads an SM (60 registers) against 1536 (40, spilling): 20 steps of the 512-system
 // ensemble, which rebuild in each, 2.57 and 2.79 ms, 50 FIRE iterations of 524288 particles
 // 4.21 and 4.42.  As one block of 1024 or four of 256 the ensemble takes 2.65 and 2.60 ms.
 template <bool LISTS, int BS>
