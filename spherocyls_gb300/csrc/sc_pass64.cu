@@ -140,6 +140,9 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_rebuild64(Dev d,
       [&](int i, int, double2 p, double, double2 ra, double2, int, int) {
         const double2 n = d.s_nxy[i];
         d.nxy[i] = n;
+        // the records take the memory of this slot's scratch, as other types: no store of
+        // theirs before the loads of put_back
+        asm volatile("" ::: "memory");
         d.rec[i] = screen_record(p, n);
         d.rf[i] = (float)ra.x;
         d.rsf[i] = (float)(ra.x + ra.y);

@@ -438,7 +438,6 @@ __device__ __forceinline__ void put_back(const Dev& d, const Work<BS>& work, boo
     const double2 p = d.s_xy[i], ra = d.s_ra[i], irc = d.s_irc[i];
     const double phi = d.s_ph[i];
     const int id = d.s_id[i], c = d.s_cell[i];
-    asm volatile("" ::: "memory");  // no store of the records' types before these loads
     if (!records) {
       d.xy[i] = p;
       d.ph[i] = phi;
